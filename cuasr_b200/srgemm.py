@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import dataclasses
+import struct
 from typing import Any, Optional, Tuple
 
 import numpy as np
@@ -18,25 +19,35 @@ from . import _lib
 from .semiring import DType, Layout, NUMPY_DTYPE, Op, Status, annihilator, identity
 
 
-def _ptr(x: Any) -> Optional[int]:
+def _ptr(x: Any) -> int:
+    """Device address of a tensor or an address; 0 for None."""
     if x is None:
-        return None
-    if hasattr(x, "data_ptr"):
-        return int(x.data_ptr())
-    return int(x)
+        return 0
+    if type(x) is int:
+        return x
+    data_ptr = getattr(x, "data_ptr", None)
+    return int(x) if data_ptr is None else data_ptr()
 
 
-def _scalar(value, dtype: DType) -> _lib.Scalar:
-    s = _lib.Scalar()
-    raw = np.asarray(value).astype(NUMPY_DTYPE[dtype]).tobytes()
-    for i, b in enumerate(raw):
-        s.bytes[i] = b
-    return s
+# One call packs its arguments with a single struct.pack and makes a single call into the library: a 64 x 64 x 64
+# product runs for about 5 us on the device, so what the host does per call decides how often it can be made.
+_PACK_SCALAR = {DType.F32: struct.Struct("<f4x").pack, DType.F64: struct.Struct("<d").pack,
+                DType.S32: struct.Struct("<i4x").pack, DType.U32: struct.Struct("<I4x").pack}
+# the layout of _lib.Args
+_PACK_ARGS = struct.Struct("4iQqQqQqQq8s8s8s8sQNQ").pack
+assert struct.calcsize("4iQqQqQqQq8s8s8s8sQNQ") == ctypes.sizeof(_lib.Args)
+_STATUS = {int(st): st for st in Status}
 
 
-def _stream_handle(stream) -> Optional[int]:
+def _scalar(value, dtype: DType) -> bytes:
+    """The element `value` of type `dtype`, in eight bytes: for values _PACK_SCALAR refuses, because the element type
+    cannot hold them or they need a conversion first."""
+    return np.asarray(value).astype(NUMPY_DTYPE[dtype]).tobytes().ljust(8, b"\0")
+
+
+def _stream_handle(stream) -> int:
     if stream is None:
-        return None
+        return 0
     if hasattr(stream, "cuda_stream"):
         return int(stream.cuda_stream)
     return int(stream)
@@ -70,31 +81,34 @@ class _Operator:
         self._lib = _lib.load()
         self._desc = _lib.Desc(int(self.add_op), int(self.mul_op), int(self.dtype), int(self.layout_a),
                                int(self.layout_b), int(self.layout_c), int(self.kSplitKSerial), 0)
+        self._pack_scalar = _PACK_SCALAR[self.dtype]
+        self._desc_ref = ctypes.byref(self._desc)
+        name = "cuasr_b200_srgemm_splitk" if self._splitk_parallel else "cuasr_b200_srgemm"
+        self._run_fn = getattr(self._lib, name)
+        # EpilogueOutputOp::Params defaults (semiring_linear_combination.h:67-85)
+        self._default_beta = annihilator(self.mul_op, self.dtype)
         self._args: Optional[_lib.Args] = None
         self._keepalive = None
 
     # -- helpers ---------------------------------------------------------------------------------------
     def _pack(self, args: Arguments, workspace=None, workspace_bytes: int = 0, stream=None) -> _lib.Args:
         m, n, k = args.problem_size
-        epi = tuple(args.epilogue)
-        # EpilogueOutputOp::Params defaults (semiring_linear_combination.h:67-85)
+        epi = args.epilogue
         alpha = epi[0] if len(epi) >= 1 else self.mul_identity
-        beta = epi[1] if len(epi) >= 2 else annihilator(self.mul_op, self.dtype)
-        a = _lib.Args()
-        a.m, a.n, a.k, a.split_k_slices = int(m), int(n), int(k), int(args.split_k_slices)
-        a.A, a.lda = _ptr(args.ref_A[0]), int(args.ref_A[1])
-        a.B, a.ldb = _ptr(args.ref_B[0]), int(args.ref_B[1])
-        a.C, a.ldc = _ptr(args.ref_C[0]), int(args.ref_C[1])
-        a.D, a.ldd = _ptr(args.ref_D[0]), int(args.ref_D[1])
-        a.alpha, a.beta = _scalar(alpha, self.dtype), _scalar(beta, self.dtype)
-        a.add_identity = _scalar(self.add_identity, self.dtype)
-        a.mul_identity = _scalar(self.mul_identity, self.dtype)
-        a.workspace = _ptr(workspace)
+        beta = epi[1] if len(epi) >= 2 else self._default_beta
+        pack = self._pack_scalar
+        try:
+            alpha, beta, add_identity, mul_identity = pack(alpha), pack(beta), pack(self.add_identity), pack(self.mul_identity)
+        except (struct.error, OverflowError, TypeError):
+            alpha, beta, add_identity, mul_identity = (_scalar(v, self.dtype) for v in
+                                                       (alpha, beta, self.add_identity, self.mul_identity))
+        (A, lda), (B, ldb), (C, ldc), (D, ldd) = args.ref_A, args.ref_B, args.ref_C, args.ref_D
         if workspace is not None and workspace_bytes == 0 and hasattr(workspace, "numel"):
             workspace_bytes = workspace.numel() * workspace.element_size()
-        a.workspace_bytes = int(workspace_bytes)
-        a.stream = _stream_handle(stream)
-        return a
+        return _lib.Args.from_buffer_copy(_PACK_ARGS(
+            int(m), int(n), int(k), int(args.split_k_slices), _ptr(A), int(lda), _ptr(B), int(ldb), _ptr(C), int(ldc),
+            _ptr(D), int(ldd), alpha, beta, add_identity, mul_identity, _ptr(workspace), int(workspace_bytes),
+            0 if stream is None else _stream_handle(stream)))
 
     def _fn(self, base: str):
         name = "cuasr_b200_srgemm_splitk" if self._splitk_parallel else "cuasr_b200_srgemm"
@@ -139,7 +153,7 @@ class _Operator:
             return Status.kErrorInternal
         if stream is not None:
             self._args.stream = _stream_handle(stream)
-        return Status(self._fn("")(ctypes.byref(self._desc), ctypes.byref(self._args)))
+        return _STATUS[self._run_fn(self._desc_ref, ctypes.byref(self._args))]
 
     def run_push(self, extra_outputs, stream=None) -> Status:
         """run(), with every element of D also stored to each matrix in `extra_outputs` (pointers or tensors
@@ -154,11 +168,15 @@ class _Operator:
 
     def __call__(self, args: Optional[Arguments] = None, workspace=None, stream=None,
                  workspace_bytes: int = 0) -> Status:
-        if args is not None:
-            status = self.initialize(args, workspace, stream, workspace_bytes)
-            if status != Status.kSuccess:
-                return status
-        return self.run(stream)
+        if args is None:
+            return self.run(stream)
+        # initialize + run: the library's run entry point makes every check that initialize() makes
+        packed = self._pack(args, workspace, workspace_bytes, stream)
+        status = _STATUS[self._run_fn(self._desc_ref, ctypes.byref(packed))]
+        if status is Status.kSuccess:
+            self._args = packed
+            self._keepalive = (args, workspace)
+        return status
 
     # -- extras ------------------------------------------------------------------------------------------
     def last_kernel(self) -> str:
