@@ -76,17 +76,18 @@ template <> struct TmaType<int32_t>  { static constexpr CUtensorMapDataType v = 
 template <> struct TmaType<uint32_t> { static constexpr CUtensorMapDataType v = CU_TENSOR_MAP_DATA_TYPE_UINT32; };
 
 // Describes one operand of `rows` x K elements to TMA.
-//   K-contiguous:  tensor {K, rows}, box {128 bytes of k, 128 rows}, 128-byte swizzle
+//   K-contiguous:  tensor {K, rows}, box {128 bytes of k, box_rows rows}, 128-byte swizzle
 //   MN-contiguous: tensor {rows, K}, box {128 rows, 128 bytes worth of k}, no swizzle
 template <typename T>
-bool make_operand_map(CUtensorMap* map, const T* ptr, long long ld, int rows, int K, bool kcontig, bool nan_fill) {
+bool make_operand_map(CUtensorMap* map, const T* ptr, long long ld, int rows, int K, bool kcontig, bool nan_fill,
+                      int box_rows = kTileM) {
   EncodeTiledFn encode = encode_tiled_fn();
   if (encode == nullptr) return false;
   const cuuint32_t tk = kTileKBytes / sizeof(T);
   cuuint64_t dims[2];
   cuuint32_t box[2];
-  if (kcontig) { dims[0] = K; dims[1] = rows; box[0] = tk; box[1] = kTileM; }
-  else         { dims[0] = rows; dims[1] = K; box[0] = kTileM; box[1] = tk; }
+  if (kcontig) { dims[0] = K; dims[1] = rows; box[0] = tk; box[1] = box_rows; }
+  else         { dims[0] = rows; dims[1] = K; box[0] = box_rows; box[1] = tk; }
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * sizeof(T)};
   const cuuint32_t elem_strides[2] = {1, 1};
   const CUresult r = encode(map, TmaType<T>::v, 2, const_cast<T*>(ptr), dims, strides, box, elem_strides,
@@ -200,8 +201,7 @@ size_t tile_count(const cuasr_b200_args_t& args) {
 size_t ticket_bytes_for(const cuasr_b200_args_t& args) { return align_up(tile_count(args) * sizeof(unsigned int), 256); }
 
 // Scratch layout: [tickets: one u32 per 128 x 128 tile, padded to 256 B][partials: one full 128 x 128 block per
-// (split tile, slice)].  With every tile split (explicit split-K) that is tiles * slices blocks, which also
-// covers the slices * m * n elements the fallback kernel needs.
+// (split tile, slice)].  With every tile split (explicit split-K) that is tiles * slices blocks.
 size_t splitk_bytes_for_pieces(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, long long pieces) {
   const size_t es = desc.dtype == CUASR_F64 ? 8 : 4;
   return ticket_bytes_for(args) + es * tile_count(args) * kTileM * kTileN * static_cast<size_t>(pieces);
@@ -302,29 +302,11 @@ struct ExtraOutputs {
   void* ptr[kMaxDestinations - 1] = {};
 };
 
-// Re-packing of MN-contiguous fp32 operands into K-contiguous scratch, so that the kernel variant with packed
-// fp32x2 adds (both operands deliver (k, k+1) register pairs) can run.  Worth it only for the rings that variant
-// speeds up, for problems large enough for the TMA kernel, and when the copy is cheap against what it buys: the
-// variant is about 7 % faster (8192^3: 31.0 ms against 33.4), the copy moves 8 bytes per re-packed element, which
-// breaks even near m n = 700 x (re-packed rows).  One rank's share of a sharded SRGEMM or one chunk of the host
-// pipeline (8192 x 1024 x 8192) passes that test, thinner slices do not; copies of less than 16 MB are always taken
-// (512^3: 0.076 -> 0.050 ms).
-bool repack_pays(const cuasr_b200_desc_t& desc, const Normalised& p) {
-  const bool ring = (desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM) &&
-                    (desc.mul_op == CUASR_OP_PLUS || desc.mul_op == CUASR_OP_MULTIPLIES);
-  if (!(desc.dtype == CUASR_F32 && ring && static_cast<long long>(p.m) * p.n >= 256 * 256 && p.k >= 256 &&
-        (!p.a_kcontig || !p.b_kcontig)))
-    return false;
-  const long long rows = (p.a_kcontig ? 0LL : p.m) + (p.b_kcontig ? 0LL : p.n);
-  const bool small_copy = rows * p.k < 4LL * 1024 * 1024;
-  return small_copy || static_cast<long long>(p.m) * p.n >= 700LL * rows;
-}
-// Which operands a launch copies into K-contiguous, 16-byte aligned scratch before the TMA kernel runs:
-//   * an operand TMA cannot describe (its address or its leading dimension is not a multiple of 16 bytes; the
-//     reference accepts alignment 1, include/cuasr/gemm/device/default_srgemm_configuration.h:88-89) - otherwise the
-//     whole product would fall back to the generic kernel;
-//   * an MN-contiguous fp32 operand of a ring with a packed-add variant, where that pays (repack_pays).
-// Rows are padded to a multiple of 16 bytes; the padding is never read (the tensor map ends at K).
+// Which operands a launch with an optional workspace copies into K-contiguous, 16-byte aligned scratch, so that TMA
+// brings them in: an operand TMA cannot describe (its address or its leading dimension is not a multiple of 16 bytes;
+// the reference accepts alignment 1, include/cuasr/gemm/device/default_srgemm_configuration.h:88-89).  Without the
+// workspace the kernel gathers such an operand itself.  Rows are padded to a multiple of 16 bytes; the padding is never
+// read (the tensor map ends at K).
 struct RepackPlan {
   bool a = false, b = false;
   int k_padded = 0;      // > 0: both copies are extended along K to this length (a multiple of the kernel's K step)
@@ -361,21 +343,91 @@ bool ring_pads_itself(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& ar
 RepackPlan repack_plan(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, const Normalised& p) {
   RepackPlan plan;
   const size_t es = desc.dtype == CUASR_F64 ? 8 : 4;
-  // only problems the TMA kernel would take: not tiny, storage lines that do not overlap
+  // not for tiny outputs, nor for storage lines that overlap
   if (static_cast<long long>(p.m) * p.n < 64 * 64) return plan;
   if (p.lda < (p.a_kcontig ? p.k : p.m) || p.ldb < (p.b_kcontig ? p.k : p.n)) return plan;
   const int tk = kTileKBytes / static_cast<int>(es);
   if (p.k % tk != 0 && !ring_pads_itself(desc, args)) {
     plan.a = plan.b = true;
-    plan.k_padded = (p.k + tk - 1) / tk * tk;
+    plan.k_padded = (p.k + 2 * tk - 1) / (2 * tk) * (2 * tk);     // the longest K step of any tile
   } else {
-    const bool pays = repack_pays(desc, p);
-    plan.a = !tma_describable(p.a, p.lda, es) || (pays && !p.a_kcontig);
-    plan.b = !tma_describable(p.b, p.ldb, es) || (pays && !p.b_kcontig);
+    plan.a = !tma_describable(p.a, p.lda, es);
+    plan.b = !tma_describable(p.b, p.ldb, es);
   }
   const int k_copy = plan.k_padded > 0 ? plan.k_padded : p.k;
   plan.bytes = (plan.a ? repack_operand_bytes(p.m, k_copy, es) : 0) + (plan.b ? repack_operand_bytes(p.n, k_copy, es) : 0);
   return plan;
+}
+
+// ---- which tile, and how K is shared ---------------------------------------------------------------------------
+// Clocks the 8 consumer warps of a CTA (two per scheduler, 64 products per lane and k) take for one k: measured per
+// product and scheduler 2.07 (fp32 with a packed add and a three-input minimum, fused integer add-min, one logic
+// instruction), 3.0 (two-instruction bottleneck products), 6.5 (fp64 minima), 2.1 (fp64 sums on the tensor cores).
+double clocks_per_k(const cuasr_b200_desc_t& desc) {
+  const bool sum = desc.add_op == CUASR_OP_PLUS;
+  double per_product = 2.1;
+  if (desc.dtype == CUASR_F64) per_product = sum ? 2.1 : 6.5;
+  else if (desc.mul_op == CUASR_OP_MINIMUM || desc.mul_op == CUASR_OP_MAXIMUM) per_product = 3.0;
+  else if (desc.mul_op == CUASR_OP_BINARY_AND) per_product = 5.0;
+  return 2 * 64 * per_product;
+}
+
+struct LaunchPlan {
+  int tile = kSmallTile;
+  int cluster = 1;                 // CTAs that share a tile's K range through a cluster
+  int whole_tiles = 0, pieces = 1; // ticket pieces (cluster == 1)
+  double cost = 1e300;             // modelled clocks
+};
+constexpr int kTileRows[3] = {LargeTile::kM, MediumTile::kM, SmallTile::kM};
+constexpr int kTileCols[3] = {LargeTile::kN, MediumTile::kN, SmallTile::kN};
+constexpr int kTileWk[3] = {LargeTile::WK, MediumTile::WK, SmallTile::WK};
+constexpr int kTileSub[3] = {LargeTile::kSub, MediumTile::kSub, SmallTile::kSub};
+
+// The fastest of the launches that need no workspace, by a model in clocks: start of the launch and first tile of
+// operands 3000, then per wave of CTAs the contraction (above) and the tile's end (2000 for the large tile, 1500 for the
+// fold of the small ones, twice that for 8-byte elements), 2500 for the exchange inside a cluster.  Clusters of four
+// and eight do not fill every SM (a cluster lives in one GPC): 144 and 128 of the 148.
+LaunchPlan plan_without_workspace(const cuasr_b200_desc_t& desc, int m, int n, int k, int sms, bool all_tiles) {
+  const int tk = kTileKBytes / (desc.dtype == CUASR_F64 ? 8 : 4);
+  const double per_k = clocks_per_k(desc), wide = desc.dtype == CUASR_F64 ? 2.0 : 1.0;
+  LaunchPlan best;
+  for (int tile = all_tiles ? kLargeTile : kSmallTile; tile <= kSmallTile; ++tile) {
+    const long long tiles = static_cast<long long>((m + kTileRows[tile] - 1) / kTileRows[tile]) * ((n + kTileCols[tile] - 1) / kTileCols[tile]);
+    const int step = tk * kTileSub[tile];
+    const int k_steps = (k + step - 1) / step;
+    for (int z = 1; z <= (tile == kLargeTile ? 1 : 8); z *= 2) {
+      const int per_piece = (k_steps + z - 1) / z;
+      if ((z - 1) * per_piece >= k_steps) break;                        // every CTA of a cluster has work
+      const long long room = z <= 2 ? sms : z == 4 ? sms * 36LL / 37 : sms * 32LL / 37;
+      const long long waves = (tiles * z + room - 1) / room;
+      const double end = (tile == kLargeTile ? 2000 : 1500) * wide + (z > 1 ? 2500 : 0);
+      const double cost = 3000 + static_cast<double>(waves) * (per_k * step * per_piece / kTileWk[tile] + end);
+      if (cost < best.cost) {
+        best.tile = tile; best.cluster = z; best.cost = cost;
+        best.whole_tiles = z > 1 ? 0 : static_cast<int>(tiles); best.pieces = z;
+      }
+    }
+  }
+  return best;
+}
+// Modelled clocks of a launch of large tiles whose pieces meet through tickets in a workspace.
+double ticket_plan_cost(const cuasr_b200_desc_t& desc, long long tiles, int whole_tiles, int pieces, int k, int sms) {
+  const int tk = kTileKBytes / (desc.dtype == CUASR_F64 ? 8 : 4);
+  const double wide = desc.dtype == CUASR_F64 ? 2.0 : 1.0;
+  const int k_steps = (k + tk - 1) / tk, per_piece = (k_steps + pieces - 1) / pieces;
+  const double per_step = clocks_per_k(desc) * tk;
+  const long long waves = whole_tiles / sms, tail = ((tiles - whole_tiles) * pieces + sms - 1) / sms;
+  // the tickets are cleared by a memset in front of the launch; a piece is parked and read back by the last one
+  return 3000 + 4000 + waves * (per_step * k_steps + 2000 * wide) + tail * (per_step * per_piece + 1000 * wide) + 1000 * wide * pieces;
+}
+
+template <typename T>
+bool ring_has_all_tiles(const cuasr_b200_desc_t& desc) {
+#define X(ADD, MUL) if (desc.add_op == ADD && desc.mul_op == MUL) return all_tiles_instantiated<ADD, MUL, T>();
+  CUASR_FLOAT_RINGS(X)
+  if constexpr (std::is_integral<T>::value) { CUASR_BIT_RINGS(X) }
+#undef X
+  return false;
 }
 
 template <typename T>
@@ -389,30 +441,47 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   const T add_id = load_scalar<T>(args.add_identity), mul_id = load_scalar<T>(args.mul_identity);
   // semiring_linear_combination.h:118-125: C is read unless mult(beta, mult-identity) is the add-identity
   const bool read_c = !(host_op<T>(desc.mul_op, beta, mul_id) == add_id);
-  if (read_c && p.c == nullptr) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
 
-  // split-K scratch
-  unsigned int* tickets = nullptr;
-  T* partial = nullptr;
-  BalancePlan plan{static_cast<int>(tile_count(args)), 1};
+  constexpr int TK = kTileKBytes / sizeof(T);
+  const long long tiles = static_cast<long long>(tile_count(args));
+  const bool all_tiles = ring_has_all_tiles<T>(desc);
+  LaunchPlan plan = plan_without_workspace(desc, p.m, p.n, p.k, dev->sms, all_tiles);
+  bool tickets_used = false, balanced = false;
   // partials are moved 16 bytes at a time and re-packed operands are read by TMA: a workspace that does not start
   // on a 16-byte boundary is an error where it is required and is left unused where it is optional
   const bool workspace_aligned = reinterpret_cast<uintptr_t>(args.workspace) % 16 == 0;
+  auto take_ticket_plan = [&](int whole_tiles, int pieces, double cost) {
+    plan.tile = kLargeTile; plan.cluster = 1; plan.whole_tiles = whole_tiles; plan.pieces = pieces; plan.cost = cost;
+    tickets_used = true;
+  };
+  if (slices > 1 && args.workspace == nullptr) return CUASR_STATUS_ERROR_WORKSPACE_NULL;
+  if (read_c && p.c == nullptr) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
   if (slices > 1) {
     const size_t need = splitk_workspace_bytes(desc, args);
-    if (args.workspace == nullptr) return CUASR_STATUS_ERROR_WORKSPACE_NULL;
     if (args.workspace_bytes < need) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
     if (!workspace_aligned) return CUASR_STATUS_ERROR_MISALIGNED_OPERAND;
-    // as many pieces as the workspace at hand has room for (it always has room for `slices`)
-    const size_t per_piece = splitk_bytes_for_pieces(desc, args, 1) - splitk_bytes_for_pieces(desc, args, 0);
-    const long long room = static_cast<long long>((args.workspace_bytes - splitk_bytes_for_pieces(desc, args, 0)) / per_piece);
-    plan = BalancePlan{0, static_cast<int>(splitk_pieces(desc, args, dev->sms, room))};
-  } else if (args.workspace != nullptr && workspace_aligned) {
+    if (all_tiles) {
+      // as many pieces as the workspace at hand has room for (it always has room for `slices`), unless a cluster does
+      // it sooner; floating-point sums keep the cutting that was asked for
+      const size_t per_piece = splitk_bytes_for_pieces(desc, args, 1) - splitk_bytes_for_pieces(desc, args, 0);
+      const long long room = static_cast<long long>((args.workspace_bytes - splitk_bytes_for_pieces(desc, args, 0)) / per_piece);
+      const int pieces = static_cast<int>(splitk_pieces(desc, args, dev->sms, room));
+      const double cost = ticket_plan_cost(desc, tiles, 0, pieces, p.k, dev->sms);
+      if (cost < plan.cost || !splitk_order_independent(desc)) take_ticket_plan(0, pieces, cost);
+    }
+  } else if (args.workspace != nullptr && workspace_aligned && all_tiles) {
     // an optional workspace on an unsplit launch buys load balancing, if it is large enough for the plan
-    constexpr int tk = kTileKBytes / sizeof(T);
-    const BalancePlan wish = balance_plan(static_cast<long long>(tile_count(args)), dev->sms, (args.k + tk - 1) / tk);
-    if (wish.pieces > 1 && args.workspace_bytes >= balance_workspace_bytes(desc, args, dev->sms)) plan = wish;
+    const BalancePlan wish = balance_plan(tiles, dev->sms, (args.k + TK - 1) / TK);
+    if (wish.pieces > 1 && args.workspace_bytes >= balance_workspace_bytes(desc, args, dev->sms)) {
+      balanced = true;
+      const double cost = ticket_plan_cost(desc, tiles, wish.whole_tiles, wish.pieces, p.k, dev->sms);
+      if (cost < plan.cost) take_ticket_plan(wish.whole_tiles, wish.pieces, cost);
+    }
   }
+  const bool pads_itself = ring_pads_itself(desc, args);
+  // operands whose storage lines overlap (leading dimension below the contiguous extent) stay off the TMA path
+  const bool dense = p.lda >= (p.a_kcontig ? p.k : p.m) && p.ldb >= (p.b_kcontig ? p.k : p.n);
+  const bool small = static_cast<long long>(p.m) * p.n < 64 * 64;
   // the rest of an optional workspace holds K-contiguous, aligned copies of operands (see RepackPlan)
   bool repacked = false;
   int k_map = p.k;              // K extent the tensor maps describe
@@ -443,110 +512,74 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
       k_map = k_copy;
     }
   }
-  if (plan.pieces > 1) {
-    const size_t ticket_bytes = ticket_bytes_for(args);
-    tickets = static_cast<unsigned int*>(args.workspace);
-    partial = reinterpret_cast<T*>(static_cast<char*>(args.workspace) + ticket_bytes);
-    // same role as the semaphore memset of device/srgemm.h:253-259
-    if (cudaMemsetAsync(tickets, 0, ticket_bytes, stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
+
+  const bool describable = tma_describable(p.a, p.lda, sizeof(T)) && tma_describable(p.b, p.ldb, sizeof(T));
+  // the name a caller sees: "tma..." where the storage lines are what TMA could describe
+  const bool aligned_name = (pads_itself || k_map % TK == 0) && !small && dense && describable;
+  const int step = TK * kTileSub[plan.tile];
+  const bool nan_pad = std::is_floating_point<T>::value && (desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM);
+  // TMA brings in what lies along k on aligned lines, unless a ragged last step needs padding it cannot write
+  const bool fill_ok = encode_tiled_fn() != nullptr && dense && (pads_itself || k_map % step == 0);
+  TmaParams<T> tp;
+  tp.M = p.m; tp.N = p.n; tp.K = p.k;
+  tp.A = static_cast<const T*>(p.a); tp.lda = p.lda;
+  tp.B = static_cast<const T*>(p.b); tp.ldb = p.ldb;
+  tp.a_mode = p.a_kcontig ? (fill_ok && tma_describable(p.a, p.lda, sizeof(T)) ? kLoadTma : kLoadGatherK) : kLoadGatherMN;
+  tp.b_mode = p.b_kcontig ? (fill_ok && tma_describable(p.b, p.ldb, sizeof(T)) ? kLoadTma : kLoadGatherK) : kLoadGatherMN;
+  CUtensorMap map_a = {}, map_b = {};
+  if (tp.a_mode == kLoadTma &&
+      !make_operand_map<T>(&map_a, tp.A, p.lda, p.m, k_map, true, nan_pad, kTileRows[plan.tile])) tp.a_mode = kLoadGatherK;
+  if (tp.b_mode == kLoadTma &&
+      !make_operand_map<T>(&map_b, tp.B, p.ldb, p.n, k_map, true, nan_pad, kTileCols[plan.tile])) tp.b_mode = kLoadGatherK;
+  if (k_map != p.k && (tp.a_mode != kLoadTma || tp.b_mode != kLoadTma)) tp.K = k_map;   // copies that hold their own padding
+  tp.pad_a = tp.pad_b = T(0);
+  if (nan_pad) tp.pad_a = tp.pad_b = static_cast<T>(NAN);
+  else if (!pads_itself) { tp.pad_a = add_id; tp.pad_b = mul_id; }
+  tp.C = static_cast<const T*>(p.c); tp.ldc = p.ldc;
+  tp.D = static_cast<T*>(p.d); tp.ldd = p.ldd;
+  tp.alpha = alpha; tp.beta = beta; tp.add_identity = add_id; tp.read_c = read_c;
+  tp.part_identity = desc.add_op == CUASR_OP_PLUS || desc.add_op == CUASR_OP_BIT_XOR ? T(0) : add_id;
+  tp.n_extra = extra.count;
+  bool vec = tma_describable(p.d, p.ldd, sizeof(T)) && (!read_c || tma_describable(p.c, p.ldc, sizeof(T))) && p.n % (16 / (int)sizeof(T)) == 0;
+  for (int x = 0; x < extra.count; ++x) {
+    tp.extra_d[x] = static_cast<T*>(extra.ptr[x]);
+    vec = vec && reinterpret_cast<uintptr_t>(extra.ptr[x]) % 16 == 0;
   }
-
-  constexpr int TK = kTileKBytes / sizeof(T);
-  const bool is_float = std::is_floating_point<T>::value;
-  const bool min_or_max = desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM;
-  const bool zero_pad_ok =
-      (desc.add_op == CUASR_OP_PLUS && desc.mul_op == CUASR_OP_MULTIPLIES) ||
-      ((desc.add_op == CUASR_OP_BIT_OR || desc.add_op == CUASR_OP_BIT_XOR) &&
-       (desc.mul_op == CUASR_OP_BINARY_AND || desc.mul_op == CUASR_OP_BIT_AND)) ||
-      (desc.add_op == CUASR_OP_BINARY_OR && desc.mul_op == CUASR_OP_BINARY_AND && (add_id == T(0) || add_id == T(1)));
-  const bool nan_pad = is_float && min_or_max;
-  const bool paddable = nan_pad || zero_pad_ok || (k_map % TK == 0);
-  auto tma_ok = [&](const void* ptr, long long ld) {
-    return reinterpret_cast<uintptr_t>(ptr) % 16 == 0 && (ld * (long long)sizeof(T)) % 16 == 0;
-  };
-  const bool small = static_cast<long long>(p.m) * p.n < 64 * 64;
-  // operands whose storage lines overlap (leading dimension below the contiguous extent) stay off the TMA path
-  const bool dense = p.lda >= (p.a_kcontig ? p.k : p.m) && p.ldb >= (p.b_kcontig ? p.k : p.n);
-  bool use_tma = paddable && !small && dense && tma_ok(p.a, p.lda) && tma_ok(p.b, p.ldb) && encode_tiled_fn() != nullptr;
-
+  tp.vector_epilogue = vec;
+  tp.tiles_m = (p.m + kTileRows[plan.tile] - 1) / kTileRows[plan.tile];
+  tp.tiles_n = (p.n + kTileCols[plan.tile] - 1) / kTileCols[plan.tile];
+  tp.status = dev->status;
+  tp.whole_tiles = plan.whole_tiles;
+  tp.slices = plan.pieces;
+  tp.cluster = plan.cluster > 1;
+  const int k_steps = (p.k + step - 1) / step;
+  tp.k_tiles_per_slice = (k_steps + plan.pieces - 1) / plan.pieces;
+  tp.partial = nullptr; tp.tickets = nullptr;
+  if (tickets_used && plan.pieces > 1) {
+    const size_t ticket_bytes = ticket_bytes_for(args);
+    tp.tickets = static_cast<unsigned int*>(args.workspace);
+    tp.partial = reinterpret_cast<T*>(static_cast<char*>(args.workspace) + ticket_bytes);
+    // same role as the semaphore memset of device/srgemm.h:253-259
+    if (cudaMemsetAsync(tp.tickets, 0, ticket_bytes, stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
+  }
+  const long long all = static_cast<long long>(tp.tiles_m) * tp.tiles_n;
+  const long long work = plan.whole_tiles + (all - plan.whole_tiles) * plan.pieces;
+  if (work > 2147483647LL) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
+  const int grid = static_cast<int>(plan.cluster > 1 || work < dev->sms ? work : dev->sms);
   cudaError_t err = cudaErrorInvalidValue;
   bool launched = false;
-  if (use_tma) {
-    CUtensorMap map_a, map_b;
-    if (make_operand_map<T>(&map_a, static_cast<const T*>(p.a), p.lda, p.m, k_map, p.a_kcontig, nan_pad) &&
-        make_operand_map<T>(&map_b, static_cast<const T*>(p.b), p.ldb, p.n, k_map, p.b_kcontig, nan_pad)) {
-      TmaParams<T> tp;
-      tp.M = p.m; tp.N = p.n; tp.K = p.k;
-      tp.C = static_cast<const T*>(p.c); tp.ldc = p.ldc;
-      tp.D = static_cast<T*>(p.d); tp.ldd = p.ldd;
-      tp.alpha = alpha; tp.beta = beta; tp.add_identity = add_id; tp.read_c = read_c;
-      tp.n_extra = extra.count;
-      bool vec = tma_ok(p.d, p.ldd) && (!read_c || tma_ok(p.c, p.ldc)) && p.n % (16 / (int)sizeof(T)) == 0;
-      for (int x = 0; x < extra.count; ++x) {
-        tp.extra_d[x] = static_cast<T*>(extra.ptr[x]);
-        vec = vec && reinterpret_cast<uintptr_t>(extra.ptr[x]) % 16 == 0;
-      }
-      tp.vector_epilogue = vec;
-      tp.tiles_m = (p.m + kTileM - 1) / kTileM; tp.tiles_n = (p.n + kTileN - 1) / kTileN;
-      tp.status = dev->status;
-      tp.whole_tiles = plan.whole_tiles;
-      tp.slices = plan.pieces;
-      const int k_tiles = (p.k + TK - 1) / TK;
-      tp.k_tiles_per_slice = (k_tiles + plan.pieces - 1) / plan.pieces;
-      tp.partial = partial; tp.tickets = tickets;
-      const long long all_tiles = static_cast<long long>(tp.tiles_m) * tp.tiles_n;
-      const long long work = plan.whole_tiles + (all_tiles - plan.whole_tiles) * plan.pieces;
-      const int grid = static_cast<int>(work < dev->sms ? work : dev->sms);
-#define X(ADD, MUL)                                                                                       \
-      if (!launched && desc.add_op == ADD && desc.mul_op == MUL) {                                        \
-        if constexpr (tma_instantiated<ADD, MUL, T>()) {                                                  \
-          err = launch_tma<ADD, MUL, T>(p.a_kcontig, p.b_kcontig, map_a, map_b, tp, grid, stream);        \
-          launched = true;                                                                                \
-        }                                                                                                 \
-      }
-      CUASR_FLOAT_RINGS(X)
-      if constexpr (std::is_integral<T>::value) { CUASR_BIT_RINGS(X) }
-#undef X
-      if (launched)
-        t_last_kernel = slices > 1 ? "tma_splitk" : plan.pieces > 1 ? "tma_balanced" : repacked ? "tma_repacked" : "tma";
-    }
+#define X(ADD, MUL)                                                                                    \
+  if (!launched && desc.add_op == ADD && desc.mul_op == MUL) {                                         \
+    err = launch_tma<ADD, MUL, T>(plan.tile, map_a, map_b, tp, grid, plan.cluster, stream);            \
+    launched = true;                                                                                   \
   }
-  if (!launched) {
-    GenericParams<T> gp;
-    gp.M = p.m; gp.N = p.n; gp.K = p.k;
-    gp.A = static_cast<const T*>(p.a); gp.a_row = p.a_kcontig ? p.lda : 1; gp.a_col = p.a_kcontig ? 1 : p.lda;
-    gp.B = static_cast<const T*>(p.b); gp.b_row = p.b_kcontig ? 1 : p.ldb; gp.b_col = p.b_kcontig ? p.ldb : 1;
-    gp.C = static_cast<const T*>(p.c); gp.ldc = p.ldc;
-    gp.D = static_cast<T*>(p.d); gp.ldd = p.ldd;
-    gp.n_extra = extra.count;
-    for (int x = 0; x < extra.count; ++x) gp.extra_d[x] = static_cast<T*>(extra.ptr[x]);
-    gp.alpha = alpha; gp.beta = beta; gp.add_identity = add_id; gp.read_c = read_c;
-    gp.k_per_slice = (p.k + slices - 1) / slices;
-    gp.partial = slices > 1 ? partial : nullptr;
-#define X(ADD, MUL)                                                   \
-    if (!launched && desc.add_op == ADD && desc.mul_op == MUL) {      \
-      err = launch_generic<ADD, MUL, T>(gp, slices, stream);          \
-      launched = true;                                                \
-    }
-    CUASR_FLOAT_RINGS(X)
-    if constexpr (std::is_integral<T>::value) { CUASR_BIT_RINGS(X) }
+  CUASR_FLOAT_RINGS(X)
+  if constexpr (std::is_integral<T>::value) { CUASR_BIT_RINGS(X) }
 #undef X
-    if (launched && err == cudaSuccess && slices > 1) {
-      g_launches.fetch_add(1);
-      bool reduced = false;
-#define X(ADD, MUL)                                                   \
-      if (!reduced && desc.add_op == ADD && desc.mul_op == MUL) {     \
-        err = launch_generic_reduce<ADD, MUL, T>(gp, slices, stream); \
-        reduced = true;                                               \
-      }
-      CUASR_FLOAT_RINGS(X)
-      if constexpr (std::is_integral<T>::value) { CUASR_BIT_RINGS(X) }
-#undef X
-    }
-    if (launched) t_last_kernel = slices > 1 ? "generic_splitk" : "generic";
-  }
   if (!launched) return CUASR_STATUS_ERROR_NOT_SUPPORTED;
   if (err != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
+  t_last_kernel = !aligned_name ? (slices > 1 ? "generic_splitk" : "generic")
+                  : slices > 1 ? "tma_splitk" : balanced ? "tma_balanced" : repacked ? "tma_repacked" : "tma";
   g_launches.fetch_add(1);
   return CUASR_STATUS_SUCCESS;
 }

@@ -1,0 +1,96 @@
+// Operand staging by ordinary loads: copies a tile of an operand with ANY leading dimension, alignment and layout
+// into the shared-memory layout the contraction reads, [rows][128 bytes of k] with TMA's 128-byte swizzle.
+//
+// TMA describes an operand only if its address and leading dimension are multiples of 16 bytes, cannot transpose,
+// and fills out-of-range elements with zero or NaN only.  The four producer warps of a CTA have nothing to do while
+// TMA works, so where TMA cannot deliver the K-contiguous layout they bring the elements themselves with 4- or 8-byte
+// cp.async, transposing on the way, and write any padding value a ring needs past the end of K.
+// Cost: 128 threads issue 64 cp.async each per 32 KiB stage, about 1000 of the 8500 clocks that stage's arithmetic takes.
+#pragma once
+
+#include "ring.cuh"
+
+namespace cuasr_b200 {
+
+// How an operand reaches shared memory.
+enum LoadMode : int {
+  kLoadTma = 0,          // contiguous along k, 16-byte aligned storage lines: TMA
+  kLoadGatherK = 1,      // contiguous along k, any alignment: lanes along k
+  kLoadGatherMN = 2,     // contiguous along rows, any alignment: 8 rows x 4 k per warp instruction
+};
+
+template <int kBytes>
+__device__ __forceinline__ void cp_async(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(kBytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// The barrier receives this thread's arrival when all cp.async the thread has issued so far have landed.
+__device__ __forceinline__ void cp_async_arrive_noinc(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void sts(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
+__device__ __forceinline__ void sts(uint32_t addr, int32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts(uint32_t addr, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts(uint32_t addr, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory"); }
+
+// Stages rows [r0, r0 + kRows) x k [k0, k0 + kSub * 128 bytes) of an operand whose element (r, k) is base[r * ld + k]
+// (kLoadGatherK) or base[r + k * ld] (kLoadGatherMN).  Rows at or beyond `rows` are left alone (their results are
+// never stored); k at or beyond K is set to `pad` by plain stores, so a stage that reaches beyond K must not be announced
+// with cp_async_arrive_noinc alone.  Called by all 128 producer threads; `pw` is the producer warp (0..3).
+template <typename T, int kRows, int kSub>
+__device__ __forceinline__ void gather_tile(uint32_t dst, const T* __restrict__ base, long long ld, int mode, int r0,
+                                            int rows, int k0, int K, T pad, int pw, int lane) {
+  constexpr int TK = 128 / (int)sizeof(T);         // k per 128-byte row
+  constexpr int ES = (int)sizeof(T);
+  // opaque: the lane's offsets are computed here, per stage, instead of being held in the producers' few registers
+  asm volatile("" : "+r"(lane), "+r"(pw));
+  if (mode == kLoadGatherMN) {
+    // A warp instruction covers 8 rows x 4 k: four 32-byte (64-byte for 8-byte elements) pieces of global memory, and
+    // (row & 7) spreads the 8 rows over the 8 swizzled chunks, so the shared-memory writes do not conflict.
+    const int r8 = lane & 7, kq = lane >> 3;
+    const int left = rows - r0 - r8;               // row block i is inside if 8 i < left
+#pragma unroll 1
+    for (int sub = 0; sub < kSub; ++sub) {
+#pragma unroll 1
+      for (int step = 0; step < TK / 16; ++step) {
+        const int kk = step * 16 + pw * 4 + kq;
+        const int k = k0 + sub * TK + kk;
+        const uint32_t d = dst + sub * (kRows * 128) + r8 * 128 + ((((kk * ES) >> 4) ^ r8) << 4) + ((kk * ES) & 15);
+        if (k < K) {
+          const T* s = base + (long long)k * ld + (r0 + r8);
+          if (rows - r0 >= kRows) {
+#pragma unroll
+            for (int i = 0; i < kRows / 8; ++i) cp_async<ES>(d + i * 1024, s + 8 * i);
+          } else {
+#pragma unroll
+            for (int i = 0; i < kRows / 8; ++i)
+              if (8 * i < left) cp_async<ES>(d + i * 1024, s + 8 * i);
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < kRows / 8; ++i) sts(d + i * 1024, pad);
+        }
+      }
+    }
+  } else {
+    constexpr int kRowsPerInstr = ES == 8 ? 2 : 1;
+    const int kk = ES == 8 ? (lane & 15) : lane;
+    const int rr = ES == 8 ? pw * 2 + (lane >> 4) : pw;
+#pragma unroll 1
+    for (int sub = 0; sub < kSub; ++sub) {
+      const int k = k0 + sub * TK + kk;
+      const bool in_k = k < K;
+      const T* s = base + (long long)(r0 + rr) * ld + k;
+#pragma unroll 4
+      for (int i = 0; i < kRows / (4 * kRowsPerInstr); ++i) {
+        const int row = rr + 4 * kRowsPerInstr * i;
+        const uint32_t d = dst + sub * (kRows * 128) + row * 128 + ((((kk * ES) >> 4) ^ (row & 7)) << 4) + ((kk * ES) & 15);
+        if (!in_k) sts(d, pad);
+        else if (r0 + row < rows) cp_async<ES>(d, s);
+        s += 4 * kRowsPerInstr * ld;
+      }
+    }
+  }
+}
+
+}  // namespace cuasr_b200

@@ -1,25 +1,7 @@
-// Every supported ring on the generic (any alignment, any shape) kernel.
-#include "srgemm_launch_impl.cuh"
+// Launcher of the operand copies.
+#include "repack.cuh"
+#include "srgemm_launch.h"
 namespace cuasr_b200 {
-#define CUASR_ALL_TYPES(ADD, MUL)              \
-  CUASR_INSTANTIATE_GENERIC(ADD, MUL, float)   \
-  CUASR_INSTANTIATE_GENERIC(ADD, MUL, double)  \
-  CUASR_INSTANTIATE_GENERIC(ADD, MUL, int32_t) \
-  CUASR_INSTANTIATE_GENERIC(ADD, MUL, uint32_t)
-#define CUASR_INT_TYPES(ADD, MUL)              \
-  CUASR_INSTANTIATE_GENERIC(ADD, MUL, int32_t) \
-  CUASR_INSTANTIATE_GENERIC(ADD, MUL, uint32_t)
-CUASR_ALL_TYPES(CUASR_OP_PLUS, CUASR_OP_MULTIPLIES)
-CUASR_ALL_TYPES(CUASR_OP_MINIMUM, CUASR_OP_PLUS)
-CUASR_ALL_TYPES(CUASR_OP_MAXIMUM, CUASR_OP_PLUS)
-CUASR_ALL_TYPES(CUASR_OP_MINIMUM, CUASR_OP_MAXIMUM)
-CUASR_ALL_TYPES(CUASR_OP_MAXIMUM, CUASR_OP_MINIMUM)
-CUASR_ALL_TYPES(CUASR_OP_MINIMUM, CUASR_OP_MULTIPLIES)
-CUASR_ALL_TYPES(CUASR_OP_MAXIMUM, CUASR_OP_MULTIPLIES)
-CUASR_ALL_TYPES(CUASR_OP_BINARY_OR, CUASR_OP_BINARY_AND)
-CUASR_INT_TYPES(CUASR_OP_BIT_XOR, CUASR_OP_BIT_AND)
-CUASR_INT_TYPES(CUASR_OP_BIT_OR, CUASR_OP_BIT_AND)
-CUASR_INT_TYPES(CUASR_OP_BIT_XOR, CUASR_OP_BINARY_AND)
 cudaError_t launch_repack(const void* src, long long ld_src, bool src_kcontig, int rows, int K, int K_out,
                           unsigned long long pad_bits, void* dst, long long ld_dst, size_t element_bytes,
                           cudaStream_t stream) {

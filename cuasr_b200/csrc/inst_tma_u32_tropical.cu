@@ -1,5 +1,5 @@
 // Tropical (min-plus, max-plus) and bottleneck (min-max, max-min) rings over unsigned 32-bit integers on the TMA
-// kernel (only when K is a multiple of the K step: there is no padding value for them).
+// kernel.
 #include "srgemm_launch_impl.cuh"
 namespace cuasr_b200 {
 CUASR_INSTANTIATE_TMA(CUASR_OP_MINIMUM, CUASR_OP_PLUS, uint32_t)

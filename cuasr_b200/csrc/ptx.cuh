@@ -108,6 +108,12 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
+// Programmatic dependent launch: a kernel that is launched while the one before it in the stream still runs waits here
+// until that kernel has completed and its writes are visible ...
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// ... and lets the next one start its own set-up as soon as every CTA of this grid has come this far.
+__device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- packed / three-input arithmetic (sm_100 and later) ----
 
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {

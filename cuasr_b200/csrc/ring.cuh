@@ -9,6 +9,7 @@
 
 #include <cstdint>
 #include <type_traits>
+#include <utility>
 
 #include "../../include/cuasr_b200_types.h"
 #include "ptx.cuh"

@@ -1,25 +1,25 @@
-// Host-side launchers of the SRGEMM kernels, one template per kernel family.  The definitions live in
-// srgemm_launch_impl.cuh and are instantiated explicitly, ring by ring, in the inst_*.cu files so that
-// the rings compile in parallel; abi.cu only sees these declarations.
+// Host-side launchers of the SRGEMM kernel.  The definitions live in srgemm_launch_impl.cuh and are instantiated
+// explicitly, ring by ring, in the inst_*.cu files so that the rings compile in parallel; abi.cu only sees these
+// declarations.
 #pragma once
 
 #include <cuda.h>
 #include <cuda_runtime.h>
 
-#include "srgemm_generic.cuh"
 #include "srgemm_tma.cuh"
 
 namespace cuasr_b200 {
 
-// Launches srgemm_tma_kernel<Ring<ADD, MUL, T>, a_kcontig, b_kcontig> on `grid` persistent CTAs.
-template <int ADD, int MUL, typename T>
-cudaError_t launch_tma(bool a_kcontig, bool b_kcontig, const CUtensorMap& map_a, const CUtensorMap& map_b,
-                       const TmaParams<T>& params, int grid, cudaStream_t stream);
+enum TileKind : int { kLargeTile = 0, kMediumTile = 1, kSmallTile = 2 };
 
-// Which (ring, element type) pairs have the TMA kernel compiled in (see the inst_tma_*.cu files); every
-// other supported pair runs on the generic kernel.
+// Launches srgemm_tma_kernel<Ring<ADD, MUL, T>, tile> on `grid` CTAs in clusters of `cluster`.
 template <int ADD, int MUL, typename T>
-constexpr bool tma_instantiated() {
+cudaError_t launch_tma(int tile, const CUtensorMap& map_a, const CUtensorMap& map_b, const TmaParams<T>& params,
+                       int grid, int cluster, cudaStream_t stream);
+
+// (ring, element type) pairs that have every tile shape compiled in; the others run on the small tile alone.
+template <int ADD, int MUL, typename T>
+constexpr bool all_tiles_instantiated() {
   constexpr bool tropical = (ADD == CUASR_OP_MINIMUM || ADD == CUASR_OP_MAXIMUM) && MUL == CUASR_OP_PLUS;
   constexpr bool minmax = (ADD == CUASR_OP_MINIMUM && MUL == CUASR_OP_MAXIMUM) ||
                           (ADD == CUASR_OP_MAXIMUM && MUL == CUASR_OP_MINIMUM);
@@ -28,19 +28,9 @@ constexpr bool tma_instantiated() {
   constexpr bool bits = (ADD == CUASR_OP_BIT_XOR || ADD == CUASR_OP_BIT_OR) &&
                         (MUL == CUASR_OP_BIT_AND || MUL == CUASR_OP_BINARY_AND) &&
                         !(ADD == CUASR_OP_BIT_OR && MUL == CUASR_OP_BINARY_AND);
-  if (std::is_same<T, float>::value) return tropical || minmax || times;
-  if (std::is_same<T, double>::value) return tropical || minmax || times;
+  if (std::is_floating_point<T>::value) return tropical || minmax || times;
   return bits || tropical || minmax;  // int32_t, uint32_t
 }
-
-// Launches srgemm_generic_kernel<Ring<ADD, MUL, T>> on a (ceil(N/64), ceil(M/64), slices) grid.
-template <int ADD, int MUL, typename T>
-cudaError_t launch_generic(const GenericParams<T>& params, int slices, cudaStream_t stream);
-
-// Second step of a split-K run on the generic kernel: D = epilogue((+) over slices of partial), the work of
-// the reference's ReduceSplitK (include/cuasr/reduction/kernel/reduce_split_k.h:162-236).
-template <int ADD, int MUL, typename T>
-cudaError_t launch_generic_reduce(const GenericParams<T>& params, int slices, cudaStream_t stream);
 
 // Copies a rows x K operand of 4- or 8-byte elements, K-contiguous or MN-contiguous with any leading dimension and
 // alignment, into K-contiguous storage with leading dimension ld_dst; columns K .. K_out - 1 of the copy are set to
@@ -48,5 +38,26 @@ cudaError_t launch_generic_reduce(const GenericParams<T>& params, int slices, cu
 cudaError_t launch_repack(const void* src, long long ld_src, bool src_kcontig, int rows, int K, int K_out,
                           unsigned long long pad_bits, void* dst, long long ld_dst, size_t element_bytes,
                           cudaStream_t stream);
+
+// Kernel launch that lets the kernel's set-up overlap the end of the kernel before it in the stream (the kernel must
+// call grid_dependency_wait() before it touches global memory).
+template <typename... Params, typename... Args>
+cudaError_t launch_overlapped(void (*kernel)(Params...), int grid, int block, int smem_bytes, int cluster,
+                              cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(static_cast<unsigned>(grid));
+  config.blockDim = dim3(static_cast<unsigned>(block));
+  config.dynamicSmemBytes = static_cast<size_t>(smem_bytes);
+  config.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  config.attrs = attr;
+  config.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
+}
 
 }  // namespace cuasr_b200

@@ -40,6 +40,9 @@ struct PathTmaParams {
   unsigned int* status;
 };
 
+constexpr int kStages = 5;
+constexpr int kOperandStageBytes = kTileM * kTileKBytes;   // 16 KiB
+constexpr int kStageBytes = 2 * kOperandStageBytes;
 constexpr int kPathTmaSmemBytes = kStages * kStageBytes + 1024 /* alignment slack */ + 256 /* barriers */;
 
 template <bool kMaximize, bool kAK, bool kBK>

@@ -4,53 +4,78 @@
 // its threadblock mainloop SrmmaPipelined (include/cuasr/gemm/threadblock/srmma_pipelined.h:153-288),
 // the warp/thread level (include/cuasr/gemm/warp/srmma_simt.h:139-199,
 // include/cuasr/gemm/thread/srmma_sm50.h:118-146) and the epilogue functor
-// (include/cuasr/gemm/epilogue/thread/semiring_linear_combination.h:118-183); with `partial` set it is
-// also the first half of kernel::SrgemmSplitKParallel (include/cuasr/gemm/kernel/srgemm_splitk_parallel.h:86-219).
+// (include/cuasr/gemm/epilogue/thread/semiring_linear_combination.h:118-183); with split tiles it is
+// also kernel::SrgemmSplitKParallel (include/cuasr/gemm/kernel/srgemm_splitk_parallel.h:86-219).
 //
-// Structure (one persistent CTA per SM, 12 warps = 2 consumer warpgroups + 1 producer warpgroup that
-// hands most of its registers to the consumers with setmaxnreg):
-//   warp 8, lane 0      producer: for every K tile of every output tile this CTA owns, waits for a free
-//                       stage and issues two TMA tile loads (A, B) that complete on the stage's mbarrier.
-//   warps 0..7          consumers: 2 x 4 warps over a 128 x 128 output tile, 8 x 4 lanes per warp, an
-//                       8 x 8 register micro-tile per lane.  They wait for a stage, read 16-byte vectors
-//                       from shared memory and run the contraction two k steps at a time:
-//                       acc = add(acc, a0 (x) b0, a1 (x) b1)  — for fp32 min/max rings one add per product
-//                       plus ONE three-input min/max per two products.
-// Shared-memory tile layouts (per stage, 16 KiB per operand):
-//   K-contiguous operand  (row-major A, column-major B): [128 rows][128 bytes of k], TMA 128-byte swizzle;
-//                         a lane owns rows lane_row + 8 i (A) / lane_col + 4 j (B) and loads 16 bytes of k.
-//   MN-contiguous operand (column-major A, row-major B): [k][128 rows], no swizzle; a lane owns groups of
-//                         16/sizeof(T) adjacent rows and loads one k of a group per 16-byte vector.
-// Ragged edges: TMA fills out-of-range elements with NaN (fp min/max rings; min/max never select a NaN
-// product) or zero (rings where 0 (x) 0 is neutral); stores are predicated on m < M, n < N.
+// Structure (one CTA per SM, 12 warps = 2 consumer warpgroups + 1 producer warpgroup that hands most of its
+// registers to the consumers with setmaxnreg):
+//   warps 8..11         producers: for every K step of every output tile this CTA owns, wait for a free stage and
+//                       fill it: operands that lie contiguous along k on 16-byte storage lines by TMA (one lane),
+//                       all others by the cp.async gather of gather.cuh (all 128 threads).  Either way the stage
+//                       holds [rows][128 bytes of k] with the 128-byte swizzle, so there is one contraction loop.
+//   warps 0..7          consumers: WM x WN x WK warps.  A warp owns a 64 x 32 block of the tile (8 x 4 lanes, an
+//                       8 x 8 register micro-tile per lane) and every WK-th part of each stage's k range.
+//                       They wait for a stage, read 16-byte vectors and run the contraction two k steps at a time:
+//                       acc = add(acc, a0 (x) b0, a1 (x) b1)  — for fp32 min/max rings one packed add for both
+//                       products plus ONE three-input min/max.
+// Tiles: WM x WN x WK = 2 x 4 x 1 is a 128 x 128 tile, for outputs with enough of them to fill the GPU.  Smaller
+// outputs leave most SMs idle with it, and a smaller micro-tile would be bound by shared-memory reads, so the smaller
+// tiles keep the 8 x 8 micro-tile and put the spare warps on other parts of k: 2 x 2 x 2 (128 x 64) and 1 x 2 x 4
+// (64 x 64).  Their partial results meet in shared memory, in a fixed order, on the way to the output.
+// Clusters: where even the 64 x 64 tiles are fewer than the SMs, the CTAs of a thread-block cluster share a tile's k
+// range and fold their partial tiles through distributed shared memory: no workspace, no second launch.
 #pragma once
 
-#include "ring.cuh"
+#include "gather.cuh"
 
 namespace cuasr_b200 {
 
-constexpr int kTileM = 128;
+constexpr int kTileM = 128;                       // the large tile; also the unit of the split-K scratch
 constexpr int kTileN = 128;
-constexpr int kTileKBytes = 128;                 // bytes of k per stage and row
-constexpr int kStages = 5;
+constexpr int kTileKBytes = 128;                 // bytes of k per swizzled shared-memory row
 constexpr int kConsumerWarps = 8;
-constexpr int kProducerWarps = 4;                 // one warpgroup; only its first lane issues TMA
+constexpr int kProducerWarps = 4;                 // one warpgroup
+constexpr int kConsumerThreads = kConsumerWarps * 32;
 constexpr int kTmaThreads = (kConsumerWarps + kProducerWarps) * 32;
-// Registers per thread after the warpgroups re-balance with setmaxnreg: the two consumer warps and
-// the one producer warp that share an SM sub-partition fit its 16384 registers (2 * 232 + 40 = 504 <= 512).
-constexpr int kConsumerRegs = 232;
-constexpr int kProducerRegs = 40;
-constexpr int kOperandStageBytes = kTileM * kTileKBytes;   // 16 KiB
-constexpr int kStageBytes = 2 * kOperandStageBytes;
+// Registers per thread after the warpgroups re-balance with setmaxnreg: 256 x 224 + 128 x 56 = the 64512 registers
+// the CTA is launched with (384 x 168).
+constexpr int kConsumerRegs = 224;
+constexpr int kProducerRegs = 56;
 constexpr int kEpilogueWarpBytes = 8192;          // per consumer warp: staging for coalesced output rows
-constexpr int kEpilogueBytes = kConsumerWarps * kEpilogueWarpBytes;
 constexpr int kMaxDestinations = 8;               // output copies one launch can write (this GPU + peers)
-constexpr int kTmaSmemBytes =
-    kStages * kStageBytes + kEpilogueBytes + 1024 /* alignment slack */ + 256 /* barriers */;
+constexpr int kMaxSmemBytes = 232448;             // 227 KiB: what one CTA may have
+
+// Tile shape of a kernel variant.
+template <int WM_, int WN_, int WK_>
+struct TileShape {
+  static constexpr int WM = WM_, WN = WN_, WK = WK_;
+  static_assert(WM * WN * WK == kConsumerWarps, "eight consumer warps");
+  static constexpr int kM = 64 * WM, kN = 32 * WN;
+  // 128-byte k columns per stage: two where the k range is shared by four warps, so that each warp gets four of the
+  // 16-byte chunks of a stage (one unrolled pass of the contraction loop)
+  static constexpr int kSub = WK == 4 ? 2 : 1;
+  static constexpr int kABytes = kM * kTileKBytes * kSub;
+  static constexpr int kBBytes = kN * kTileKBytes * kSub;
+  static constexpr int kStageBytes = kABytes + kBBytes;
+  // WK > 1: every warp's 64 x 32 partial block, for the fold; WK = 1: 8 KiB of staging per warp
+  template <typename T>
+  static constexpr int kFoldBytes = WK > 1 ? kConsumerWarps * 64 * 32 * (int)sizeof(T) : kConsumerWarps * kEpilogueWarpBytes;
+  template <typename T>
+  static constexpr int kStages = (kMaxSmemBytes - 1024 - 512 - kFoldBytes<T>) / kStageBytes;
+  template <typename T>
+  static constexpr int kSmemBytes = kStages<T> * kStageBytes + kFoldBytes<T> + 1024 /* alignment */ + 512 /* barriers */;
+};
+using LargeTile = TileShape<2, 4, 1>;    // 128 x 128
+using MediumTile = TileShape<2, 2, 2>;   // 128 x 64
+using SmallTile = TileShape<1, 2, 4>;    // 64 x 64
 
 template <typename T>
 struct TmaParams {
   int M, N, K;
+  const T* A;  long long lda;   // gathered operands only
+  const T* B;  long long ldb;
+  int a_mode, b_mode;           // LoadMode
+  T pad_a, pad_b;               // what a gather writes for k >= K
   const T* C;  long long ldc;   // row-major; may alias D; may be null when !read_c
   T* D;        long long ldd;   // row-major
   // Extra copies of the output: when n_extra > 0 every element of D is also stored to extra_d[i] (same
@@ -59,18 +84,24 @@ struct TmaParams {
   int n_extra;
   T* extra_d[kMaxDestinations - 1];
   T alpha, beta, add_identity;
+  // start value of accumulators beyond the first of an element whose k range is shared (by warps, CTAs or pieces):
+  // the additive identity where (+) is idempotent, the neutral 0 for sums and exclusive ors
+  T part_identity;
   int read_c;
   int vector_epilogue;          // D, C and every extra_d are 16-byte aligned, ld * sizeof(T) % 16 == 0, N % EV == 0
   int tiles_m, tiles_n;
   unsigned int* status;         // device status word (see DeviceStatus)
   // Work decomposition.  Tiles [0, whole_tiles) are computed whole by one CTA each.  Every later tile is cut
-  // along K into `slices` pieces: piece z handles K tiles [z * k_tiles_per_slice, ...), the last piece takes the
-  // rest, and writes its raw accumulators to partial + ((tile - whole_tiles) * slices + z) * 128 * 128 (a full
-  // 128 x 128 block, row-major).  tickets[tile - whole_tiles] counts the pieces written; the CTA that draws the
-  // last ticket folds the pieces in slice order and runs the epilogue, so nobody ever waits and the result does
-  // not depend on which CTA finishes last.  tickets must be zero at launch; the kernel leaves them zero.
-  // Explicit split-K is whole_tiles = 0; a balanced launch splits only the tiles of the last, partial wave.
-  int whole_tiles, slices, k_tiles_per_slice;
+  // along K into `slices` pieces: piece z handles K steps [z * k_tiles_per_slice, ...), the last piece takes the
+  // rest.
+  //  * cluster == 0 (large tile only): a piece writes its raw accumulators to partial +
+  //    ((tile - whole_tiles) * slices + z) * 128 * 128.  tickets[tile - whole_tiles] counts the pieces written; the
+  //    CTA that draws the last ticket folds the pieces in slice order and runs the epilogue, so nobody ever waits
+  //    and the result does not depend on which CTA finishes last.  tickets must be zero at launch; the kernel leaves
+  //    them zero.  Explicit split-K is whole_tiles = 0; a balanced launch splits only the tiles of the last wave.
+  //  * cluster == 1 (WK > 1 only): whole_tiles = 0 and the `slices` CTAs of a cluster hold the pieces of one tile;
+  //    CTA r of the cluster folds and writes the r-th part of the tile.
+  int whole_tiles, slices, k_tiles_per_slice, cluster;
   T* partial;
   unsigned int* tickets;
 };
@@ -88,6 +119,20 @@ __device__ __forceinline__ void lds16(uint32_t addr, int32_t (&v)[4]) {
 __device__ __forceinline__ void lds16(uint32_t addr, double (&v)[2]) {
   asm volatile("ld.shared.v2.f64 {%0,%1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "r"(addr));
 }
+// The same from the shared memory of CTA `rank` of the cluster (own-CTA address).
+__device__ __forceinline__ uint4 lds16_cluster(uint32_t addr, int rank) {
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+  uint4 v;
+  asm volatile("ld.shared::cluster.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(remote) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void consumer_sync() {
+  asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads) : "memory");
+}
 
 // Tile rasterisation: bands of kBand tile columns, rows fastest inside a band, so that the CTAs that
 // run at the same time share A row-panels and B column-panels in L2.
@@ -102,116 +147,150 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
 }
 
 // Work item w of a launch -> (tile, K piece z, number of pieces of that tile).
-__device__ __forceinline__ void decode_work(int w, int num_tiles, int whole_tiles, int slices, int& tile, int& z,
-                                            int& pieces) {
-  if (w < whole_tiles) {
+template <typename T>
+__device__ __forceinline__ void decode_work(const TmaParams<T>& p, int w, int num_tiles, int& tile, int& z, int& pieces) {
+  if (p.cluster) {                       // the CTAs of a cluster are consecutive
+    tile = w / p.slices; z = w - tile * p.slices; pieces = p.slices;
+  } else if (w < p.whole_tiles) {
     tile = w; z = 0; pieces = 1;
   } else {
-    const int tail = num_tiles - whole_tiles;
-    const int v = w - whole_tiles;
+    const int tail = num_tiles - p.whole_tiles;
+    const int v = w - p.whole_tiles;
     z = v / tail;
-    tile = whole_tiles + (v - z * tail);
-    pieces = slices;
+    tile = p.whole_tiles + (v - z * tail);
+    pieces = p.slices;
   }
 }
 
-template <typename RingT, bool kAK, bool kBK>
+template <typename RingT, typename Tile>
 __global__ void __launch_bounds__(kTmaThreads, 1)
 srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                  const TmaParams<typename RingT::Element> p) {
+                  const __grid_constant__ TmaParams<typename RingT::Element> p) {
   using T = typename RingT::Element;
+  constexpr int WM = Tile::WM, WN = Tile::WN, WK = Tile::WK, kSub = Tile::kSub;
+  constexpr int kStages = Tile::template kStages<T>;
+  static_assert(kStages >= 2, "at least double-buffered");
   constexpr int EV = 16 / sizeof(T);              // elements per 16-byte vector: 4 (fp32/int32) or 2 (fp64)
-  constexpr int TK = kTileKBytes / sizeof(T);     // k per stage: 32 or 16
-  constexpr int kChunks = TK / EV;                // 16-byte k chunks per stage: 8
+  constexpr int TK = kTileKBytes / sizeof(T);     // k per 128-byte column: 32 or 16
+  constexpr int kStep = TK * kSub;                // k per stage
+  constexpr int kChunks = 8 * kSub / WK;          // 16-byte k chunks of a stage that one warp works on
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* epi_smem = smem + kStages * kStageBytes;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(epi_smem + kEpilogueBytes);
+  uint8_t* epi_smem = smem + kStages * Tile::kStageBytes;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(epi_smem + Tile::template kFoldBytes<T>);
   uint64_t* empty_bar = full_bar + kStages;
   unsigned int* ticket_smem = reinterpret_cast<unsigned int*>(empty_bar + kStages);
   volatile unsigned int* abandoned = ticket_smem + 1;     // raised when a consumer's wait ran out (see ptx.cuh)
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const bool gathers = p.a_mode != kLoadTma || p.b_mode != kLoadTma;
+  const bool tmas = p.a_mode == kLoadTma || p.b_mode == kLoadTma;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
-      mbar_init(&full_bar[s], 1);
+      mbar_init(&full_bar[s], (tmas ? 1 : 0) + (gathers ? kProducerWarps * 32 : 0));
       mbar_init(&empty_bar[s], kConsumerWarps);
     }
     *abandoned = 0;
     fence_barrier_init();
   }
   __syncthreads();
+  // Launched with programmatic stream serialisation: everything above overlaps the end of the kernel before this one;
+  // nothing below touches global memory before that kernel's results are there.
+  grid_dependency_wait();
+  grid_dependency_launch();
 
-  const int k_tiles_total = (p.K + TK - 1) / TK;
+  const int k_tiles_total = (p.K + kStep - 1) / kStep;
   const int num_tiles = p.tiles_m * p.tiles_n;
   const int num_work = p.whole_tiles + (num_tiles - p.whole_tiles) * p.slices;
 
   if (warp >= kConsumerWarps) {
-    // ---------------------------------------------------------------- producer
+    // ---------------------------------------------------------------- producers
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kProducerRegs));
-    if (warp == kConsumerWarps && lane == 0) {
+    const int pw = warp - kConsumerWarps;
+    const bool issuer = pw == 0 && lane == 0;
+    bool working = gathers || issuer;
+    if (issuer && tmas) {
       prefetch_tensormap(&map_a);
       prefetch_tensormap(&map_b);
-      uint32_t it = 0;  // running K-tile counter across all work items: stage = it % kStages
-      for (int w = blockIdx.x; w < num_work; w += gridDim.x) {
-        int tile, z, pieces, tm, tn;
-        decode_work(w, num_tiles, p.whole_tiles, p.slices, tile, z, pieces);
-        tile_coords(tile, p.tiles_m, p.tiles_n, tm, tn);
-        const int kt_begin = pieces == 1 ? 0 : z * p.k_tiles_per_slice;
-        const int kt_end = (z == pieces - 1) ? k_tiles_total : min(k_tiles_total, kt_begin + p.k_tiles_per_slice);
-        for (int kt = kt_begin; kt < kt_end; ++kt, ++it) {
-          const int s = it % kStages;
-          const uint32_t round = it / kStages;
-          if (round > 0 && !mbar_wait(&empty_bar[s], (round - 1) & 1, p.status, kDeviceTimeoutEmpty)) return;
-          mbar_arrive_expect_tx(&full_bar[s], kStageBytes);
-          uint8_t* sa = smem + s * kStageBytes;
-          uint8_t* sb = sa + kOperandStageBytes;
-          if (kAK) tma_load_2d(sa, &map_a, &full_bar[s], kt * TK, tm * kTileM);
-          else     tma_load_2d(sa, &map_a, &full_bar[s], tm * kTileM, kt * TK);
-          if (kBK) tma_load_2d(sb, &map_b, &full_bar[s], kt * TK, tn * kTileN);
-          else     tma_load_2d(sb, &map_b, &full_bar[s], tn * kTileN, kt * TK);
+    }
+    uint32_t it = 0;  // running K-step counter across all work items: stage = it % kStages
+    for (int w = blockIdx.x; working && w < num_work; w += gridDim.x) {
+      int tile, z, pieces, tm, tn;
+      decode_work(p, w, num_tiles, tile, z, pieces);
+      tile_coords(tile, p.tiles_m, p.tiles_n, tm, tn);
+      const int m0 = tm * Tile::kM, n0 = tn * Tile::kN;
+      const int kt_begin = pieces == 1 ? 0 : z * p.k_tiles_per_slice;
+      const int kt_end = (z == pieces - 1) ? k_tiles_total : min(k_tiles_total, kt_begin + p.k_tiles_per_slice);
+      for (int kt = kt_begin; kt < kt_end; ++kt, ++it) {
+        const int s = it % kStages;
+        const uint32_t round = it / kStages;
+        if (round > 0 && !mbar_wait(&empty_bar[s], (round - 1) & 1, p.status, kDeviceTimeoutEmpty)) { working = false; break; }
+        uint8_t* sa = smem + s * Tile::kStageBytes;
+        uint8_t* sb = sa + Tile::kABytes;
+        const int k0 = kt * kStep;
+        if (issuer && tmas) {
+          mbar_arrive_expect_tx(&full_bar[s], (p.a_mode == kLoadTma ? Tile::kABytes : 0) + (p.b_mode == kLoadTma ? Tile::kBBytes : 0));
+#pragma unroll
+          for (int sub = 0; sub < kSub; ++sub) {
+            if (p.a_mode == kLoadTma) tma_load_2d(sa + sub * (Tile::kM * 128), &map_a, &full_bar[s], k0 + sub * TK, m0);
+            if (p.b_mode == kLoadTma) tma_load_2d(sb + sub * (Tile::kN * 128), &map_b, &full_bar[s], k0 + sub * TK, n0);
+          }
+        }
+        if (gathers) {
+          if (p.a_mode != kLoadTma)
+            gather_tile<T, Tile::kM, kSub>(smem_u32(sa), p.A, p.lda, p.a_mode, m0, p.M, k0, p.K, p.pad_a, pw, lane);
+          if (p.b_mode != kLoadTma)
+            gather_tile<T, Tile::kN, kSub>(smem_u32(sb), p.B, p.ldb, p.b_mode, n0, p.N, k0, p.K, p.pad_b, pw, lane);
+          if (k0 + kStep > p.K) {         // padding was written by ordinary stores: announce with an ordinary arrival
+            cp_async_wait_all();
+            mbar_arrive(&full_bar[s]);
+          } else {
+            cp_async_arrive_noinc(&full_bar[s]);
+          }
         }
       }
+    }
+    // every copy has landed before the thread goes away
+    if (gathers) cp_async_wait_all();
+    if (p.cluster) {                       // the two barriers of the consumers' fold are for all threads of the cluster
+      __syncwarp();
+      cluster_sync();
+      cluster_sync();
     }
     return;
   }
 
   // ------------------------------------------------------------------ consumers
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kConsumerRegs));
-  const int wm = warp / 4, wn = warp % 4;        // 2 x 4 warps
+  const int wk = warp / (WM * WN), wm = (warp / WN) % WM, wn = warp % WN;
   const int lr = lane / 4, lc = lane % 4;        // 8 x 4 lanes
   // Row i (0..7) of this lane inside the warp's 64 rows; column j (0..7) inside the warp's 32 columns.
   // Plus-times fp64 runs on the tensor cores (DMMA): acc[mb][2 nb + e] is then element e of the lane's
   // accumulator pair of the 8 x 8 block (mb, nb) of the warp tile; its row inside the block is lr, its column
-  // 2 lc + e.  Blocks fed from an MN-contiguous operand are interleaved in pairs (see the loaders below).
+  // 2 lc + e.
   constexpr bool kDmma = std::is_same<T, double>::value && RingT::kAdd == CUASR_OP_PLUS &&
                          RingT::kMul == CUASR_OP_MULTIPLIES;
-  auto row_of = [&](int i) {
-    if (kDmma) return kAK ? (8 * i + lr) : (16 * (i / 2) + 2 * lr + (i % 2));
-    return kAK ? (lr + 8 * i) : (EV * lr + (i % EV) + 8 * EV * (i / EV));
-  };
-  auto col_of = [&](int j) {
-    if (kDmma) return kBK ? (8 * (j / 2) + 2 * lc + (j % 2)) : (16 * (j / 4) + 4 * lc + 2 * (j % 2) + ((j / 2) % 2));
-    return kBK ? (lc + 4 * j) : (EV * lc + (j % EV) + 4 * EV * (j / EV));
-  };
+  auto row_of = [&](int i) { return 8 * i + lr; };
+  auto col_of = [&](int j) { return kDmma ? (8 * (j / 2) + 2 * lc + (j % 2)) : (lc + 4 * j); };
 
   // Byte offset of this lane's first operand vector inside a stage; every other vector of the lane is a
-  // compile-time constant away from it.
-  //   K-contiguous:  row * 128 + ((chunk ^ (row & 7)) * 16)        (TMA 128-byte swizzle)
-  //                  A rows are lr + 8 i  -> + i * 1024 bytes, row & 7 == lr for every i
-  //                  B rows are lc + 4 j  -> + j * 512 bytes,  row & 7 == lc + 4 (j & 1)
-  //   MN-contiguous: k * (128 * sizeof(T)) + first_row_of_group * sizeof(T); groups are 8 EV (A) or
-  //                  4 EV (B) rows apart -> + g * 128 / + g * 64 bytes
+  // compile-time constant away from it:  row * 128 + ((chunk ^ (row & 7)) * 16)
+  //   A rows are lr + 8 i  -> + i * 1024 bytes, row & 7 == lr for every i
+  //   B rows are lc + 4 j  -> + j * 512 bytes,  row & 7 == lc + 4 (j & 1)
+  // The warp's first chunk of a stage: column wk * kChunks / 8, chunk wk * kChunks % 8 (0 or 4) of it.
+  constexpr int kChunksPerColumn = 8;
+  const int first_chunk = WK == 1 ? 0 : (wk * kChunks) % kChunksPerColumn;
+  const int column = WK == 1 ? 0 : (wk * kChunks) / kChunksPerColumn;
   const uint32_t smem_base = smem_u32(smem);
-  const uint32_t a_base = kAK ? (wm * 64 + lr) * 128 : (wm * 64 + EV * lr) * (int)sizeof(T);
-  const uint32_t b_base = kBK ? (wn * 32 + lc) * 128 : (wn * 32 + EV * lc) * (int)sizeof(T);
+  const uint32_t a_base = column * (Tile::kM * 128) + (wm * 64 + lr) * 128;
+  const uint32_t b_base = Tile::kABytes + column * (Tile::kN * 128) + (wn * 32 + lc) * 128;
 
   T acc[8][8];
 
-  // Per-lane byte offsets of the eight 16-byte k chunks of a K-contiguous operand row, swizzle applied: computed
-  // once, so that inside the contraction an operand vector is addressed as (stage base + one of these + a constant).
+  // Per-lane byte offsets of the 16-byte k chunks of an operand row, swizzle applied: computed once, so that inside
+  // the contraction an operand vector is addressed as (stage base + one of these + a constant).
   // Only for 4-byte elements: with 8-byte elements the accumulators leave no registers for the table, and the
   // offsets are computed where they are used.
   constexpr bool kOffsetTable = sizeof(T) == 4;
@@ -224,83 +303,53 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   uint32_t a_off[kOffsetTable ? kUnroll : 1], b_off[kOffsetTable ? 8 : 1];
   if constexpr (kOffsetTable) {
 #pragma unroll
-    for (int c = 0; c < kUnroll; ++c) a_off[c] = a_base + (((c ^ lr) & 7) << 4);
+    for (int c = 0; c < kUnroll; ++c) a_off[c] = a_base + ((((c + first_chunk) ^ lr) & 7) << 4);
 #pragma unroll
-    for (int c = 0; c < 8; ++c) b_off[c] = b_base + (((c ^ lc) & 7) << 4);      // rows lc + 4 j with odd j use b_off[c ^ 4]
+    for (int c = 0; c < 8; ++c) b_off[c] = b_base + ((((c + first_chunk) ^ lc) & 7) << 4);   // rows lc + 4 j with odd j use b_off[c ^ 4]
   }
 
   uint32_t it = 0;
   for (int w = blockIdx.x; w < num_work; w += gridDim.x) {
     int tile, z, pieces, tm, tn;
-    decode_work(w, num_tiles, p.whole_tiles, p.slices, tile, z, pieces);
+    decode_work(p, w, num_tiles, tile, z, pieces);
     tile_coords(tile, p.tiles_m, p.tiles_n, tm, tn);
     const int kt_begin = pieces == 1 ? 0 : z * p.k_tiles_per_slice;
     const int kt_end = (z == pieces - 1) ? k_tiles_total : min(k_tiles_total, kt_begin + p.k_tiles_per_slice);
 
+    const T start = (wk == 0 && z == 0) ? p.add_identity : p.part_identity;
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = p.add_identity;
+      for (int j = 0; j < 8; ++j) acc[i][j] = start;
 
     for (int kt = kt_begin; kt < kt_end; ++kt, ++it) {
       const int s = it % kStages;
       mbar_wait_or_abandon(&full_bar[s], (it / kStages) & 1, p.status, kDeviceTimeoutFull, abandoned);
-      const uint32_t sa = smem_base + s * kStageBytes;
-      const uint32_t sb = sa + kOperandStageBytes;
+      const uint32_t st = smem_base + s * Tile::kStageBytes;
 
       // fragment loaders for one 16-byte k chunk: a[i][e] = A(row i, k = chunk * EV + e).  With the offset table the
       // chunk is given as (c, h): chunk = h * kUnroll + c with c a compile-time constant; without it h is 0.
       auto load_a = [&](T (&a)[8][EV], int c, int h = 0) {
-        const int chunk = kOffsetTable ? h * kUnroll + c : c;
-        if (kAK) {
-          uint32_t base;
-          if constexpr (kOffsetTable) base = sa + (a_off[c] ^ (h << 6));
-          else base = sa + a_base + (((chunk ^ lr) & 7) << 4);
+        uint32_t base;
+        if constexpr (kOffsetTable) base = st + (a_off[c] ^ (h << 6));
+        else base = st + a_base + ((((c + first_chunk) ^ lr) & 7) << 4);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) lds16(base + i * 1024, a[i]);
-        } else {
-          const uint32_t base = sa + a_base + chunk * (EV * kTileM * (int)sizeof(T));
-#pragma unroll
-          for (int e = 0; e < EV; ++e) {
-#pragma unroll
-            for (int g = 0; g < 8 / EV; ++g) {
-              T v[EV];
-              lds16(base + e * (kTileM * (int)sizeof(T)) + g * 128, v);
-#pragma unroll
-              for (int t = 0; t < EV; ++t) a[g * EV + t][e] = v[t];
-            }
-          }
-        }
+        for (int i = 0; i < 8; ++i) lds16(base + i * 1024, a[i]);
       };
       auto load_b = [&](T (&b)[8][EV], int c, int h = 0) {
-        const int chunk = kOffsetTable ? h * kUnroll + c : c;
-        if (kBK) {
-          uint32_t base0, base1;
-          if constexpr (kOffsetTable) {
-            base0 = sb + (b_off[c] ^ (h << 6));
-            base1 = sb + (b_off[c ^ 4] ^ (h << 6));
-          } else {
-            base0 = sb + b_base + (((chunk ^ lc) & 7) << 4);
-            base1 = sb + b_base + (((chunk ^ (lc + 4)) & 7) << 4);
-          }
-#pragma unroll
-          for (int j = 0; j < 8; ++j) lds16(((j & 1) ? base1 : base0) + j * 512, b[j]);
+        uint32_t base0, base1;
+        if constexpr (kOffsetTable) {
+          base0 = st + (b_off[c] ^ (h << 6));
+          base1 = st + (b_off[c ^ 4] ^ (h << 6));
         } else {
-          const uint32_t base = sb + b_base + chunk * (EV * kTileN * (int)sizeof(T));
-#pragma unroll
-          for (int e = 0; e < EV; ++e) {
-#pragma unroll
-            for (int g = 0; g < 8 / EV; ++g) {
-              T v[EV];
-              lds16(base + e * (kTileN * (int)sizeof(T)) + g * 64, v);
-#pragma unroll
-              for (int t = 0; t < EV; ++t) b[g * EV + t][e] = v[t];
-            }
-          }
+          base0 = st + b_base + ((((c + first_chunk) ^ lc) & 7) << 4);
+          base1 = st + b_base + ((((c + first_chunk) ^ (lc + 4)) & 7) << 4);
         }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) lds16(((j & 1) ? base1 : base0) + j * 512, b[j]);
       };
       auto compute = [&](const T (&a)[8][EV], const T (&b)[8][EV]) {
-        if constexpr (kAK && kBK && RingT::kPackedPairs) {
+        if constexpr (RingT::kPackedPairs) {
           // both fragments came from 16-byte loads along k: (k, k+1) are adjacent registers, so the pairs below
           // are register renames, not moves
 #pragma unroll
@@ -326,46 +375,20 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
       if constexpr (kDmma) {
         // Tensor-core path.  The fp64 mma takes, per lane, A(row lr [+8], k slot lc [+4]) and B(k slot lc [+4], column lr).
-        // The contraction index may be permuted freely as long as A and B agree: within a group of 8 k the
-        // slot lc of step s (s = 0, 1) stands for k = 2 lc + s, so a K-contiguous operand delivers both steps of
-        // a block with one 16-byte load.  An MN-contiguous operand delivers two adjacent rows with one 16-byte
-        // load; they feed the two blocks of an interleaved pair (block rows 2 lr and 2 lr + 1).
-        static_assert(!kDmma || TK == 16, "two groups of 8 k per stage");
+        // The contraction index may be permuted freely as long as A and B agree: within a group of 8 k (four
+        // chunks) the slot lc of step s (s = 0, 1) stands for k = 2 lc + s, so one 16-byte load delivers both steps
+        // of a block.
+        constexpr int kGroups = kChunks / 4;
+        static_assert(!kDmma || (kGroups >= 1 && kGroups <= 2), "one or two groups of 8 k per warp and stage");
         auto load_group = [&](double (&a)[8][2], double (&b)[4][2], int group) {
-          if (kAK) {
-            const uint32_t base = sa + (wm * 64 + lr) * 128 + ((((group * 4 + lc) ^ lr) & 7) << 4);
+          const uint32_t chunk = ((((group * 4 + first_chunk + lc) ^ lr) & 7) << 4);
+          const uint32_t abase = st + a_base + chunk;
 #pragma unroll
-            for (int mb = 0; mb < 8; ++mb) lds16(base + mb * 1024, a[mb]);
-          } else {
+          for (int mb = 0; mb < 8; ++mb) lds16(abase + mb * 1024, a[mb]);
+          // B rows (columns of the product) of this path are lr + 8 nb
+          const uint32_t bbase = st + Tile::kABytes + column * (Tile::kN * 128) + (wn * 32 + lr) * 128 + chunk;
 #pragma unroll
-            for (int sstep = 0; sstep < 2; ++sstep) {
-              const uint32_t base = sa + (group * 8 + 2 * lc + sstep) * (kTileM * 8) + (wm * 64 + 2 * lr) * 8;
-#pragma unroll
-              for (int pr = 0; pr < 4; ++pr) {
-                double v[2];
-                lds16(base + pr * 128, v);
-                a[2 * pr][sstep] = v[0];
-                a[2 * pr + 1][sstep] = v[1];
-              }
-            }
-          }
-          if (kBK) {
-            const uint32_t base = sb + (wn * 32 + lr) * 128 + ((((group * 4 + lc) ^ lr) & 7) << 4);
-#pragma unroll
-            for (int nb = 0; nb < 4; ++nb) lds16(base + nb * 1024, b[nb]);
-          } else {
-#pragma unroll
-            for (int sstep = 0; sstep < 2; ++sstep) {
-              const uint32_t base = sb + (group * 8 + 2 * lc + sstep) * (kTileN * 8) + (wn * 32 + 2 * lr) * 8;
-#pragma unroll
-              for (int pr = 0; pr < 2; ++pr) {
-                double v[2];
-                lds16(base + pr * 128, v);
-                b[2 * pr][sstep] = v[0];
-                b[2 * pr + 1][sstep] = v[1];
-              }
-            }
-          }
+          for (int nb = 0; nb < 4; ++nb) lds16(bbase + nb * 1024, b[nb]);
         };
         auto mma_group = [&](const double (&a)[8][2], const double (&b)[4][2]) {
           // m16n8k8: rows lr and lr + 8 of the instruction are the two 8-row blocks 2 h and 2 h + 1, k slots lc and
@@ -384,9 +407,9 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         };
         double a0[8][2], b0[4][2], a1[8][2], b1[4][2];
         load_group(a0, b0, 0);
-        load_group(a1, b1, 1);
+        if constexpr (kGroups == 2) load_group(a1, b1, 1);
         mma_group(a0, b0);
-        mma_group(a1, b1);
+        if constexpr (kGroups == 2) mma_group(a1, b1);
       } else if constexpr (sizeof(T) == 4) {
         // 4-byte elements: operand fragments are double-buffered in registers (64 + 4 x 32 registers)
         T a0[8][EV], b0[8][EV], a1[8][EV], b1[8][EV];
@@ -430,59 +453,155 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
 
     // ---------------------------------------------------------------- epilogue
-    const int m_base = tm * kTileM + wm * 64, n_base = tn * kTileN + wn * 32;
-    if (pieces > 1) {
-      // A piece of a split tile: park the raw accumulators in the tile's scratch block, in "fragment order"
-      // ([16 vectors][256 consumer threads][16 bytes], so that every access is a coalesced 16-byte vector and the
-      // thread that folds reads exactly the layout it would have written), then take a ticket.
-      constexpr int kVecPerThread = 64 / EV;
-      const int split = tile - p.whole_tiles;                     // index among the split tiles
-      T* block = p.partial + (long long)split * pieces * (kTileM * kTileN);
-      uint4* mine = reinterpret_cast<uint4*>(block + (long long)z * (kTileM * kTileN)) + threadIdx.x;
+    // 16 bytes of an output row: C is read, the epilogue applied and the vector stored to D and to every extra copy;
+    // element by element where the row is not 16-byte aligned or the vector crosses N.
+    auto store_vector = [&](T (&v)[EV], int m, int n) {
+      if (m >= p.M || n >= p.N) return;
 #pragma unroll
-      for (int v = 0; v < kVecPerThread; ++v) {
-        alignas(16) T tmp[EV];
+      for (int e = 0; e < EV; ++e) v[e] = RingT::mul(p.alpha, v[e]);
+      const long long off = (long long)m * p.ldd + n;
+      if (p.vector_epilogue) {
+        if (p.read_c) {
+          alignas(16) T c[EV];
+          *reinterpret_cast<uint4*>(c) = *reinterpret_cast<const uint4*>(p.C + (long long)m * p.ldc + n);
 #pragma unroll
-        for (int e = 0; e < EV; ++e) tmp[e] = acc[(v * EV + e) / 8][(v * EV + e) % 8];
-        mine[v * (kConsumerWarps * 32)] = *reinterpret_cast<const uint4*>(tmp);
-      }
-      __threadfence();
-      asm volatile("bar.sync 1, %0;" ::"n"(kConsumerWarps * 32) : "memory");
-      if (threadIdx.x == 0) *ticket_smem = atomicAdd(&p.tickets[split], 1u);
-      asm volatile("bar.sync 1, %0;" ::"n"(kConsumerWarps * 32) : "memory");
-      const bool last = (*ticket_smem == (unsigned)pieces - 1);
-      asm volatile("bar.sync 1, %0;" ::"n"(kConsumerWarps * 32) : "memory");
-      if (!last) continue;
-      // This CTA completed the tile: fold all pieces in slice order (a fixed order, whoever comes last), then
-      // fall through to the ordinary epilogue with the folded accumulators.
-      __threadfence();
-      if (threadIdx.x == 0) p.tickets[split] = 0;
+          for (int e = 0; e < EV; ++e) v[e] = RingT::add(v[e], RingT::mul(p.beta, c[e]));
+        }
+        *reinterpret_cast<uint4*>(p.D + off) = *reinterpret_cast<const uint4*>(v);
+        for (int x = 0; x < p.n_extra; ++x) *reinterpret_cast<uint4*>(p.extra_d[x] + off) = *reinterpret_cast<const uint4*>(v);
+      } else {
+        T c[EV];
+        if (p.read_c) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+          for (int e = 0; e < EV; ++e) c[e] = n + e < p.N ? p.C[(long long)m * p.ldc + n + e] : p.add_identity;
+        }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = p.add_identity;
-      for (int zz = 0; zz < pieces; ++zz) {
-        const uint4* theirs = reinterpret_cast<const uint4*>(block + (long long)zz * (kTileM * kTileN)) + threadIdx.x;
-        uint4 raw[kVecPerThread];
-#pragma unroll
-        for (int v = 0; v < kVecPerThread; ++v) raw[v] = __ldcg(theirs + v * (kConsumerWarps * 32));
-#pragma unroll
-        for (int v = 0; v < kVecPerThread; ++v) {
-          alignas(16) T tmp[EV];
-          *reinterpret_cast<uint4*>(tmp) = raw[v];
-#pragma unroll
-          for (int e = 0; e < EV; ++e) {
-            T& a = acc[(v * EV + e) / 8][(v * EV + e) % 8];
-            a = RingT::add(tmp[e], a);
+        for (int e = 0; e < EV; ++e) {
+          if (p.read_c) v[e] = RingT::add(v[e], RingT::mul(p.beta, c[e]));
+          if (n + e < p.N) {
+            p.D[off + e] = v[e];
+            for (int x = 0; x < p.n_extra; ++x) p.extra_d[x][off + e] = v[e];
           }
         }
       }
-    }
-    if (p.vector_epilogue) {
+    };
 
-      // Coalesced path: the warp's 64 x 32 block goes through its private staging area (rows of 32
-      // elements, the 16-byte column groups XOR-swizzled by row & 7), then every lane handles 16 bytes of
-      // a row: C is read, the epilogue applied and the vector stored to D and to every extra copy.
+    if constexpr (WK > 1) {
+      // Every warp leaves its block in shared memory ([wk][row][column], the 16-byte column groups XOR-swizzled by
+      // row & 7); then the 256 threads fold the WK partial values of an output vector in k-group order and store it,
+      // one vector per thread at a time.
+      constexpr int kRowGroups = Tile::kN / EV;                      // 16-byte groups per tile row
+      constexpr int kVectors = Tile::kM * kRowGroups;
+      T* fold = reinterpret_cast<T*>(epi_smem);
+      consumer_sync();                                               // the previous tile's fold has been read
+      {
+        T* mine = fold + wk * (Tile::kM * Tile::kN);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = wm * 64 + row_of(i);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const int c = wn * 32 + col_of(j);
+            mine[r * Tile::kN + (((c / EV) ^ (r & 7)) * EV) + (c % EV)] = acc[i][j];
+          }
+        }
+      }
+      consumer_sync();
+      auto folded = [&](int r, int g, T (&v)[EV]) {
+        const int at = r * Tile::kN + ((g ^ (r & 7)) * EV);
+        *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(fold + at);
+#pragma unroll
+        for (int q = 1; q < WK; ++q) {
+          alignas(16) T t[EV];
+          *reinterpret_cast<uint4*>(t) = *reinterpret_cast<const uint4*>(fold + q * (Tile::kM * Tile::kN) + at);
+#pragma unroll
+          for (int e = 0; e < EV; ++e) v[e] = RingT::add(t[e], v[e]);
+        }
+        return at;
+      };
+      if (!p.cluster) {
+#pragma unroll 4
+        for (int idx = threadIdx.x; idx < kVectors; idx += kConsumerThreads) {
+          const int r = idx / kRowGroups, g = idx % kRowGroups;
+          alignas(16) T v[EV];
+          folded(r, g, v);
+          store_vector(v, tm * Tile::kM + r, tn * Tile::kN + g * EV);
+        }
+      } else {
+        // fold this CTA's k groups into block 0, then the cluster's blocks, CTA by CTA in k order; CTA z of the cluster
+        // finishes the z-th part of the tile.  The hardware barriers also keep every CTA's memory in place until
+        // all of them have read it.
+#pragma unroll 4
+        for (int idx = threadIdx.x; idx < kVectors; idx += kConsumerThreads) {
+          const int r = idx / kRowGroups, g = idx % kRowGroups;
+          alignas(16) T v[EV];
+          const int at = folded(r, g, v);
+          *reinterpret_cast<uint4*>(fold + at) = *reinterpret_cast<const uint4*>(v);
+        }
+        cluster_sync();
+        const int share = kVectors / p.slices;
+        for (int idx = z * share + threadIdx.x; idx < (z + 1) * share; idx += kConsumerThreads) {
+          const int r = idx / kRowGroups, g = idx % kRowGroups;
+          const uint32_t at = smem_u32(fold + r * Tile::kN + ((g ^ (r & 7)) * EV));
+          alignas(16) T v[EV];
+          *reinterpret_cast<uint4*>(v) = lds16_cluster(at, 0);
+          for (int q = 1; q < p.slices; ++q) {
+            alignas(16) T t[EV];
+            *reinterpret_cast<uint4*>(t) = lds16_cluster(at, q);
+#pragma unroll
+            for (int e = 0; e < EV; ++e) v[e] = RingT::add(t[e], v[e]);
+          }
+          store_vector(v, tm * Tile::kM + r, tn * Tile::kN + g * EV);
+        }
+        cluster_sync();
+      }
+    } else {
+      const int m_base = tm * Tile::kM + wm * 64, n_base = tn * Tile::kN + wn * 32;
+      if (pieces > 1) {
+        // A piece of a split tile: park the raw accumulators in the tile's scratch block, in "fragment order"
+        // ([16 vectors][256 consumer threads][16 bytes], so that every access is a coalesced 16-byte vector and the
+        // thread that folds reads exactly the layout it would have written), then take a ticket.
+        constexpr int kVecPerThread = 64 / EV;
+        const int split = tile - p.whole_tiles;                     // index among the split tiles
+        T* block = p.partial + (long long)split * pieces * (kTileM * kTileN);
+        uint4* mine = reinterpret_cast<uint4*>(block + (long long)z * (kTileM * kTileN)) + threadIdx.x;
+#pragma unroll
+        for (int v = 0; v < kVecPerThread; ++v) {
+          alignas(16) T tmp[EV];
+#pragma unroll
+          for (int e = 0; e < EV; ++e) tmp[e] = acc[(v * EV + e) / 8][(v * EV + e) % 8];
+          mine[v * kConsumerThreads] = *reinterpret_cast<const uint4*>(tmp);
+        }
+        __threadfence();
+        consumer_sync();
+        if (threadIdx.x == 0) *ticket_smem = atomicAdd(&p.tickets[split], 1u);
+        consumer_sync();
+        const bool last = (*ticket_smem == (unsigned)pieces - 1);
+        consumer_sync();
+        if (!last) continue;
+        // This CTA completed the tile: fold all pieces in slice order (a fixed order, whoever comes last), then
+        // fall through to the ordinary epilogue with the folded accumulators.
+        __threadfence();
+        if (threadIdx.x == 0) p.tickets[split] = 0;
+        for (int zz = 0; zz < pieces; ++zz) {
+          const uint4* theirs = reinterpret_cast<const uint4*>(block + (long long)zz * (kTileM * kTileN)) + threadIdx.x;
+          uint4 raw[kVecPerThread];
+#pragma unroll
+          for (int v = 0; v < kVecPerThread; ++v) raw[v] = __ldcg(theirs + v * kConsumerThreads);
+#pragma unroll
+          for (int v = 0; v < kVecPerThread; ++v) {
+            alignas(16) T tmp[EV];
+            *reinterpret_cast<uint4*>(tmp) = raw[v];
+#pragma unroll
+            for (int e = 0; e < EV; ++e) {
+              T& a = acc[(v * EV + e) / 8][(v * EV + e) % 8];
+              a = zz == 0 ? tmp[e] : RingT::add(tmp[e], a);
+            }
+          }
+        }
+      }
+      // The warp's 64 x 32 block goes through its private staging area (rows of 32 elements, the 16-byte column
+      // groups XOR-swizzled by row & 7), then every lane handles 16 bytes of a row.
       constexpr int kRowsPerPass = kEpilogueWarpBytes / (32 * (int)sizeof(T));   // 64 (4-byte) or 32 (8-byte)
       constexpr int kGroups = 32 / EV;                                            // 16-byte groups per row
       T* stage = reinterpret_cast<T*>(epi_smem + warp * kEpilogueWarpBytes);
@@ -504,39 +623,10 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 #pragma unroll 4
         for (int idx = lane; idx < kRowsPerPass * kGroups; idx += 32) {
           const int r = idx / kGroups, g = idx % kGroups;
-          const int m = m_base + pass * kRowsPerPass + r;
-          const int n = n_base + g * EV;
-          if (m >= p.M || n >= p.N) continue;
           const int group = (g ^ (r & 7)) & (kGroups - 1);
           alignas(16) T v[EV];
           *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(stage + r * 32 + group * EV);
-#pragma unroll
-          for (int e = 0; e < EV; ++e) v[e] = RingT::mul(p.alpha, v[e]);
-          if (p.read_c) {
-            alignas(16) T c[EV];
-            *reinterpret_cast<uint4*>(c) = *reinterpret_cast<const uint4*>(p.C + (long long)m * p.ldc + n);
-#pragma unroll
-            for (int e = 0; e < EV; ++e) v[e] = RingT::add(v[e], RingT::mul(p.beta, c[e]));
-          }
-          const long long off = (long long)m * p.ldd + n;
-          *reinterpret_cast<uint4*>(p.D + off) = *reinterpret_cast<const uint4*>(v);
-          for (int x = 0; x < p.n_extra; ++x) *reinterpret_cast<uint4*>(p.extra_d[x] + off) = *reinterpret_cast<const uint4*>(v);
-        }
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int m = m_base + row_of(i);
-        if (m >= p.M) continue;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int n = n_base + col_of(j);
-          if (n >= p.N) continue;
-          T v = RingT::mul(p.alpha, acc[i][j]);
-          if (p.read_c) v = RingT::add(v, RingT::mul(p.beta, p.C[(long long)m * p.ldc + n]));
-          const long long off = (long long)m * p.ldd + n;
-          p.D[off] = v;
-          for (int x = 0; x < p.n_extra; ++x) p.extra_d[x][off] = v;
+          store_vector(v, m_base + pass * kRowsPerPass + r, n_base + g * EV);
         }
       }
     }
