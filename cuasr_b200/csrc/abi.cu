@@ -343,8 +343,9 @@ bool ring_pads_itself(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& ar
 RepackPlan repack_plan(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, const Normalised& p) {
   RepackPlan plan;
   const size_t es = desc.dtype == CUASR_F64 ? 8 : 4;
-  // not for tiny outputs, nor for storage lines that overlap
-  if (static_cast<long long>(p.m) * p.n < 64 * 64) return plan;
+  // not for storage lines that overlap, nor for small products: up to about 128^3 the copy's launch costs as much as
+  // the product itself, which gathers its operands just as well
+  if (static_cast<double>(p.m) * p.n * p.k < 128.0 * 128 * 128 || static_cast<long long>(p.m) * p.n < 64 * 64) return plan;
   if (p.lda < (p.a_kcontig ? p.k : p.m) || p.ldb < (p.b_kcontig ? p.k : p.n)) return plan;
   const int tk = kTileKBytes / static_cast<int>(es);
   if (p.k % tk != 0 && !ring_pads_itself(desc, args)) {
@@ -495,19 +496,19 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
       unsigned long long pad_a = 0, pad_b = 0;
       std::memcpy(&pad_a, &add_id, sizeof(T));
       std::memcpy(&pad_b, &mul_id, sizeof(T));
+      RepackRequest requests[2];
+      int count = 0;
       if (rp.a) {
-        if (launch_repack(p.a, p.lda, p.a_kcontig, p.m, p.k, k_copy, pad_a, cursor, ldt, sizeof(T), stream) != cudaSuccess)
-          return CUASR_STATUS_ERROR_INTERNAL;
-        g_launches.fetch_add(1);
+        requests[count++] = {p.a, p.lda, p.a_kcontig, p.m, p.k, k_copy, pad_a, cursor, ldt};
         p.a = cursor; p.lda = ldt; p.a_kcontig = true;
         cursor += repack_operand_bytes(p.m, k_copy, sizeof(T));
       }
       if (rp.b) {
-        if (launch_repack(p.b, p.ldb, p.b_kcontig, p.n, p.k, k_copy, pad_b, cursor, ldt, sizeof(T), stream) != cudaSuccess)
-          return CUASR_STATUS_ERROR_INTERNAL;
-        g_launches.fetch_add(1);
+        requests[count++] = {p.b, p.ldb, p.b_kcontig, p.n, p.k, k_copy, pad_b, cursor, ldt};
         p.b = cursor; p.ldb = ldt; p.b_kcontig = true;
       }
+      if (launch_repack(requests, count, sizeof(T), stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
+      g_launches.fetch_add(1);
       repacked = true;
       k_map = k_copy;
     }
@@ -819,8 +820,8 @@ int cuasr_b200_pack_k_contiguous(int32_t dtype, const void* src, int64_t ld_src,
   const size_t es = dtype == CUASR_F64 ? 8 : 4;
   if (reinterpret_cast<uintptr_t>(src) % es != 0 || reinterpret_cast<uintptr_t>(dst) % es != 0)
     return CUASR_STATUS_ERROR_MISALIGNED_OPERAND;
-  if (launch_repack(src, ld_src, src_k_contiguous != 0, rows, k, k, 0ull, dst, ld_dst, es,
-                    static_cast<cudaStream_t>(stream)) != cudaSuccess)
+  const RepackRequest request = {src, ld_src, src_k_contiguous != 0, rows, k, k, 0ull, dst, ld_dst};
+  if (launch_repack(&request, 1, es, static_cast<cudaStream_t>(stream)) != cudaSuccess)
     return CUASR_STATUS_ERROR_INTERNAL;
   g_launches.fetch_add(1);
   t_last_kernel = "pack";

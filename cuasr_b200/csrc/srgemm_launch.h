@@ -32,12 +32,17 @@ constexpr bool all_tiles_instantiated() {
   return bits || tropical || minmax;  // int32_t, uint32_t
 }
 
-// Copies a rows x K operand of 4- or 8-byte elements, K-contiguous or MN-contiguous with any leading dimension and
-// alignment, into K-contiguous storage with leading dimension ld_dst; columns K .. K_out - 1 of the copy are set to
-// the element whose bits are `pad_bits` (see repack_to_kcontig_kernel).
-cudaError_t launch_repack(const void* src, long long ld_src, bool src_kcontig, int rows, int K, int K_out,
-                          unsigned long long pad_bits, void* dst, long long ld_dst, size_t element_bytes,
-                          cudaStream_t stream);
+// Copies of up to two operands of 4- or 8-byte elements into K-contiguous storage, in one launch (see repack.cuh).
+struct RepackRequest {
+  const void* src;
+  long long ld_src;
+  bool kcontig;
+  int rows, K, K_out;
+  unsigned long long pad_bits;
+  void* dst;
+  long long ld_dst;
+};
+cudaError_t launch_repack(const RepackRequest* requests, int count, size_t element_bytes, cudaStream_t stream);
 
 // Kernel launch that lets the kernel's set-up overlap the end of the kernel before it in the stream (the kernel must
 // call grid_dependency_wait() before it touches global memory).
