@@ -17,10 +17,12 @@
 #include <vector>
 
 #include "../../include/cuasr_b200_apsp.h"
+#include "srgemm_launch.h"
 
 namespace {
 
-constexpr int kDefaultBlock = 1024;
+constexpr int kDefaultBlock = 1024;     // of the workspace layout, and of the solve with predecessors
+constexpr int kClosureBlock = 128;       // vertices fw_closure_kernel closes at once
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 size_t elem_size(int dtype) { return dtype == CUASR_F64 ? 8 : 4; }
@@ -220,20 +222,20 @@ int squaring(const cuasr_b200_apsp_args_t& a) {
   return CUASR_STATUS_SUCCESS;
 }
 
-int floyd_warshall(const cuasr_b200_apsp_args_t& a) {
-  if (a.parent != nullptr) return floyd_warshall_with_parents(a);
+// Scratch of one level of the blocked solve below: panels of n x b and b x n elements, and the closed b x b block.
+struct FwScratch {
+  void* p_col;            // leading dimension n
+  void* p_row;            // leading dimension b
+  void* star;             // leading dimension b
+};
+
+// The three-phase blocked scheme on the n x n matrix D, b vertices at a time; `close` closes a diagonal block into
+// scratch.star (leading dimension b).
+template <typename Close>
+int blocked_floyd_warshall(const cuasr_b200_apsp_args_t& a, char* D, long long ldd, int n, int b, const FwScratch& w,
+                           void* scratch, size_t scratch_bytes, Close&& close) {
   const cuasr_b200_desc_t desc = minplus_desc(a.dtype);
   const size_t es = elem_size(a.dtype);
-  const int n = a.n, b = block_of(a);
-  const FwLayout l = fw_layout(a);
-  char* ws = static_cast<char*>(a.workspace);
-  char* D = static_cast<char*>(a.D);
-  void* p_col = ws + l.p_col;             // n x bk, leading dimension n
-  void* p_row = ws + l.p_row;             // bk x n, leading dimension b
-  void* diag[2] = {ws + l.diag[0], ws + l.diag[1]};   // bk x bk, leading dimension b
-  void* scratch = a.workspace_bytes > l.srgemm ? ws + l.srgemm : nullptr;
-  const size_t scratch_bytes = a.workspace_bytes - l.srgemm;
-  cudaStream_t stream = static_cast<cudaStream_t>(a.stream);
   auto product = [&](int m, int nn, int k, const void* A, long long lda, const void* B, long long ldb, const void* C,
                      long long ldc, void* out, long long ldo) {
     cuasr_b200_args_t s = minplus_args(a.dtype, m, nn, k, A, lda, B, ldb, C, ldc, out, ldo, scratch, scratch_bytes,
@@ -242,28 +244,51 @@ int floyd_warshall(const cuasr_b200_apsp_args_t& a) {
   };
   for (int k0 = 0; k0 < n; k0 += b) {
     const int bk = std::min(b, n - k0);
-    // phase 1: paths inside the block, by squaring a private copy of the diagonal block
-    const char* dkk = D + (static_cast<size_t>(k0) + static_cast<size_t>(k0) * a.ldd) * es;
-    if (cudaMemcpy2DAsync(diag[0], b * es, dkk, a.ldd * es, bk * es, bk, cudaMemcpyDeviceToDevice, stream) != cudaSuccess)
-      return CUASR_STATUS_ERROR_INTERNAL;
-    int cur = 0;
-    for (int it = 0; it < std::max(1, ceil_log2(bk)); ++it, cur = 1 - cur) {
-      const int st = product(bk, bk, bk, diag[cur], b, diag[cur], b, diag[cur], b, diag[1 - cur], b);
-      if (st != CUASR_STATUS_SUCCESS) return st;
-    }
-    const void* star = diag[cur];
-    // phase 2: the column panel D[:, K] and the row panel D[K, :] through the closed block, out of place
-    const char* col = D + static_cast<size_t>(k0) * a.ldd * es;
-    const char* row = D + static_cast<size_t>(k0) * es;
-    int st = product(n, bk, bk, col, a.ldd, star, b, col, a.ldd, p_col, n);
+    // phase 1: paths inside the block
+    int st = close(D + (static_cast<size_t>(k0) + static_cast<size_t>(k0) * ldd) * es, ldd, bk);
     if (st != CUASR_STATUS_SUCCESS) return st;
-    st = product(bk, n, bk, star, b, row, a.ldd, row, a.ldd, p_row, b);
+    if (bk == n) return copy_block(a, D, ldd, w.star, b, n, n) == cudaSuccess ? CUASR_STATUS_SUCCESS : CUASR_STATUS_ERROR_INTERNAL;
+    // phase 2: the column panel D[:, K] and the row panel D[K, :] through the closed block, out of place
+    const char* col = D + static_cast<size_t>(k0) * ldd * es;
+    const char* row = D + static_cast<size_t>(k0) * es;
+    st = product(n, bk, bk, col, ldd, w.star, b, col, ldd, w.p_col, n);
+    if (st != CUASR_STATUS_SUCCESS) return st;
+    st = product(bk, n, bk, w.star, b, row, ldd, row, ldd, w.p_row, b);
     if (st != CUASR_STATUS_SUCCESS) return st;
     // phase 3: everything through the two panels, in place (the operands are copies)
-    st = product(n, n, bk, p_col, n, p_row, b, D, a.ldd, D, a.ldd);
+    st = product(n, n, bk, w.p_col, n, w.p_row, b, D, ldd, D, ldd);
     if (st != CUASR_STATUS_SUCCESS) return st;
   }
   return CUASR_STATUS_SUCCESS;
+}
+
+// Without predecessors.  The serial part of a step is the closure of its diagonal block, one CTA's work for 128 vertices
+// (15 us); larger blocks would only be closed by this same scheme one level down, and a step of 128 vertices already
+// runs at the rate of long products (n = 2000: 2.9 ms with blocks of 1024 closed by ten squarings each).  So 128 is
+// the block where the caller leaves it open; a block the caller asked for is closed in steps of 128.
+int floyd_warshall(const cuasr_b200_apsp_args_t& a) {
+  if (a.parent != nullptr) return floyd_warshall_with_parents(a);
+  const FwLayout l = fw_layout(a);
+  const int b = a.block > 0 ? block_of(a) : std::min(kClosureBlock, block_of(a));
+  char* ws = static_cast<char*>(a.workspace);
+  void* scratch = a.workspace_bytes > l.srgemm ? ws + l.srgemm : nullptr;
+  const size_t scratch_bytes = a.workspace_bytes - l.srgemm;
+  auto close_small = [&](const char* block, long long ld, void* star, long long ld_star, int n) {
+    const cudaError_t err = cuasr_b200::launch_fw_closure(block, ld, star, ld_star, n, elem_size(a.dtype), static_cast<cudaStream_t>(a.stream));
+    return err == cudaSuccess ? CUASR_STATUS_SUCCESS : CUASR_STATUS_ERROR_INTERNAL;
+  };
+  const FwScratch outer = {ws + l.p_col, ws + l.p_row, ws + l.diag[0]};
+  return blocked_floyd_warshall(a, static_cast<char*>(a.D), a.ldd, a.n, b, outer, scratch, scratch_bytes,
+                                [&](const char* block, long long ld, int bk) -> int {
+    if (bk <= kClosureBlock) return close_small(block, ld, outer.star, b, bk);
+    // in place on a copy; the panels of the outer level are free until phase 2
+    if (copy_block(a, outer.star, b, block, ld, bk, bk) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
+    const FwScratch inner = {outer.p_col, outer.p_row, ws + l.diag[1]};
+    return blocked_floyd_warshall(a, static_cast<char*>(outer.star), b, bk, kClosureBlock, inner, scratch, scratch_bytes,
+                                  [&](const char* sub, long long ld_sub, int n) -> int {
+      return close_small(sub, ld_sub, inner.star, kClosureBlock, n);
+    });
+  });
 }
 
 }  // namespace

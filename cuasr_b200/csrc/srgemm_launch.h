@@ -44,6 +44,10 @@ struct RepackRequest {
 };
 cudaError_t launch_repack(const RepackRequest* requests, int count, size_t element_bytes, cudaStream_t stream);
 
+// Closure of a diagonal block of n <= 128 vertices (see fw_closure.cuh); 4- or 8-byte floating-point elements.
+cudaError_t launch_fw_closure(const void* src, long long ld_src, void* dst, long long ld_dst, int n, size_t element_bytes,
+                              cudaStream_t stream);
+
 // Kernel launch that lets the kernel's set-up overlap the end of the kernel before it in the stream (the kernel must
 // call grid_dependency_wait() before it touches global memory).
 template <typename... Params, typename... Args>
