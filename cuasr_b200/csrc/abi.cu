@@ -15,8 +15,7 @@
 #include "../../include/cuasr_b200.h"
 #include "../../include/cuasr_b200_apsp.h"
 #include "srgemm_launch.h"
-#include "srgemm_path.cuh"
-#include "srgemm_path_tma.cuh"
+#include "srgemm_screened.cuh"
 
 namespace cuasr_b200 {
 namespace {
@@ -411,6 +410,31 @@ LaunchPlan plan_without_workspace(const cuasr_b200_desc_t& desc, int m, int n, i
   }
   return best;
 }
+// ---- the screened kernel (srgemm_screened.cuh) -------------------------------------------------------------------
+struct ScreenPlan {
+  int pieces = 1, blocks_per_piece = 0;
+  double cost = 1e300;
+};
+// Modelled clocks.  Measured per product and scheduler: 1.45 (fp32), 1.75 (fp64) with the tests, the conversions and
+// the usual number of recomputed elements; the first blocks of a tile, done exactly or with many recomputed elements,
+// cost about as much again as four exact blocks.
+ScreenPlan screen_plan(int dtype, int m, int n, int k, int sms, bool may_split) {
+  const int kb = dtype == CUASR_F64 ? 32 : 64;
+  const int blocks = (k + kb - 1) / kb;
+  const long long tiles = static_cast<long long>((m + kTileM - 1) / kTileM) * ((n + kTileN - 1) / kTileN);
+  const double per_block = 128.0 * kb * (dtype == CUASR_F64 ? 1.75 : 1.45);
+  const double first = 128.0 * kb * 4 * (dtype == CUASR_F64 ? 6.5 : 2.1);
+  ScreenPlan best;
+  for (int pieces = 1; pieces <= (may_split ? 128 : 1) && pieces <= blocks; ++pieces) {
+    const int per_piece = (blocks + pieces - 1) / pieces;
+    if ((pieces - 1) * per_piece >= blocks) continue;                     // every piece has work
+    const long long waves = (tiles * pieces + sms - 1) / sms;
+    const double cost = 4000 + (pieces > 1 ? 4000 : 0) + static_cast<double>(waves) * (per_block * per_piece + first + 2000);
+    if (cost < best.cost) { best.cost = cost; best.pieces = pieces; best.blocks_per_piece = per_piece; }
+  }
+  return best;
+}
+
 // Modelled clocks of a launch of large tiles whose pieces meet through tickets in a workspace.
 double ticket_plan_cost(const cuasr_b200_desc_t& desc, long long tiles, int whole_tiles, int pieces, int k, int sms) {
   const int tk = kTileKBytes / (desc.dtype == CUASR_F64 ? 8 : 4);
@@ -420,6 +444,45 @@ double ticket_plan_cost(const cuasr_b200_desc_t& desc, long long tiles, int whol
   const long long waves = whole_tiles / sms, tail = ((tiles - whole_tiles) * pieces + sms - 1) / sms;
   // the tickets are cleared by a memset in front of the launch; a piece is parked and read back by the last one
   return 3000 + 4000 + waves * (per_step * k_steps + 2000 * wide) + tail * (per_step * per_piece + 1000 * wide) + 1000 * wide * pieces;
+}
+
+// Launches the screened kernel on a normalised problem (row-major D).  parent != nullptr: with predecessors.
+template <typename T>
+int run_screened(bool maximize, const Normalised& p, T beta, T add_id, bool read_c, const ScreenPlan& plan,
+                 const ExtraOutputs& extra, int32_t* parent, long long ld_parent, int k_offset, DeviceState* dev,
+                 cudaStream_t stream) {
+  ScreenParams<T> sp = {};
+  sp.M = p.m; sp.N = p.n; sp.K = p.k;
+  sp.A = static_cast<const T*>(p.a); sp.lda = p.lda;
+  sp.B = static_cast<const T*>(p.b); sp.ldb = p.ldb;
+  auto mode = [&](const void* ptr, long long ld, bool kcontig) {
+    if (!kcontig) return kLoadGatherMN;
+    return encode_tiled_fn() != nullptr && ld >= p.k && tma_describable(ptr, ld, sizeof(T)) ? kLoadTma : kLoadGatherK;
+  };
+  sp.a_mode = mode(p.a, p.lda, p.a_kcontig);
+  sp.b_mode = mode(p.b, p.ldb, p.b_kcontig);
+  CUtensorMap map_a = {}, map_b = {};
+  if (sp.a_mode == kLoadTma && !make_operand_map<T>(&map_a, sp.A, p.lda, p.m, p.k, true, true)) sp.a_mode = kLoadGatherK;
+  if (sp.b_mode == kLoadTma && !make_operand_map<T>(&map_b, sp.B, p.ldb, p.n, p.k, true, true)) sp.b_mode = kLoadGatherK;
+  sp.C = static_cast<const T*>(p.c); sp.ldc = p.ldc;
+  sp.D = static_cast<T*>(p.d); sp.ldd = p.ldd;
+  sp.parent = parent; sp.ld_parent = ld_parent; sp.k_offset = k_offset;
+  sp.beta = beta; sp.add_identity = add_id; sp.read_c = read_c;
+  sp.n_extra = extra.count;
+  for (int x = 0; x < extra.count; ++x) sp.extra_d[x] = static_cast<T*>(extra.ptr[x]);
+  sp.tiles_m = (p.m + kTileM - 1) / kTileM; sp.tiles_n = (p.n + kTileN - 1) / kTileN;
+  sp.pieces = plan.pieces; sp.blocks_per_piece = plan.blocks_per_piece;
+  sp.status = dev->status;
+  const long long work = static_cast<long long>(sp.tiles_m) * sp.tiles_n * sp.pieces;
+  if (work > 2147483647LL) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
+  if (plan.pieces > 1) {
+    if (launch_screened_init<T>(maximize, sp, dev->sms, stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
+    g_launches.fetch_add(1);
+  }
+  const int grid = static_cast<int>(work < dev->sms ? work : dev->sms);
+  if (launch_screened<T>(maximize, map_a, map_b, sp, grid, stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
+  g_launches.fetch_add(1);
+  return CUASR_STATUS_SUCCESS;
 }
 
 template <typename T>
@@ -483,6 +546,24 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   // operands whose storage lines overlap (leading dimension below the contiguous extent) stay off the TMA path
   const bool dense = p.lda >= (p.a_kcontig ? p.k : p.m) && p.ldb >= (p.b_kcontig ? p.k : p.n);
   const bool small = static_cast<long long>(p.m) * p.n < 64 * 64;
+  if constexpr (std::is_same<T, double>::value) {
+    // the screened kernel, where it is modelled faster: no factor on the product (alpha is the identity of +), so that
+    // the running minimum can live in D
+    if ((desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM) && desc.mul_op == CUASR_OP_PLUS && alpha == T(0)) {
+      const ScreenPlan screened = screen_plan(desc.dtype, p.m, p.n, p.k, dev->sms, extra.count == 0);
+      if (screened.cost < plan.cost) {
+        const bool name = !small && dense && tma_describable(p.a, p.lda, sizeof(T)) && tma_describable(p.b, p.ldb, sizeof(T));
+        const bool copies = slices == 1 && args.workspace != nullptr && workspace_aligned && repack_plan(desc, args, p).bytes > 0 &&
+                            args.workspace_bytes >= align_up(balance_workspace_bytes(desc, args, dev->sms), 256) + repack_plan(desc, args, p).bytes;
+        if (!copies) {
+          const int st = run_screened<T>(desc.add_op == CUASR_OP_MAXIMUM, p, beta, add_id, read_c, screened, extra, nullptr, 0, 0, dev, stream);
+          if (st == CUASR_STATUS_SUCCESS)
+            t_last_kernel = !name ? (slices > 1 ? "generic_splitk" : "generic") : slices > 1 ? "tma_splitk" : balanced ? "tma_balanced" : "tma";
+          return st;
+        }
+      }
+    }
+  }
   // the rest of an optional workspace holds K-contiguous, aligned copies of operands (see RepackPlan)
   bool repacked = false;
   int k_map = p.k;              // K extent the tensor maps describe
@@ -755,60 +836,22 @@ int cuasr_b200_srgemm_path(const cuasr_b200_desc_t* desc, const cuasr_b200_args_
   if (parent == nullptr || reinterpret_cast<uintptr_t>(parent) % 4 != 0) return CUASR_STATUS_ERROR_MISALIGNED_OPERAND;
   const bool row_c = desc->layout_c == CUASR_ROW_MAJOR;
   if (ld_parent < (row_c ? args->n : args->m)) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
-  auto fill = [&](auto* pp) {
-    pp->M = args->m; pp->N = args->n; pp->K = args->k;
-    const bool row_a = desc->layout_a == CUASR_ROW_MAJOR, row_b = desc->layout_b == CUASR_ROW_MAJOR;
-    pp->a_row = row_a ? args->lda : 1; pp->a_col = row_a ? 1 : args->lda;
-    pp->b_row = row_b ? args->ldb : 1; pp->b_col = row_b ? 1 : args->ldb;
-    pp->d_row = row_c ? args->ldd : 1; pp->d_col = row_c ? 1 : args->ldd;
-    pp->p_row = row_c ? ld_parent : 1; pp->p_col = row_c ? 1 : ld_parent;
-    pp->parent = parent; pp->k_offset = k_offset;
-  };
+  DeviceState* dev = nullptr;
+  if (!device_state(&dev)) return CUASR_STATUS_ERROR_INTERNAL;
+  // the normalised problem has a row-major D: element (m, n) at D[m * ldd + n], whatever the caller's layout
+  const Normalised p = normalise(*desc, *args);
   cudaStream_t stream = static_cast<cudaStream_t>(args->stream);
-  cudaError_t err;
-  // fp32 operands TMA can describe take the pipelined kernel; everything else the any-layout one
-  if (desc->dtype == CUASR_F32 && static_cast<long long>(args->m) * args->n >= 64 * 64 && encode_tiled_fn() != nullptr) {
-    const Normalised p = normalise(*desc, *args);
-    const bool dense = p.lda >= (p.a_kcontig ? p.k : p.m) && p.ldb >= (p.b_kcontig ? p.k : p.n);
-    DeviceState* dev = nullptr;
-    CUtensorMap map_a, map_b;
-    if (dense && tma_describable(p.a, p.lda, 4) && tma_describable(p.b, p.ldb, 4) && device_state(&dev) &&
-        make_operand_map<float>(&map_a, static_cast<const float*>(p.a), p.lda, p.m, p.k, p.a_kcontig, true) &&
-        make_operand_map<float>(&map_b, static_cast<const float*>(p.b), p.ldb, p.n, p.k, p.b_kcontig, true)) {
-      PathTmaParams tp;
-      tp.M = p.m; tp.N = p.n; tp.K = p.k;
-      // the normalised problem has a row-major D: element (m, n) at D[m * ldd + n], whatever the caller's layout
-      tp.dist = static_cast<float*>(args->D); tp.d_row = args->ldd; tp.d_col = 1;
-      tp.parent = parent; tp.p_row = ld_parent; tp.p_col = 1;
-      tp.k_offset = k_offset;
-      tp.tiles_m = (p.m + kTileM - 1) / kTileM; tp.tiles_n = (p.n + kTileN - 1) / kTileN;
-      tp.status = dev->status;
-      const long long tiles = static_cast<long long>(tp.tiles_m) * tp.tiles_n;
-      const int grid = static_cast<int>(tiles < dev->sms ? tiles : dev->sms);
-      if (launch_path_tma(maximize, p.a_kcontig, p.b_kcontig, map_a, map_b, tp, grid, stream) != cudaSuccess)
-        return CUASR_STATUS_ERROR_INTERNAL;
-      g_launches.fetch_add(1);
-      t_last_kernel = "path_tma";
-      return CUASR_STATUS_SUCCESS;
-    }
-  }
-  if (desc->dtype == CUASR_F32) {
-    PathParams<float> pp;
-    fill(&pp);
-    pp.A = static_cast<const float*>(args->A); pp.B = static_cast<const float*>(args->B);
-    pp.dist = static_cast<float*>(args->D);
-    err = launch_path<float>(pp, maximize, stream);
-  } else {
-    PathParams<double> pp;
-    fill(&pp);
-    pp.A = static_cast<const double*>(args->A); pp.B = static_cast<const double*>(args->B);
-    pp.dist = static_cast<double*>(args->D);
-    err = launch_path<double>(pp, maximize, stream);
-  }
-  if (err != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
-  g_launches.fetch_add(1);
-  t_last_kernel = "path";
-  return CUASR_STATUS_SUCCESS;
+  const bool f32 = desc->dtype == CUASR_F32;
+  const size_t es = f32 ? 4 : 8;
+  const bool dense = p.lda >= (p.a_kcontig ? p.k : p.m) && p.ldb >= (p.b_kcontig ? p.k : p.n);
+  const bool pipelined = f32 && dense && static_cast<long long>(args->m) * args->n >= 64 * 64 &&
+                         tma_describable(p.a, p.lda, es) && tma_describable(p.b, p.ldb, es);
+  const ScreenPlan plan = screen_plan(desc->dtype, p.m, p.n, p.k, dev->sms, false);
+  const ExtraOutputs none;
+  const int done = f32 ? run_screened<float>(maximize, p, 0.0f, 0.0f, false, plan, none, parent, ld_parent, k_offset, dev, stream)
+                       : run_screened<double>(maximize, p, 0.0, 0.0, false, plan, none, parent, ld_parent, k_offset, dev, stream);
+  if (done == CUASR_STATUS_SUCCESS) t_last_kernel = pipelined ? "path_tma" : "path";
+  return done;
 }
 
 int cuasr_b200_pack_k_contiguous(int32_t dtype, const void* src, int64_t ld_src, int32_t src_k_contiguous, int32_t rows,

@@ -34,9 +34,11 @@ __device__ __forceinline__ void sts(uint32_t addr, uint32_t v) { asm volatile("s
 __device__ __forceinline__ void sts(uint32_t addr, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory"); }
 
 // Stages rows [r0, r0 + kRows) x k [k0, k0 + kSub * 128 bytes) of an operand whose element (r, k) is base[r * ld + k]
-// (kLoadGatherK) or base[r + k * ld] (kLoadGatherMN).  Rows at or beyond `rows` are left alone (their results are
+// (kLoadGatherK) or base[r + k * ld] (kLoadGatherMN).  Rows at or beyond `rows` repeat the last row (their results are
 // never stored); k at or beyond K is set to `pad` by plain stores, so a stage that reaches beyond K must not be announced
 // with cp_async_arrive_noinc alone.  Called by all 128 producer threads; `pw` is the producer warp (0..3).
+// Inside the matrix a copy is one cp.async and at most one addition: with the bounds tested element by element a
+// 1024 x 768 x 1536 product of odd storage lines took 186 us, against 97 us with TMA.
 template <typename T, int kRows, int kSub>
 __device__ __forceinline__ void gather_tile(uint32_t dst, const T* __restrict__ base, long long ld, int mode, int r0,
                                             int rows, int k0, int K, T pad, int pw, int lane) {
@@ -44,11 +46,11 @@ __device__ __forceinline__ void gather_tile(uint32_t dst, const T* __restrict__ 
   constexpr int ES = (int)sizeof(T);
   // opaque: the lane's offsets are computed here, per stage, instead of being held in the producers' few registers
   asm volatile("" : "+r"(lane), "+r"(pw));
+  const int last = rows - 1 - r0;                  // last row, relative to the tile's first
   if (mode == kLoadGatherMN) {
     // A warp instruction covers 8 rows x 4 k: four 32-byte (64-byte for 8-byte elements) pieces of global memory, and
     // (row & 7) spreads the 8 rows over the 8 swizzled chunks, so the shared-memory writes do not conflict.
     const int r8 = lane & 7, kq = lane >> 3;
-    const int left = rows - r0 - r8;               // row block i is inside if 8 i < left
 #pragma unroll 1
     for (int sub = 0; sub < kSub; ++sub) {
 #pragma unroll 1
@@ -56,38 +58,47 @@ __device__ __forceinline__ void gather_tile(uint32_t dst, const T* __restrict__ 
         const int kk = step * 16 + pw * 4 + kq;
         const int k = k0 + sub * TK + kk;
         const uint32_t d = dst + sub * (kRows * 128) + r8 * 128 + ((((kk * ES) >> 4) ^ r8) << 4) + ((kk * ES) & 15);
-        if (k < K) {
-          const T* s = base + (long long)k * ld + (r0 + r8);
-          if (rows - r0 >= kRows) {
+        const T* line = base + (long long)k * ld + r0;
+        if (k0 + sub * TK + TK <= K && last >= kRows - 1) {          // uniform over the warp
+          const T* s = line + r8;
 #pragma unroll
-            for (int i = 0; i < kRows / 8; ++i) cp_async<ES>(d + i * 1024, s + 8 * i);
-          } else {
-#pragma unroll
-            for (int i = 0; i < kRows / 8; ++i)
-              if (8 * i < left) cp_async<ES>(d + i * 1024, s + 8 * i);
-          }
+          for (int i = 0; i < kRows / 8; ++i) cp_async<ES>(d + i * 1024, s + 8 * i);
+        } else if (k < K) {
+#pragma unroll 1
+          for (int i = 0; i < kRows / 8; ++i) cp_async<ES>(d + i * 1024, line + min(r8 + 8 * i, last));
         } else {
-#pragma unroll
+#pragma unroll 1
           for (int i = 0; i < kRows / 8; ++i) sts(d + i * 1024, pad);
         }
       }
     }
   } else {
     constexpr int kRowsPerInstr = ES == 8 ? 2 : 1;
+    constexpr int kRowStep = 4 * kRowsPerInstr;
     const int kk = ES == 8 ? (lane & 15) : lane;
     const int rr = ES == 8 ? pw * 2 + (lane >> 4) : pw;
+    // swizzled chunk of row rr + kRowStep i: the row's low three bits alternate for 4-byte elements
+    const uint32_t c0 = (((kk * ES) >> 4) ^ (rr & 7)) << 4;
+    const uint32_t c1 = ES == 8 ? c0 : c0 ^ 64;
 #pragma unroll 1
     for (int sub = 0; sub < kSub; ++sub) {
       const int k = k0 + sub * TK + kk;
-      const bool in_k = k < K;
-      const T* s = base + (long long)(r0 + rr) * ld + k;
+      const uint32_t d = dst + sub * (kRows * 128) + rr * 128 + ((kk * ES) & 15);
+      const T* column = base + (long long)r0 * ld + k;
+      if (k0 + sub * TK + TK <= K && last >= kRows - 1) {            // uniform over the warp
+        const T* s = column + (long long)rr * ld;
 #pragma unroll 4
-      for (int i = 0; i < kRows / (4 * kRowsPerInstr); ++i) {
-        const int row = rr + 4 * kRowsPerInstr * i;
-        const uint32_t d = dst + sub * (kRows * 128) + row * 128 + ((((kk * ES) >> 4) ^ (row & 7)) << 4) + ((kk * ES) & 15);
-        if (!in_k) sts(d, pad);
-        else if (r0 + row < rows) cp_async<ES>(d, s);
-        s += 4 * kRowsPerInstr * ld;
+        for (int i = 0; i < kRows / kRowStep; ++i) {
+          cp_async<ES>(d + i * (kRowStep * 128) + ((i & 1) ? c1 : c0), s);
+          s += (long long)kRowStep * ld;
+        }
+      } else if (k < K) {
+#pragma unroll 1
+        for (int i = 0; i < kRows / kRowStep; ++i)
+          cp_async<ES>(d + i * (kRowStep * 128) + ((i & 1) ? c1 : c0), column + (long long)min(rr + kRowStep * i, last) * ld);
+      } else {
+#pragma unroll 1
+        for (int i = 0; i < kRows / kRowStep; ++i) sts(d + i * (kRowStep * 128) + ((i & 1) ? c1 : c0), pad);
       }
     }
   }
