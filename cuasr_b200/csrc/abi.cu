@@ -3,6 +3,7 @@
 // Host-side counterpart of the reference's device::Srgemm (include/cuasr/gemm/device/srgemm.h:85-357 and
 // its column-major specialisation :398-567) and device::SrgemmSplitKParallel
 // (include/cuasr/gemm/device/srgemm_splitk_parallel.h:101-378, :424-607).
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -15,6 +16,7 @@
 #include "../../include/cuasr_b200.h"
 #include "../../include/cuasr_b200_apsp.h"
 #include "srgemm_launch.h"
+#include "srgemm_path.cuh"
 #include "srgemm_screened.cuh"
 
 namespace cuasr_b200 {
@@ -349,7 +351,7 @@ RepackPlan repack_plan(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& a
   const int tk = kTileKBytes / static_cast<int>(es);
   if (p.k % tk != 0 && !ring_pads_itself(desc, args)) {
     plan.a = plan.b = true;
-    plan.k_padded = (p.k + 2 * tk - 1) / (2 * tk) * (2 * tk);     // the longest K step of any tile
+    plan.k_padded = (p.k + 2 * tk - 1) / (2 * tk) * (2 * tk);     // the longest K step of a tile (rings without padding)
   } else {
     plan.a = !tma_describable(p.a, p.lda, es);
     plan.b = !tma_describable(p.b, p.ldb, es);
@@ -378,22 +380,30 @@ struct LaunchPlan {
   int whole_tiles = 0, pieces = 1; // ticket pieces (cluster == 1)
   double cost = 1e300;             // modelled clocks
 };
-constexpr int kTileRows[3] = {LargeTile::kM, MediumTile::kM, SmallTile::kM};
-constexpr int kTileCols[3] = {LargeTile::kN, MediumTile::kN, SmallTile::kN};
-constexpr int kTileWk[3] = {LargeTile::WK, MediumTile::WK, SmallTile::WK};
-constexpr int kTileSub[3] = {LargeTile::kSub, MediumTile::kSub, SmallTile::kSub};
+constexpr int kTileRows[4] = {LargeTile::kM, MediumTile::kM, SmallTile::kM, TinyTile::kM};
+constexpr int kTileCols[4] = {LargeTile::kN, MediumTile::kN, SmallTile::kN, TinyTile::kN};
+constexpr int kTileWk[4] = {LargeTile::WK, MediumTile::WK, SmallTile::WK, TinyTile::WK};
+// k columns per stage; fp64 sums use the deep form of the tiny tile
+int tile_sub(int tile, const cuasr_b200_desc_t& desc) {
+  constexpr int sub[4] = {LargeTile::kSub, MediumTile::kSub, SmallTile::kSub, TinyTile::kSub};
+  const bool dmma = desc.dtype == CUASR_F64 && desc.add_op == CUASR_OP_PLUS && desc.mul_op == CUASR_OP_MULTIPLIES;
+  return tile == kTinyTile && dmma ? TinyTileDeep::kSub : sub[tile];
+}
 
 // The fastest of the launches that need no workspace, by a model in clocks: start of the launch and first tile of
 // operands 3000, then per wave of CTAs the contraction (above) and the tile's end (2000 for the large tile, 1500 for the
 // fold of the small ones, twice that for 8-byte elements), 2500 for the exchange inside a cluster.  Clusters of four
 // and eight do not fill every SM (a cluster lives in one GPC): 144 and 128 of the 148.
-LaunchPlan plan_without_workspace(const cuasr_b200_desc_t& desc, int m, int n, int k, int sms, bool all_tiles) {
+// A gathered element costs 0.17 clocks on the small tiles (2048^3 with both operands transposed on 64 x 64 tiles takes
+// 694 us against 519 with TMA) and 0.07 on the large one (4096^3: 4.30 ms against 3.97).
+LaunchPlan plan_without_workspace(const cuasr_b200_desc_t& desc, int m, int n, int k, int sms, bool all_tiles, bool gather_a,
+                                  bool gather_b) {
   const int tk = kTileKBytes / (desc.dtype == CUASR_F64 ? 8 : 4);
   const double per_k = clocks_per_k(desc), wide = desc.dtype == CUASR_F64 ? 2.0 : 1.0;
   LaunchPlan best;
-  for (int tile = all_tiles ? kLargeTile : kSmallTile; tile <= kSmallTile; ++tile) {
+  for (int tile = all_tiles ? kLargeTile : kSmallTile; tile <= kTinyTile; ++tile) {
     const long long tiles = static_cast<long long>((m + kTileRows[tile] - 1) / kTileRows[tile]) * ((n + kTileCols[tile] - 1) / kTileCols[tile]);
-    const int step = tk * kTileSub[tile];
+    const int step = tk * tile_sub(tile, desc);
     const int k_steps = (k + step - 1) / step;
     for (int z = 1; z <= (tile == kLargeTile ? 1 : 8); z *= 2) {
       const int per_piece = (k_steps + z - 1) / z;
@@ -401,7 +411,9 @@ LaunchPlan plan_without_workspace(const cuasr_b200_desc_t& desc, int m, int n, i
       const long long room = z <= 2 ? sms : z == 4 ? sms * 36LL / 37 : sms * 32LL / 37;
       const long long waves = (tiles * z + room - 1) / room;
       const double end = (tile == kLargeTile ? 2000 : 1500) * wide + (z > 1 ? 2500 : 0);
-      const double cost = 3000 + static_cast<double>(waves) * (per_k * step * per_piece / kTileWk[tile] + end);
+      const double gathered = (tile == kLargeTile ? 0.07 : 0.17) * step * ((gather_a ? kTileRows[tile] : 0) + (gather_b ? kTileCols[tile] : 0));
+      const double per_stage = per_k * step / kTileWk[tile] + gathered;
+      const double cost = 3000 + static_cast<double>(waves) * (per_stage * per_piece + end);
       if (cost < best.cost) {
         best.tile = tile; best.cluster = z; best.cost = cost;
         best.whole_tiles = z > 1 ? 0 : static_cast<int>(tiles); best.pieces = z;
@@ -415,15 +427,15 @@ struct ScreenPlan {
   int pieces = 1, blocks_per_piece = 0;
   double cost = 1e300;
 };
-// Modelled clocks.  Measured per product and scheduler: 1.45 (fp32), 1.75 (fp64) with the tests, the conversions and
-// the usual number of recomputed elements; the first blocks of a tile, done exactly or with many recomputed elements,
-// cost about as much again as four exact blocks.
-ScreenPlan screen_plan(int dtype, int m, int n, int k, int sms, bool may_split) {
-  const int kb = dtype == CUASR_F64 ? 32 : 64;
+// Modelled clocks.  Measured per product and scheduler: 3.0 with the tests, the conversions and the usual number of
+// recomputed elements; the first blocks of a tile, done exactly or with many recomputed elements, cost about as much
+// again as four exact blocks.
+ScreenPlan screen_plan(int m, int n, int k, int sms, bool may_split) {
+  const int kb = 32;
   const int blocks = (k + kb - 1) / kb;
   const long long tiles = static_cast<long long>((m + kTileM - 1) / kTileM) * ((n + kTileN - 1) / kTileN);
-  const double per_block = 128.0 * kb * (dtype == CUASR_F64 ? 1.75 : 1.45);
-  const double first = 128.0 * kb * 4 * (dtype == CUASR_F64 ? 6.5 : 2.1);
+  const double per_block = 128.0 * kb * 3.0;
+  const double first = 128.0 * kb * 4 * 6.5;
   ScreenPlan best;
   for (int pieces = 1; pieces <= (may_split ? 128 : 1) && pieces <= blocks; ++pieces) {
     const int per_piece = (blocks + pieces - 1) / pieces;
@@ -446,27 +458,29 @@ double ticket_plan_cost(const cuasr_b200_desc_t& desc, long long tiles, int whol
   return 3000 + 4000 + waves * (per_step * k_steps + 2000 * wide) + tail * (per_step * per_piece + 1000 * wide) + 1000 * wide * pieces;
 }
 
-// Launches the screened kernel on a normalised problem (row-major D).  parent != nullptr: with predecessors.
+// How the kernels that can fill in NaN or an infinity bring in one operand, and its tensor map if that is TMA.
+template <typename T>
+int operand_mode(CUtensorMap* map, const void* ptr, long long ld, bool kcontig, int rows, int k, int box_rows) {
+  if (!kcontig) return kLoadGatherMN;
+  if (encode_tiled_fn() != nullptr && ld >= k && tma_describable(ptr, ld, sizeof(T)) &&
+      make_operand_map<T>(map, static_cast<const T*>(ptr), ld, rows, k, true, true, box_rows))
+    return kLoadTma;
+  return kLoadGatherK;
+}
+
+// Launches the screened kernel on a normalised problem (row-major D).
 template <typename T>
 int run_screened(bool maximize, const Normalised& p, T beta, T add_id, bool read_c, const ScreenPlan& plan,
-                 const ExtraOutputs& extra, int32_t* parent, long long ld_parent, int k_offset, DeviceState* dev,
-                 cudaStream_t stream) {
+                 const ExtraOutputs& extra, DeviceState* dev, cudaStream_t stream) {
   ScreenParams<T> sp = {};
   sp.M = p.m; sp.N = p.n; sp.K = p.k;
   sp.A = static_cast<const T*>(p.a); sp.lda = p.lda;
   sp.B = static_cast<const T*>(p.b); sp.ldb = p.ldb;
-  auto mode = [&](const void* ptr, long long ld, bool kcontig) {
-    if (!kcontig) return kLoadGatherMN;
-    return encode_tiled_fn() != nullptr && ld >= p.k && tma_describable(ptr, ld, sizeof(T)) ? kLoadTma : kLoadGatherK;
-  };
-  sp.a_mode = mode(p.a, p.lda, p.a_kcontig);
-  sp.b_mode = mode(p.b, p.ldb, p.b_kcontig);
   CUtensorMap map_a = {}, map_b = {};
-  if (sp.a_mode == kLoadTma && !make_operand_map<T>(&map_a, sp.A, p.lda, p.m, p.k, true, true)) sp.a_mode = kLoadGatherK;
-  if (sp.b_mode == kLoadTma && !make_operand_map<T>(&map_b, sp.B, p.ldb, p.n, p.k, true, true)) sp.b_mode = kLoadGatherK;
+  sp.a_mode = operand_mode<T>(&map_a, p.a, p.lda, p.a_kcontig, p.m, p.k, kTileM);
+  sp.b_mode = operand_mode<T>(&map_b, p.b, p.ldb, p.b_kcontig, p.n, p.k, kTileN);
   sp.C = static_cast<const T*>(p.c); sp.ldc = p.ldc;
   sp.D = static_cast<T*>(p.d); sp.ldd = p.ldd;
-  sp.parent = parent; sp.ld_parent = ld_parent; sp.k_offset = k_offset;
   sp.beta = beta; sp.add_identity = add_id; sp.read_c = read_c;
   sp.n_extra = extra.count;
   for (int x = 0; x < extra.count; ++x) sp.extra_d[x] = static_cast<T*>(extra.ptr[x]);
@@ -481,6 +495,57 @@ int run_screened(bool maximize, const Normalised& p, T beta, T add_id, bool read
   }
   const int grid = static_cast<int>(work < dev->sms ? work : dev->sms);
   if (launch_screened<T>(maximize, map_a, map_b, sp, grid, stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
+  g_launches.fetch_add(1);
+  return CUASR_STATUS_SUCCESS;
+}
+
+// ---- the path-tracking kernel (srgemm_path.cuh) -------------------------------------------------------------------
+// Its launch by the model of plan_without_workspace, with the work that comes on top of the contraction: per stage a
+// test of 64 elements (256 clocks per warp), and the look-ups, about 64 / t + 1.5 per lane after stage t of cold data, of
+// 60 clocks per four chunks of the stage that a warp works on.
+template <typename T>
+int run_path(bool maximize, const Normalised& p, int32_t* parent, long long ld_parent, int k_offset, DeviceState* dev,
+             cudaStream_t stream) {
+  constexpr int TK = kTileKBytes / sizeof(T);
+  const double per_k = 2 * 64 * (sizeof(T) == 8 ? 6.5 : 2.1);
+  double best = 1e300;
+  int tile = kLargeTile, cluster = 1;
+  for (int candidate : {kLargeTile, kSmallTile}) {
+    if (candidate == kSmallTile && sizeof(T) == 8) continue;                  // its partial values would not fit beside a pipeline
+    const bool large = candidate == kLargeTile;
+    const long long tiles = static_cast<long long>((p.m + kTileRows[candidate] - 1) / kTileRows[candidate]) * ((p.n + kTileCols[candidate] - 1) / kTileCols[candidate]);
+    const int step = large ? TK : 2 * TK;
+    const int k_steps = (p.k + step - 1) / step;
+    for (int z = 1; z <= (large ? 1 : 8); z *= 2) {
+      const int per_piece = (k_steps + z - 1) / z;
+      if ((z - 1) * per_piece >= k_steps) break;
+      const long long room = z <= 2 ? dev->sms : z == 4 ? dev->sms * 36LL / 37 : dev->sms * 32LL / 37;
+      const long long waves = (tiles * z + room - 1) / room;
+      const double per_stage = per_k * step / kTileWk[candidate] + 2 * 256 + 2 * 1.5 * 60 * (large ? 2 : 1);
+      const double lookups = 2 * 64 * 60 * (large ? 2 : 1) * std::log(1.0 + per_piece);
+      const double cost = 3000 + static_cast<double>(waves) * (per_stage * per_piece + lookups + 3000 + (z > 1 ? 3000 : 0));
+      if (cost < best) { best = cost; tile = candidate; cluster = z; }
+    }
+  }
+  PathParams<T> pp = {};
+  pp.M = p.m; pp.N = p.n; pp.K = p.k;
+  pp.A = static_cast<const T*>(p.a); pp.lda = p.lda;
+  pp.B = static_cast<const T*>(p.b); pp.ldb = p.ldb;
+  CUtensorMap map_a = {}, map_b = {};
+  pp.a_mode = operand_mode<T>(&map_a, p.a, p.lda, p.a_kcontig, p.m, p.k, kTileRows[tile]);
+  pp.b_mode = operand_mode<T>(&map_b, p.b, p.ldb, p.b_kcontig, p.n, p.k, kTileCols[tile]);
+  pp.pad = static_cast<T>(NAN);
+  pp.dist = static_cast<T*>(p.d); pp.ldd = p.ldd;
+  pp.parent = parent; pp.ld_parent = ld_parent; pp.k_offset = k_offset;
+  pp.tiles_m = (p.m + kTileRows[tile] - 1) / kTileRows[tile]; pp.tiles_n = (p.n + kTileCols[tile] - 1) / kTileCols[tile];
+  const int step = tile == kLargeTile ? TK : 2 * TK;
+  const int k_steps = (p.k + step - 1) / step;
+  pp.cluster = cluster; pp.k_tiles_per_slice = (k_steps + cluster - 1) / cluster;
+  pp.status = dev->status;
+  const long long work = static_cast<long long>(pp.tiles_m) * pp.tiles_n * cluster;
+  if (work > 2147483647LL) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
+  const int grid = static_cast<int>(cluster > 1 || work < dev->sms ? work : dev->sms);
+  if (launch_path<T>(maximize, tile == kSmallTile, map_a, map_b, pp, grid, stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
   g_launches.fetch_add(1);
   return CUASR_STATUS_SUCCESS;
 }
@@ -509,7 +574,9 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   constexpr int TK = kTileKBytes / sizeof(T);
   const long long tiles = static_cast<long long>(tile_count(args));
   const bool all_tiles = ring_has_all_tiles<T>(desc);
-  LaunchPlan plan = plan_without_workspace(desc, p.m, p.n, p.k, dev->sms, all_tiles);
+  LaunchPlan plan = plan_without_workspace(desc, p.m, p.n, p.k, dev->sms, all_tiles,
+                                           !p.a_kcontig || !tma_describable(p.a, p.lda, sizeof(T)),
+                                           !p.b_kcontig || !tma_describable(p.b, p.ldb, sizeof(T)));
   bool tickets_used = false, balanced = false;
   // partials are moved 16 bytes at a time and re-packed operands are read by TMA: a workspace that does not start
   // on a 16-byte boundary is an error where it is required and is left unused where it is optional
@@ -550,13 +617,13 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
     // the screened kernel, where it is modelled faster: no factor on the product (alpha is the identity of +), so that
     // the running minimum can live in D
     if ((desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM) && desc.mul_op == CUASR_OP_PLUS && alpha == T(0)) {
-      const ScreenPlan screened = screen_plan(desc.dtype, p.m, p.n, p.k, dev->sms, extra.count == 0);
+      const ScreenPlan screened = screen_plan(p.m, p.n, p.k, dev->sms, extra.count == 0);
       if (screened.cost < plan.cost) {
         const bool name = !small && dense && tma_describable(p.a, p.lda, sizeof(T)) && tma_describable(p.b, p.ldb, sizeof(T));
         const bool copies = slices == 1 && args.workspace != nullptr && workspace_aligned && repack_plan(desc, args, p).bytes > 0 &&
                             args.workspace_bytes >= align_up(balance_workspace_bytes(desc, args, dev->sms), 256) + repack_plan(desc, args, p).bytes;
         if (!copies) {
-          const int st = run_screened<T>(desc.add_op == CUASR_OP_MAXIMUM, p, beta, add_id, read_c, screened, extra, nullptr, 0, 0, dev, stream);
+          const int st = run_screened<T>(desc.add_op == CUASR_OP_MAXIMUM, p, beta, add_id, read_c, screened, extra, dev, stream);
           if (st == CUASR_STATUS_SUCCESS)
             t_last_kernel = !name ? (slices > 1 ? "generic_splitk" : "generic") : slices > 1 ? "tma_splitk" : balanced ? "tma_balanced" : "tma";
           return st;
@@ -598,7 +665,7 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   const bool describable = tma_describable(p.a, p.lda, sizeof(T)) && tma_describable(p.b, p.ldb, sizeof(T));
   // the name a caller sees: "tma..." where the storage lines are what TMA could describe
   const bool aligned_name = (pads_itself || k_map % TK == 0) && !small && dense && describable;
-  const int step = TK * kTileSub[plan.tile];
+  const int step = TK * tile_sub(plan.tile, desc);
   const bool nan_pad = std::is_floating_point<T>::value && (desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM);
   // TMA brings in what lies along k on aligned lines, unless a ragged last step needs padding it cannot write
   const bool fill_ok = encode_tiled_fn() != nullptr && dense && (pads_itself || k_map % step == 0);
@@ -846,10 +913,8 @@ int cuasr_b200_srgemm_path(const cuasr_b200_desc_t* desc, const cuasr_b200_args_
   const bool dense = p.lda >= (p.a_kcontig ? p.k : p.m) && p.ldb >= (p.b_kcontig ? p.k : p.n);
   const bool pipelined = f32 && dense && static_cast<long long>(args->m) * args->n >= 64 * 64 &&
                          tma_describable(p.a, p.lda, es) && tma_describable(p.b, p.ldb, es);
-  const ScreenPlan plan = screen_plan(desc->dtype, p.m, p.n, p.k, dev->sms, false);
-  const ExtraOutputs none;
-  const int done = f32 ? run_screened<float>(maximize, p, 0.0f, 0.0f, false, plan, none, parent, ld_parent, k_offset, dev, stream)
-                       : run_screened<double>(maximize, p, 0.0, 0.0, false, plan, none, parent, ld_parent, k_offset, dev, stream);
+  const int done = f32 ? run_path<float>(maximize, p, parent, ld_parent, k_offset, dev, stream)
+                       : run_path<double>(maximize, p, parent, ld_parent, k_offset, dev, stream);
   if (done == CUASR_STATUS_SUCCESS) t_last_kernel = pipelined ? "path_tma" : "path";
   return done;
 }

@@ -1,11 +1,11 @@
-// Screened tropical kernels: fp32 and fp64, min-plus and max-plus, with and without predecessors.
+// Screened tropical kernels: fp64 min-plus and max-plus.
 #include "srgemm_launch_impl.cuh"
 #include "srgemm_screened.cuh"
 namespace cuasr_b200 {
-template <typename T, bool kMax, bool kPath>
+template <typename T, bool kMax>
 static cudaError_t launch_variant(const CUtensorMap& map_a, const CUtensorMap& map_b, const ScreenParams<T>& params, int grid,
                                   cudaStream_t stream) {
-  auto kernel = srgemm_screened_kernel<T, kMax, kPath>;
+  auto kernel = srgemm_screened_kernel<T, kMax>;
   static std::atomic<unsigned long long> done{0};
   const cudaError_t err = opt_in_shared_memory(kernel, kScreenSmemBytes<T>, done);
   if (err != cudaSuccess) return err;
@@ -14,11 +14,8 @@ static cudaError_t launch_variant(const CUtensorMap& map_a, const CUtensorMap& m
 template <typename T>
 cudaError_t launch_screened(bool maximize, const CUtensorMap& map_a, const CUtensorMap& map_b, const ScreenParams<T>& params,
                             int grid, cudaStream_t stream) {
-  if (params.parent != nullptr)
-    return maximize ? launch_variant<T, true, true>(map_a, map_b, params, grid, stream)
-                    : launch_variant<T, false, true>(map_a, map_b, params, grid, stream);
-  return maximize ? launch_variant<T, true, false>(map_a, map_b, params, grid, stream)
-                  : launch_variant<T, false, false>(map_a, map_b, params, grid, stream);
+  return maximize ? launch_variant<T, true>(map_a, map_b, params, grid, stream)
+                  : launch_variant<T, false>(map_a, map_b, params, grid, stream);
 }
 template <typename T>
 cudaError_t launch_screened_init(bool maximize, const ScreenParams<T>& params, int sms, cudaStream_t stream) {
@@ -27,8 +24,6 @@ cudaError_t launch_screened_init(bool maximize, const ScreenParams<T>& params, i
   return maximize ? launch_overlapped(screened_init_kernel<Ring<CUASR_OP_MAXIMUM, CUASR_OP_PLUS, T>>, grid, 256, 0, 1, stream, params)
                   : launch_overlapped(screened_init_kernel<Ring<CUASR_OP_MINIMUM, CUASR_OP_PLUS, T>>, grid, 256, 0, 1, stream, params);
 }
-template cudaError_t launch_screened<float>(bool, const CUtensorMap&, const CUtensorMap&, const ScreenParams<float>&, int, cudaStream_t);
 template cudaError_t launch_screened<double>(bool, const CUtensorMap&, const CUtensorMap&, const ScreenParams<double>&, int, cudaStream_t);
-template cudaError_t launch_screened_init<float>(bool, const ScreenParams<float>&, int, cudaStream_t);
 template cudaError_t launch_screened_init<double>(bool, const ScreenParams<double>&, int, cudaStream_t);
 }  // namespace cuasr_b200

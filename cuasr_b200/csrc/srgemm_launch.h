@@ -10,14 +10,14 @@
 
 namespace cuasr_b200 {
 
-enum TileKind : int { kLargeTile = 0, kMediumTile = 1, kSmallTile = 2 };
+enum TileKind : int { kLargeTile = 0, kMediumTile = 1, kSmallTile = 2, kTinyTile = 3 };
 
 // Launches srgemm_tma_kernel<Ring<ADD, MUL, T>, tile> on `grid` CTAs in clusters of `cluster`.
 template <int ADD, int MUL, typename T>
 cudaError_t launch_tma(int tile, const CUtensorMap& map_a, const CUtensorMap& map_b, const TmaParams<T>& params,
                        int grid, int cluster, cudaStream_t stream);
 
-// (ring, element type) pairs that have every tile shape compiled in; the others run on the small tile alone.
+// (ring, element type) pairs that have every tile shape compiled in; the others run on the two smallest alone.
 template <int ADD, int MUL, typename T>
 constexpr bool all_tiles_instantiated() {
   constexpr bool tropical = (ADD == CUASR_OP_MINIMUM || ADD == CUASR_OP_MAXIMUM) && MUL == CUASR_OP_PLUS;

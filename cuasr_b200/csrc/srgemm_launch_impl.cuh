@@ -41,6 +41,10 @@ cudaError_t launch_tma(int tile, const CUtensorMap& map_a, const CUtensorMap& ma
     if (tile == kLargeTile) return launch_tma_variant<R, LargeTile>(map_a, map_b, params, grid, cluster, stream);
     if (tile == kMediumTile) return launch_tma_variant<R, MediumTile>(map_a, map_b, params, grid, cluster, stream);
   }
+  if (tile == kTinyTile) {
+    constexpr bool dmma = std::is_same<T, double>::value && ADD == CUASR_OP_PLUS && MUL == CUASR_OP_MULTIPLIES;
+    return launch_tma_variant<R, std::conditional_t<dmma, TinyTileDeep, TinyTile>>(map_a, map_b, params, grid, cluster, stream);
+  }
   return launch_tma_variant<R, SmallTile>(map_a, map_b, params, grid, cluster, stream);
 }
 

@@ -19,8 +19,6 @@
 // and blocks are independent of order, so K may be cut into pieces for different CTAs, which then meet in D by
 // compare-and-swap (pieces > 1; D initialised by an earlier launch).
 //
-// With kPath the k that first attains the best value goes to `parent` (blocks in ascending k, strict improvements).
-//
 // Structure: one persistent CTA per SM.  Warps 8..11 bring exact tiles in (TMA or gather), turn them into 16-bit tiles;
 // warps 0..7 own 64 x 32 blocks of the 128 x 128 tile, 8 x 8 elements per lane.  A stage is 512 bytes of exact operand
 // rows' worth of k: 64 k (fp32) or 32 k (fp64), two stages.
@@ -38,8 +36,6 @@ struct ScreenParams {
   int a_mode, b_mode;              // LoadMode
   const T* C;  long long ldc;      // row-major; may alias D
   T* D;        long long ldd;      // row-major
-  int32_t* parent; long long ld_parent;   // kPath
-  int k_offset;                           // kPath: added to every recorded k
   T beta, add_identity;
   int read_c;
   int n_extra;
@@ -160,7 +156,7 @@ __device__ __forceinline__ void merge_into(double* at, double value) {
   else      atomicMin(reinterpret_cast<long long*>(at), __double_as_longlong(value));
 }
 
-template <typename T, bool kMax, bool kPath>
+template <typename T, bool kMax>
 __global__ void __launch_bounds__(kTmaThreads, 1)
 srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                        const __grid_constant__ ScreenParams<T> p) {
@@ -209,10 +205,9 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   const int num_work = p.tiles_m * p.tiles_n * p.pieces;
   const int tiles = p.tiles_m * p.tiles_n;
   // A piece walks its blocks in a scattered order (stride near the golden section, coprime to the count), so that data
-  // whose products improve steadily along k does not let an element improve in every block.  With kPath the order is
-  // ascending: the first k wins.
+  // whose products improve steadily along k does not let an element improve in every block.
   auto stride_of = [&](int count) {
-    if (kPath || count < 8) return 1;
+    if (count < 8) return 1;
     int st = (int)(count * 0.618f) | 1;
     auto gcd = [](int a, int b) { while (b) { const int t = a % b; a = b; b = t; } return a; };
     while (gcd(count, st) != 1) st += 2;
@@ -399,8 +394,8 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     const int m_base = tm * 128 + wm * 64, n_base = tn * 128 + wn * 32;
     int my_exp = 1 << 30;             // exponent the bounds were made with
     int pos = 0;
-    int exact_left = kPath ? 0 : 1;   // blocks to do exactly before the screen is worth its tests
-    bool opened = kPath;              // D holds the running values of this tile
+    int exact_left = 1;               // blocks to do exactly before the screen is worth its tests
+    bool opened = false;              // D holds the running values of this tile
 
     for (int b = 0; b < count; ++b, ++it) {
       const int s = it % kScreenStages;
@@ -417,11 +412,10 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       const int exponent = stage_exp[s];
       const bool unfit = top > S::kFiniteLimit || low < 0.0f;
       const T scale = (T)__int_as_float((exponent + 127) << 23);
-      const int k0 = (begin + pos) * KB;
       pos += stride;
       if (pos >= count) pos -= count;
 
-      if (!kPath && (unfit || exact_left > 0)) {
+      if (unfit || exact_left > 0) {
         // ---- the whole block exactly, for all 64 elements of the lane; then merged into D
         T acc[8][8];
 #pragma unroll
@@ -503,9 +497,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       }
 
       uint32_t mask_lo = 0, mask_hi = 0;              // bit 8 i + j: element (i, j) might improve in this block
-      if (kPath && unfit) {
-        mask_lo = mask_hi = ~0u;
-      } else {
+      {
         // ---- the screen: two products per instruction
         uint32_t bound[8][8], q[8][8];
 #pragma unroll
@@ -563,7 +555,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       }
       const int total = __shfl_sync(~0u, slot_of_next, 31);
       slot_of_next -= mine;
-      if (!kPath && total > kExactAbove) exact_left = 3;
+      if (total > kExactAbove) exact_left = 3;
       for (int first = 0; first < total; first += kListed) {
         while (slot_of_next < first + kListed && (mask_lo | mask_hi) != 0) {
           int bit;
@@ -578,7 +570,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         for (int base = 0; base < listed; base += 16) {
           // two groups of eight elements, so that their loads and exchanges overlap
           T best[2];
-          int best_k[2], code[2];
+          int code[2];
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
             const int slot = base + u * 8 + (lane >> 2);
@@ -589,19 +581,12 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             // the lane's chunks of 16 bytes: t and t + 4 of both 128-byte columns
             const uint32_t fa = (row & 4) << 4, fb = (col & 4) << 4;
             best[u] = kMax ? -static_cast<T>(INFINITY) : static_cast<T>(INFINITY);
-            best_k[u] = 1 << 20;
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
               T a[EV], bb[EV];
               lds16(ra + (h >> 1) * kColumn + (((h & 1) << 6) ^ fa), a);
               lds16(rb + (h >> 1) * kColumn + (((h & 1) << 6) ^ fb), bb);
-              if constexpr (kPath) {
-#pragma unroll
-                for (int e = 0; e < EV; ++e) {
-                  const T v = a[e] + bb[e];
-                  if (S::better(v, best[u])) { best[u] = v; best_k[u] = (h >> 1) * TK + (t + 4 * (h & 1)) * EV + e; }
-                }
-              } else if constexpr (RingT::kPackedPairs) {
+              if constexpr (RingT::kPackedPairs) {
                 best[u] = RingT::mac_packed(best[u], pack2(a[0], a[1]), pack2(bb[0], bb[1]));
                 best[u] = RingT::mac_packed(best[u], pack2(a[2], a[3]), pack2(bb[2], bb[3]));
               } else {
@@ -614,12 +599,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
               const T other = __shfl_xor_sync(~0u, best[u], d);
-              if constexpr (kPath) {
-                const int other_k = __shfl_xor_sync(~0u, best_k[u], d);
-                if (S::better(other, best[u]) || (other == best[u] && other_k < best_k[u])) { best[u] = other; best_k[u] = other_k; }
-              } else {
-                best[u] = RingT::add(other, best[u]);
-              }
+              best[u] = RingT::add(other, best[u]);
             }
           }
 #pragma unroll
@@ -631,17 +611,9 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
               const uint32_t where = warp_bounds + i * 512 + el * 16 + j * 2;
               const uint32_t was = lds2(where), now = S::bound(best[u], scale);
               // Which of two values with the same 16-bit bound is better only D can tell; there a minimum (maximum) in
-              // memory does, without waiting for its answer, unless the predecessor depends on it.
-              bool improved = S::sooner(now, was);
-              if (kPath) {
-                if (now == was || (unfit && !improved)) improved = S::better(best[u], *at);
-                if (improved) {
-                  *at = best[u];
-                  p.parent[(long long)m * p.ld_parent + n] = k0 + best_k[u] + p.k_offset;
-                }
-              } else if ((improved || now == was) && best[u] >= T(0)) {
-                merge_into<kMax>(at, best[u]);
-              }
+              // memory does, without waiting for its answer.
+              const bool improved = S::sooner(now, was);
+              if ((improved || now == was) && best[u] >= T(0)) merge_into<kMax>(at, best[u]);
               if (improved) sts2(where, now);
             }
           }
@@ -683,7 +655,7 @@ screened_init_kernel(const __grid_constant__ ScreenParams<typename RingT::Elemen
   }
 }
 
-// Launches srgemm_screened_kernel (params.parent != nullptr: with predecessors) on `grid` persistent CTAs, and the
+// Launches srgemm_screened_kernel on `grid` persistent CTAs, and the
 // kernel that prepares D where its pieces share it.
 template <typename T>
 cudaError_t launch_screened(bool maximize, const CUtensorMap& map_a, const CUtensorMap& map_b, const ScreenParams<T>& params,

@@ -46,14 +46,14 @@ constexpr int kMaxDestinations = 8;               // output copies one launch ca
 constexpr int kMaxSmemBytes = 232448;             // 227 KiB: what one CTA may have
 
 // Tile shape of a kernel variant.
-template <int WM_, int WN_, int WK_>
+template <int WM_, int WN_, int WK_, int kSub_ = WK_ == 4 ? 2 : 1>
 struct TileShape {
   static constexpr int WM = WM_, WN = WN_, WK = WK_;
   static_assert(WM * WN * WK == kConsumerWarps, "eight consumer warps");
   static constexpr int kM = 64 * WM, kN = 32 * WN;
   // 128-byte k columns per stage: two where the k range is shared by four warps, so that each warp gets four of the
   // 16-byte chunks of a stage (one unrolled pass of the contraction loop)
-  static constexpr int kSub = WK == 4 ? 2 : 1;
+  static constexpr int kSub = kSub_;
   static constexpr int kABytes = kM * kTileKBytes * kSub;
   static constexpr int kBBytes = kN * kTileKBytes * kSub;
   static constexpr int kStageBytes = kABytes + kBBytes;
@@ -68,6 +68,10 @@ struct TileShape {
 using LargeTile = TileShape<2, 4, 1>;    // 128 x 128
 using MediumTile = TileShape<2, 2, 2>;   // 128 x 64
 using SmallTile = TileShape<1, 2, 4>;    // 64 x 64
+// 64 x 32, one 16-byte chunk of k per warp and stage: the shortest chain for the smallest products, and the finest
+// pieces of k for a cluster (fp64 sums take their chunks in fours, so their stage is four columns deep)
+using TinyTile = TileShape<1, 1, 8>;
+using TinyTileDeep = TileShape<1, 1, 8, 4>;
 
 template <typename T>
 struct TmaParams {
@@ -279,7 +283,7 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   // compile-time constant away from it:  row * 128 + ((chunk ^ (row & 7)) * 16)
   //   A rows are lr + 8 i  -> + i * 1024 bytes, row & 7 == lr for every i
   //   B rows are lc + 4 j  -> + j * 512 bytes,  row & 7 == lc + 4 (j & 1)
-  // The warp's first chunk of a stage: column wk * kChunks / 8, chunk wk * kChunks % 8 (0 or 4) of it.
+  // The warp's first chunk of a stage: column wk * kChunks / 8, chunk wk * kChunks % 8 of it.
   constexpr int kChunksPerColumn = 8;
   const int first_chunk = WK == 1 ? 0 : (wk * kChunks) % kChunksPerColumn;
   const int column = WK == 1 ? 0 : (wk * kChunks) / kChunksPerColumn;
@@ -299,13 +303,14 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   // multiples of 128, so the flip commutes with adding them)
   // (four chunks keep the loop body near 16 KiB of instructions; unrolling all eight measured the same on min-plus
   // and 25 % slower on max-min, whose body is half as large again)
-  constexpr int kUnroll = 4;
-  uint32_t a_off[kOffsetTable ? kUnroll : 1], b_off[kOffsetTable ? 8 : 1];
+  constexpr int kUnroll = kChunks < 4 ? kChunks : 4;
+  uint32_t a_off[kOffsetTable ? kUnroll : 1], b_off[kOffsetTable ? kUnroll : 1];
   if constexpr (kOffsetTable) {
 #pragma unroll
-    for (int c = 0; c < kUnroll; ++c) a_off[c] = a_base + ((((c + first_chunk) ^ lr) & 7) << 4);
-#pragma unroll
-    for (int c = 0; c < 8; ++c) b_off[c] = b_base + ((((c + first_chunk) ^ lc) & 7) << 4);   // rows lc + 4 j with odd j use b_off[c ^ 4]
+    for (int c = 0; c < kUnroll; ++c) {
+      a_off[c] = a_base + ((((c + first_chunk) ^ lr) & 7) << 4);
+      b_off[c] = b_base + ((((c + first_chunk) ^ lc) & 7) << 4);       // rows lc + 4 j with odd j: bit 6 flipped
+    }
   }
 
   uint32_t it = 0;
@@ -340,7 +345,7 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         uint32_t base0, base1;
         if constexpr (kOffsetTable) {
           base0 = st + (b_off[c] ^ (h << 6));
-          base1 = st + (b_off[c ^ 4] ^ (h << 6));
+          base1 = st + (b_off[c] ^ ((h << 6) ^ 64));
         } else {
           base0 = st + b_base + ((((c + first_chunk) ^ lc) & 7) << 4);
           base1 = st + b_base + ((((c + first_chunk) ^ (lc + 4)) & 7) << 4);
@@ -364,6 +369,16 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           }
           return;
         }
+        if constexpr (sizeof(T) == 8) {
+          // one k at a time: neighbouring instructions are independent
+#pragma unroll
+          for (int e = 0; e < EV; ++e)
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+              for (int j = 0; j < 8; ++j) acc[i][j] = RingT::add(RingT::mul(a[i][e], b[j][e]), acc[i][j]);
+          return;
+        }
 #pragma unroll
         for (int e = 0; e < EV; e += 2)
 #pragma unroll
@@ -379,7 +394,7 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         // chunks) the slot lc of step s (s = 0, 1) stands for k = 2 lc + s, so one 16-byte load delivers both steps
         // of a block.
         constexpr int kGroups = kChunks / 4;
-        static_assert(!kDmma || (kGroups >= 1 && kGroups <= 2), "one or two groups of 8 k per warp and stage");
+        static_assert(kGroups == 1 || kGroups == 2, "one or two groups of 8 k per warp and stage");
         auto load_group = [&](double (&a)[8][2], double (&b)[4][2], int group) {
           const uint32_t chunk = ((((group * 4 + first_chunk + lc) ^ lr) & 7) << 4);
           const uint32_t abase = st + a_base + chunk;
@@ -415,24 +430,28 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         T a0[8][EV], b0[8][EV], a1[8][EV], b1[8][EV];
         load_a(a0, 0, 0);
         load_b(b0, 0, 0);
-        // kUnroll chunks at a time with compile-time chunk indices, so that the only integer work left per chunk is
-        // combining the stage base with a table entry (integer instructions share the half-rate pipe with the
-        // three-input min: each one costs as much as a product pair)
+        if constexpr (kChunks == 1) {
+          compute(a0, b0);
+        } else {
+          // kUnroll chunks at a time with compile-time chunk indices, so that the only integer work left per chunk is
+          // combining the stage base with a table entry (integer instructions share the half-rate pipe with the
+          // three-input min: each one costs as much as a product pair)
 #pragma unroll 1
-        for (int h = 0; h < kChunks / kUnroll; ++h) {
+          for (int h = 0; h < kChunks / kUnroll; ++h) {
 #pragma unroll
-          for (int c = 0; c < kUnroll; c += 2) {
-            load_a(a1, c + 1, h);
-            load_b(b1, c + 1, h);
-            compute(a0, b0);
-            if (c + 2 < kUnroll) {
-              load_a(a0, c + 2, h);
-              load_b(b0, c + 2, h);
-            } else if (h + 1 < kChunks / kUnroll) {
-              load_a(a0, 0, h + 1);
-              load_b(b0, 0, h + 1);
+            for (int c = 0; c < kUnroll; c += 2) {
+              load_a(a1, c + 1, h);
+              load_b(b1, c + 1, h);
+              compute(a0, b0);
+              if (c + 2 < kUnroll) {
+                load_a(a0, c + 2, h);
+                load_b(b0, c + 2, h);
+              } else if (h + 1 < kChunks / kUnroll) {
+                load_a(a0, 0, h + 1);
+                load_b(b0, 0, h + 1);
+              }
+              compute(a1, b1);
             }
-            compute(a1, b1);
           }
         }
       } else {
