@@ -614,9 +614,9 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   const bool dense = p.lda >= (p.a_kcontig ? p.k : p.m) && p.ldb >= (p.b_kcontig ? p.k : p.n);
   const bool small = static_cast<long long>(p.m) * p.n < 64 * 64;
   if constexpr (std::is_same<T, double>::value) {
-    // the screened kernel, where it is modelled faster: no factor on the product (alpha is the identity of +), so that
-    // the running minimum can live in D
-    if ((desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM) && desc.mul_op == CUASR_OP_PLUS && alpha == T(0)) {
+    // the screened kernel, where it is modelled faster: no factor on the product (alpha is the identity of +) and a
+    // start value that compares, so that the running minimum can live in D
+    if (add_id == add_id && (desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM) && desc.mul_op == CUASR_OP_PLUS && alpha == T(0)) {
       const ScreenPlan screened = screen_plan(p.m, p.n, p.k, dev->sms, extra.count == 0);
       if (screened.cost < plan.cost) {
         const bool name = !small && dense && tma_describable(p.a, p.lda, sizeof(T)) && tma_describable(p.b, p.ldb, sizeof(T));
@@ -681,9 +681,9 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   if (tp.b_mode == kLoadTma &&
       !make_operand_map<T>(&map_b, tp.B, p.ldb, p.n, k_map, true, nan_pad, kTileCols[plan.tile])) tp.b_mode = kLoadGatherK;
   if (k_map != p.k && (tp.a_mode != kLoadTma || tp.b_mode != kLoadTma)) tp.K = k_map;   // copies that hold their own padding
-  tp.pad_a = tp.pad_b = T(0);
-  if (nan_pad) tp.pad_a = tp.pad_b = static_cast<T>(NAN);
-  else if (!pads_itself) { tp.pad_a = add_id; tp.pad_b = mul_id; }
+  tp.pad = nan_pad ? static_cast<T>(NAN) : T(0);
+  // the other rings (integer minima and maxima, logical or from an odd start value) are idempotent
+  tp.repeat_k = !pads_itself;
   tp.C = static_cast<const T*>(p.c); tp.ldc = p.ldc;
   tp.D = static_cast<T*>(p.d); tp.ldd = p.ldd;
   tp.alpha = alpha; tp.beta = beta; tp.add_identity = add_id; tp.read_c = read_c;

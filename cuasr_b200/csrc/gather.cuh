@@ -35,13 +35,14 @@ __device__ __forceinline__ void sts(uint32_t addr, double v) { asm volatile("st.
 
 // Stages rows [r0, r0 + kRows) x k [k0, k0 + kSub * 128 bytes) of an operand whose element (r, k) is base[r * ld + k]
 // (kLoadGatherK) or base[r + k * ld] (kLoadGatherMN).  Rows at or beyond `rows` repeat the last row (their results are
-// never stored); k at or beyond K is set to `pad` by plain stores, so a stage that reaches beyond K must not be announced
+// never stored); k at or beyond K repeats the last k too where `repeat_k` is set (rings whose (+) is idempotent: a product
+// twice changes nothing) and is else set to `pad` by plain stores, so a stage that reaches beyond K must not be announced
 // with cp_async_arrive_noinc alone.  Called by all 128 producer threads; `pw` is the producer warp (0..3).
 // Inside the matrix a copy is one cp.async and at most one addition: with the bounds tested element by element a
 // 1024 x 768 x 1536 product of odd storage lines took 186 us, against 97 us with TMA.
 template <typename T, int kRows, int kSub>
 __device__ __forceinline__ void gather_tile(uint32_t dst, const T* __restrict__ base, long long ld, int mode, int r0,
-                                            int rows, int k0, int K, T pad, int pw, int lane) {
+                                            int rows, int k0, int K, T pad, bool repeat_k, int pw, int lane) {
   constexpr int TK = 128 / (int)sizeof(T);         // k per 128-byte row
   constexpr int ES = (int)sizeof(T);
   // opaque: the lane's offsets are computed here, per stage, instead of being held in the producers' few registers
@@ -56,7 +57,7 @@ __device__ __forceinline__ void gather_tile(uint32_t dst, const T* __restrict__ 
 #pragma unroll 1
       for (int step = 0; step < TK / 16; ++step) {
         const int kk = step * 16 + pw * 4 + kq;
-        const int k = k0 + sub * TK + kk;
+        const int k = repeat_k ? min(k0 + sub * TK + kk, K - 1) : k0 + sub * TK + kk;
         const uint32_t d = dst + sub * (kRows * 128) + r8 * 128 + ((((kk * ES) >> 4) ^ r8) << 4) + ((kk * ES) & 15);
         const T* line = base + (long long)k * ld + r0;
         if (k0 + sub * TK + TK <= K && last >= kRows - 1) {          // uniform over the warp
@@ -82,7 +83,7 @@ __device__ __forceinline__ void gather_tile(uint32_t dst, const T* __restrict__ 
     const uint32_t c1 = ES == 8 ? c0 : c0 ^ 64;
 #pragma unroll 1
     for (int sub = 0; sub < kSub; ++sub) {
-      const int k = k0 + sub * TK + kk;
+      const int k = repeat_k ? min(k0 + sub * TK + kk, K - 1) : k0 + sub * TK + kk;
       const uint32_t d = dst + sub * (kRows * 128) + rr * 128 + ((kk * ES) & 15);
       const T* column = base + (long long)r0 * ld + k;
       if (k0 + sub * TK + TK <= K && last >= kRows - 1) {            // uniform over the warp

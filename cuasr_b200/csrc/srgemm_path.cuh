@@ -135,9 +135,9 @@ srgemm_path_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         }
         if (gathers) {
           if (p.a_mode != kLoadTma)
-            gather_tile<T, Tile::kM, kSub>(smem_u32(sa), p.A, p.lda, p.a_mode, m0, p.M, k0, p.K, p.pad, pw, lane);
+            gather_tile<T, Tile::kM, kSub>(smem_u32(sa), p.A, p.lda, p.a_mode, m0, p.M, k0, p.K, p.pad, false, pw, lane);
           if (p.b_mode != kLoadTma)
-            gather_tile<T, Tile::kN, kSub>(smem_u32(sb), p.B, p.ldb, p.b_mode, n0, p.N, k0, p.K, p.pad, pw, lane);
+            gather_tile<T, Tile::kN, kSub>(smem_u32(sb), p.B, p.ldb, p.b_mode, n0, p.N, k0, p.K, p.pad, false, pw, lane);
           if (k0 + kStep > p.K) {
             cp_async_wait_all();
             mbar_arrive(&full_bar[s]);
@@ -195,7 +195,9 @@ srgemm_path_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int m = m_base + lr + 8 * i, n = n_base + lc + 4 * j;
-        acc[i][j] = (m < p.M && n < p.N) ? p.dist[(long long)m * p.ldd + n] : T(0);
+        const T x = (m < p.M && n < p.N) ? p.dist[(long long)m * p.ldd + n] : T(0);
+        // nothing is better than a NaN; the minimum instruction would drop it for the first product
+        acc[i][j] = x == x ? x : kMaximize ? static_cast<T>(INFINITY) : -static_cast<T>(INFINITY);
       }
     keep();
 
@@ -286,7 +288,10 @@ srgemm_path_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int m = m_base + lr + 8 * i + zero, n = n_base + lc + 4 * j + zero;
-          if (m < p.M && n < p.N) p.dist[(long long)m * p.ldd + n] = acc[i][j];
+          if (m < p.M && n < p.N) {
+            T* at = p.dist + (long long)m * p.ldd + n;
+            if (better(acc[i][j], *at)) *at = acc[i][j];
+          }
         }
     } else {
       // Partial values to shared memory ([wk][row][column], column groups swizzled), then one element per thread at a

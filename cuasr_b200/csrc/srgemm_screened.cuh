@@ -82,9 +82,12 @@ __device__ __forceinline__ bool producers_agree(bool ok) {
 template <bool kMax>
 struct Screen {
   static constexpr float kFiniteLimit = 16382.0f;
-  // fp64 -> fp32 without losing the direction of the bound
-  static __device__ __forceinline__ float narrow(float x) { return x; }
-  static __device__ __forceinline__ float narrow(double x) { return kMax ? __double2float_ru(x) : __double2float_rd(x); }
+  // scaled fp32 image of an element, rounded towards "better" in both steps (the scaling is inexact where it underflows:
+  // rounded to nearest, a tiny negative value would come out as a zero and a tiny maximum would lose its upper bound)
+  static __device__ __forceinline__ float scaled(float x, float scale) { return kMax ? __fmul_ru(x, scale) : __fmul_rd(x, scale); }
+  static __device__ __forceinline__ float scaled(double x, float scale) {
+    return scaled(kMax ? __double2float_ru(x) : __double2float_rd(x), scale);
+  }
   static constexpr uint32_t kNever = kMax ? 0x8000u : 0x7FFFu;       // the infinity no sum improves with
   static constexpr uint32_t kNothing = kMax ? 0x7FFFu : 0u;          // bound no sum beats (elements outside the matrix)
   // Widens [smallest, largest] by two scaled values.  The infinity that never improves (+inf for min) is legal and
@@ -109,6 +112,7 @@ struct Screen {
   template <typename T>
   static __device__ __forceinline__ uint32_t bound(T v, T scale) {
     const T y = v * scale;
+    if (y != y) return kNothing;                                        // a NaN (from C) stays: nothing is better than it
     if (kMax) {
       if (!(y >= T(0))) return (uint32_t)(uint16_t)-1;                  // any sum of finite values
       if (y >= T(32766)) return 32766u;
@@ -143,15 +147,17 @@ __device__ __forceinline__ double improve_shared(double* at, double value, doubl
   return seen;
 }
 
-// *at = better(*at, value) without reading it back.  `value` is a sum of a fit stage, i.e. not negative, and then the
-// bit patterns of any float compare with it like signed integers.
+// *at = better(*at, value) without reading it back.  `value` is not negative, and then the bit patterns of any float
+// compare with it like signed integers; adding zero makes a negative zero a positive one, whose pattern does.
 template <bool kMax>
 __device__ __forceinline__ void merge_into(float* at, float value) {
+  value += 0.0f;
   if (kMax) atomicMax(reinterpret_cast<int*>(at), __float_as_int(value));
   else      atomicMin(reinterpret_cast<int*>(at), __float_as_int(value));
 }
 template <bool kMax>
 __device__ __forceinline__ void merge_into(double* at, double value) {
+  value += 0.0;
   if (kMax) atomicMax(reinterpret_cast<long long*>(at), __double_as_longlong(value));
   else      atomicMin(reinterpret_cast<long long*>(at), __double_as_longlong(value));
 }
@@ -258,8 +264,8 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       if (alive && gathers) {
         // beyond K: infinities of the kind that never improves
         const T pad = kMax ? -static_cast<T>(INFINITY) : static_cast<T>(INFINITY);
-        if (p.a_mode != kLoadTma) gather_tile<T, 128, 2>(smem_u32(sa), p.A, p.lda, p.a_mode, lm0, p.M, k0, p.K, pad, pw, lane);
-        if (p.b_mode != kLoadTma) gather_tile<T, 128, 2>(smem_u32(sb), p.B, p.ldb, p.b_mode, ln0, p.N, k0, p.K, pad, pw, lane);
+        if (p.a_mode != kLoadTma) gather_tile<T, 128, 2>(smem_u32(sa), p.A, p.lda, p.a_mode, lm0, p.M, k0, p.K, pad, false, pw, lane);
+        if (p.b_mode != kLoadTma) gather_tile<T, 128, 2>(smem_u32(sb), p.B, p.ldb, p.b_mode, ln0, p.N, k0, p.K, pad, false, pw, lane);
         if (k0 + KB > p.K) {
           cp_async_wait_all();
           mbar_arrive(&full_bar[s]);
@@ -309,7 +315,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             }
 #pragma unroll
             for (int w = 0; w < 4; ++w) {
-              const float y0 = x[w >> 1][(w & 1) * 2] * scale, y1 = x[w >> 1][(w & 1) * 2 + 1] * scale;
+              const float y0 = S::scaled(x[w >> 1][(w & 1) * 2], scale), y1 = S::scaled(x[w >> 1][(w & 1) * 2 + 1], scale);
               S::survey(y0, y1, largest, smallest);
               words[w] = S::quantise(y0) | (S::quantise(y1) << 16);
             }
@@ -319,7 +325,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
               double x[2];
               const int chunk = 4 * c + w;                            // 2 k
               lds16(src + (chunk >> 3) * kColumn + (((chunk & 7) ^ r8) << 4), x);
-              const float y0 = S::narrow(x[0]) * scale, y1 = S::narrow(x[1]) * scale;
+              const float y0 = S::scaled(x[0], scale), y1 = S::scaled(x[1], scale);
               S::survey(y0, y1, largest, smallest);
               words[w] = S::quantise(y0) | (S::quantise(y1) << 16);
             }
@@ -459,7 +465,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
               if (shared_d) {
                 v = improve_shared<kMax>(at, v, __ldcg(at));
               } else if (opened) {
-                const T cur = *at;
+                const T cur = __ldcg(at);                          // lanes of this warp improve it at the L2
                 if (S::better(v, cur)) *at = v;
                 else v = cur;
               } else {
@@ -613,7 +619,10 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
               // Which of two values with the same 16-bit bound is better only D can tell; there a minimum (maximum) in
               // memory does, without waiting for its answer.
               const bool improved = S::sooner(now, was);
-              if ((improved || now == was) && best[u] >= T(0)) merge_into<kMax>(at, best[u]);
+              if (improved || now == was) {
+                if (best[u] >= T(0)) merge_into<kMax>(at, best[u]);
+                else improve_shared<kMax>(at, best[u], __ldcg(at));   // max only: sums of values that round up to zero
+              }
               if (improved) sts2(where, now);
             }
           }

@@ -79,7 +79,8 @@ struct TmaParams {
   const T* A;  long long lda;   // gathered operands only
   const T* B;  long long ldb;
   int a_mode, b_mode;           // LoadMode
-  T pad_a, pad_b;               // what a gather writes for k >= K
+  T pad;                        // what a gather writes for k >= K ...
+  int repeat_k;                 // ... unless it repeats the last k there: (+) is idempotent and there is no such value
   const T* C;  long long ldc;   // row-major; may alias D; may be null when !read_c
   T* D;        long long ldd;   // row-major
   // Extra copies of the output: when n_extra > 0 every element of D is also stored to extra_d[i] (same
@@ -244,9 +245,9 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         }
         if (gathers) {
           if (p.a_mode != kLoadTma)
-            gather_tile<T, Tile::kM, kSub>(smem_u32(sa), p.A, p.lda, p.a_mode, m0, p.M, k0, p.K, p.pad_a, pw, lane);
+            gather_tile<T, Tile::kM, kSub>(smem_u32(sa), p.A, p.lda, p.a_mode, m0, p.M, k0, p.K, p.pad, p.repeat_k, pw, lane);
           if (p.b_mode != kLoadTma)
-            gather_tile<T, Tile::kN, kSub>(smem_u32(sb), p.B, p.ldb, p.b_mode, n0, p.N, k0, p.K, p.pad_b, pw, lane);
+            gather_tile<T, Tile::kN, kSub>(smem_u32(sb), p.B, p.ldb, p.b_mode, n0, p.N, k0, p.K, p.pad, p.repeat_k, pw, lane);
           if (k0 + kStep > p.K) {         // padding was written by ordinary stores: announce with an ordinary arrival
             cp_async_wait_all();
             mbar_arrive(&full_bar[s]);

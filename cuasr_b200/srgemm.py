@@ -36,6 +36,7 @@ _PACK_SCALAR = {DType.F32: struct.Struct("<f4x").pack, DType.F64: struct.Struct(
 # the layout of _lib.Args
 _PACK_ARGS = struct.Struct("4iQqQqQqQq8s8s8s8sQNQ").pack
 assert struct.calcsize("4iQqQqQqQq8s8s8s8sQNQ") == ctypes.sizeof(_lib.Args)
+_WRAPPED = (ctypes.c_int32, ctypes.c_int64, ctypes.c_size_t, ctypes.c_void_p)
 _STATUS = {int(st): st for st in Status}
 
 
@@ -105,10 +106,14 @@ class _Operator:
         (A, lda), (B, ldb), (C, ldc), (D, ldd) = args.ref_A, args.ref_B, args.ref_C, args.ref_D
         if workspace is not None and workspace_bytes == 0 and hasattr(workspace, "numel"):
             workspace_bytes = workspace.numel() * workspace.element_size()
-        return _lib.Args.from_buffer_copy(_PACK_ARGS(
-            int(m), int(n), int(k), int(args.split_k_slices), _ptr(A), int(lda), _ptr(B), int(ldb), _ptr(C), int(ldc),
-            _ptr(D), int(ldd), alpha, beta, add_identity, mul_identity, _ptr(workspace), int(workspace_bytes),
-            0 if stream is None else _stream_handle(stream)))
+        fields = (int(m), int(n), int(k), int(args.split_k_slices), _ptr(A), int(lda), _ptr(B), int(ldb), _ptr(C), int(ldc),
+                  _ptr(D), int(ldd), alpha, beta, add_identity, mul_identity, _ptr(workspace), int(workspace_bytes),
+                  0 if stream is None else _stream_handle(stream))
+        try:
+            return _lib.Args.from_buffer_copy(_PACK_ARGS(*fields))
+        except struct.error:                # a number its C field cannot hold: wrapped around, as ctypes assigns it
+            return _lib.Args(*(kind(v).value if kind in _WRAPPED else _lib.Scalar.from_buffer_copy(v)
+                               for v, (_, kind) in zip(fields, _lib.Args._fields_)))
 
     def _fn(self, base: str):
         name = "cuasr_b200_srgemm_splitk" if self._splitk_parallel else "cuasr_b200_srgemm"
