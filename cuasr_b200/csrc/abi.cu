@@ -364,11 +364,11 @@ RepackPlan repack_plan(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& a
 // ---- which tile, and how K is shared ---------------------------------------------------------------------------
 // Clocks the 8 consumer warps of a CTA (two per scheduler, 64 products per lane and k) take for one k: measured per
 // product and scheduler 2.07 (fp32 with a packed add and a three-input minimum, fused integer add-min, one logic
-// instruction), 3.0 (two-instruction bottleneck products), 6.5 (fp64 minima), 2.1 (fp64 sums on the tensor cores).
+// instruction), 3.0 (two-instruction bottleneck products), 8.2 (fp64 minima), 2.1 (fp64 sums on the tensor cores).
 double clocks_per_k(const cuasr_b200_desc_t& desc) {
   const bool sum = desc.add_op == CUASR_OP_PLUS;
   double per_product = 2.1;
-  if (desc.dtype == CUASR_F64) per_product = sum ? 2.1 : 6.5;
+  if (desc.dtype == CUASR_F64) per_product = sum ? 2.1 : 8.2;
   else if (desc.mul_op == CUASR_OP_MINIMUM || desc.mul_op == CUASR_OP_MAXIMUM) per_product = 3.0;
   else if (desc.mul_op == CUASR_OP_BINARY_AND) per_product = 5.0;
   return 2 * 64 * per_product;
@@ -427,15 +427,16 @@ struct ScreenPlan {
   int pieces = 1, blocks_per_piece = 0;
   double cost = 1e300;
 };
-// Modelled clocks.  Measured per product and scheduler: 3.0 with the tests, the conversions and the usual number of
-// recomputed elements; the first blocks of a tile, done exactly or with many recomputed elements, cost about as much
-// again as four exact blocks.
+// Modelled clocks: 3.7 per product and scheduler with the tests, the conversions and the usual number of recomputed
+// elements (1000 x 1000 x 3000 takes 250 us more than 1000^3 with 31 blocks more per CTA), and 400000 per tile or piece for
+// its first blocks, which are done exactly or with many recomputed elements.  So 2048^3 is screened (1.46 - 1.55 ms
+// against 1.90 exact) and 1000^3 is not (334 - 379 us against 276).
 ScreenPlan screen_plan(int m, int n, int k, int sms, bool may_split) {
   const int kb = 32;
   const int blocks = (k + kb - 1) / kb;
   const long long tiles = static_cast<long long>((m + kTileM - 1) / kTileM) * ((n + kTileN - 1) / kTileN);
-  const double per_block = 128.0 * kb * 3.0;
-  const double first = 128.0 * kb * 4 * 6.5;
+  const double per_block = 128.0 * kb * 3.7;
+  const double first = 400000;
   ScreenPlan best;
   for (int pieces = 1; pieces <= (may_split ? 128 : 1) && pieces <= blocks; ++pieces) {
     const int per_piece = (blocks + pieces - 1) / pieces;

@@ -7,13 +7,17 @@
 // sum of two such numbers is never worse than the exact sum, and one fused packed add-min instruction handles two
 // products in 2 clocks (measured 1.08 per product with its shared-memory reads).  A block of k whose 16-bit sums
 // cannot beat the element's current value cannot contain an improvement and is done; the few (element, block) pairs
-// that might improve are recomputed exactly, by eight lanes each, from the exact tile in shared memory.  The result is
+// that might improve are recomputed exactly, by four lanes each, from the exact tile in shared memory.  The result is
 // bit for bit that of the exact computation: the screen only ever lets too much through.
 //
 // Fixed point: q(x) = floor(x * 2^e) (ceil for max), finite values at most 16382, +inf (-inf for max) = 32767 (-16384),
 // so sums of finite values and sums with an infinity do not overlap.  2^e comes from the largest finite value of the
 // tiles seen so far.  A stage with a negative or too large finite value is "unfit" and done exactly; a larger 2^-e
 // follows for the next.
+//
+// What the screen saves depends on the data (4096^3, 12.3 ms before it, 14.4 with the exact kernel of srgemm_tma.cuh): sparse
+// edges 7.7 ms, uniform values 8.0, small whole numbers 4.7, sums that improve along k 7.5; values it cannot hold, negative
+// ones or magnitudes over hundreds of decades, are done exactly in runs of blocks, 18.5.
 //
 // The running result lives in D itself: an element is written when it improves, by the lane that found it.  Elements
 // and blocks are independent of order, so K may be cut into pieces for different CTAs, which then meet in D by
@@ -49,6 +53,7 @@ template <typename T>
 constexpr int kScreenStageBytes = kScreenExactBytes + 2 * 128 * (256 / (int)sizeof(T)) * 2;
 constexpr int kScreenStages = 2;
 constexpr int kScreenBoundBytes = 8 * 64 * 32 * 2;   // per warp, element and lane: the value a 16-bit sum has to beat
+constexpr int kListGroups = 4;                       // groups of eight elements that a warp recomputes at a time
 constexpr int kListed = 96;                          // elements to recompute that a warp lists at a time
 constexpr int kScreenListBytes = 8 * kListed * 2;
 template <typename T>
@@ -108,19 +113,24 @@ struct Screen {
     return kMax ? __viaddmax_s16x2(a, b, acc) : __viaddmin_u16x2(a, b, acc);
   }
   // The bound of an element with current value v: a 16-bit sum may stand for an improvement only if it is below
-  // (min) or above (max) it.  min: exact sum < v implies floor sums <= floor(v * s).
+  // (min) or above (max) it.  min: exact sum < v implies (sum of floors) < v * s, i.e. < ceil(v * s); the product is
+  // rounded up, so that it only ever gets larger where it is inexact.
   template <typename T>
-  static __device__ __forceinline__ uint32_t bound(T v, T scale) {
-    const T y = v * scale;
+  static __device__ __forceinline__ uint32_t bound(T v, float scale) {
+    const T y = rescaled(v, scale);
     if (y != y) return kNothing;                                        // a NaN (from C) stays: nothing is better than it
     if (kMax) {
       if (!(y >= T(0))) return (uint32_t)(uint16_t)-1;                  // any sum of finite values
       if (y >= T(32766)) return 32766u;
-      return (uint32_t)(uint16_t)((int)ceil(y) - 1);
+      return (uint32_t)(int)y;
     }
     if (!(y < T(32766))) return 32767u;                                 // any sum of finite values
     if (y < T(0)) return 0u;                                            // nothing: no negative values in a fit stage
-    return (uint32_t)((int)floor(y) + 1);
+    return (uint32_t)(int)ceil(y);
+  }
+  static __device__ __forceinline__ float rescaled(float v, float scale) { return kMax ? __fmul_rd(v, scale) : __fmul_ru(v, scale); }
+  static __device__ __forceinline__ double rescaled(double v, float scale) {
+    return kMax ? __dmul_rd(v, (double)scale) : __dmul_ru(v, (double)scale);
   }
   static __device__ __forceinline__ bool sooner(uint32_t a, uint32_t b) { return kMax ? (int16_t)a > (int16_t)b : a < b; }
   template <typename T>
@@ -175,9 +185,10 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   constexpr int kCoarseChunks = kCoarseRow / 16;    // 8 or 4 chunks of 8 k
   constexpr int kExactOperand = 32768, kColumn = 16384;
   constexpr int kCoarseOperand = 128 * kCoarseRow;
-  // elements of a warp (of 2048) above which recomputing them one by one costs more than the whole block: about 9 clocks
-  // each against the difference between the exact and the screened block
-  constexpr int kExactAbove = sizeof(T) == 8 ? 1200 : 400;
+  // Elements of a warp (of 2048) above which recomputing them one by one costs more than doing the block exactly, and how
+  // many blocks are then done exactly: two, and twice as many each time the next block screened is no better.
+  // (4096^3: 8.15 ms with 350 elements on uniform data and 8.25 on sparse edges, 7.98 and 7.68 with 600, 8.21 and 7.66 with 1000)
+  constexpr int kExactAbove = 600, kPatience = 2, kMaxPatience = 256;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -189,7 +200,9 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   // per stage: largest and smallest finite scaled value seen by each producer warp, and the exponent
   volatile float* range = reinterpret_cast<volatile float*>(empty_bar + kScreenStages);   // [stage][warp][2]
   volatile int* stage_exp = reinterpret_cast<volatile int*>(range + kScreenStages * kProducerWarps * 2);
-  volatile unsigned int* abandoned = reinterpret_cast<volatile unsigned int*>(stage_exp + kScreenStages);
+  // per consumer warp: it does the blocks before this one (counted over the CTA's whole work) exactly
+  volatile int* exact_until = stage_exp + kScreenStages;
+  volatile unsigned int* abandoned = reinterpret_cast<volatile unsigned int*>(exact_until + kConsumerWarps);
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const bool gathers = p.a_mode != kLoadTma || p.b_mode != kLoadTma;
@@ -201,6 +214,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       mbar_init(&empty_bar[s], kConsumerWarps);
     }
     *abandoned = 0;
+    for (int v = 0; v < kConsumerWarps; ++v) exact_until[v] = 0;
     fence_barrier_init();
   }
   __syncthreads();
@@ -295,6 +309,19 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       const uint32_t exact = smem_u32(smem + s * kScreenStageBytes<T>);
       const uint32_t coarse = exact + kScreenExactBytes;
       const int k_left = p.K - (s == 0 ? k0_even : k0_odd);          // below KB in the block that reaches beyond K
+      // No 16-bit tile for a block that all consumers do exactly (what they promise, they keep).
+      bool wanted = false;
+#pragma unroll
+      for (int v = 0; v < kConsumerWarps; ++v) wanted |= exact_until[v] <= (int)it;
+      if (producers_agree(!wanted)) {
+        if (lane == 0) {
+          range[(s * kProducerWarps + pw) * 2] = INFINITY;            // unfit
+          if (pw == 0) stage_exp[s] = exponent;
+        }
+        mbar_arrive(&ready_bar[s]);
+        if (lw < num_work) load_next();
+        continue;
+      }
       // Two passes where the scale has to be found first (the first stage of the CTA), one otherwise.
       for (int pass = have_exponent ? 1 : 0; pass < 2; ++pass) {     // (uniform: all producers saw the same ranges)
         const float scale = __int_as_float((exponent + 127) << 23);
@@ -390,25 +417,26 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   const bool shared_d = p.pieces > 1;
 
   uint32_t it = 0;
+  int until = 0, patience = kPatience;      // blocks before `until` are done exactly; length of the next such run
+  auto do_exactly = [&](uint32_t from, int blocks) {
+    until = max(until, (int)from + blocks);
+    if (lane == 0) exact_until[warp] = until;
+  };
   for (int w = blockIdx.x; w < num_work; w += gridDim.x) {
     const int piece = w / tiles, tile = w - piece * tiles;
     int tm, tn;
     tile_coords(tile, p.tiles_m, p.tiles_n, tm, tn);
     const int begin = piece * p.blocks_per_piece;
     const int count = min(blocks_total - begin, p.blocks_per_piece);
-    const int stride = stride_of(count);
     const int m_base = tm * 128 + wm * 64, n_base = tn * 128 + wn * 32;
     int my_exp = 1 << 30;             // exponent the bounds were made with
-    int pos = 0;
-    int exact_left = 1;               // blocks to do exactly before the screen is worth its tests
     bool opened = false;              // D holds the running values of this tile
+    do_exactly(it, 1);                // the first block has nothing to be screened against
 
-    for (int b = 0; b < count; ++b, ++it) {
+    for (int b = 0; b < count;) {
       const int s = it % kScreenStages;
       mbar_wait_or_abandon(&ready_bar[s], (it / kScreenStages) & 1, p.status, kDeviceTimeoutFull, abandoned);
       mbar_wait_or_abandon(&full_bar[s], (it / kScreenStages) & 1, p.status, kDeviceTimeoutFull, abandoned);
-      const uint32_t exact = smem_base + s * kScreenStageBytes<T>;
-      const uint32_t coarse = exact + kScreenExactBytes;
       float top = -INFINITY, low = INFINITY;
 #pragma unroll
       for (int v = 0; v < kProducerWarps; ++v) {
@@ -416,44 +444,63 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         low = fminf(low, range[(s * kProducerWarps + v) * 2 + 1]);
       }
       const int exponent = stage_exp[s];
+      const float scale = __int_as_float((exponent + 127) << 23);
       const bool unfit = top > S::kFiniteLimit || low < 0.0f;
-      const T scale = (T)__int_as_float((exponent + 127) << 23);
-      pos += stride;
-      if (pos >= count) pos -= count;
 
-      if (unfit || exact_left > 0) {
-        // ---- the whole block exactly, for all 64 elements of the lane; then merged into D
+      if (unfit || (int)it < until) {
+        if (unfit && (int)it >= until) {
+          do_exactly(it, patience);
+          patience = min(2 * patience, kMaxPatience);
+        }
+        // ---- a run of whole blocks exactly, for all 64 elements of the lane; then merged into D
         T acc[8][8];
 #pragma unroll
         for (int i = 0; i < 8; ++i)
 #pragma unroll
           for (int j = 0; j < 8; ++j) acc[i][j] = p.add_identity;
-        const uint32_t a_base = exact + (wm * 64 + lr) * 128, b_base = exact + kExactOperand + (wn * 32 + lc) * 128;
+        for (;;) {
+          const int sx = it % kScreenStages;
+          const uint32_t exact = smem_base + sx * kScreenStageBytes<T>;
+          const uint32_t a_base = exact + (wm * 64 + lr) * 128, b_base = exact + kExactOperand + (wn * 32 + lc) * 128;
 #pragma unroll 1
-        for (int chunk = 0; chunk < 16; ++chunk) {
-          const uint32_t column = (chunk >> 3) * kColumn;
-          const uint32_t ab = a_base + column + (((chunk ^ lr) & 7) << 4);
-          const uint32_t b0 = b_base + column + (((chunk ^ lc) & 7) << 4), b1 = b_base + column + (((chunk ^ (lc + 4)) & 7) << 4);
-          T a[8][EV], bb[8][EV];
+          for (int chunk = 0; chunk < 16; ++chunk) {
+            const uint32_t at = (chunk >> 3) * kColumn;
+            const uint32_t ab = a_base + at + (((chunk ^ lr) & 7) << 4);
+            const uint32_t b0 = b_base + at + (((chunk ^ lc) & 7) << 4), b1 = b_base + at + (((chunk ^ (lc + 4)) & 7) << 4);
+            T a[8][EV];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) lds16(ab + i * 1024, a[i]);
+            for (int i = 0; i < 8; ++i) lds16(ab + i * 1024, a[i]);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) lds16(((j & 1) ? b1 : b0) + j * 512, bb[j]);
+            for (int j = 0; j < 8; ++j) {
+              T bj[EV];
+              lds16(((j & 1) ? b1 : b0) + j * 512, bj);
 #pragma unroll
-          for (int e = 0; e < EV; e += 2)
+              for (int e = 0; e < EV; e += 2)
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                if constexpr (RingT::kPackedPairs)
-                  acc[i][j] = RingT::mac_packed(acc[i][j], pack2(a[i][e], a[i][e + 1]), pack2(bb[j][e], bb[j][e + 1]));
-                else
-                  acc[i][j] = RingT::mac2(acc[i][j], a[i][e], bb[j][e], a[i][e + 1], bb[j][e + 1]);
-              }
+                for (int i = 0; i < 8; ++i) acc[i][j] = RingT::mac2(acc[i][j], a[i][e], bj[e], a[i][e + 1], bj[e + 1]);
+            }
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&empty_bar[sx]);
+          ++it;
+          if (++b == count || (int)it >= until) break;
+          // (the 16-bit tile of the next block is not waited for)
+          mbar_wait_or_abandon(&full_bar[it % kScreenStages], (it / kScreenStages) & 1, p.status, kDeviceTimeoutFull, abandoned);
         }
+        // (the opaque zero: the addresses are computed here instead of being carried through the contraction)
+        int zero;
+        asm volatile("mov.s32 %0, 0;" : "=r"(zero));
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const int m = m_base + lr + 8 * i;
+          const int m = m_base + lr + 8 * i + zero;
+          T cur[8];                      // a row's loads together: none of them can pass a store
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const int n = n_base + lc + 4 * j;
+            if (m >= p.M || n >= p.N) continue;
+            if (shared_d || opened) cur[j] = __ldcg(p.D + (long long)m * p.ldd + n);   // improved at the L2 by other lanes
+            else if (p.read_c) cur[j] = p.C[(long long)m * p.ldc + n];
+          }
           uint32_t q[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
@@ -463,13 +510,14 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             if (inside) {
               T* at = p.D + (long long)m * p.ldd + n;
               if (shared_d) {
-                v = improve_shared<kMax>(at, v, __ldcg(at));
+                if (!S::better(v, cur[j])) v = cur[j];
+                else if (v >= T(0)) merge_into<kMax>(at, v);       // without waiting for the answer
+                else v = improve_shared<kMax>(at, v, cur[j]);
               } else if (opened) {
-                const T cur = __ldcg(at);                          // lanes of this warp improve it at the L2
-                if (S::better(v, cur)) *at = v;
-                else v = cur;
+                if (S::better(v, cur[j])) *at = v;
+                else v = cur[j];
               } else {
-                if (p.read_c) v = RingT::add(v, RingT::mul(p.beta, p.C[(long long)m * p.ldc + n]));
+                if (p.read_c) v = RingT::add(v, RingT::mul(p.beta, cur[j]));
                 *at = v;
               }
             }
@@ -479,11 +527,11 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         }
         opened = true;
         my_exp = exponent;
-        if (exact_left > 0) --exact_left;
         __syncwarp();
-        if (lane == 0) mbar_arrive(&empty_bar[s]);
         continue;
       }
+      const uint32_t exact = smem_base + s * kScreenStageBytes<T>;
+      const uint32_t coarse = exact + kScreenExactBytes;
 
       if (my_exp != exponent) {
         // bounds at this stage's scale, from the running values
@@ -505,17 +553,17 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       uint32_t mask_lo = 0, mask_hi = 0;              // bit 8 i + j: element (i, j) might improve in this block
       {
         // ---- the screen: two products per instruction
-        uint32_t bound[8][8], q[8][8];
+        uint32_t q[8][8];
+        // row i of the lane's bounds, each in both halves of a word; read again after the contraction, which has no
+        // registers for them
+        auto bounds = [&](int i, uint32_t (&v)[8]) {
+          const uint4 x = lds16u(my_bounds + i * 512);
+          const uint32_t packed[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const uint4 v = lds16u(my_bounds + i * 512);
-          const uint32_t packed[4] = {v.x, v.y, v.z, v.w};
+          for (int j = 0; j < 8; ++j) v[j] = __byte_perm(packed[j >> 1], 0, (j & 1) ? 0x3232 : 0x1010);
+        };
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            bound[i][j] = __byte_perm(packed[j >> 1], 0, (j & 1) ? 0x3232 : 0x1010);
-            q[i][j] = bound[i][j];
-          }
-        }
+        for (int i = 0; i < 8; ++i) bounds(i, q[i]);
         const uint32_t qa = coarse + (wm * 64 + lr) * kCoarseRow, qb = coarse + kCoarseOperand + (wn * 32 + lc) * kCoarseRow;
 #pragma unroll 2
         for (int c = 0; c < kCoarseChunks; ++c) {
@@ -543,13 +591,16 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             }
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < 8; ++i) {
+          uint32_t bound[8];
+          bounds(i, bound);
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            if (q[i][j] != bound[i][j]) {
+            if (q[i][j] != bound[j]) {
               if (i < 4) mask_lo |= 1u << (8 * i + j);
               else       mask_hi |= 1u << (8 * (i - 4) + j);
             }
+        }
       }
       // ---- exact values of the elements that might improve, four lanes each, listed kListed at a time
       const int mine = __popc(mask_lo) + __popc(mask_hi);
@@ -561,7 +612,12 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       }
       const int total = __shfl_sync(~0u, slot_of_next, 31);
       slot_of_next -= mine;
-      if (total > kExactAbove) exact_left = 3;
+      if (total > kExactAbove) {        // this block and the next ones exactly
+        do_exactly(it, patience);
+        patience = min(2 * patience, kMaxPatience);
+        continue;
+      }
+      patience = kPatience;
       for (int first = 0; first < total; first += kListed) {
         while (slot_of_next < first + kListed && (mask_lo | mask_hi) != 0) {
           int bit;
@@ -573,12 +629,12 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         __syncwarp();
         const int listed = min(kListed, total - first);
         const int t = lane & 3;
-        for (int base = 0; base < listed; base += 16) {
-          // two groups of eight elements, so that their loads and exchanges overlap
-          T best[2];
-          int code[2];
+        for (int base = 0; base < listed; base += 8 * kListGroups) {
+          // groups of eight elements, so that their loads and exchanges overlap
+          T best[kListGroups];
+          int code[kListGroups];
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
+          for (int u = 0; u < kListGroups; ++u) {
             const int slot = base + u * 8 + (lane >> 2);
             code[u] = lds2(list + 2 * (slot < listed ? slot : base));
             const int el = code[u] >> 6, i = (code[u] >> 3) & 7, j = code[u] & 7;
@@ -603,13 +659,13 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 #pragma unroll
           for (int d = 2; d > 0; d >>= 1) {
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
+            for (int u = 0; u < kListGroups; ++u) {
               const T other = __shfl_xor_sync(~0u, best[u], d);
               best[u] = RingT::add(other, best[u]);
             }
           }
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
+          for (int u = 0; u < kListGroups; ++u) {
             const int el = code[u] >> 6, i = (code[u] >> 3) & 7, j = code[u] & 7;
             const int m = m_base + (el >> 2) + 8 * i, n = n_base + (el & 3) + 4 * j;
             if (t == u && base + u * 8 + (lane >> 2) < listed && m < p.M && n < p.N) {
@@ -631,6 +687,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty_bar[s]);
+      ++b; ++it;
     }
     // further copies of the finished tile (pieces == 1)
     if (p.n_extra > 0) {
