@@ -184,7 +184,7 @@ int validate(const cuasr_b200_desc_t* desc, const cuasr_b200_args_t* args) {
   // alias it) that would be a race, so it is refused.  A and B are only read: the reference never looks at their
   // leading dimensions (its own examples/02_splitk_srgemm/splitk_srgemm.cu:247-248 passes 128 for a row-major
   // 128 x 4096 operand), and an overlapping view is well defined, so any positive value is accepted; such views
-  // run on the generic kernel.
+  // are gathered.
   const long long c_min = desc->layout_c == CUASR_ROW_MAJOR ? args->n : args->m;
   if (args->lda < 1 || args->ldb < 1 || args->ldd < c_min) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
   if (args->C != nullptr && args->ldc < c_min) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
@@ -338,28 +338,6 @@ bool ring_pads_itself(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& ar
   }
   return false;
 }
-// Every other ring (the integer min/max rings) has no value TMA could fill in.  With the optional workspace both
-// operands are copied and their K range is extended to a whole number of K steps: A with the additive identity, B
-// with the multiplicative one, so that every padded product is the additive identity.
-RepackPlan repack_plan(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, const Normalised& p) {
-  RepackPlan plan;
-  const size_t es = desc.dtype == CUASR_F64 ? 8 : 4;
-  // not for storage lines that overlap, nor for small products: up to about 128^3 the copy's launch costs as much as
-  // the product itself, which gathers its operands just as well
-  if (static_cast<double>(p.m) * p.n * p.k < 128.0 * 128 * 128 || static_cast<long long>(p.m) * p.n < 64 * 64) return plan;
-  if (p.lda < (p.a_kcontig ? p.k : p.m) || p.ldb < (p.b_kcontig ? p.k : p.n)) return plan;
-  const int tk = kTileKBytes / static_cast<int>(es);
-  if (p.k % tk != 0 && !ring_pads_itself(desc, args)) {
-    plan.a = plan.b = true;
-    plan.k_padded = (p.k + 2 * tk - 1) / (2 * tk) * (2 * tk);     // the longest K step of a tile (rings without padding)
-  } else {
-    plan.a = !tma_describable(p.a, p.lda, es);
-    plan.b = !tma_describable(p.b, p.ldb, es);
-  }
-  const int k_copy = plan.k_padded > 0 ? plan.k_padded : p.k;
-  plan.bytes = (plan.a ? repack_operand_bytes(p.m, k_copy, es) : 0) + (plan.b ? repack_operand_bytes(p.n, k_copy, es) : 0);
-  return plan;
-}
 
 // ---- which tile, and how K is shared ---------------------------------------------------------------------------
 // Clocks the 8 consumer warps of a CTA (two per scheduler, 64 products per lane and k) take for one k: measured per
@@ -394,8 +372,17 @@ int tile_sub(int tile, const cuasr_b200_desc_t& desc) {
 // operands 3000, then per wave of CTAs the contraction (above) and the tile's end (2000 for the large tile, 1500 for the
 // fold of the small ones, twice that for 8-byte elements), 2500 for the exchange inside a cluster.  Clusters of four
 // and eight do not fill every SM (a cluster lives in one GPC): 144 and 128 of the 148.
-// A gathered element costs 0.17 clocks on the small tiles (2048^3 with both operands transposed on 64 x 64 tiles takes
-// 694 us against 519 with TMA) and 0.07 on the large one (4096^3: 4.30 ms against 3.97).
+// A cluster launch is not persistent: each further wave starts its CTAs anew, 4000.  The 64 x 32 tile hands a stage over
+// for every chunk of a warp: 250 clocks a stage (a 512 x 4096 x 4096 product as seven waves of it took 635 us instead of
+// the 514 modelled without; the 128 x 128 tile takes 580).
+// A gathered element costs 0.17 clocks on the small tiles where the contraction is bound by register reads (2048^3
+// min-plus with one operand transposed on 64 x 64 tiles: 589 us against 522 with TMA), 0.08 in the other rings (max-min:
+// 795 against 765), and 0.07 and 0.02 on the large one (4096^3: 3998 against 3969, both operands 4096).
+double gather_clocks(const cuasr_b200_desc_t& desc, bool large) {
+  const bool packed = desc.dtype == CUASR_F32 && (desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM) &&
+                      (desc.mul_op == CUASR_OP_PLUS || desc.mul_op == CUASR_OP_MULTIPLIES);
+  return packed ? (large ? 0.07 : 0.17) : (large ? 0.02 : 0.08);
+}
 LaunchPlan plan_without_workspace(const cuasr_b200_desc_t& desc, int m, int n, int k, int sms, bool all_tiles, bool gather_a,
                                   bool gather_b) {
   const int tk = kTileKBytes / (desc.dtype == CUASR_F64 ? 8 : 4);
@@ -410,9 +397,9 @@ LaunchPlan plan_without_workspace(const cuasr_b200_desc_t& desc, int m, int n, i
       if ((z - 1) * per_piece >= k_steps) break;                        // every CTA of a cluster has work
       const long long room = z <= 2 ? sms : z == 4 ? sms * 36LL / 37 : sms * 32LL / 37;
       const long long waves = (tiles * z + room - 1) / room;
-      const double end = (tile == kLargeTile ? 2000 : 1500) * wide + (z > 1 ? 2500 : 0);
-      const double gathered = (tile == kLargeTile ? 0.07 : 0.17) * step * ((gather_a ? kTileRows[tile] : 0) + (gather_b ? kTileCols[tile] : 0));
-      const double per_stage = per_k * step / kTileWk[tile] + gathered;
+      const double end = (tile == kLargeTile ? 2000 : 1500) * wide + (z > 1 ? 2500 + (waves > 1 ? 4000 : 0) : 0);
+      const double gathered = gather_clocks(desc, tile == kLargeTile) * step * ((gather_a ? kTileRows[tile] : 0) + (gather_b ? kTileCols[tile] : 0));
+      const double per_stage = per_k * step / kTileWk[tile] + gathered + (tile == kTinyTile ? 250 : 0);
       const double cost = 3000 + static_cast<double>(waves) * (per_stage * per_piece + end);
       if (cost < best.cost) {
         best.tile = tile; best.cluster = z; best.cost = cost;
@@ -422,6 +409,59 @@ LaunchPlan plan_without_workspace(const cuasr_b200_desc_t& desc, int m, int n, i
   }
   return best;
 }
+template <typename T>
+bool ring_has_all_tiles(const cuasr_b200_desc_t& desc) {
+#define X(ADD, MUL) if (desc.add_op == ADD && desc.mul_op == MUL) return all_tiles_instantiated<ADD, MUL, T>();
+  CUASR_FLOAT_RINGS(X)
+  if constexpr (std::is_integral<T>::value) { CUASR_BIT_RINGS(X) }
+#undef X
+  return false;
+}
+
+bool has_all_tiles(const cuasr_b200_desc_t& desc) {
+  switch (desc.dtype) {
+    case CUASR_F32: return ring_has_all_tiles<float>(desc);
+    case CUASR_F64: return ring_has_all_tiles<double>(desc);
+    case CUASR_S32: return ring_has_all_tiles<int32_t>(desc);
+    default:        return ring_has_all_tiles<uint32_t>(desc);
+  }
+}
+
+// Every other ring (the integer min/max rings) has no value TMA could fill in.  With the optional workspace both
+// operands are copied and their K range is extended to a whole number of K steps: A with the additive identity, B
+// with the multiplicative one, so that every padded product is the additive identity.
+// An operand that lies along its rows is copied, transposed, where that makes the modelled launch faster by more than the
+// copy takes (4000 clocks for its launch, 2200 bytes per clock): 2048^3 min-plus with one such operand 589 us gathered,
+// 538 copied; 4096^3 3998 and 4007.
+RepackPlan repack_plan(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, const Normalised& p, int sms) {
+  RepackPlan plan;
+  const size_t es = desc.dtype == CUASR_F64 ? 8 : 4;
+  // not for storage lines that overlap, nor for small products: up to about 128^3 the copy's launch costs as much as
+  // the product itself, which gathers its operands just as well
+  if (static_cast<double>(p.m) * p.n * p.k < 128.0 * 128 * 128 || static_cast<long long>(p.m) * p.n < 64 * 64) return plan;
+  if (p.lda < (p.a_kcontig ? p.k : p.m) || p.ldb < (p.b_kcontig ? p.k : p.n)) return plan;
+  const int tk = kTileKBytes / static_cast<int>(es);
+  if (p.k % tk != 0 && !ring_pads_itself(desc, args)) {
+    plan.a = plan.b = true;
+    plan.k_padded = (p.k + 2 * tk - 1) / (2 * tk) * (2 * tk);     // the longest K step of a tile (rings without padding)
+  } else {
+    plan.a = !tma_describable(p.a, p.lda, es);
+    plan.b = !tma_describable(p.b, p.ldb, es);
+    const bool all_tiles = has_all_tiles(desc);
+    auto cost = [&](bool gather_a, bool gather_b) {
+      return plan_without_workspace(desc, p.m, p.n, p.k, sms, all_tiles, gather_a, gather_b).cost;
+    };
+    auto copy = [&](bool first, int rows) { return (first ? 4000.0 : 0.0) + 2.0 * es * rows * p.k / 2200; };
+    const bool along_a = !p.a_kcontig && !plan.a, along_b = !p.b_kcontig && !plan.b;
+    if (along_a && cost(true, along_b) - cost(false, along_b) > copy(!plan.b, p.m)) plan.a = true;
+    const bool gather_a = along_a && !plan.a;
+    if (along_b && cost(gather_a, true) - cost(gather_a, false) > copy(!plan.a, p.n)) plan.b = true;
+  }
+  const int k_copy = plan.k_padded > 0 ? plan.k_padded : p.k;
+  plan.bytes = (plan.a ? repack_operand_bytes(p.m, k_copy, es) : 0) + (plan.b ? repack_operand_bytes(p.n, k_copy, es) : 0);
+  return plan;
+}
+
 // ---- the screened kernel (srgemm_screened.cuh) -------------------------------------------------------------------
 struct ScreenPlan {
   int pieces = 1, blocks_per_piece = 0;
@@ -449,11 +489,11 @@ ScreenPlan screen_plan(int m, int n, int k, int sms, bool may_split) {
 }
 
 // Modelled clocks of a launch of large tiles whose pieces meet through tickets in a workspace.
-double ticket_plan_cost(const cuasr_b200_desc_t& desc, long long tiles, int whole_tiles, int pieces, int k, int sms) {
+double ticket_plan_cost(const cuasr_b200_desc_t& desc, long long tiles, int whole_tiles, int pieces, int k, int sms, int gathered) {
   const int tk = kTileKBytes / (desc.dtype == CUASR_F64 ? 8 : 4);
   const double wide = desc.dtype == CUASR_F64 ? 2.0 : 1.0;
   const int k_steps = (k + tk - 1) / tk, per_piece = (k_steps + pieces - 1) / pieces;
-  const double per_step = clocks_per_k(desc) * tk;
+  const double per_step = (clocks_per_k(desc) + gather_clocks(desc, true) * kTileM * gathered) * tk;
   const long long waves = whole_tiles / sms, tail = ((tiles - whole_tiles) * pieces + sms - 1) / sms;
   // the tickets are cleared by a memset in front of the launch; a piece is parked and read back by the last one
   return 3000 + 4000 + waves * (per_step * k_steps + 2000 * wide) + tail * (per_step * per_piece + 1000 * wide) + 1000 * wide * pieces;
@@ -552,15 +592,6 @@ int run_path(bool maximize, const Normalised& p, int32_t* parent, long long ld_p
 }
 
 template <typename T>
-bool ring_has_all_tiles(const cuasr_b200_desc_t& desc) {
-#define X(ADD, MUL) if (desc.add_op == ADD && desc.mul_op == MUL) return all_tiles_instantiated<ADD, MUL, T>();
-  CUASR_FLOAT_RINGS(X)
-  if constexpr (std::is_integral<T>::value) { CUASR_BIT_RINGS(X) }
-#undef X
-  return false;
-}
-
-template <typename T>
 int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int slices, const ExtraOutputs& extra) {
   DeviceState* dev = nullptr;
   if (!device_state(&dev)) return CUASR_STATUS_ERROR_INTERNAL;
@@ -572,22 +603,31 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   // semiring_linear_combination.h:118-125: C is read unless mult(beta, mult-identity) is the add-identity
   const bool read_c = !(host_op<T>(desc.mul_op, beta, mul_id) == add_id);
 
-  constexpr int TK = kTileKBytes / sizeof(T);
-  const long long tiles = static_cast<long long>(tile_count(args));
-  const bool all_tiles = ring_has_all_tiles<T>(desc);
-  LaunchPlan plan = plan_without_workspace(desc, p.m, p.n, p.k, dev->sms, all_tiles,
-                                           !p.a_kcontig || !tma_describable(p.a, p.lda, sizeof(T)),
-                                           !p.b_kcontig || !tma_describable(p.b, p.ldb, sizeof(T)));
-  bool tickets_used = false, balanced = false;
+  if (slices > 1 && args.workspace == nullptr) return CUASR_STATUS_ERROR_WORKSPACE_NULL;
+  if (read_c && p.c == nullptr) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
   // partials are moved 16 bytes at a time and re-packed operands are read by TMA: a workspace that does not start
   // on a 16-byte boundary is an error where it is required and is left unused where it is optional
   const bool workspace_aligned = reinterpret_cast<uintptr_t>(args.workspace) % 16 == 0;
+  // the copies an optional workspace has room for, behind the scratch of a balanced launch
+  RepackPlan copies;
+  size_t copies_at = 0;
+  if (slices == 1 && args.workspace != nullptr && workspace_aligned) {
+    copies = repack_plan(desc, args, p, dev->sms);
+    copies_at = align_up(balance_workspace_bytes(desc, args, dev->sms), 256);
+    if (copies.bytes == 0 || args.workspace_bytes < copies_at + copies.bytes) copies = RepackPlan();
+  }
+
+  constexpr int TK = kTileKBytes / sizeof(T);
+  const long long tiles = static_cast<long long>(tile_count(args));
+  const bool all_tiles = ring_has_all_tiles<T>(desc);
+  const bool gather_a = !copies.a && (!p.a_kcontig || !tma_describable(p.a, p.lda, sizeof(T)));
+  const bool gather_b = !copies.b && (!p.b_kcontig || !tma_describable(p.b, p.ldb, sizeof(T)));
+  LaunchPlan plan = plan_without_workspace(desc, p.m, p.n, p.k, dev->sms, all_tiles, gather_a, gather_b);
+  bool tickets_used = false, balanced = false;
   auto take_ticket_plan = [&](int whole_tiles, int pieces, double cost) {
     plan.tile = kLargeTile; plan.cluster = 1; plan.whole_tiles = whole_tiles; plan.pieces = pieces; plan.cost = cost;
     tickets_used = true;
   };
-  if (slices > 1 && args.workspace == nullptr) return CUASR_STATUS_ERROR_WORKSPACE_NULL;
-  if (read_c && p.c == nullptr) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
   if (slices > 1) {
     const size_t need = splitk_workspace_bytes(desc, args);
     if (args.workspace_bytes < need) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
@@ -598,7 +638,7 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
       const size_t per_piece = splitk_bytes_for_pieces(desc, args, 1) - splitk_bytes_for_pieces(desc, args, 0);
       const long long room = static_cast<long long>((args.workspace_bytes - splitk_bytes_for_pieces(desc, args, 0)) / per_piece);
       const int pieces = static_cast<int>(splitk_pieces(desc, args, dev->sms, room));
-      const double cost = ticket_plan_cost(desc, tiles, 0, pieces, p.k, dev->sms);
+      const double cost = ticket_plan_cost(desc, tiles, 0, pieces, p.k, dev->sms, gather_a + gather_b);
       if (cost < plan.cost || !splitk_order_independent(desc)) take_ticket_plan(0, pieces, cost);
     }
   } else if (args.workspace != nullptr && workspace_aligned && all_tiles) {
@@ -606,7 +646,7 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
     const BalancePlan wish = balance_plan(tiles, dev->sms, (args.k + TK - 1) / TK);
     if (wish.pieces > 1 && args.workspace_bytes >= balance_workspace_bytes(desc, args, dev->sms)) {
       balanced = true;
-      const double cost = ticket_plan_cost(desc, tiles, wish.whole_tiles, wish.pieces, p.k, dev->sms);
+      const double cost = ticket_plan_cost(desc, tiles, wish.whole_tiles, wish.pieces, p.k, dev->sms, gather_a + gather_b);
       if (cost < plan.cost) take_ticket_plan(wish.whole_tiles, wish.pieces, cost);
     }
   }
@@ -614,58 +654,48 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   // operands whose storage lines overlap (leading dimension below the contiguous extent) stay off the TMA path
   const bool dense = p.lda >= (p.a_kcontig ? p.k : p.m) && p.ldb >= (p.b_kcontig ? p.k : p.n);
   const bool small = static_cast<long long>(p.m) * p.n < 64 * 64;
+  // the rest of an optional workspace holds K-contiguous, aligned copies of operands (see RepackPlan)
+  const bool repacked = copies.bytes > 0;
+  int k_map = p.k;              // K extent the tensor maps describe
+  if (repacked) {
+    char* cursor = static_cast<char*>(args.workspace) + copies_at;
+    k_map = copies.k_padded > 0 ? copies.k_padded : p.k;
+    const long long ldt = static_cast<long long>(align_up(static_cast<size_t>(k_map), 16 / sizeof(T)));
+    unsigned long long pad_a = 0, pad_b = 0;
+    std::memcpy(&pad_a, &add_id, sizeof(T));
+    std::memcpy(&pad_b, &mul_id, sizeof(T));
+    RepackRequest requests[2];
+    int count = 0;
+    if (copies.a) {
+      requests[count++] = {p.a, p.lda, p.a_kcontig, p.m, p.k, k_map, pad_a, cursor, ldt};
+      p.a = cursor; p.lda = ldt; p.a_kcontig = true;
+      cursor += repack_operand_bytes(p.m, k_map, sizeof(T));
+    }
+    if (copies.b) {
+      requests[count++] = {p.b, p.ldb, p.b_kcontig, p.n, p.k, k_map, pad_b, cursor, ldt};
+      p.b = cursor; p.ldb = ldt; p.b_kcontig = true;
+    }
+    if (launch_repack(requests, count, sizeof(T), stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
+    g_launches.fetch_add(1);
+  }
+
+  const bool describable = tma_describable(p.a, p.lda, sizeof(T)) && tma_describable(p.b, p.ldb, sizeof(T));
+  // the name a caller sees: "tma..." where the storage lines are what TMA could describe
+  const bool aligned_name = (pads_itself || k_map % TK == 0) && !small && dense && describable;
+  const char* const name = !aligned_name ? (slices > 1 ? "generic_splitk" : "generic")
+                           : slices > 1 ? "tma_splitk" : balanced ? "tma_balanced" : repacked ? "tma_repacked" : "tma";
   if constexpr (std::is_same<T, double>::value) {
     // the screened kernel, where it is modelled faster: no factor on the product (alpha is the identity of +) and a
     // start value that compares, so that the running minimum can live in D
     if (add_id == add_id && (desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM) && desc.mul_op == CUASR_OP_PLUS && alpha == T(0)) {
       const ScreenPlan screened = screen_plan(p.m, p.n, p.k, dev->sms, extra.count == 0);
       if (screened.cost < plan.cost) {
-        const bool name = !small && dense && tma_describable(p.a, p.lda, sizeof(T)) && tma_describable(p.b, p.ldb, sizeof(T));
-        const bool copies = slices == 1 && args.workspace != nullptr && workspace_aligned && repack_plan(desc, args, p).bytes > 0 &&
-                            args.workspace_bytes >= align_up(balance_workspace_bytes(desc, args, dev->sms), 256) + repack_plan(desc, args, p).bytes;
-        if (!copies) {
-          const int st = run_screened<T>(desc.add_op == CUASR_OP_MAXIMUM, p, beta, add_id, read_c, screened, extra, dev, stream);
-          if (st == CUASR_STATUS_SUCCESS)
-            t_last_kernel = !name ? (slices > 1 ? "generic_splitk" : "generic") : slices > 1 ? "tma_splitk" : balanced ? "tma_balanced" : "tma";
-          return st;
-        }
+        const int st = run_screened<T>(desc.add_op == CUASR_OP_MAXIMUM, p, beta, add_id, read_c, screened, extra, dev, stream);
+        if (st == CUASR_STATUS_SUCCESS) t_last_kernel = name;
+        return st;
       }
     }
   }
-  // the rest of an optional workspace holds K-contiguous, aligned copies of operands (see RepackPlan)
-  bool repacked = false;
-  int k_map = p.k;              // K extent the tensor maps describe
-  if (slices == 1 && args.workspace != nullptr && workspace_aligned) {
-    const size_t first = align_up(balance_workspace_bytes(desc, args, dev->sms), 256);
-    const RepackPlan rp = repack_plan(desc, args, p);
-    if (rp.bytes > 0 && args.workspace_bytes >= first + rp.bytes) {
-      char* cursor = static_cast<char*>(args.workspace) + first;
-      const int k_copy = rp.k_padded > 0 ? rp.k_padded : p.k;
-      const long long ldt = static_cast<long long>(align_up(static_cast<size_t>(k_copy), 16 / sizeof(T)));
-      unsigned long long pad_a = 0, pad_b = 0;
-      std::memcpy(&pad_a, &add_id, sizeof(T));
-      std::memcpy(&pad_b, &mul_id, sizeof(T));
-      RepackRequest requests[2];
-      int count = 0;
-      if (rp.a) {
-        requests[count++] = {p.a, p.lda, p.a_kcontig, p.m, p.k, k_copy, pad_a, cursor, ldt};
-        p.a = cursor; p.lda = ldt; p.a_kcontig = true;
-        cursor += repack_operand_bytes(p.m, k_copy, sizeof(T));
-      }
-      if (rp.b) {
-        requests[count++] = {p.b, p.ldb, p.b_kcontig, p.n, p.k, k_copy, pad_b, cursor, ldt};
-        p.b = cursor; p.ldb = ldt; p.b_kcontig = true;
-      }
-      if (launch_repack(requests, count, sizeof(T), stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
-      g_launches.fetch_add(1);
-      repacked = true;
-      k_map = k_copy;
-    }
-  }
-
-  const bool describable = tma_describable(p.a, p.lda, sizeof(T)) && tma_describable(p.b, p.ldb, sizeof(T));
-  // the name a caller sees: "tma..." where the storage lines are what TMA could describe
-  const bool aligned_name = (pads_itself || k_map % TK == 0) && !small && dense && describable;
   const int step = TK * tile_sub(plan.tile, desc);
   const bool nan_pad = std::is_floating_point<T>::value && (desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM);
   // TMA brings in what lies along k on aligned lines, unless a ragged last step needs padding it cannot write
@@ -728,8 +758,7 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
 #undef X
   if (!launched) return CUASR_STATUS_ERROR_NOT_SUPPORTED;
   if (err != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
-  t_last_kernel = !aligned_name ? (slices > 1 ? "generic_splitk" : "generic")
-                  : slices > 1 ? "tma_splitk" : balanced ? "tma_balanced" : repacked ? "tma_repacked" : "tma";
+  t_last_kernel = name;
   g_launches.fetch_add(1);
   return CUASR_STATUS_SUCCESS;
 }
@@ -835,7 +864,7 @@ size_t cuasr_b200_srgemm_optional_workspace_size(const cuasr_b200_desc_t* desc, 
   if (args->split_k_slices > 1) return 0;
   DeviceState* dev = nullptr;
   if (!device_state(&dev)) return 0;
-  const size_t repack = repack_plan(*desc, *args, normalise(*desc, *args)).bytes;
+  const size_t repack = repack_plan(*desc, *args, normalise(*desc, *args), dev->sms).bytes;
   const size_t balance = balance_workspace_bytes(*desc, *args, dev->sms);
   return repack > 0 ? align_up(balance, 256) + repack : balance;
 }

@@ -34,13 +34,15 @@ __device__ __forceinline__ void sts(uint32_t addr, uint32_t v) { asm volatile("s
 __device__ __forceinline__ void sts(uint32_t addr, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory"); }
 
 // Stages rows [r0, r0 + kRows) x k [k0, k0 + kSub * 128 bytes) of an operand whose element (r, k) is base[r * ld + k]
-// (kLoadGatherK) or base[r + k * ld] (kLoadGatherMN).  Rows at or beyond `rows` repeat the last row (their results are
-// never stored); k at or beyond K repeats the last k too where `repeat_k` is set (rings whose (+) is idempotent: a product
+// (kLoadGatherK) or base[r + k * ld] (kLoadGatherMN).  Rows at or beyond `rows` are left as they are (their results are
+// never stored) or, where the kernel looks at the whole stage (kRepeatRow), repeat the last row, which takes more
+// instructions.
+// k at or beyond K repeats the last k where `repeat_k` is set (rings whose (+) is idempotent: a product
 // twice changes nothing) and is else set to `pad` by plain stores, so a stage that reaches beyond K must not be announced
 // with cp_async_arrive_noinc alone.  Called by all 128 producer threads; `pw` is the producer warp (0..3).
 // Inside the matrix a copy is one cp.async and at most one addition: with the bounds tested element by element a
 // 1024 x 768 x 1536 product of odd storage lines took 186 us, against 97 us with TMA.
-template <typename T, int kRows, int kSub>
+template <typename T, int kRows, int kSub, bool kRepeatRow = false>
 __device__ __forceinline__ void gather_tile(uint32_t dst, const T* __restrict__ base, long long ld, int mode, int r0,
                                             int rows, int k0, int K, T pad, bool repeat_k, int pw, int lane) {
   constexpr int TK = 128 / (int)sizeof(T);         // k per 128-byte row
@@ -65,8 +67,15 @@ __device__ __forceinline__ void gather_tile(uint32_t dst, const T* __restrict__ 
 #pragma unroll
           for (int i = 0; i < kRows / 8; ++i) cp_async<ES>(d + i * 1024, s + 8 * i);
         } else if (k < K) {
+          if constexpr (kRepeatRow) {
 #pragma unroll 1
-          for (int i = 0; i < kRows / 8; ++i) cp_async<ES>(d + i * 1024, line + min(r8 + 8 * i, last));
+            for (int i = 0; i < kRows / 8; ++i) cp_async<ES>(d + i * 1024, line + min(r8 + 8 * i, last));
+          } else {
+            const T* s = line + r8;
+#pragma unroll
+            for (int i = 0; i < kRows / 8; ++i)
+              if (8 * i <= last - r8) cp_async<ES>(d + i * 1024, s + 8 * i);
+          }
         } else {
 #pragma unroll 1
           for (int i = 0; i < kRows / 8; ++i) sts(d + i * 1024, pad);
@@ -94,9 +103,18 @@ __device__ __forceinline__ void gather_tile(uint32_t dst, const T* __restrict__ 
           s += (long long)kRowStep * ld;
         }
       } else if (k < K) {
+        if constexpr (kRepeatRow) {
 #pragma unroll 1
-        for (int i = 0; i < kRows / kRowStep; ++i)
-          cp_async<ES>(d + i * (kRowStep * 128) + ((i & 1) ? c1 : c0), column + (long long)min(rr + kRowStep * i, last) * ld);
+          for (int i = 0; i < kRows / kRowStep; ++i)
+            cp_async<ES>(d + i * (kRowStep * 128) + ((i & 1) ? c1 : c0), column + (long long)min(rr + kRowStep * i, last) * ld);
+        } else {
+          const T* s = column + (long long)rr * ld;
+#pragma unroll 4
+          for (int i = 0; i < kRows / kRowStep; ++i) {
+            if (kRowStep * i <= last - rr) cp_async<ES>(d + i * (kRowStep * 128) + ((i & 1) ? c1 : c0), s);
+            s += (long long)kRowStep * ld;
+          }
+        }
       } else {
 #pragma unroll 1
         for (int i = 0; i < kRows / kRowStep; ++i) sts(d + i * (kRowStep * 128) + ((i & 1) ? c1 : c0), pad);

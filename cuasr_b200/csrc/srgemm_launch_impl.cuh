@@ -38,7 +38,10 @@ cudaError_t launch_tma(int tile, const CUtensorMap& map_a, const CUtensorMap& ma
                        int grid, int cluster, cudaStream_t stream) {
   using R = Ring<ADD, MUL, T>;
   if constexpr (all_tiles_instantiated<ADD, MUL, T>()) {
-    if (tile == kLargeTile) return launch_tma_variant<R, LargeTile>(map_a, map_b, params, grid, cluster, stream);
+    if (tile == kLargeTile)
+      return params.a_mode == kLoadTma && params.b_mode == kLoadTma
+                 ? launch_tma_variant<R, LargeTmaTile>(map_a, map_b, params, grid, cluster, stream)
+                 : launch_tma_variant<R, LargeTile>(map_a, map_b, params, grid, cluster, stream);
     if (tile == kMediumTile) return launch_tma_variant<R, MediumTile>(map_a, map_b, params, grid, cluster, stream);
   }
   if (tile == kTinyTile) {

@@ -278,8 +278,8 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       if (alive && gathers) {
         // beyond K: infinities of the kind that never improves
         const T pad = kMax ? -static_cast<T>(INFINITY) : static_cast<T>(INFINITY);
-        if (p.a_mode != kLoadTma) gather_tile<T, 128, 2>(smem_u32(sa), p.A, p.lda, p.a_mode, lm0, p.M, k0, p.K, pad, false, pw, lane);
-        if (p.b_mode != kLoadTma) gather_tile<T, 128, 2>(smem_u32(sb), p.B, p.ldb, p.b_mode, ln0, p.N, k0, p.K, pad, false, pw, lane);
+        if (p.a_mode != kLoadTma) gather_tile<T, 128, 2, true>(smem_u32(sa), p.A, p.lda, p.a_mode, lm0, p.M, k0, p.K, pad, false, pw, lane);
+        if (p.b_mode != kLoadTma) gather_tile<T, 128, 2, true>(smem_u32(sb), p.B, p.ldb, p.b_mode, ln0, p.N, k0, p.K, pad, false, pw, lane);
         if (k0 + KB > p.K) {
           cp_async_wait_all();
           mbar_arrive(&full_bar[s]);

@@ -46,8 +46,13 @@ constexpr int kMaxDestinations = 8;               // output copies one launch ca
 constexpr int kMaxSmemBytes = 232448;             // 227 KiB: what one CTA may have
 
 // Tile shape of a kernel variant.
-template <int WM_, int WN_, int WK_, int kSub_ = WK_ == 4 ? 2 : 1>
+template <int WM_, int WN_, int WK_, int kSub_ = WK_ == 4 ? 2 : 1, bool kGathers_ = true>
 struct TileShape {
+  // Without the gather the producers need no more than 40 registers, and the consumers of the 128 x 128 tile get the 232
+  // that hold their fragments and tables without spilling (see LargeTmaTile).
+  static constexpr bool kGathers = kGathers_;
+  static constexpr int kConsumerRegisters = kGathers ? kConsumerRegs : 232, kProducerRegisters = kGathers ? kProducerRegs : 40;
+  static_assert(2 * kConsumerRegisters + kProducerRegisters <= 3 * 168, "the registers the CTA is launched with");
   static constexpr int WM = WM_, WN = WN_, WK = WK_;
   static_assert(WM * WN * WK == kConsumerWarps, "eight consumer warps");
   static constexpr int kM = 64 * WM, kN = 32 * WN;
@@ -66,6 +71,9 @@ struct TileShape {
   static constexpr int kSmemBytes = kStages<T> * kStageBytes + kFoldBytes<T> + 1024 /* alignment */ + 512 /* barriers */;
 };
 using LargeTile = TileShape<2, 4, 1>;    // 128 x 128
+// The same where TMA brings in both operands.  With the gather compiled in (224 registers) the fp32 tropical contraction
+// spills 64 bytes: 256 x 256 x 262144 split along K takes 1049 us with it and 1036 without, 8192^3 31.38 and 31.20 ms.
+using LargeTmaTile = TileShape<2, 4, 1, 1, false>;
 using MediumTile = TileShape<2, 2, 2>;   // 128 x 64
 using SmallTile = TileShape<1, 2, 4>;    // 64 x 64
 // 64 x 32, one 16-byte chunk of k per warp and stage: the shortest chain for the smallest products, and the finest
@@ -189,8 +197,8 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   volatile unsigned int* abandoned = ticket_smem + 1;     // raised when a consumer's wait ran out (see ptx.cuh)
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const bool gathers = p.a_mode != kLoadTma || p.b_mode != kLoadTma;
-  const bool tmas = p.a_mode == kLoadTma || p.b_mode == kLoadTma;
+  const bool a_tma = !Tile::kGathers || p.a_mode == kLoadTma, b_tma = !Tile::kGathers || p.b_mode == kLoadTma;
+  const bool gathers = !a_tma || !b_tma, tmas = a_tma || b_tma;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -212,7 +220,7 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
   if (warp >= kConsumerWarps) {
     // ---------------------------------------------------------------- producers
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kProducerRegs));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Tile::kProducerRegisters));
     const int pw = warp - kConsumerWarps;
     const bool issuer = pw == 0 && lane == 0;
     bool working = gathers || issuer;
@@ -236,17 +244,17 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         uint8_t* sb = sa + Tile::kABytes;
         const int k0 = kt * kStep;
         if (issuer && tmas) {
-          mbar_arrive_expect_tx(&full_bar[s], (p.a_mode == kLoadTma ? Tile::kABytes : 0) + (p.b_mode == kLoadTma ? Tile::kBBytes : 0));
+          mbar_arrive_expect_tx(&full_bar[s], (a_tma ? Tile::kABytes : 0) + (b_tma ? Tile::kBBytes : 0));
 #pragma unroll
           for (int sub = 0; sub < kSub; ++sub) {
-            if (p.a_mode == kLoadTma) tma_load_2d(sa + sub * (Tile::kM * 128), &map_a, &full_bar[s], k0 + sub * TK, m0);
-            if (p.b_mode == kLoadTma) tma_load_2d(sb + sub * (Tile::kN * 128), &map_b, &full_bar[s], k0 + sub * TK, n0);
+            if (a_tma) tma_load_2d(sa + sub * (Tile::kM * 128), &map_a, &full_bar[s], k0 + sub * TK, m0);
+            if (b_tma) tma_load_2d(sb + sub * (Tile::kN * 128), &map_b, &full_bar[s], k0 + sub * TK, n0);
           }
         }
         if (gathers) {
-          if (p.a_mode != kLoadTma)
+          if (!a_tma)
             gather_tile<T, Tile::kM, kSub>(smem_u32(sa), p.A, p.lda, p.a_mode, m0, p.M, k0, p.K, p.pad, p.repeat_k, pw, lane);
-          if (p.b_mode != kLoadTma)
+          if (!b_tma)
             gather_tile<T, Tile::kN, kSub>(smem_u32(sb), p.B, p.ldb, p.b_mode, n0, p.N, k0, p.K, p.pad, p.repeat_k, pw, lane);
           if (k0 + kStep > p.K) {         // padding was written by ordinary stores: announce with an ordinary arrival
             cp_async_wait_all();
@@ -268,7 +276,7 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   }
 
   // ------------------------------------------------------------------ consumers
-  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kConsumerRegs));
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Tile::kConsumerRegisters));
   const int wk = warp / (WM * WN), wm = (warp / WN) % WM, wn = warp % WN;
   const int lr = lane / 4, lc = lane % 4;        // 8 x 4 lanes
   // Row i (0..7) of this lane inside the warp's 64 rows; column j (0..7) inside the warp's 32 columns.
@@ -299,18 +307,22 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   // Only for 4-byte elements: with 8-byte elements the accumulators leave no registers for the table, and the
   // offsets are computed where they are used.
   constexpr bool kOffsetTable = sizeof(T) == 4;
-  // chunks unrolled in the contraction loop; the table holds the offsets of that many chunks, and chunk c + kUnroll
-  // of a stage is reached by flipping bit 6 of the offset (bit 2 of the chunk index; a_base and b_base are
-  // multiples of 128, so the flip commutes with adding them)
+  // Chunks unrolled in the contraction loop; the table holds the offsets of that many chunks.  Chunk c + kUnroll of a
+  // stage differs in bit 6 of the offset (bit 2 of the chunk index), and so do the B rows of odd j.  That bit is the same
+  // for all entries of a lane's table, so the flip is an addition of 64 or -64 that goes into the stage's base once:
+  // 4096^3 max-min 5952 -> 5920 us.  The packed rings with the gather compiled in have no registers for it (4096^3
+  // min-plus, one operand gathered: 3998 -> 4090 us) and flip the bit of each offset.
+  constexpr bool kFlipBase = !Tile::kGathers || !RingT::kPackedPairs;
   // (four chunks keep the loop body near 16 KiB of instructions; unrolling all eight measured the same on min-plus
   // and 25 % slower on max-min, whose body is half as large again)
   constexpr int kUnroll = kChunks < 4 ? kChunks : 4;
   uint32_t a_off[kOffsetTable ? kUnroll : 1], b_off[kOffsetTable ? kUnroll : 1];
+  const int a_flip = ((first_chunk ^ lr) & 4) ? -64 : 64, b_flip = ((first_chunk ^ lc) & 4) ? -64 : 64;
   if constexpr (kOffsetTable) {
 #pragma unroll
     for (int c = 0; c < kUnroll; ++c) {
       a_off[c] = a_base + ((((c + first_chunk) ^ lr) & 7) << 4);
-      b_off[c] = b_base + ((((c + first_chunk) ^ lc) & 7) << 4);       // rows lc + 4 j with odd j: bit 6 flipped
+      b_off[c] = b_base + ((((c + first_chunk) ^ lc) & 7) << 4);       // rows lc + 4 j with even j
     }
   }
 
@@ -337,7 +349,7 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       // chunk is given as (c, h): chunk = h * kUnroll + c with c a compile-time constant; without it h is 0.
       auto load_a = [&](T (&a)[8][EV], int c, int h = 0) {
         uint32_t base;
-        if constexpr (kOffsetTable) base = st + (a_off[c] ^ (h << 6));
+        if constexpr (kOffsetTable) base = kFlipBase ? st + h * a_flip + a_off[c] : st + (a_off[c] ^ (h << 6));
         else base = st + a_base + ((((c + first_chunk) ^ lr) & 7) << 4);
 #pragma unroll
         for (int i = 0; i < 8; ++i) lds16(base + i * 1024, a[i]);
@@ -345,8 +357,8 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       auto load_b = [&](T (&b)[8][EV], int c, int h = 0) {
         uint32_t base0, base1;
         if constexpr (kOffsetTable) {
-          base0 = st + (b_off[c] ^ (h << 6));
-          base1 = st + (b_off[c] ^ ((h << 6) ^ 64));
+          base0 = kFlipBase ? st + h * b_flip + b_off[c] : st + (b_off[c] ^ (h << 6));
+          base1 = kFlipBase ? st + (1 - h) * b_flip + b_off[c] : st + (b_off[c] ^ ((h << 6) ^ 64));
         } else {
           base0 = st + b_base + ((((c + first_chunk) ^ lc) & 7) << 4);
           base1 = st + b_base + ((((c + first_chunk) ^ (lc + 4)) & 7) << 4);
@@ -640,6 +652,39 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           }
         }
         __syncwarp();
+        if constexpr (kDmma) {
+          // C may be D, so a load of C after a store to D cannot be moved in front of it: one by one, the 32 vectors of a
+          // lane are as many memory latencies in a row.  Here they are loaded four at a time (every element is read and
+          // written by one thread only): 1500^3 230 -> 219 us, 4096^3 3991 -> 3901.  The rings with more registers in
+          // use lose as much in the contraction as they gain (8192^3 min-plus 31.2 -> 31.9 ms).
+          if (p.vector_epilogue && p.read_c) {
+            constexpr int kBatch = 4;
+#pragma unroll 1
+            for (int at = lane; at < kRowsPerPass * kGroups; at += kBatch * 32) {
+              alignas(16) T c[kBatch][EV];
+#pragma unroll
+              for (int u = 0; u < kBatch; ++u) {
+                const int m = m_base + pass * kRowsPerPass + (at + u * 32) / kGroups, n = n_base + (at + u * 32) % kGroups * EV;
+                if (m < p.M && n < p.N)
+                  *reinterpret_cast<uint4*>(c[u]) = *reinterpret_cast<const uint4*>(p.C + (long long)m * p.ldc + n);
+              }
+#pragma unroll
+              for (int u = 0; u < kBatch; ++u) {
+                const int r = (at + u * 32) / kGroups, g = (at + u * 32) % kGroups;
+                const int m = m_base + pass * kRowsPerPass + r, n = n_base + g * EV;
+                if (m >= p.M || n >= p.N) continue;
+                alignas(16) T v[EV];
+                *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(stage + r * 32 + ((g ^ (r & 7)) & (kGroups - 1)) * EV);
+#pragma unroll
+                for (int e = 0; e < EV; ++e) v[e] = RingT::add(RingT::mul(p.alpha, v[e]), RingT::mul(p.beta, c[u][e]));
+                const long long off = (long long)m * p.ldd + n;
+                *reinterpret_cast<uint4*>(p.D + off) = *reinterpret_cast<const uint4*>(v);
+                for (int x = 0; x < p.n_extra; ++x) *reinterpret_cast<uint4*>(p.extra_d[x] + off) = *reinterpret_cast<const uint4*>(v);
+              }
+            }
+            continue;
+          }
+        }
 #pragma unroll 4
         for (int idx = lane; idx < kRowsPerPass * kGroups; idx += 32) {
           const int r = idx / kGroups, g = idx % kGroups;
