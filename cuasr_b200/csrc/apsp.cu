@@ -263,13 +263,16 @@ int blocked_floyd_warshall(const cuasr_b200_apsp_args_t& a, char* D, long long l
 }
 
 // Without predecessors.  The serial part of a step is the closure of its diagonal block, one CTA's work for 128 vertices
-// (15 us); larger blocks would only be closed by this same scheme one level down, and a step of 128 vertices already
-// runs at the rate of long products (n = 2000: 2.9 ms with blocks of 1024 closed by ten squarings each).  So 128 is
-// the block where the caller leaves it open; a block the caller asked for is closed in steps of 128.
+// (15 us); larger blocks are closed by this same scheme one level down, in steps of 128.  Small blocks keep the serial part
+// short, large ones the number of times all of D is read and written.  ms with blocks of 128 / 256 / 512 / 1024:
+//   n = 2000  1.71 / 1.83 / 1.84 / 2.26     n = 4000  7.71 / 7.53 / 7.65 / 8.45
+//   n = 8192  57.3 / 48.0 / 45.0 / 46.6     n = 16384  423 / 346 / 314 / 309
+// (closed by squarings in blocks of 1024: 3.01, 10.0, 49.5, 314), so where the caller leaves it open the block grows with n.
 int floyd_warshall(const cuasr_b200_apsp_args_t& a) {
   if (a.parent != nullptr) return floyd_warshall_with_parents(a);
   const FwLayout l = fw_layout(a);
-  const int b = a.block > 0 ? block_of(a) : std::min(kClosureBlock, block_of(a));
+  const int best = a.n <= 3000 ? kClosureBlock : a.n <= 6000 ? 256 : a.n <= 12000 ? 512 : kDefaultBlock;
+  const int b = a.block > 0 ? block_of(a) : std::min(best, block_of(a));
   char* ws = static_cast<char*>(a.workspace);
   void* scratch = a.workspace_bytes > l.srgemm ? ws + l.srgemm : nullptr;
   const size_t scratch_bytes = a.workspace_bytes - l.srgemm;

@@ -34,7 +34,7 @@ typedef struct cuasr_b200_apsp_args {
   int32_t dtype;       /* CUASR_F32 or CUASR_F64 */
   int32_t algorithm;   /* cuasr_apsp_algorithm_t */
   int32_t n;           /* vertices */
-  int32_t block;       /* Floyd-Warshall block size, a multiple of 4; 0 = 1024 (the measured optimum at n = 16384) */
+  int32_t block;       /* Floyd-Warshall block size, a multiple of 4; 0 = chosen by n (1024 with predecessors) */
   int32_t iterations;  /* repeated squaring: number of squarings; 0 = ceil(log2 n), enough for any graph */
   int32_t reserved;
   void *D;             /* distances, read and overwritten with the closure */
