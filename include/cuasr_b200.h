@@ -88,14 +88,12 @@ CUASR_B200_API int cuasr_b200_srgemm(const cuasr_b200_desc_t *desc, const cuasr_
  * cuasr_b200_srgemm or cuasr_b200_srgemm_push with split_k_slices == 1 gets two things, with identical results:
  *  - load balance: when the tile count is not a multiple of the SM count, the tiles of the last wave are cut along
  *    K, their pieces fill the SMs, and the CTA that finishes a tile last folds the pieces in a fixed order;
- *  - fp32 min/max-plus and min/max-times rings: operands whose contiguous dimension is not K are first copied into
- *    K-contiguous scratch (a bandwidth-bound pre-pass of well under 1 % of the run time), which lets the kernel use
- *    packed fp32x2 adds for both products of a three-input min/max;
- *  - operands the fast kernel cannot read in place are copied into scratch it can read: an operand whose address
+ *  - operands that TMA cannot bring in as they lie are first copied into scratch where it can: an operand whose
+ *    contiguous dimension is not K (where the copy is expected to take less time than it saves), one whose address
  *    or leading dimension is not a multiple of 16 bytes (the reference accepts alignment 1,
- *    device/default_srgemm_configuration.h:88-89; without the workspace such a product runs on the slower generic
- *    kernel), and both operands of an integer min/max ring whose K is not a multiple of the kernel's K step (the
- *    copies are extended along K: A by the additive identity, B by the multiplicative one).
+ *    device/default_srgemm_configuration.h:88-89), and both operands of an integer min/max ring whose K is not a
+ *    multiple of the kernel's K step (the copies are extended along K: A by the additive identity, B by the
+ *    multiplicative one).  Without the workspace the kernel gathers such operands element by element.
  * The size depends on the operand addresses in `args`.  Needs a current device. */
 CUASR_B200_API size_t cuasr_b200_srgemm_optional_workspace_size(const cuasr_b200_desc_t *desc, const cuasr_b200_args_t *args);
 
@@ -178,7 +176,9 @@ CUASR_B200_API int cuasr_b200_pack_k_contiguous(int32_t dtype, const void *src, 
  * (1: tile never arrived, 2: stage never released, 3: peer flag never set).  This call blocks. */
 CUASR_B200_API int cuasr_b200_device_status(void *stream);
 
-/* Name of the kernel the last cuasr_b200_srgemm* call on this thread launched ("tma", "generic", ...). */
+/* How the last cuasr_b200_srgemm* call on this thread ran: "tma", "tma_balanced", "tma_repacked", "tma_splitk", "path_tma"
+ * where the storage lines of the operands (or of their copies) are what TMA can describe, "generic", "generic_splitk",
+ * "path" where they are not. */
 CUASR_B200_API const char *cuasr_b200_last_kernel(void);
 
 /* Number of kernels this library has launched in this process so far. */
