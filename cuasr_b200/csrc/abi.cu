@@ -548,22 +548,23 @@ template <typename T>
 int run_path(bool maximize, const Normalised& p, int32_t* parent, long long ld_parent, int k_offset, DeviceState* dev,
              cudaStream_t stream) {
   constexpr int TK = kTileKBytes / sizeof(T);
-  const double per_k = 2 * 64 * (sizeof(T) == 8 ? 6.5 : 2.1);
+  constexpr int small = sizeof(T) == 4 ? kSmallTile : kTinyTile;
+  const double per_k = 2 * 64 * (sizeof(T) == 8 ? 8.2 : 2.1);
   double best = 1e300;
   int tile = kLargeTile, cluster = 1;
-  for (int candidate : {kLargeTile, kSmallTile}) {
-    if (candidate == kSmallTile && sizeof(T) == 8) continue;                  // its partial values would not fit beside a pipeline
+  for (int candidate : {(int)kLargeTile, small}) {
     const bool large = candidate == kLargeTile;
     const long long tiles = static_cast<long long>((p.m + kTileRows[candidate] - 1) / kTileRows[candidate]) * ((p.n + kTileCols[candidate] - 1) / kTileCols[candidate]);
-    const int step = large ? TK : 2 * TK;
+    const int step = candidate == kSmallTile ? 2 * TK : TK;
+    const double chunks = large ? 2 : candidate == kSmallTile ? 1 : 0.25;           // in fours, of a warp and stage
     const int k_steps = (p.k + step - 1) / step;
     for (int z = 1; z <= (large ? 1 : 8); z *= 2) {
       const int per_piece = (k_steps + z - 1) / z;
       if ((z - 1) * per_piece >= k_steps) break;
       const long long room = z <= 2 ? dev->sms : z == 4 ? dev->sms * 36LL / 37 : dev->sms * 32LL / 37;
       const long long waves = (tiles * z + room - 1) / room;
-      const double per_stage = per_k * step / kTileWk[candidate] + 2 * 256 + 2 * 1.5 * 60 * (large ? 2 : 1);
-      const double lookups = 2 * 64 * 60 * (large ? 2 : 1) * std::log(1.0 + per_piece);
+      const double per_stage = per_k * step / kTileWk[candidate] + 2 * 256 + 2 * 1.5 * 60 * chunks;
+      const double lookups = 2 * 64 * 60 * chunks * std::log(1.0 + per_piece);
       const double cost = 3000 + static_cast<double>(waves) * (per_stage * per_piece + lookups + 3000 + (z > 1 ? 3000 : 0));
       if (cost < best) { best = cost; tile = candidate; cluster = z; }
     }
@@ -579,14 +580,14 @@ int run_path(bool maximize, const Normalised& p, int32_t* parent, long long ld_p
   pp.dist = static_cast<T*>(p.d); pp.ldd = p.ldd;
   pp.parent = parent; pp.ld_parent = ld_parent; pp.k_offset = k_offset;
   pp.tiles_m = (p.m + kTileRows[tile] - 1) / kTileRows[tile]; pp.tiles_n = (p.n + kTileCols[tile] - 1) / kTileCols[tile];
-  const int step = tile == kLargeTile ? TK : 2 * TK;
+  const int step = tile == kSmallTile ? 2 * TK : TK;
   const int k_steps = (p.k + step - 1) / step;
   pp.cluster = cluster; pp.k_tiles_per_slice = (k_steps + cluster - 1) / cluster;
   pp.status = dev->status;
   const long long work = static_cast<long long>(pp.tiles_m) * pp.tiles_n * cluster;
   if (work > 2147483647LL) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
   const int grid = static_cast<int>(cluster > 1 || work < dev->sms ? work : dev->sms);
-  if (launch_path<T>(maximize, tile == kSmallTile, map_a, map_b, pp, grid, stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
+  if (launch_path<T>(maximize, tile != kLargeTile, map_a, map_b, pp, grid, stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
   g_launches.fetch_add(1);
   return CUASR_STATUS_SUCCESS;
 }

@@ -14,11 +14,10 @@ static cudaError_t launch_variant(const CUtensorMap& map_a, const CUtensorMap& m
 template <typename T>
 cudaError_t launch_path(bool maximize, bool small_tile, const CUtensorMap& map_a, const CUtensorMap& map_b,
                         const PathParams<T>& params, int grid, cudaStream_t stream) {
-  if constexpr (sizeof(T) == 4) {
-    if (small_tile)
-      return maximize ? launch_variant<T, true, SmallTile>(map_a, map_b, params, grid, stream)
-                      : launch_variant<T, false, SmallTile>(map_a, map_b, params, grid, stream);
-  }
+  using Small = std::conditional_t<sizeof(T) == 4, SmallTile, TinyTile>;
+  if (small_tile)
+    return maximize ? launch_variant<T, true, Small>(map_a, map_b, params, grid, stream)
+                    : launch_variant<T, false, Small>(map_a, map_b, params, grid, stream);
   return maximize ? launch_variant<T, true, LargeTile>(map_a, map_b, params, grid, stream)
                   : launch_variant<T, false, LargeTile>(map_a, map_b, params, grid, stream);
 }

@@ -10,11 +10,12 @@
 // that changed in a 64-bit mask: 2 instructions per element and stage.  One pass per noted element then finds the k:
 // it reads the operand rows again from the stage, which is still there, and takes the first sum that equals the new
 // value.  The n-th product of random data is a new minimum with probability 1/n, so late stages note next to nothing.
-//   Against a test every four k and an index per improvement among those (2048^3 from +inf: 1.69 ms): see the figures at
-//   launch_path's caller.
+// With a test every four k and an index per improvement among those, 2048^3 from +inf took 1.69 ms and 0.96 once nothing
+// improves; now 1.36 and 0.65 (the plain product: 0.52).
 // Tiles: 128 x 128 with whole k ranges per warp (the index then goes straight to `parent`: a lane meets its k in
-// ascending order), and for fp32 outputs too small to fill the GPU with those, 64 x 64 with the k range shared by four
-// warps and, beyond that, by the CTAs of a cluster; their (value, k) candidates meet in shared memory, the smaller k
+// ascending order), and for outputs too small to fill the GPU with those, 64 x 64 (fp32) or 64 x 32 (fp64, whose partial
+// values leave no room for a pipeline beside the larger one) with the k range shared by four or eight warps and, beyond
+// that, by the CTAs of a cluster; their (value, k) candidates meet in shared memory, the smaller k
 // winning ties.
 #pragma once
 
@@ -48,6 +49,16 @@ constexpr int kPathStages = (kMaxSmemBytes - 1024 - 512 - kPathKeptBytes<T, Tile
 template <typename T, typename Tile>
 constexpr int kPathSmemBytes = kPathStages<T, Tile> * Tile::kStageBytes + kPathKeptBytes<T, Tile> + kPathIndexBytes<Tile> + 1024 + 512;
 
+__device__ __forceinline__ void ld_cluster(uint32_t addr, int rank, float& v) {
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+}
+__device__ __forceinline__ void ld_cluster(uint32_t addr, int rank, double& v) {
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(remote) : "memory");
+}
 __device__ __forceinline__ uint32_t ld4_cluster(uint32_t addr, int rank) {
   uint32_t remote, v;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
@@ -284,15 +295,20 @@ srgemm_path_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       int zero;
       asm volatile("mov.s32 %0, 0;" : "=r"(zero));
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < 8; ++i) {
+        const int m = m_base + lr + 8 * i + zero;
+        T cur[8];                      // a row's loads together: none of them can pass a store
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const int m = m_base + lr + 8 * i + zero, n = n_base + lc + 4 * j + zero;
-          if (m < p.M && n < p.N) {
-            T* at = p.dist + (long long)m * p.ldd + n;
-            if (better(acc[i][j], *at)) *at = acc[i][j];
-          }
+          const int n = n_base + lc + 4 * j + zero;
+          cur[j] = m < p.M && n < p.N ? p.dist[(long long)m * p.ldd + n] : acc[i][j];
         }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int n = n_base + lc + 4 * j + zero;
+          if (better(acc[i][j], cur[j])) p.dist[(long long)m * p.ldd + n] = acc[i][j];
+        }
+      }
     } else {
       // Partial values to shared memory ([wk][row][column], column groups swizzled), then one element per thread at a
       // time: the best value, and among equal ones the smallest k.  A value that is not better than dist has no k.
@@ -347,10 +363,11 @@ srgemm_path_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         for (int idx = z * share + threadIdx.x; idx < (z + 1) * share; idx += kConsumerThreads) {
           const int r = idx / Tile::kN, c = idx % Tile::kN;
           const uint32_t at = smem_u32(fold + r * Tile::kN + (((c / EV) ^ (r & 7)) * EV) + (c % EV));
-          float best = __uint_as_float(ld4_cluster(at, 0));
+          T best, v;
+          ld_cluster(at, 0, best);
           int k = (int)ld4_cluster(smem_u32(tile_k + idx), 0);
           for (int q = 1; q < p.cluster; ++q) {
-            const float v = __uint_as_float(ld4_cluster(at, q));
+            ld_cluster(at, q, v);
             const int kq = (int)ld4_cluster(smem_u32(tile_k + idx), q);
             if (better(v, best) || (v == best && kq < k)) { best = v; k = kq; }
           }
@@ -366,7 +383,8 @@ srgemm_path_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   }
 }
 
-// Launches srgemm_path_kernel on `grid` CTAs: the 128 x 128 tile, or (fp32) the 64 x 64 one in clusters of params.cluster.
+// Launches srgemm_path_kernel on `grid` CTAs: the 128 x 128 tile, or the small one (fp32 64 x 64, fp64 64 x 32) in clusters of
+// params.cluster.
 template <typename T>
 cudaError_t launch_path(bool maximize, bool small_tile, const CUtensorMap& map_a, const CUtensorMap& map_b,
                         const PathParams<T>& params, int grid, cudaStream_t stream);
