@@ -373,7 +373,7 @@ int tile_sub(int tile, const cuasr_b200_desc_t& desc) {
 // fold of the small ones, twice that for 8-byte elements), 2500 for the exchange inside a cluster.  Clusters of four
 // and eight do not fill every SM (a cluster lives in one GPC): 144 and 128 of the 148.
 // A cluster launch is not persistent: each further wave starts its CTAs anew, 4000.  The 64 x 32 tile hands a stage over
-// for every chunk of a warp: 250 clocks a stage (a 512 x 4096 x 4096 product as seven waves of it took 635 us instead of
+// for every chunk of a warp: 250 clocks a stage, twice that for 8-byte elements (a 512 x 4096 x 4096 product as seven waves of it took 635 us instead of
 // the 514 modelled without; the 128 x 128 tile takes 580).
 // A gathered element costs 0.17 clocks on the small tiles where the contraction is bound by register reads (2048^3
 // min-plus with one operand transposed on 64 x 64 tiles: 589 us against 522 with TMA), 0.08 in the other rings (max-min:
@@ -399,7 +399,7 @@ LaunchPlan plan_without_workspace(const cuasr_b200_desc_t& desc, int m, int n, i
       const long long waves = (tiles * z + room - 1) / room;
       const double end = (tile == kLargeTile ? 2000 : 1500) * wide + (z > 1 ? 2500 + (waves > 1 ? 4000 : 0) : 0);
       const double gathered = gather_clocks(desc, tile == kLargeTile) * step * ((gather_a ? kTileRows[tile] : 0) + (gather_b ? kTileCols[tile] : 0));
-      const double per_stage = per_k * step / kTileWk[tile] + gathered + (tile == kTinyTile ? 250 : 0);
+      const double per_stage = per_k * step / kTileWk[tile] + gathered + (tile == kTinyTile ? 250 * wide : 0);
       const double cost = 3000 + static_cast<double>(waves) * (per_stage * per_piece + end);
       if (cost < best.cost) {
         best.tile = tile; best.cluster = z; best.cost = cost;
@@ -564,7 +564,10 @@ int run_path(bool maximize, const Normalised& p, int32_t* parent, long long ld_p
       const long long room = z <= 2 ? dev->sms : z == 4 ? dev->sms * 36LL / 37 : dev->sms * 32LL / 37;
       const long long waves = (tiles * z + room - 1) / room;
       const double per_stage = per_k * step / kTileWk[candidate] + 2 * 256 + 2 * 1.5 * 60 * chunks;
-      const double lookups = 2 * 64 * 60 * chunks * std::log(1.0 + per_piece);
+      // fp64: 180 clocks and 60 per four chunks for each look-up of the slowest lane (1000^3 from +inf: 907 us on 64 x 32 tiles
+      // against 764 on 128 x 128 ones, 300^3: 78 against 340)
+      const double lookups = sizeof(T) == 8 ? 2 * (96 * std::log(1.0 + per_piece) + 4 * per_piece) * (180 + 60 * chunks)
+                                            : 2 * 64 * 60 * chunks * std::log(1.0 + per_piece);
       const double cost = 3000 + static_cast<double>(waves) * (per_stage * per_piece + lookups + 3000 + (z > 1 ? 3000 : 0));
       if (cost < best) { best = cost; tile = candidate; cluster = z; }
     }
