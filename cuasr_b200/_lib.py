@@ -102,6 +102,7 @@ PROTOTYPES = {
                                                     ctypes.c_void_p]),
     "cuasr_b200_device_status": (ctypes.c_int, [ctypes.c_void_p]),
     "cuasr_b200_last_kernel": (ctypes.c_char_p, []),
+    "cuasr_b200_last_route": (ctypes.c_char_p, []),
     "cuasr_b200_launch_count": (ctypes.c_uint64, []),
     "cuasr_b200_status_string": (ctypes.c_char_p, [ctypes.c_int]),
     "cuasr_b200_version": (ctypes.c_char_p, []),

@@ -25,6 +25,22 @@ namespace {
 std::atomic<uint64_t> g_launches{0};
 thread_local const char* t_last_kernel = "none";
 
+// What the last call on this thread launched, for cuasr_b200_last_route: kept as numbers, written out when asked for.
+struct Route {
+  const char* kernel = "none";
+  int tile_m = 0, tile_n = 0, cluster = 1, pieces = 1;
+  const char* load_a = "";
+  const char* load_b = "";
+  bool tickets = false, copied_a = false, copied_b = false;
+};
+thread_local Route t_route;
+thread_local char t_route_text[160];
+
+const char* load_name(int mode) {
+  static const char* const names[4] = {"tma", "gather", "gather", "tma-rows"};      // LoadMode
+  return names[mode];
+}
+
 // ---- per-device state: SM count and the device status word --------------------------------------
 __device__ unsigned int g_status_word;  // zero-initialised when the module loads
 
@@ -537,6 +553,7 @@ int run_screened(bool maximize, const Normalised& p, T beta, T add_id, bool read
   const int grid = static_cast<int>(work < dev->sms ? work : dev->sms);
   if (launch_screened<T>(maximize, map_a, map_b, sp, grid, stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
   g_launches.fetch_add(1);
+  t_route = {"screened", kTileM, kTileN, 1, plan.pieces, load_name(sp.a_mode), load_name(sp.b_mode)};
   return CUASR_STATUS_SUCCESS;
 }
 
@@ -592,6 +609,7 @@ int run_path(bool maximize, const Normalised& p, int32_t* parent, long long ld_p
   const int grid = static_cast<int>(cluster > 1 || work < dev->sms ? work : dev->sms);
   if (launch_path<T>(maximize, tile != kLargeTile, map_a, map_b, pp, grid, stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
   g_launches.fetch_add(1);
+  t_route = {"path", kTileRows[tile], kTileCols[tile], cluster, cluster, load_name(pp.a_mode), load_name(pp.b_mode)};
   return CUASR_STATUS_SUCCESS;
 }
 
@@ -695,7 +713,10 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
       const ScreenPlan screened = screen_plan(p.m, p.n, p.k, dev->sms, extra.count == 0);
       if (screened.cost < plan.cost) {
         const int st = run_screened<T>(desc.add_op == CUASR_OP_MAXIMUM, p, beta, add_id, read_c, screened, extra, dev, stream);
-        if (st == CUASR_STATUS_SUCCESS) t_last_kernel = name;
+        if (st == CUASR_STATUS_SUCCESS) {
+          t_last_kernel = name;
+          t_route.copied_a = copies.a; t_route.copied_b = copies.b;
+        }
         return st;
       }
     }
@@ -763,6 +784,8 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   if (!launched) return CUASR_STATUS_ERROR_NOT_SUPPORTED;
   if (err != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
   t_last_kernel = name;
+  t_route = {"product", kTileRows[plan.tile], kTileCols[plan.tile], plan.cluster, plan.pieces, load_name(tp.a_mode), load_name(tp.b_mode),
+             tickets_used && plan.pieces > 1, copies.a, copies.b};
   g_launches.fetch_add(1);
   return CUASR_STATUS_SUCCESS;
 }
@@ -967,6 +990,8 @@ int cuasr_b200_pack_k_contiguous(int32_t dtype, const void* src, int64_t ld_src,
     return CUASR_STATUS_ERROR_INTERNAL;
   g_launches.fetch_add(1);
   t_last_kernel = "pack";
+  t_route = Route();
+  t_route.kernel = "pack";
   return CUASR_STATUS_SUCCESS;
 }
 
@@ -1009,6 +1034,14 @@ int cuasr_b200_flag_wait(const void* words, int count, uint32_t value, uint32_t 
 }
 
 const char* cuasr_b200_last_kernel(void) { return t_last_kernel; }
+
+const char* cuasr_b200_last_route(void) {
+  const Route& r = t_route;
+  if (r.tile_m == 0) return r.kernel;
+  std::snprintf(t_route_text, sizeof(t_route_text), "%s tile=%dx%d cluster=%d pieces=%d tickets=%d a=%s%s b=%s%s", r.kernel, r.tile_m,
+                r.tile_n, r.cluster, r.pieces, (int)r.tickets, r.copied_a ? "copy+" : "", r.load_a, r.copied_b ? "copy+" : "", r.load_b);
+  return t_route_text;
+}
 
 uint64_t cuasr_b200_launch_count(void) { return g_launches.load(); }
 

@@ -187,6 +187,10 @@ class _Operator:
     def last_kernel(self) -> str:
         return self._lib.cuasr_b200_last_kernel().decode()
 
+    def last_route(self) -> str:
+        """What the last product call of this thread launched (cuasr_b200_last_route)."""
+        return self._lib.cuasr_b200_last_route().decode()
+
 
 class Srgemm(_Operator):
     """cuasr::gemm::device::Srgemm."""

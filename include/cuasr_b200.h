@@ -176,10 +176,19 @@ CUASR_B200_API int cuasr_b200_pack_k_contiguous(int32_t dtype, const void *src, 
  * (1: tile never arrived, 2: stage never released, 3: peer flag never set).  This call blocks. */
 CUASR_B200_API int cuasr_b200_device_status(void *stream);
 
-/* How the last cuasr_b200_srgemm* call on this thread ran: "tma", "tma_balanced", "tma_repacked", "tma_splitk", "path_tma"
- * where the storage lines of the operands (or of their copies) are what TMA can describe, "generic", "generic_splitk",
- * "path" where they are not. */
+/* A label for the last cuasr_b200_srgemm* call on this thread that depends on its arguments alone: "tma...", "path_tma" where
+ * the storage lines of the operands (or of their copies) are what TMA can describe, "generic", "generic_splitk", "path" where
+ * they are not; "..._splitk", "..._balanced", "..._repacked": what was asked for or had room in the workspace.  Which
+ * kernel the call launched is answered by cuasr_b200_last_route. */
 CUASR_B200_API const char *cuasr_b200_last_kernel(void);
+
+/* What the last cuasr_b200_srgemm* call on this thread launched: the kernel ("product", "screened", "path", "pack"; "none"
+ * before the first call), its tile, the CTAs that share a tile's K through a cluster or in pieces, whether the pieces meet
+ * through tickets in the workspace, and how each operand of the row-major problem came in ("tma", "tma-rows", "gather",
+ * "copy+tma"; with a column-major C that problem's operands are B and A), e.g.
+ * "product tile=128x128 cluster=1 pieces=3 tickets=1 a=tma b=copy+tma".  For people and tests: the words may change.  The text
+ * is valid until the next call of this function on the thread. */
+CUASR_B200_API const char *cuasr_b200_last_route(void);
 
 /* Number of kernels this library has launched in this process so far. */
 CUASR_B200_API uint64_t cuasr_b200_launch_count(void);
