@@ -435,8 +435,11 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 
     for (int b = 0; b < count;) {
       const int s = it % kScreenStages;
-      mbar_wait_or_abandon(&ready_bar[s], (it / kScreenStages) & 1, p.status, kDeviceTimeoutFull, abandoned);
+      // In this order: an exact run below passes blocks without looking at ready_bar, and a parity wait is only sound if
+      // the phase before its own is complete.  The loads of block `it` are issued after all producers met in block it - 1,
+      // hence after each of them arrived for block it - 2; so once block `it` has landed, that phase is complete.
       mbar_wait_or_abandon(&full_bar[s], (it / kScreenStages) & 1, p.status, kDeviceTimeoutFull, abandoned);
+      mbar_wait_or_abandon(&ready_bar[s], (it / kScreenStages) & 1, p.status, kDeviceTimeoutFull, abandoned);
       float top = -INFINITY, low = INFINITY;
 #pragma unroll
       for (int v = 0; v < kProducerWarps; ++v) {

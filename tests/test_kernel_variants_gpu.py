@@ -68,6 +68,7 @@ def check_product(ring, dtype, A, B, C, layouts, pads=(0, 0, 0), workspace=False
     # nothing beyond the matrix was written
     lines = fd.reshape(-1, ldc)
     assert (lines[:, m if layouts[2] == COL else n:] == 77).all()
+    return op.last_route()
 
 
 def whole_numbers(g, shape, dtype, lo=-9, hi=10):
@@ -124,16 +125,22 @@ def distances(kind, g, shape, along):
     if kind == "almost zero":        # negative values and differences far below the resolution of the largest one
         small = torch.randint(-3, 4, shape, generator=g, device=dev).double() * 1e-310
         return torch.where(x < 0.01, 3e38, torch.where(x < 0.5, 0.0, small))
+    if kind == "bursts":             # stretches of k with negative values between ones that fit the screen: exact runs of
+        k = torch.arange(shape[along], device=dev)        # blocks, screened blocks behind them
+        burst = ((k // 32) % 7 < 3) & (k % 32 == 5)
+        return torch.where(burst[None, :] if along == 1 else burst[:, None], 90 - 100 * x, 100 * x + 1)
     if kind == "nan":
         return torch.where(x < 0.002, torch.nan, torch.where(x < 0.3, torch.inf, 100 * x))
     return torch.where(x < 0.002, -torch.inf, 100 * x)
 
 
-# one piece of K per tile of the output, and several (which then meet in D)
-@pytest.mark.parametrize("m, n, k", [(700, 650, 1500), (1021, 1023, 517), (129, 1290, 2000), (64, 70, 20001), (2305, 1025, 650)])
-@pytest.mark.parametrize("kind", ["edges", "signed", "ties", "falling", "wide", "almost zero", "nan", "infinite"])
+# Sizes the screened kernel gets: several pieces of K per tile of the output (which then meet in D), on even and odd lines, and
+# one; and sizes just below, which run exactly.
+@pytest.mark.parametrize("m, n, k, screened", [(1000, 1000, 3000, True), (1021, 1023, 4099, True), (129, 1290, 9001, True),
+                                               (2049, 2047, 2050, True), (700, 650, 1500, False), (64, 70, 5001, False)])
+@pytest.mark.parametrize("kind", ["edges", "signed", "ties", "falling", "wide", "almost zero", "bursts", "nan", "infinite"])
 @pytest.mark.parametrize("ring", ["minimum_plus", "maximum_plus"])
-def test_double_precision_tropical_products(cuda_device, ring, kind, m, n, k):
+def test_double_precision_tropical_products(cuda_device, ring, kind, m, n, k, screened):
     import torch
     g = torch.Generator(device="cuda").manual_seed(k)
     A, B = distances(kind, g, (m, k), 1), distances(kind, g, (k, n), 0)
@@ -144,9 +151,12 @@ def test_double_precision_tropical_products(cuda_device, ring, kind, m, n, k):
             A, B = A.flip(1), B.flip(0)
     if ring == "maximum_plus" and kind == "infinite":
         A, B = (torch.where(x == -torch.inf, torch.inf, x) for x in (A, B))
-    check_product(ring, "f64", A, B, C, (ROW, COL, ROW), (-k % 2, -k % 2, 0))
-    check_product(ring, "f64", A, B, C, (COL, COL, COL), (1, 0, 1), in_place=True)
-    check_product(ring, "f64", A, B, torch.full_like(C, -5.0 if ring == "minimum_plus" else 1e12), (COL, ROW, ROW))
+    want = "screened " if screened else "product "
+    for layouts, pads, C, in_place in (((ROW, COL, ROW), (-k % 2, -k % 2, 0), C, False), ((COL, COL, COL), (1, 0, 1), C, True),
+                                       ((COL, ROW, ROW), (0, 0, 0), torch.full_like(C, -5.0 if ring == "minimum_plus" else 1e12), False)):
+        route = check_product(ring, "f64", A, B, C, layouts, pads, in_place=in_place)
+        assert route.startswith(want), route
+        assert not screened or ("pieces=1 " in route) == (m == 2049), route
     assert device_status() == 0
 
 
