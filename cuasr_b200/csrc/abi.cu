@@ -708,8 +708,11 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
                            : slices > 1 ? "tma_splitk" : balanced ? "tma_balanced" : repacked ? "tma_repacked" : "tma";
   if constexpr (std::is_same<T, double>::value) {
     // the screened kernel, where it is modelled faster: no factor on the product (alpha is the identity of +) and a
-    // start value that compares, so that the running minimum can live in D
-    if (add_id == add_id && (desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM) && desc.mul_op == CUASR_OP_PLUS && alpha == T(0)) {
+    // start value that compares, so that the running minimum can live in D; and no negative zeros among the factors, so
+    // that D holds none and values that compare equal are the same
+    auto negative_zero = [](T x) { return x == T(0) && std::signbit(x); };
+    if (add_id == add_id && (desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM) && desc.mul_op == CUASR_OP_PLUS &&
+        alpha == T(0) && !negative_zero(alpha) && !(read_c && negative_zero(beta))) {
       const ScreenPlan screened = screen_plan(p.m, p.n, p.k, dev->sms, extra.count == 0);
       if (screened.cost < plan.cost) {
         const int st = run_screened<T>(desc.add_op == CUASR_OP_MAXIMUM, p, beta, add_id, read_c, screened, extra, dev, stream);

@@ -8,7 +8,8 @@
 // products in 2 clocks (measured 1.08 per product with its shared-memory reads).  A block of k whose 16-bit sums
 // cannot beat the element's current value cannot contain an improvement and is done; the few (element, block) pairs
 // that might improve are recomputed exactly, by four lanes each, from the exact tile in shared memory.  The result is
-// bit for bit that of the exact computation: the screen only ever lets too much through.
+// bit for bit that of the exact computation: the screen only ever lets too much through.  That includes the sign of zeros:
+// alpha and beta are not negative zeros here, so no term of D is one, and every product gets the + 0 that alpha stands for.
 //
 // Fixed point: q(x) = floor(x * 2^e) (ceil for max), finite values at most 16382, +inf (-inf for max) = 32767 (-16384),
 // so sums of finite values and sums with an infinity do not overlap.  2^e comes from the largest finite value of the
@@ -508,7 +509,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const int n = n_base + lc + 4 * j;
-            T v = acc[i][j];
+            T v = acc[i][j] + T(0);                          // alpha (x) product
             const bool inside = m < p.M && n < p.N;
             if (inside) {
               T* at = p.D + (long long)m * p.ldd + n;
@@ -718,7 +719,7 @@ screened_init_kernel(const __grid_constant__ ScreenParams<typename RingT::Elemen
   const long long total = (long long)p.M * p.N;
   for (long long idx = (long long)blockIdx.x * 256 + threadIdx.x; idx < total; idx += (long long)gridDim.x * 256) {
     const int m = static_cast<int>(idx / p.N), n = static_cast<int>(idx - (long long)m * p.N);
-    T v = p.add_identity;
+    T v = p.add_identity + T(0);                             // alpha (x) identity
     if (p.read_c) v = RingT::add(v, RingT::mul(p.beta, p.C[(long long)m * p.ldc + n]));
     p.D[(long long)m * p.ldd + n] = v;
   }

@@ -160,6 +160,32 @@ def test_double_precision_tropical_products(cuda_device, ring, kind, m, n, k, sc
     assert device_status() == 0
 
 
+@pytest.mark.parametrize("ring", ["minimum_plus", "maximum_plus"])
+@pytest.mark.parametrize("m, n, k", [(1000, 1000, 3000), (2049, 2047, 2050), (300, 200, 100)])
+def test_double_precision_tropical_zeros_are_positive(cuda_device, ring, m, n, k):
+    """D = (0 + A B) (+) (0 + C): adding zero makes every zero a positive one, whichever kernel does it."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(m)
+    sign = -1.0 if ring == "minimum_plus" else 1.0
+    better = Op.MINIMUM if ring == "minimum_plus" else Op.MAXIMUM
+    A, B = (torch.where(torch.rand(s, generator=g, device="cuda") < 0.001, -0.0, -sign) for s in ((m, k), (k, n)))
+    A, B = A.double(), B.double()
+    if ring == "maximum_plus":
+        A, B = -A.abs(), -B.abs()                 # best sums: -0 + -0
+    for beta in (0.0, -0.0):
+        C = torch.full((m, n), -sign * 5, dtype=torch.float64, device="cuda")
+        C[::2] = -0.0
+        D = torch.empty_like(C)
+        op = Srgemm(better, Op.PLUS, DType.F64, ROW, ROW, ROW, add_identity=-sign * np.inf)
+        assert op(Arguments((m, n, k), (A, k), (B, n), (C, n), (D, n), (0.0, beta))) == Status.kSuccess
+        zero = D == 0
+        assert zero.any() and (zero == (by_loop(ring, A, B, C) == 0)).all()
+        if beta == 0.0 and not np.signbit(beta):
+            assert not torch.signbit(D[zero]).any(), (int(torch.signbit(D[zero]).sum()), op.last_route())
+        else:
+            assert op.last_route().startswith("product ")
+
+
 # ---- distances with predecessors ----------------------------------------------------------------------------------
 # the 128 x 128 tile, and the 64 x 64 one with K shared by the CTAs of clusters
 @pytest.mark.parametrize("dtype", ["f32", "f64"])
