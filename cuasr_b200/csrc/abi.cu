@@ -525,6 +525,18 @@ int operand_mode(CUtensorMap* map, const void* ptr, long long ld, bool kcontig, 
   return kLoadGatherK;
 }
 
+// The screened kernel reads D back and updates it with atomics: only where D lies in this GPU's memory (or migrates there).
+// In host memory or on a peer every one of these crosses a link, where the exact kernel writes each element once.
+bool in_device_memory(const void* ptr) {
+  cudaPointerAttributes at = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&at, ptr) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeManaged || (at.type == cudaMemoryTypeDevice && at.device == dev);
+}
+
 // Launches the screened kernel on a normalised problem (row-major D).
 template <typename T>
 int run_screened(bool maximize, const Normalised& p, T beta, T add_id, bool read_c, const ScreenPlan& plan,
@@ -714,7 +726,7 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
     if (add_id == add_id && (desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM) && desc.mul_op == CUASR_OP_PLUS &&
         alpha == T(0) && !negative_zero(alpha) && !(read_c && negative_zero(beta))) {
       const ScreenPlan screened = screen_plan(p.m, p.n, p.k, dev->sms, extra.count == 0);
-      if (screened.cost < plan.cost) {
+      if (screened.cost < plan.cost && in_device_memory(p.d)) {
         const int st = run_screened<T>(desc.add_op == CUASR_OP_MAXIMUM, p, beta, add_id, read_c, screened, extra, dev, stream);
         if (st == CUASR_STATUS_SUCCESS) {
           t_last_kernel = name;

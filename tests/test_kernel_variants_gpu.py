@@ -186,6 +186,33 @@ def test_double_precision_tropical_zeros_are_positive(cuda_device, ring, m, n, k
             assert op.last_route().startswith("product ")
 
 
+def test_double_precision_tropical_product_into_host_memory(cuda_device):
+    """A D in mapped host memory is written once, by the exact kernel; under capture the question where D lies is asked too."""
+    import torch
+    m, n, k = 1000, 1000, 3000
+    g = torch.Generator(device="cuda").manual_seed(2)
+    A, B = (torch.rand(s, generator=g, device="cuda", dtype=torch.float64) for s in ((m, k), (k, n)))
+    C = torch.full((m, n), torch.inf, dtype=torch.float64, device="cuda")
+    host = torch.zeros((m, n), dtype=torch.float64).pin_memory()
+    here, captured = torch.zeros_like(C), torch.zeros_like(C)
+    op = Srgemm(Op.MINIMUM, Op.PLUS, DType.F64, ROW, ROW, ROW, add_identity=np.inf)
+
+    def product(D):
+        args = Arguments((m, n, k), (A, k), (B, n), (C, n), (D, n), (0.0, 0.0))
+        assert op(args, None, torch.cuda.current_stream()) == Status.kSuccess
+        return op.last_route()
+    assert product(host).startswith("product ")
+    assert product(here).startswith("screened ")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        assert product(captured).startswith("screened ")
+    graph.replay()
+    torch.cuda.synchronize()
+    want = by_loop("minimum_plus", A, B, C)
+    assert (here == want).all() and (captured == want).all() and (host.cuda() == want).all()
+    assert device_status() == 0
+
+
 # ---- distances with predecessors ----------------------------------------------------------------------------------
 # the 128 x 128 tile, and the 64 x 64 one with K shared by the CTAs of clusters
 @pytest.mark.parametrize("dtype", ["f32", "f64"])
