@@ -444,8 +444,8 @@ bool has_all_tiles(const cuasr_b200_desc_t& desc) {
 }
 
 // Every other ring (the integer min/max rings) has no value TMA could fill in.  With the optional workspace both
-// operands are copied and their K range is extended to a whole number of K steps: A with the additive identity, B
-// with the multiplicative one, so that every padded product is the additive identity.
+// operands are copied and their K range is extended to a whole number of K steps by repeating the last k, as the gather
+// does without the workspace: these rings are idempotent, and nothing depends on the caller's identities.
 // An operand that lies along its rows is copied, transposed, where that makes the modelled launch faster by more than the
 // copy takes (4000 clocks for its launch, 2200 bytes per clock): 2048^3 min-plus with one such operand 589 us gathered,
 // 538 copied; 4096^3 3998 and 4007.
@@ -695,18 +695,15 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
     char* cursor = static_cast<char*>(args.workspace) + copies_at;
     k_map = copies.k_padded > 0 ? copies.k_padded : p.k;
     const long long ldt = static_cast<long long>(align_up(static_cast<size_t>(k_map), 16 / sizeof(T)));
-    unsigned long long pad_a = 0, pad_b = 0;
-    std::memcpy(&pad_a, &add_id, sizeof(T));
-    std::memcpy(&pad_b, &mul_id, sizeof(T));
     RepackRequest requests[2];
     int count = 0;
     if (copies.a) {
-      requests[count++] = {p.a, p.lda, p.a_kcontig, p.m, p.k, k_map, pad_a, cursor, ldt};
+      requests[count++] = {p.a, p.lda, p.a_kcontig, p.m, p.k, k_map, cursor, ldt};
       p.a = cursor; p.lda = ldt; p.a_kcontig = true;
       cursor += repack_operand_bytes(p.m, k_map, sizeof(T));
     }
     if (copies.b) {
-      requests[count++] = {p.b, p.ldb, p.b_kcontig, p.n, p.k, k_map, pad_b, cursor, ldt};
+      requests[count++] = {p.b, p.ldb, p.b_kcontig, p.n, p.k, k_map, cursor, ldt};
       p.b = cursor; p.ldb = ldt; p.b_kcontig = true;
     }
     if (launch_repack(requests, count, sizeof(T), stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
@@ -1000,7 +997,7 @@ int cuasr_b200_pack_k_contiguous(int32_t dtype, const void* src, int64_t ld_src,
   const size_t es = dtype == CUASR_F64 ? 8 : 4;
   if (reinterpret_cast<uintptr_t>(src) % es != 0 || reinterpret_cast<uintptr_t>(dst) % es != 0)
     return CUASR_STATUS_ERROR_MISALIGNED_OPERAND;
-  const RepackRequest request = {src, ld_src, src_k_contiguous != 0, rows, k, k, 0ull, dst, ld_dst};
+  const RepackRequest request = {src, ld_src, src_k_contiguous != 0, rows, k, k, dst, ld_dst};
   if (launch_repack(&request, 1, es, static_cast<cudaStream_t>(stream)) != cudaSuccess)
     return CUASR_STATUS_ERROR_INTERNAL;
   g_launches.fetch_add(1);

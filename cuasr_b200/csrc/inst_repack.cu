@@ -11,7 +11,7 @@ static cudaError_t launch(const RepackRequest* requests, int count, cudaStream_t
     const long long tiles_r = (q.rows + 31) / 32, tiles_k = (q.K_out + 31) / 32;
     grid += tiles_r * tiles_k;
     if (grid > 2147483647LL) return cudaErrorInvalidValue;
-    op[i] = {static_cast<const W*>(q.src), q.ld_src, q.kcontig, q.rows, q.K, q.K_out, static_cast<W>(q.pad_bits),
+    op[i] = {static_cast<const W*>(q.src), q.ld_src, q.kcontig, q.rows, q.K, q.K_out,
              static_cast<W*>(q.dst), q.ld_dst, static_cast<int>(tiles_r), static_cast<int>(tiles_r * tiles_k)};
   }
   return launch_overlapped(repack_to_kcontig_kernel<W>, static_cast<int>(grid), 256, 0, 1, stream, op[0], op[1]);

@@ -7,13 +7,12 @@ namespace cuasr_b200 {
 
 // One operand to copy: rows x K elements (r, k) at src[r * ld_src + k] (kcontig: a copy, for addresses and leading
 // dimensions TMA cannot use) or src[r + k * ld_src] (a transposition), to dst[r * ld_dst + k]; columns K .. K_out - 1 of
-// the copy are set to `pad`.
+// the copy repeat column K - 1 (for an idempotent (+) a product taken twice changes nothing).
 template <typename W>
 struct RepackOperand {
   const W* src;
   long long ld_src;
   int kcontig, rows, K, K_out;
-  W pad;
   W* dst;
   long long ld_dst;
   int tiles_r, tiles;
@@ -38,7 +37,7 @@ repack_to_kcontig_kernel(const RepackOperand<W> first, const RepackOperand<W> se
 #pragma unroll
     for (int i = 0; i < 32; i += 8) {
       const int r = r0 + tx, k = k0 + ty + i;
-      if (r < o.rows && k < o.K) tile[ty + i][tx] = o.src[r + (long long)k * o.ld_src];
+      if (r < o.rows && k < o.K_out) tile[ty + i][tx] = o.src[r + (long long)min(k, o.K - 1) * o.ld_src];
     }
     __syncthreads();
   }
@@ -46,7 +45,7 @@ repack_to_kcontig_kernel(const RepackOperand<W> first, const RepackOperand<W> se
   for (int i = 0; i < 32; i += 8) {
     const int r = r0 + ty + i, k = k0 + tx;
     if (r < o.rows && k < o.K_out)
-      o.dst[(long long)r * o.ld_dst + k] = k >= o.K ? o.pad : o.kcontig ? o.src[(long long)r * o.ld_src + k] : tile[tx][ty + i];
+      o.dst[(long long)r * o.ld_dst + k] = o.kcontig ? o.src[(long long)r * o.ld_src + min(k, o.K - 1)] : tile[tx][ty + i];
   }
 }
 

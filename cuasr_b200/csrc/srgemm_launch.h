@@ -38,7 +38,6 @@ struct RepackRequest {
   long long ld_src;
   bool kcontig;
   int rows, K, K_out;
-  unsigned long long pad_bits;
   void* dst;
   long long ld_dst;
 };

@@ -92,8 +92,7 @@ CUASR_B200_API int cuasr_b200_srgemm(const cuasr_b200_desc_t *desc, const cuasr_
  *    contiguous dimension is not K (where the copy is expected to take less time than it saves), one whose address
  *    or leading dimension is not a multiple of 16 bytes (the reference accepts alignment 1,
  *    device/default_srgemm_configuration.h:88-89), and both operands of an integer min/max ring whose K is not a
- *    multiple of the kernel's K step (the copies are extended along K: A by the additive identity, B by the
- *    multiplicative one).  Without the workspace the kernel gathers such operands element by element.
+ *    multiple of the kernel's K step (the copies repeat the last k).  Without the workspace the kernel gathers such operands element by element.
  * The size depends on the operand addresses in `args`.  Needs a current device. */
 CUASR_B200_API size_t cuasr_b200_srgemm_optional_workspace_size(const cuasr_b200_desc_t *desc, const cuasr_b200_args_t *args);
 

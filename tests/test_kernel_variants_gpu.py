@@ -98,11 +98,13 @@ def test_ragged_k_does_not_lean_on_the_identities(cuda_device):
     caller's identities, whatever they are."""
     import torch
     g = torch.Generator(device="cuda").manual_seed(1)
-    for m, n, k in ((40, 50, 7), (200, 150, 45)):
+    for m, n, k in ((40, 50, 7), (200, 150, 45), (256, 192, 77)):
         A, B = (whole_numbers(g, s, "s32", 100, 200) for s in ((m, k), (k, n)))
         C = torch.full((m, n), 1000, dtype=torch.int32, device="cuda")
         for layouts in ((COL, COL, COL), (ROW, COL, ROW)):
             check_product("minimum_plus", "s32", A, B, C, layouts, (1, 1, 0), mul_identity=-2**31)
+            route = check_product("minimum_plus", "s32", A, B, C, layouts, (1, 1, 0), True, mul_identity=-2**31)
+            assert ("a=copy+tma b=copy+tma" in route) == (m == 256), route
 
 
 # ---- double precision minima and maxima, screened in 16 bits -------------------------------------------------------
