@@ -235,6 +235,9 @@ size_t splitk_bytes_for_pieces(const cuasr_b200_desc_t& desc, const cuasr_b200_a
 bool splitk_order_independent(const cuasr_b200_desc_t& desc) {
   return !(desc.add_op == CUASR_OP_PLUS && (desc.dtype == CUASR_F32 || desc.dtype == CUASR_F64));
 }
+// The SM count a launch is planned for.  How K is shared decides the order of a floating-point sum and with it the last bits,
+// so sums are planned for a B200's 148 SMs wherever they run (in a partition of the GPU with fewer they run in more waves).
+int planning_sms(const cuasr_b200_desc_t& desc, int sms) { return splitk_order_independent(desc) ? sms : 148; }
 long long splitk_pieces(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int sms, long long max_pieces) {
   const long long slices = args.split_k_slices;
   if (sms <= 0 || slices <= 1 || !splitk_order_independent(desc)) return slices;
@@ -632,6 +635,8 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   cudaStream_t stream = static_cast<cudaStream_t>(args.stream);
   Normalised p = normalise(desc, args);
 
+  const int plan_sms = planning_sms(desc, dev->sms);
+
   const T alpha = load_scalar<T>(args.alpha), beta = load_scalar<T>(args.beta);
   const T add_id = load_scalar<T>(args.add_identity), mul_id = load_scalar<T>(args.mul_identity);
   // semiring_linear_combination.h:118-125: C is read unless mult(beta, mult-identity) is the add-identity
@@ -646,8 +651,8 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   RepackPlan copies;
   size_t copies_at = 0;
   if (slices == 1 && args.workspace != nullptr && workspace_aligned) {
-    copies = repack_plan(desc, args, p, dev->sms);
-    copies_at = align_up(balance_workspace_bytes(desc, args, dev->sms), 256);
+    copies = repack_plan(desc, args, p, plan_sms);
+    copies_at = align_up(balance_workspace_bytes(desc, args, plan_sms), 256);
     if (copies.bytes == 0 || args.workspace_bytes < copies_at + copies.bytes) copies = RepackPlan();
   }
 
@@ -656,7 +661,7 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   const bool all_tiles = ring_has_all_tiles<T>(desc);
   const bool gather_a = !copies.a && (!p.a_kcontig || !tma_describable(p.a, p.lda, sizeof(T)));
   const bool gather_b = !copies.b && (!p.b_kcontig || !tma_describable(p.b, p.ldb, sizeof(T)));
-  LaunchPlan plan = plan_without_workspace(desc, p.m, p.n, p.k, dev->sms, all_tiles, gather_a, gather_b);
+  LaunchPlan plan = plan_without_workspace(desc, p.m, p.n, p.k, plan_sms, all_tiles, gather_a, gather_b);
   bool tickets_used = false, balanced = false;
   auto take_ticket_plan = [&](int whole_tiles, int pieces, double cost) {
     plan.tile = kLargeTile; plan.cluster = 1; plan.whole_tiles = whole_tiles; plan.pieces = pieces; plan.cost = cost;
@@ -671,16 +676,16 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
       // it sooner; floating-point sums keep the cutting that was asked for
       const size_t per_piece = splitk_bytes_for_pieces(desc, args, 1) - splitk_bytes_for_pieces(desc, args, 0);
       const long long room = static_cast<long long>((args.workspace_bytes - splitk_bytes_for_pieces(desc, args, 0)) / per_piece);
-      const int pieces = static_cast<int>(splitk_pieces(desc, args, dev->sms, room));
-      const double cost = ticket_plan_cost(desc, tiles, 0, pieces, p.k, dev->sms, gather_a + gather_b);
+      const int pieces = static_cast<int>(splitk_pieces(desc, args, plan_sms, room));
+      const double cost = ticket_plan_cost(desc, tiles, 0, pieces, p.k, plan_sms, gather_a + gather_b);
       if (cost < plan.cost || !splitk_order_independent(desc)) take_ticket_plan(0, pieces, cost);
     }
   } else if (args.workspace != nullptr && workspace_aligned && all_tiles) {
     // an optional workspace on an unsplit launch buys load balancing, if it is large enough for the plan
-    const BalancePlan wish = balance_plan(tiles, dev->sms, (args.k + TK - 1) / TK);
-    if (wish.pieces > 1 && args.workspace_bytes >= balance_workspace_bytes(desc, args, dev->sms)) {
+    const BalancePlan wish = balance_plan(tiles, plan_sms, (args.k + TK - 1) / TK);
+    if (wish.pieces > 1 && args.workspace_bytes >= balance_workspace_bytes(desc, args, plan_sms)) {
       balanced = true;
-      const double cost = ticket_plan_cost(desc, tiles, wish.whole_tiles, wish.pieces, p.k, dev->sms, gather_a + gather_b);
+      const double cost = ticket_plan_cost(desc, tiles, wish.whole_tiles, wish.pieces, p.k, plan_sms, gather_a + gather_b);
       if (cost < plan.cost) take_ticket_plan(wish.whole_tiles, wish.pieces, cost);
     }
   }
@@ -903,8 +908,9 @@ size_t cuasr_b200_srgemm_optional_workspace_size(const cuasr_b200_desc_t* desc, 
   if (args->split_k_slices > 1) return 0;
   DeviceState* dev = nullptr;
   if (!device_state(&dev)) return 0;
-  const size_t repack = repack_plan(*desc, *args, normalise(*desc, *args), dev->sms).bytes;
-  const size_t balance = balance_workspace_bytes(*desc, *args, dev->sms);
+  const int sms = planning_sms(*desc, dev->sms);
+  const size_t repack = repack_plan(*desc, *args, normalise(*desc, *args), sms).bytes;
+  const size_t balance = balance_workspace_bytes(*desc, *args, sms);
   return repack > 0 ? align_up(balance, 256) + repack : balance;
 }
 
