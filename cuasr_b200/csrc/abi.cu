@@ -329,6 +329,7 @@ struct ExtraOutputs {
 // read (the tensor map ends at K).
 struct RepackPlan {
   bool a = false, b = false;
+  bool faster_a = false, faster_b = false;   // copied although TMA could bring in the operand's lines as they are
   int k_padded = 0;      // > 0: both copies are extended along K to this length (a multiple of the kernel's K step)
   size_t bytes = 0;
 };
@@ -361,13 +362,17 @@ bool ring_pads_itself(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& ar
 // ---- which tile, and how K is shared ---------------------------------------------------------------------------
 // Clocks the 8 consumer warps of a CTA (two per scheduler, 64 products per lane and k) take for one k: measured per
 // product and scheduler 2.07 (fp32 with a packed add and a three-input minimum, fused integer add-min, one logic
-// instruction), 3.0 (two-instruction bottleneck products), 8.2 (fp64 minima), 2.1 (fp64 sums on the tensor cores).
-double clocks_per_k(const cuasr_b200_desc_t& desc) {
-  const bool sum = desc.add_op == CUASR_OP_PLUS;
+// instruction), 3.0 (two-instruction bottleneck products), 1.55 (fp32 sums), 2.1 (fp64 sums on the tensor cores), and for fp64
+// minima by tile (4096^3 on the large tile, 1000^3 on 128 x 64, 2048^3 on 64 x 64).
+double clocks_per_k(const cuasr_b200_desc_t& desc, int tile) {
+  static constexpr double f64_min[4] = {6.6, 7.1, 7.2, 7.3}, f64_bottleneck[4] = {9.1, 9.6, 9.5, 9.7};
+  const bool sum = desc.add_op == CUASR_OP_PLUS, logical = desc.mul_op == CUASR_OP_BINARY_AND;
+  const bool bottleneck = desc.mul_op == CUASR_OP_MINIMUM || desc.mul_op == CUASR_OP_MAXIMUM;
   double per_product = 2.1;
-  if (desc.dtype == CUASR_F64) per_product = sum ? 2.1 : 8.2;
-  else if (desc.mul_op == CUASR_OP_MINIMUM || desc.mul_op == CUASR_OP_MAXIMUM) per_product = 3.0;
-  else if (desc.mul_op == CUASR_OP_BINARY_AND) per_product = 5.0;
+  if (desc.dtype == CUASR_F64) per_product = sum ? 2.1 : logical ? 10.0 : bottleneck ? f64_bottleneck[tile] : f64_min[tile];
+  else if (desc.dtype == CUASR_F32 && sum) per_product = 1.55;
+  else if (bottleneck) per_product = 3.0;
+  else if (logical) per_product = 9.0;
   return 2 * 64 * per_product;
 }
 
@@ -395,17 +400,49 @@ int tile_sub(int tile, const cuasr_b200_desc_t& desc) {
 // for every chunk of a warp: 250 clocks a stage, twice that for 8-byte elements (a 512 x 4096 x 4096 product as seven waves of it took 635 us instead of
 // the 514 modelled without; the 128 x 128 tile takes 580).
 // A gathered element costs 0.17 clocks on the small tiles where the contraction is bound by register reads (2048^3
-// min-plus with one operand transposed on 64 x 64 tiles: 589 us against 522 with TMA), 0.08 in the other rings (max-min:
-// 795 against 765), and 0.07 and 0.02 on the large one (4096^3: 3998 against 3969, both operands 4096).
-double gather_clocks(const cuasr_b200_desc_t& desc, bool large) {
-  const bool packed = desc.dtype == CUASR_F32 && (desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM) &&
-                      (desc.mul_op == CUASR_OP_PLUS || desc.mul_op == CUASR_OP_MULTIPLIES);
-  return packed ? (large ? 0.07 : 0.17) : (large ? 0.02 : 0.08);
+// min-plus with one operand transposed on 64 x 64 tiles: 589 us against 522 with TMA) and in fp32 sums (457 against 373), 0.08
+// in the other rings (max-min: 795 against 765), and 0.07, 0.155 and 0.02 on the large one (4096^3 min-plus: 3998 against 3969,
+// both operands 4096; fp32 sums 3240 against 2950).
+bool packs_pairs(const cuasr_b200_desc_t& desc) {          // Ring::kPackedPairs
+  return desc.dtype == CUASR_F32 && (desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM) &&
+         (desc.mul_op == CUASR_OP_PLUS || desc.mul_op == CUASR_OP_MULTIPLIES);
 }
-LaunchPlan plan_without_workspace(const cuasr_b200_desc_t& desc, int m, int n, int k, int sms, bool all_tiles, bool gather_a,
-                                  bool gather_b) {
+// Rings whose large tile has variants for operands along their rows (LargeRowsTile).
+bool takes_rows(const cuasr_b200_desc_t& desc) {
+  if (desc.dtype == CUASR_F64 && desc.add_op != CUASR_OP_PLUS) return desc.mul_op != CUASR_OP_PLUS && desc.mul_op != CUASR_OP_MULTIPLIES;
+  return !packs_pairs(desc);
+}
+double gather_clocks(const cuasr_b200_desc_t& desc, bool large) {
+  if (desc.dtype == CUASR_F32 && desc.add_op == CUASR_OP_PLUS) return large ? 0.155 : 0.18;
+  return packs_pairs(desc) ? (large ? 0.07 : 0.17) : (large ? 0.02 : 0.08);
+}
+
+// Which operands a launch has to gather, given which ones are copied first.  The large tile takes operands that lie along
+// their rows as they are where TMA can bring in both (rows_a, rows_b) and the ring gains nothing from pairs of k.
+struct Gathers {
+  bool a = false, b = false;                 // the smaller tiles
+  bool large_a = false, large_b = false;
+  bool rows_a = false, rows_b = false;       // large tile: along its rows, by TMA
+};
+Gathers gathers_of(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, const Normalised& p, bool copied_a, bool copied_b) {
+  const size_t es = desc.dtype == CUASR_F64 ? 8 : 4;
+  const int tk = kTileKBytes / static_cast<int>(es);
+  const bool by_tma_a = copied_a || tma_describable(p.a, p.lda, es), by_tma_b = copied_b || tma_describable(p.b, p.ldb, es);
+  const bool along_k_a = copied_a || p.a_kcontig, along_k_b = copied_b || p.b_kcontig;
+  Gathers g;
+  g.a = g.large_a = !along_k_a || !by_tma_a;
+  g.b = g.large_b = !along_k_b || !by_tma_b;
+  const bool dense = p.lda >= (p.a_kcontig ? p.k : p.m) && p.ldb >= (p.b_kcontig ? p.k : p.n);
+  if (takes_rows(desc) && by_tma_a && by_tma_b && dense && (p.k % tk == 0 || ring_pads_itself(desc, args))) {
+    g.rows_a = !along_k_a; g.rows_b = !along_k_b;
+    g.large_a = g.large_b = false;
+  }
+  return g;
+}
+
+LaunchPlan plan_without_workspace(const cuasr_b200_desc_t& desc, int m, int n, int k, int sms, bool all_tiles, const Gathers& g) {
   const int tk = kTileKBytes / (desc.dtype == CUASR_F64 ? 8 : 4);
-  const double per_k = clocks_per_k(desc), wide = desc.dtype == CUASR_F64 ? 2.0 : 1.0;
+  const double wide = desc.dtype == CUASR_F64 ? 2.0 : 1.0;
   LaunchPlan best;
   for (int tile = all_tiles ? kLargeTile : kSmallTile; tile <= kTinyTile; ++tile) {
     const long long tiles = static_cast<long long>((m + kTileRows[tile] - 1) / kTileRows[tile]) * ((n + kTileCols[tile] - 1) / kTileCols[tile]);
@@ -417,8 +454,9 @@ LaunchPlan plan_without_workspace(const cuasr_b200_desc_t& desc, int m, int n, i
       const long long room = z <= 2 ? sms : z == 4 ? sms * 36LL / 37 : sms * 32LL / 37;
       const long long waves = (tiles * z + room - 1) / room;
       const double end = (tile == kLargeTile ? 2000 : 1500) * wide + (z > 1 ? 2500 + (waves > 1 ? 4000 : 0) : 0);
+      const bool gather_a = tile == kLargeTile ? g.large_a : g.a, gather_b = tile == kLargeTile ? g.large_b : g.b;
       const double gathered = gather_clocks(desc, tile == kLargeTile) * step * ((gather_a ? kTileRows[tile] : 0) + (gather_b ? kTileCols[tile] : 0));
-      const double per_stage = per_k * step / kTileWk[tile] + gathered + (tile == kTinyTile ? 250 * wide : 0);
+      const double per_stage = clocks_per_k(desc, tile) * step / kTileWk[tile] + gathered + (tile == kTinyTile ? 250 * wide : 0);
       const double cost = 3000 + static_cast<double>(waves) * (per_stage * per_piece + end);
       if (cost < best.cost) {
         best.tile = tile; best.cluster = z; best.cost = cost;
@@ -450,8 +488,16 @@ bool has_all_tiles(const cuasr_b200_desc_t& desc) {
 // operands are copied and their K range is extended to a whole number of K steps by repeating the last k, as the gather
 // does without the workspace: these rings are idempotent, and nothing depends on the caller's identities.
 // An operand that lies along its rows is copied, transposed, where that makes the modelled launch faster by more than the
-// copy takes (4000 clocks for its launch, 2200 bytes per clock): 2048^3 min-plus with one such operand 589 us gathered,
-// 538 copied; 4096^3 3998 and 4007.
+// copy takes (12000 clocks for its launch and the tail of its stores, 2200 bytes per clock): 2048^3 min-plus with one such
+// operand 589 us gathered, 538 copied; 4096^3 3998 and 4007.
+size_t copies_bytes(const RepackPlan& plan, const Normalised& p, size_t es) {
+  const int k = plan.k_padded > 0 ? plan.k_padded : p.k;
+  return (plan.a ? repack_operand_bytes(p.m, k, es) : 0) + (plan.b ? repack_operand_bytes(p.n, k, es) : 0);
+}
+double copies_clocks(const RepackPlan& plan, const Normalised& p, size_t es) {
+  if (!plan.a && !plan.b) return 0;
+  return 12000.0 + 2.0 * es * p.k * ((plan.a ? p.m : 0.0) + (plan.b ? p.n : 0.0)) / 2200;
+}
 RepackPlan repack_plan(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, const Normalised& p, int sms) {
   RepackPlan plan;
   const size_t es = desc.dtype == CUASR_F64 ? 8 : 4;
@@ -467,17 +513,18 @@ RepackPlan repack_plan(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& a
     plan.a = !tma_describable(p.a, p.lda, es);
     plan.b = !tma_describable(p.b, p.ldb, es);
     const bool all_tiles = has_all_tiles(desc);
-    auto cost = [&](bool gather_a, bool gather_b) {
-      return plan_without_workspace(desc, p.m, p.n, p.k, sms, all_tiles, gather_a, gather_b).cost;
+    auto cost = [&](bool copy_a, bool copy_b) {
+      return plan_without_workspace(desc, p.m, p.n, p.k, sms, all_tiles, gathers_of(desc, args, p, copy_a, copy_b)).cost;
     };
-    auto copy = [&](bool first, int rows) { return (first ? 4000.0 : 0.0) + 2.0 * es * rows * p.k / 2200; };
-    const bool along_a = !p.a_kcontig && !plan.a, along_b = !p.b_kcontig && !plan.b;
-    if (along_a && cost(true, along_b) - cost(false, along_b) > copy(!plan.b, p.m)) plan.a = true;
-    const bool gather_a = along_a && !plan.a;
-    if (along_b && cost(gather_a, true) - cost(gather_a, false) > copy(!plan.a, p.n)) plan.b = true;
+    for (const bool first : {true, false}) {
+      RepackPlan more = plan;
+      bool& copied = first ? more.a : more.b;
+      if (copied || (first ? p.a_kcontig : p.b_kcontig)) continue;
+      copied = (first ? more.faster_a : more.faster_b) = true;
+      if (cost(more.a, more.b) + copies_clocks(more, p, es) < cost(plan.a, plan.b) + copies_clocks(plan, p, es)) plan = more;
+    }
   }
-  const int k_copy = plan.k_padded > 0 ? plan.k_padded : p.k;
-  plan.bytes = (plan.a ? repack_operand_bytes(p.m, k_copy, es) : 0) + (plan.b ? repack_operand_bytes(p.n, k_copy, es) : 0);
+  plan.bytes = copies_bytes(plan, p, es);
   return plan;
 }
 
@@ -512,7 +559,7 @@ double ticket_plan_cost(const cuasr_b200_desc_t& desc, long long tiles, int whol
   const int tk = kTileKBytes / (desc.dtype == CUASR_F64 ? 8 : 4);
   const double wide = desc.dtype == CUASR_F64 ? 2.0 : 1.0;
   const int k_steps = (k + tk - 1) / tk, per_piece = (k_steps + pieces - 1) / pieces;
-  const double per_step = (clocks_per_k(desc) + gather_clocks(desc, true) * kTileM * gathered) * tk;
+  const double per_step = (clocks_per_k(desc, kLargeTile) + gather_clocks(desc, true) * kTileM * gathered) * tk;
   const long long waves = whole_tiles / sms, tail = ((tiles - whole_tiles) * pieces + sms - 1) / sms;
   // the tickets are cleared by a memset in front of the launch; a piece is parked and read back by the last one
   return 3000 + 4000 + waves * (per_step * k_steps + 2000 * wide) + tail * (per_step * per_piece + 1000 * wide) + 1000 * wide * pieces;
@@ -647,47 +694,61 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   // partials are moved 16 bytes at a time and re-packed operands are read by TMA: a workspace that does not start
   // on a 16-byte boundary is an error where it is required and is left unused where it is optional
   const bool workspace_aligned = reinterpret_cast<uintptr_t>(args.workspace) % 16 == 0;
-  // the copies an optional workspace has room for, behind the scratch of a balanced launch
-  RepackPlan copies;
-  size_t copies_at = 0;
-  if (slices == 1 && args.workspace != nullptr && workspace_aligned) {
-    copies = repack_plan(desc, args, p, plan_sms);
-    copies_at = align_up(balance_workspace_bytes(desc, args, plan_sms), 256);
-    if (copies.bytes == 0 || args.workspace_bytes < copies_at + copies.bytes) copies = RepackPlan();
-  }
-
   constexpr int TK = kTileKBytes / sizeof(T);
   const long long tiles = static_cast<long long>(tile_count(args));
   const bool all_tiles = ring_has_all_tiles<T>(desc);
-  const bool gather_a = !copies.a && (!p.a_kcontig || !tma_describable(p.a, p.lda, sizeof(T)));
-  const bool gather_b = !copies.b && (!p.b_kcontig || !tma_describable(p.b, p.ldb, sizeof(T)));
-  LaunchPlan plan = plan_without_workspace(desc, p.m, p.n, p.k, plan_sms, all_tiles, gather_a, gather_b);
-  bool tickets_used = false, balanced = false;
-  auto take_ticket_plan = [&](int whole_tiles, int pieces, double cost) {
-    plan.tile = kLargeTile; plan.cluster = 1; plan.whole_tiles = whole_tiles; plan.pieces = pieces; plan.cost = cost;
-    tickets_used = true;
-  };
+  const size_t balance_bytes = slices == 1 && all_tiles ? balance_workspace_bytes(desc, args, plan_sms) : 0;
+  const BalancePlan balance = balance_plan(tiles, plan_sms, (args.k + TK - 1) / TK);
+  // an optional workspace buys load balancing and, behind its scratch, copies of operands, as far as it has room for them
+  const bool optional = slices == 1 && args.workspace != nullptr && workspace_aligned;
+  const bool balanced = optional && balance_bytes > 0 && args.workspace_bytes >= balance_bytes;
+  const size_t copies_at = align_up(slices == 1 ? balance_workspace_bytes(desc, args, plan_sms) : 0, 256);
+  RepackPlan copies;
+  if (optional) {
+    copies = repack_plan(desc, args, p, plan_sms);
+    if (copies.bytes == 0 || args.workspace_bytes < copies_at + copies.bytes) copies = RepackPlan();
+  }
+  long long pieces = 1;
   if (slices > 1) {
     const size_t need = splitk_workspace_bytes(desc, args);
     if (args.workspace_bytes < need) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
     if (!workspace_aligned) return CUASR_STATUS_ERROR_MISALIGNED_OPERAND;
     if (all_tiles) {
-      // as many pieces as the workspace at hand has room for (it always has room for `slices`), unless a cluster does
-      // it sooner; floating-point sums keep the cutting that was asked for
+      // as many pieces as the workspace at hand has room for (it always has room for `slices`)
       const size_t per_piece = splitk_bytes_for_pieces(desc, args, 1) - splitk_bytes_for_pieces(desc, args, 0);
       const long long room = static_cast<long long>((args.workspace_bytes - splitk_bytes_for_pieces(desc, args, 0)) / per_piece);
-      const int pieces = static_cast<int>(splitk_pieces(desc, args, plan_sms, room));
-      const double cost = ticket_plan_cost(desc, tiles, 0, pieces, p.k, plan_sms, gather_a + gather_b);
-      if (cost < plan.cost || !splitk_order_independent(desc)) take_ticket_plan(0, pieces, cost);
+      pieces = splitk_pieces(desc, args, plan_sms, room);
     }
-  } else if (args.workspace != nullptr && workspace_aligned && all_tiles) {
-    // an optional workspace on an unsplit launch buys load balancing, if it is large enough for the plan
-    const BalancePlan wish = balance_plan(tiles, plan_sms, (args.k + TK - 1) / TK);
-    if (wish.pieces > 1 && args.workspace_bytes >= balance_workspace_bytes(desc, args, plan_sms)) {
-      balanced = true;
-      const double cost = ticket_plan_cost(desc, tiles, wish.whole_tiles, wish.pieces, p.k, plan_sms, gather_a + gather_b);
-      if (cost < plan.cost) take_ticket_plan(wish.whole_tiles, wish.pieces, cost);
-    }
+  }
+  // the fastest launch with a given set of copies: without the workspace, or in pieces that meet through tickets in it
+  Gathers gathers;
+  bool tickets_used = false;
+  auto plan_with = [&](const RepackPlan& c, Gathers& g, bool& tickets) {
+    g = gathers_of(desc, args, p, c.a, c.b);
+    LaunchPlan best = plan_without_workspace(desc, p.m, p.n, p.k, plan_sms, all_tiles, g);
+    tickets = false;
+    auto in_pieces = [&](int whole_tiles, int count, bool always) {
+      const double cost = ticket_plan_cost(desc, tiles, whole_tiles, count, p.k, plan_sms, g.large_a + g.large_b);
+      if (cost >= best.cost && !always) return;
+      best.tile = kLargeTile; best.cluster = 1; best.whole_tiles = whole_tiles; best.pieces = count; best.cost = cost;
+      tickets = true;
+    };
+    // floating-point sums keep the cutting that was asked for
+    if (slices > 1 && all_tiles) in_pieces(0, static_cast<int>(pieces), !splitk_order_independent(desc));
+    if (balanced) in_pieces(balance.whole_tiles, balance.pieces, false);
+    best.cost += copies_clocks(c, p, sizeof(T));
+    return best;
+  };
+  LaunchPlan plan = plan_with(copies, gathers, tickets_used);
+  if (copies.faster_a || copies.faster_b) {          // in pieces the large tile may do as well on the operands as they are
+    RepackPlan fewer = copies;
+    fewer.a = copies.a && !copies.faster_a; fewer.b = copies.b && !copies.faster_b;
+    fewer.faster_a = fewer.faster_b = false;
+    fewer.bytes = copies_bytes(fewer, p, sizeof(T));
+    Gathers g;
+    bool tickets;
+    const LaunchPlan other = plan_with(fewer, g, tickets);
+    if (other.cost < plan.cost) { plan = other; copies = fewer; gathers = g; tickets_used = tickets; }
   }
   const bool pads_itself = ring_pads_itself(desc, args);
   // operands whose storage lines overlap (leading dimension below the contiguous extent) stay off the TMA path
@@ -749,6 +810,12 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   tp.a_mode = p.a_kcontig ? (fill_ok && tma_describable(p.a, p.lda, sizeof(T)) ? kLoadTma : kLoadGatherK) : kLoadGatherMN;
   tp.b_mode = p.b_kcontig ? (fill_ok && tma_describable(p.b, p.ldb, sizeof(T)) ? kLoadTma : kLoadGatherK) : kLoadGatherMN;
   CUtensorMap map_a = {}, map_b = {};
+  if (plan.tile == kLargeTile && (gathers.rows_a || gathers.rows_b) && encode_tiled_fn() != nullptr &&
+      make_operand_map<T>(&map_a, tp.A, p.lda, p.m, k_map, !gathers.rows_a, nan_pad) &&
+      make_operand_map<T>(&map_b, tp.B, p.ldb, p.n, k_map, !gathers.rows_b, nan_pad)) {
+    tp.a_mode = gathers.rows_a ? kLoadTmaRows : kLoadTma;
+    tp.b_mode = gathers.rows_b ? kLoadTmaRows : kLoadTma;
+  }
   if (tp.a_mode == kLoadTma &&
       !make_operand_map<T>(&map_a, tp.A, p.lda, p.m, k_map, true, nan_pad, kTileRows[plan.tile])) tp.a_mode = kLoadGatherK;
   if (tp.b_mode == kLoadTma &&

@@ -17,6 +17,7 @@ enum LoadMode : int {
   kLoadTma = 0,          // contiguous along k, 16-byte aligned storage lines: TMA
   kLoadGatherK = 1,      // contiguous along k, any alignment: lanes along k
   kLoadGatherMN = 2,     // contiguous along rows, any alignment: 8 rows x 4 k per warp instruction
+  kLoadTmaRows = 3,      // contiguous along rows, 16-byte aligned storage lines: TMA, as it lies (large tile, see LargeRowsTile)
 };
 
 template <int kBytes>

@@ -38,6 +38,13 @@ cudaError_t launch_tma(int tile, const CUtensorMap& map_a, const CUtensorMap& ma
                        int grid, int cluster, cudaStream_t stream) {
   using R = Ring<ADD, MUL, T>;
   if constexpr (all_tiles_instantiated<ADD, MUL, T>()) {
+    constexpr bool rows = !R::kPackedPairs && (sizeof(T) == 4 || ADD == CUASR_OP_PLUS || (MUL != CUASR_OP_PLUS && MUL != CUASR_OP_MULTIPLIES));
+    if constexpr (rows) {                // takes_rows
+      const bool rows_a = params.a_mode == kLoadTmaRows, rows_b = params.b_mode == kLoadTmaRows;
+      if (rows_a && rows_b) return launch_tma_variant<R, LargeRowsTile<true, true>>(map_a, map_b, params, grid, cluster, stream);
+      if (rows_a) return launch_tma_variant<R, LargeRowsTile<true, false>>(map_a, map_b, params, grid, cluster, stream);
+      if (rows_b) return launch_tma_variant<R, LargeRowsTile<false, true>>(map_a, map_b, params, grid, cluster, stream);
+    }
     if (tile == kLargeTile)
       return params.a_mode == kLoadTma && params.b_mode == kLoadTma
                  ? launch_tma_variant<R, LargeTmaTile>(map_a, map_b, params, grid, cluster, stream)

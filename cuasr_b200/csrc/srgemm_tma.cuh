@@ -45,9 +45,10 @@ constexpr int kEpilogueWarpBytes = 8192;          // per consumer warp: staging 
 constexpr int kMaxDestinations = 8;               // output copies one launch can write (this GPU + peers)
 constexpr int kMaxSmemBytes = 232448;             // 227 KiB: what one CTA may have
 
-// Tile shape of a kernel variant.
-template <int WM_, int WN_, int WK_, int kSub_ = WK_ == 4 ? 2 : 1, bool kGathers_ = true>
+// Tile shape of a kernel variant.  kRowsA / kRowsB: the operand lies along its rows and TMA brings it in as it lies.
+template <int WM_, int WN_, int WK_, int kSub_ = WK_ == 4 ? 2 : 1, bool kGathers_ = true, bool kRowsA_ = false, bool kRowsB_ = false>
 struct TileShape {
+  static constexpr bool kRowsA = kRowsA_, kRowsB = kRowsB_;
   // Without the gather the producers need no more than 40 registers, and the consumers of the 128 x 128 tile get the 232
   // that hold their fragments and tables without spilling (see LargeTmaTile).
   static constexpr bool kGathers = kGathers_;
@@ -74,6 +75,13 @@ using LargeTile = TileShape<2, 4, 1>;    // 128 x 128
 // The same where TMA brings in both operands.  With the gather compiled in (224 registers) the fp32 tropical contraction
 // spills 64 bytes: 256 x 256 x 262144 split along K takes 1049 us with it and 1036 without, 8192^3 31.38 and 31.20 ms.
 using LargeTmaTile = TileShape<2, 4, 1, 1, false>;
+// The same with operands that lie along their rows, which TMA then brings in as they lie: a stage of such an operand is
+// [k][128 rows], a 16-byte vector holds rows of one k.  Not for the rings that need pairs of k in a register
+// (Ring::kPackedPairs), nor for fp64 products that are sums or products, which run as fast on gathered stages (see order_of).
+// 4096^3, operand B along its rows, gathered and as it lies: max-min fp32 5975 and 5871 us, s32 min-plus 4130 and 4017, fp32 sums
+// 3240 and 2935, fp64 max-min 17333 and 16581.
+template <bool kRowsA, bool kRowsB>
+using LargeRowsTile = TileShape<2, 4, 1, 1, false, kRowsA, kRowsB>;
 using MediumTile = TileShape<2, 2, 2>;   // 128 x 64
 using SmallTile = TileShape<1, 2, 4>;    // 64 x 64
 // 64 x 32, one 16-byte chunk of k per warp and stage: the shortest chain for the smallest products, and the finest
@@ -175,12 +183,29 @@ __device__ __forceinline__ void decode_work(const TmaParams<T>& p, int w, int nu
   }
 }
 
+// Order of the 128 updates of a lane for one 16-byte chunk (two k) of 8-byte elements: column by column with k outside the
+// rows or inside, by half tiles, or k outermost.  us at 4096^3 on 128 x 128 tiles / 1000^3 on 128 x 64 / 2048^3 on 64 x 64,
+// both operands K-contiguous:
+//   min-plus  by column 12255 / 258 / 1767, by element 12239 / 255 / 1689, by half 12390 / 237 / 1828, by k 12774 / 237 / 1977,
+//             rows outside columns 13770 - 14360 / 242 - 273 / 1750 - 1860; with one operand gathered by column 12295, by element 13145;
+//   max-min   by column 17500 / 323 / 2310, by half 17290 / 321 / 2233, by k 17315 / 322 / 2290; with operands along rows by k 16581
+//             (one) and 16843 (both), by half 17192 and 16971.
+enum UpdateOrder : int { kByColumn, kByElement, kByHalf, kByK };
+template <typename RingT, typename Tile>
+__host__ __device__ constexpr int order_of() {
+  constexpr bool compares_only = RingT::kMul != CUASR_OP_PLUS && RingT::kMul != CUASR_OP_MULTIPLIES;
+  if (Tile::WK == 1) return compares_only ? kByK : kByColumn;
+  return compares_only || Tile::WK == 2 ? kByHalf : kByElement;
+}
+
 template <typename RingT, typename Tile>
 __global__ void __launch_bounds__(kTmaThreads, 1)
 srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                   const __grid_constant__ TmaParams<typename RingT::Element> p) {
   using T = typename RingT::Element;
   constexpr int WM = Tile::WM, WN = Tile::WN, WK = Tile::WK, kSub = Tile::kSub;
+  constexpr bool kRowsA = Tile::kRowsA, kRowsB = Tile::kRowsB;
+  static_assert(!(kRowsA || kRowsB) || (WK == 1 && kSub == 1 && !Tile::kGathers), "operands along rows: the large tile, by TMA");
   constexpr int kStages = Tile::template kStages<T>;
   static_assert(kStages >= 2, "at least double-buffered");
   constexpr int EV = 16 / sizeof(T);              // elements per 16-byte vector: 4 (fp32/int32) or 2 (fp64)
@@ -247,8 +272,10 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           mbar_arrive_expect_tx(&full_bar[s], (a_tma ? Tile::kABytes : 0) + (b_tma ? Tile::kBBytes : 0));
 #pragma unroll
           for (int sub = 0; sub < kSub; ++sub) {
-            if (a_tma) tma_load_2d(sa + sub * (Tile::kM * 128), &map_a, &full_bar[s], k0 + sub * TK, m0);
-            if (b_tma) tma_load_2d(sb + sub * (Tile::kN * 128), &map_b, &full_bar[s], k0 + sub * TK, n0);
+            if (kRowsA)     tma_load_2d(sa, &map_a, &full_bar[s], m0, k0);
+            else if (a_tma) tma_load_2d(sa + sub * (Tile::kM * 128), &map_a, &full_bar[s], k0 + sub * TK, m0);
+            if (kRowsB)     tma_load_2d(sb, &map_b, &full_bar[s], n0, k0);
+            else if (b_tma) tma_load_2d(sb + sub * (Tile::kN * 128), &map_b, &full_bar[s], k0 + sub * TK, n0);
           }
         }
         if (gathers) {
@@ -282,23 +309,31 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   // Row i (0..7) of this lane inside the warp's 64 rows; column j (0..7) inside the warp's 32 columns.
   // Plus-times fp64 runs on the tensor cores (DMMA): acc[mb][2 nb + e] is then element e of the lane's
   // accumulator pair of the 8 x 8 block (mb, nb) of the warp tile; its row inside the block is lr, its column
-  // 2 lc + e.
+  // 2 lc + e.  Blocks fed from an operand along its rows are interleaved in pairs (see the loaders below).
   constexpr bool kDmma = std::is_same<T, double>::value && RingT::kAdd == CUASR_OP_PLUS &&
                          RingT::kMul == CUASR_OP_MULTIPLIES;
-  auto row_of = [&](int i) { return 8 * i + lr; };
-  auto col_of = [&](int j) { return kDmma ? (8 * (j / 2) + 2 * lc + (j % 2)) : (lc + 4 * j); };
+  auto row_of = [&](int i) {
+    if (!kRowsA) return 8 * i + lr;
+    return kDmma ? 16 * (i / 2) + 2 * lr + (i % 2) : EV * lr + (i % EV) + 8 * EV * (i / EV);
+  };
+  auto col_of = [&](int j) {
+    if (kDmma) return kRowsB ? 16 * (j / 4) + 4 * lc + 2 * (j % 2) + ((j / 2) % 2) : 8 * (j / 2) + 2 * lc + (j % 2);
+    return kRowsB ? EV * lc + (j % EV) + 4 * EV * (j / EV) : lc + 4 * j;
+  };
 
   // Byte offset of this lane's first operand vector inside a stage; every other vector of the lane is a
   // compile-time constant away from it:  row * 128 + ((chunk ^ (row & 7)) * 16)
   //   A rows are lr + 8 i  -> + i * 1024 bytes, row & 7 == lr for every i
   //   B rows are lc + 4 j  -> + j * 512 bytes,  row & 7 == lc + 4 (j & 1)
+  // An operand along its rows: k * (128 * sizeof(T)) + first row of the group * sizeof(T); the groups of EV rows are
+  // 8 EV (A) or 4 EV (B) rows apart -> + g * 128 or + g * 64 bytes.
   // The warp's first chunk of a stage: column wk * kChunks / 8, chunk wk * kChunks % 8 of it.
   constexpr int kChunksPerColumn = 8;
   const int first_chunk = WK == 1 ? 0 : (wk * kChunks) % kChunksPerColumn;
   const int column = WK == 1 ? 0 : (wk * kChunks) / kChunksPerColumn;
   const uint32_t smem_base = smem_u32(smem);
-  const uint32_t a_base = column * (Tile::kM * 128) + (wm * 64 + lr) * 128;
-  const uint32_t b_base = Tile::kABytes + column * (Tile::kN * 128) + (wn * 32 + lc) * 128;
+  const uint32_t a_base = kRowsA ? (wm * 64 + EV * lr) * (int)sizeof(T) : column * (Tile::kM * 128) + (wm * 64 + lr) * 128;
+  const uint32_t b_base = Tile::kABytes + (kRowsB ? (wn * 32 + EV * lc) * (int)sizeof(T) : column * (Tile::kN * 128) + (wn * 32 + lc) * 128);
 
   T acc[8][8];
 
@@ -348,6 +383,19 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       // fragment loaders for one 16-byte k chunk: a[i][e] = A(row i, k = chunk * EV + e).  With the offset table the
       // chunk is given as (c, h): chunk = h * kUnroll + c with c a compile-time constant; without it h is 0.
       auto load_a = [&](T (&a)[8][EV], int c, int h = 0) {
+        if constexpr (kRowsA) {
+          const uint32_t base = st + a_base + (kOffsetTable ? h * kUnroll + c : c) * (EV * Tile::kM * (int)sizeof(T));
+#pragma unroll
+          for (int e = 0; e < EV; ++e)
+#pragma unroll
+            for (int g = 0; g < 8 / EV; ++g) {
+              T v[EV];
+              lds16(base + e * (Tile::kM * (int)sizeof(T)) + g * 128, v);
+#pragma unroll
+              for (int t = 0; t < EV; ++t) a[g * EV + t][e] = v[t];
+            }
+          return;
+        }
         uint32_t base;
         if constexpr (kOffsetTable) base = kFlipBase ? st + h * a_flip + a_off[c] : st + (a_off[c] ^ (h << 6));
         else base = st + a_base + ((((c + first_chunk) ^ lr) & 7) << 4);
@@ -355,6 +403,19 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         for (int i = 0; i < 8; ++i) lds16(base + i * 1024, a[i]);
       };
       auto load_b = [&](T (&b)[8][EV], int c, int h = 0) {
+        if constexpr (kRowsB) {
+          const uint32_t base = st + b_base + (kOffsetTable ? h * kUnroll + c : c) * (EV * Tile::kN * (int)sizeof(T));
+#pragma unroll
+          for (int e = 0; e < EV; ++e)
+#pragma unroll
+            for (int g = 0; g < 8 / EV; ++g) {
+              T v[EV];
+              lds16(base + e * (Tile::kN * (int)sizeof(T)) + g * 64, v);
+#pragma unroll
+              for (int t = 0; t < EV; ++t) b[g * EV + t][e] = v[t];
+            }
+          return;
+        }
         uint32_t base0, base1;
         if constexpr (kOffsetTable) {
           base0 = kFlipBase ? st + h * b_flip + b_off[c] : st + (b_off[c] ^ (h << 6));
@@ -383,13 +444,16 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           return;
         }
         if constexpr (sizeof(T) == 8) {
-          // one k at a time: neighbouring instructions are independent
+          // An instruction's operands have to come from both register banks, so the rate depends on the order of the updates,
+          // which the compiler's register assignment follows (see order_of).
 #pragma unroll
-          for (int e = 0; e < EV; ++e)
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-              for (int j = 0; j < 8; ++j) acc[i][j] = RingT::add(RingT::mul(a[i][e], b[j][e]), acc[i][j]);
+          for (int x = 0; x < 128; ++x) {
+            constexpr int kOrder = order_of<RingT, Tile>();
+            const int e = kOrder == kByColumn ? (x / 8) % 2 : kOrder == kByElement ? x % 2 : x / 64;
+            const int i = kOrder == kByHalf ? (x / 32) % 2 * 4 + x % 4 : kOrder == kByElement ? (x / 2) % 8 : x % 8;
+            const int j = kOrder == kByHalf ? (x / 4) % 8 : kOrder == kByK ? (x / 8) % 8 : x / 16;
+            acc[i][j] = RingT::add(RingT::mul(a[i][e], b[j][e]), acc[i][j]);
+          }
           return;
         }
 #pragma unroll
@@ -405,18 +469,43 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         // Tensor-core path.  The fp64 mma takes, per lane, A(row lr [+8], k slot lc [+4]) and B(k slot lc [+4], column lr).
         // The contraction index may be permuted freely as long as A and B agree: within a group of 8 k (four
         // chunks) the slot lc of step s (s = 0, 1) stands for k = 2 lc + s, so one 16-byte load delivers both steps
-        // of a block.
+        // of a block.  An operand along its rows delivers two adjacent rows with one 16-byte load; they feed the two
+        // blocks of an interleaved pair (block rows 2 lr and 2 lr + 1).
         constexpr int kGroups = kChunks / 4;
         static_assert(kGroups == 1 || kGroups == 2, "one or two groups of 8 k per warp and stage");
         auto load_group = [&](double (&a)[8][2], double (&b)[4][2], int group) {
           const uint32_t chunk = ((((group * 4 + first_chunk + lc) ^ lr) & 7) << 4);
-          const uint32_t abase = st + a_base + chunk;
+          if constexpr (kRowsA) {
 #pragma unroll
-          for (int mb = 0; mb < 8; ++mb) lds16(abase + mb * 1024, a[mb]);
+            for (int step = 0; step < 2; ++step)
+#pragma unroll
+              for (int pair = 0; pair < 4; ++pair) {
+                double v[2];
+                lds16(st + (group * 8 + 2 * lc + step) * (Tile::kM * 8) + (wm * 64 + 2 * lr) * 8 + pair * 128, v);
+                a[2 * pair][step] = v[0];
+                a[2 * pair + 1][step] = v[1];
+              }
+          } else {
+            const uint32_t abase = st + a_base + chunk;
+#pragma unroll
+            for (int mb = 0; mb < 8; ++mb) lds16(abase + mb * 1024, a[mb]);
+          }
           // B rows (columns of the product) of this path are lr + 8 nb
-          const uint32_t bbase = st + Tile::kABytes + column * (Tile::kN * 128) + (wn * 32 + lr) * 128 + chunk;
+          if constexpr (kRowsB) {
 #pragma unroll
-          for (int nb = 0; nb < 4; ++nb) lds16(bbase + nb * 1024, b[nb]);
+            for (int step = 0; step < 2; ++step)
+#pragma unroll
+              for (int pair = 0; pair < 2; ++pair) {
+                double v[2];
+                lds16(st + Tile::kABytes + (group * 8 + 2 * lc + step) * (Tile::kN * 8) + (wn * 32 + 2 * lr) * 8 + pair * 128, v);
+                b[2 * pair][step] = v[0];
+                b[2 * pair + 1][step] = v[1];
+              }
+          } else {
+            const uint32_t bbase = st + Tile::kABytes + column * (Tile::kN * 128) + (wn * 32 + lr) * 128 + chunk;
+#pragma unroll
+            for (int nb = 0; nb < 4; ++nb) lds16(bbase + nb * 1024, b[nb]);
+          }
         };
         auto mma_group = [&](const double (&a)[8][2], const double (&b)[4][2]) {
           // m16n8k8: rows lr and lr + 8 of the instruction are the two 8-row blocks 2 h and 2 h + 1, k slots lc and
@@ -612,9 +701,17 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         consumer_sync();
         if (!last) continue;
         // This CTA completed the tile: fold all pieces in slice order (a fixed order, whoever comes last), then
-        // fall through to the ordinary epilogue with the folded accumulators.
+        // fall through to the ordinary epilogue with the folded accumulators.  An idempotent (+) folds them onto this
+        // CTA's own piece, which is one of them; sums start over.  (A test for the first piece inside the fold costs the
+        // fp64 contraction, which needs every register, 76 bytes of spills.)
         __threadfence();
         if (threadIdx.x == 0) p.tickets[split] = 0;
+        if constexpr (RingT::kAdd == CUASR_OP_PLUS || RingT::kAdd == CUASR_OP_BIT_XOR) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[i][j] = T(0);
+        }
         for (int zz = 0; zz < pieces; ++zz) {
           const uint4* theirs = reinterpret_cast<const uint4*>(block + (long long)zz * (kTileM * kTileN)) + threadIdx.x;
           uint4 raw[kVecPerThread];
@@ -627,7 +724,7 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 #pragma unroll
             for (int e = 0; e < EV; ++e) {
               T& a = acc[(v * EV + e) / 8][(v * EV + e) % 8];
-              a = zz == 0 ? tmp[e] : RingT::add(tmp[e], a);
+              a = RingT::add(tmp[e], a);
             }
           }
         }

@@ -23,7 +23,7 @@ cuasr_b200_args_t args_of(int m, int n, int k) {
 // How K is shared for a given SM count, as one number.
 long long k_sharing(const cuasr_b200_desc_t& d, const cuasr_b200_args_t& a, int gpu_sms) {
   const int sms = planning_sms(d, gpu_sms);
-  const LaunchPlan plan = plan_without_workspace(d, a.m, a.n, a.k, sms, has_all_tiles(d), false, false);
+  const LaunchPlan plan = plan_without_workspace(d, a.m, a.n, a.k, sms, has_all_tiles(d), Gathers());
   const BalancePlan balance = balance_plan(static_cast<long long>(tile_count(a)), sms, (a.k + 31) / 32);
   return ((plan.tile * 64LL + plan.cluster) * 64 + balance.pieces) * 1000000 + balance.whole_tiles;
 }
