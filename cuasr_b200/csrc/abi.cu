@@ -366,13 +366,13 @@ bool ring_pads_itself(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& ar
 // minima by tile (4096^3 on the large tile, 1000^3 on 128 x 64, 2048^3 on 64 x 64).
 double clocks_per_k(const cuasr_b200_desc_t& desc, int tile) {
   static constexpr double f64_min[4] = {6.6, 7.1, 7.2, 7.3}, f64_bottleneck[4] = {9.1, 9.6, 9.5, 9.7};
-  const bool sum = desc.add_op == CUASR_OP_PLUS, logical = desc.mul_op == CUASR_OP_BINARY_AND;
+  const bool sum = desc.add_op == CUASR_OP_PLUS, logical = desc.add_op == CUASR_OP_BINARY_OR;
   const bool bottleneck = desc.mul_op == CUASR_OP_MINIMUM || desc.mul_op == CUASR_OP_MAXIMUM;
   double per_product = 2.1;
-  if (desc.dtype == CUASR_F64) per_product = sum ? 2.1 : logical ? 10.0 : bottleneck ? f64_bottleneck[tile] : f64_min[tile];
+  if (logical) per_product = 3.1;
+  else if (desc.dtype == CUASR_F64) per_product = sum ? 2.1 : bottleneck ? f64_bottleneck[tile] : f64_min[tile];
   else if (desc.dtype == CUASR_F32 && sum) per_product = 1.55;
   else if (bottleneck) per_product = 3.0;
-  else if (logical) per_product = 9.0;
   return 2 * 64 * per_product;
 }
 

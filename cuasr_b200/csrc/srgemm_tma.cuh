@@ -369,7 +369,8 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     const int kt_begin = pieces == 1 ? 0 : z * p.k_tiles_per_slice;
     const int kt_end = (z == pieces - 1) ? k_tiles_total : min(k_tiles_total, kt_begin + p.k_tiles_per_slice);
 
-    const T start = (wk == 0 && z == 0) ? p.add_identity : p.part_identity;
+    T start = (wk == 0 && z == 0) ? p.add_identity : p.part_identity;
+    if constexpr (RingT::kLogical) start = static_cast<T>(start != T(0));      // as the first product makes it
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
@@ -440,6 +441,19 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             for (int i = 0; i < 8; ++i)
 #pragma unroll
               for (int j = 0; j < 8; ++j) acc[i][j] = RingT::mac_packed(acc[i][j], pa[i], pb[j]);
+          }
+          return;
+        }
+        if constexpr (RingT::kLogical) {
+#pragma unroll
+          for (int e = 0; e < EV; ++e) {
+            uint32_t ma[8], mb[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { ma[i] = RingT::mask(a[i][e]); mb[i] = RingT::mask(b[i][e]); }
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+              for (int j = 0; j < 8; ++j) acc[i][j] = RingT::or_mask(acc[i][j], ma[i] & mb[j]);
           }
           return;
         }

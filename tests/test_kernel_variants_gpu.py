@@ -80,7 +80,8 @@ def whole_numbers(g, shape, dtype, lo=-9, hi=10):
 # that clusters of 2, 4 and 8 share K, and with enough that they do not
 @pytest.mark.parametrize("ring, dtype", [("minimum_plus", "f32"), ("maximum_minimum", "f32"), ("plus_multiplies", "f64"),
                                          ("minimum_plus", "s32"), ("maximum_minimum", "s32"), ("minimum_plus", "u32"),
-                                         ("bit_xor_bit_and", "u32"), ("binary_or_binary_and", "f32")])
+                                         ("bit_xor_bit_and", "u32"), ("binary_or_binary_and", "f32"), ("binary_or_binary_and", "f64"),
+                                         ("binary_or_binary_and", "s32")])
 @pytest.mark.parametrize("m, n, k", [(1, 1, 1), (33, 65, 31), (64, 32, 257), (63, 31, 1025), (65, 129, 513), (256, 192, 700),
                                      (300, 500, 129), (640, 1024, 100), (1025, 1100, 70)])
 def test_tiles_and_clusters(cuda_device, ring, dtype, m, n, k):
@@ -91,6 +92,28 @@ def test_tiles_and_clusters(cuda_device, ring, dtype, m, n, k):
         for pads in ((0, 0, 0), (1, 3, 2), ((-k) % 4, (-k) % 4, (-n) % 4)):
             check_product(ring, dtype, A, B, C, layouts, pads, workspace=i % 2 == 1)
     assert device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f64", "s32"])
+def test_logical_ring_of_any_value(cuda_device, dtype):
+    """Everything but zero counts as true, negative zeros do not and NaN does; the result is 0 or 1 whatever the accumulation
+    starts from."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(8)
+    m, n, k = 130, 70, 67
+    A, B = (torch.where(torch.rand(s, generator=g, device="cuda") < 0.1, whole_numbers(g, s, "s32", -3, 4), 0).to(torch_type(dtype))
+            for s in ((m, k), (k, n)))
+    if dtype != "s32":
+        A, B = -A, torch.where(B == 1, torch.nan, torch.where(B == 2, torch.inf, torch.where(B == 3, 1e-42, B)))
+    want = ((A != 0).double() @ (B != 0).double()) != 0
+    assert want.any() and not want.all()
+    add, mul = RINGS["binary_or_binary_and"]
+    for start in (0, 1, 5):
+        D = torch.full((m, n), 77, dtype=torch_type(dtype), device="cuda")
+        op = Srgemm(add, mul, DTYPE[dtype], ROW, ROW, ROW, add_identity=start, mul_identity=1)
+        args = Arguments((m, n, k), (A, k), (B, n), (torch.zeros_like(D), n), (D, n), (1, 0))
+        assert op(args) == Status.kSuccess
+        assert (D == (want | (start != 0)).to(D.dtype)).all(), start
 
 
 def test_ragged_k_does_not_lean_on_the_identities(cuda_device):
