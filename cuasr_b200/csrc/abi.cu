@@ -538,10 +538,9 @@ struct ScreenPlan {
 // its first blocks, which are done exactly or with many recomputed elements.  So 2048^3 is screened (1.46 - 1.55 ms
 // against 1.90 exact) and 1000^3 is not (334 - 379 us against 276).
 ScreenPlan screen_plan(int m, int n, int k, int sms, bool may_split) {
-  const int kb = 32;
-  const int blocks = (k + kb - 1) / kb;
+  const int blocks = (k + kScreenBlock - 1) / kScreenBlock;
   const long long tiles = static_cast<long long>((m + kTileM - 1) / kTileM) * ((n + kTileN - 1) / kTileN);
-  const double per_block = 128.0 * kb * 3.7;
+  const double per_block = 128.0 * kScreenBlock * 3.7;
   const double first = 400000;
   ScreenPlan best;
   for (int pieces = 1; pieces <= (may_split ? 128 : 1) && pieces <= blocks; ++pieces) {
@@ -588,32 +587,31 @@ bool in_device_memory(const void* ptr) {
 }
 
 // Launches the screened kernel on a normalised problem (row-major D).
-template <typename T>
-int run_screened(bool maximize, const Normalised& p, T beta, T add_id, bool read_c, const ScreenPlan& plan,
+int run_screened(bool maximize, const Normalised& p, double beta, double add_id, bool read_c, const ScreenPlan& plan,
                  const ExtraOutputs& extra, DeviceState* dev, cudaStream_t stream) {
-  ScreenParams<T> sp = {};
+  ScreenParams sp = {};
   sp.M = p.m; sp.N = p.n; sp.K = p.k;
-  sp.A = static_cast<const T*>(p.a); sp.lda = p.lda;
-  sp.B = static_cast<const T*>(p.b); sp.ldb = p.ldb;
+  sp.A = static_cast<const double*>(p.a); sp.lda = p.lda;
+  sp.B = static_cast<const double*>(p.b); sp.ldb = p.ldb;
   CUtensorMap map_a = {}, map_b = {};
-  sp.a_mode = operand_mode<T>(&map_a, p.a, p.lda, p.a_kcontig, p.m, p.k, kTileM);
-  sp.b_mode = operand_mode<T>(&map_b, p.b, p.ldb, p.b_kcontig, p.n, p.k, kTileN);
-  sp.C = static_cast<const T*>(p.c); sp.ldc = p.ldc;
-  sp.D = static_cast<T*>(p.d); sp.ldd = p.ldd;
+  sp.a_mode = operand_mode<double>(&map_a, p.a, p.lda, p.a_kcontig, p.m, p.k, kTileM);
+  sp.b_mode = operand_mode<double>(&map_b, p.b, p.ldb, p.b_kcontig, p.n, p.k, kTileN);
+  sp.C = static_cast<const double*>(p.c); sp.ldc = p.ldc;
+  sp.D = static_cast<double*>(p.d); sp.ldd = p.ldd;
   sp.beta = beta; sp.add_identity = add_id; sp.read_c = read_c;
   sp.n_extra = extra.count;
-  for (int x = 0; x < extra.count; ++x) sp.extra_d[x] = static_cast<T*>(extra.ptr[x]);
+  for (int x = 0; x < extra.count; ++x) sp.extra_d[x] = static_cast<double*>(extra.ptr[x]);
   sp.tiles_m = (p.m + kTileM - 1) / kTileM; sp.tiles_n = (p.n + kTileN - 1) / kTileN;
   sp.pieces = plan.pieces; sp.blocks_per_piece = plan.blocks_per_piece;
   sp.status = dev->status;
   const long long work = static_cast<long long>(sp.tiles_m) * sp.tiles_n * sp.pieces;
   if (work > 2147483647LL) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
   if (plan.pieces > 1) {
-    if (launch_screened_init<T>(maximize, sp, dev->sms, stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
+    if (launch_screened_init(maximize, sp, dev->sms, stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
     g_launches.fetch_add(1);
   }
   const int grid = static_cast<int>(work < dev->sms ? work : dev->sms);
-  if (launch_screened<T>(maximize, map_a, map_b, sp, grid, stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
+  if (launch_screened(maximize, map_a, map_b, sp, grid, stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
   g_launches.fetch_add(1);
   t_route = {"screened", kTileM, kTileN, 1, plan.pieces, load_name(sp.a_mode), load_name(sp.b_mode)};
   return CUASR_STATUS_SUCCESS;
@@ -790,7 +788,7 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
         alpha == T(0) && !negative_zero(alpha) && !(read_c && negative_zero(beta))) {
       const ScreenPlan screened = screen_plan(p.m, p.n, p.k, dev->sms, extra.count == 0);
       if (screened.cost < plan.cost && in_device_memory(p.d)) {
-        const int st = run_screened<T>(desc.add_op == CUASR_OP_MAXIMUM, p, beta, add_id, read_c, screened, extra, dev, stream);
+        const int st = run_screened(desc.add_op == CUASR_OP_MAXIMUM, p, beta, add_id, read_c, screened, extra, dev, stream);
         if (st == CUASR_STATUS_SUCCESS) {
           t_last_kernel = name;
           t_route.copied_a = copies.a; t_route.copied_b = copies.b;

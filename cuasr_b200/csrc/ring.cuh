@@ -123,18 +123,6 @@ struct Ring {
     else if constexpr (std::is_same<T, double>::value) return __hiloint2double(__double2hiint(acc) | static_cast<int>(m), 0);
     else return static_cast<T>(static_cast<uint32_t>(acc) | m);
   }
-
-  // True when an out-of-range operand element may be replaced by NaN (float min/max rings: the NaN
-  // product is ignored by min/max) — otherwise by zero, which must then be harmless: 0 (x) 0 has to be
-  // the additive identity in effect (plus-times, or-and, xor-and, or-bitand).
-  static constexpr bool kNanPadding =
-      (ADD == CUASR_OP_MINIMUM || ADD == CUASR_OP_MAXIMUM) && std::is_floating_point<T>::value;
-  static constexpr bool kZeroPadding =
-      (ADD == CUASR_OP_PLUS && MUL == CUASR_OP_MULTIPLIES) ||
-      ((ADD == CUASR_OP_BINARY_OR || ADD == CUASR_OP_BIT_OR || ADD == CUASR_OP_BIT_XOR) &&
-       (MUL == CUASR_OP_BINARY_AND || MUL == CUASR_OP_BIT_AND));
-  // Rings for which padding K by out-of-range elements is safe inside the TMA kernel.
-  static constexpr bool kPaddable = kNanPadding || kZeroPadding;
 };
 
 }  // namespace cuasr_b200

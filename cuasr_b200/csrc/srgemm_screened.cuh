@@ -1,7 +1,7 @@
 // Screened tropical SRGEMM: D = min(A + B, beta + C) (or max) with most products looked at in 16 bits only.
 //
-// What bounds the ordinary kernel: a product of the min-plus ring costs 2.07 clocks per scheduler in fp32 (register
-// file reads of a packed add and a three-input minimum) and 6.5 in fp64 (add, compare, two selects).  But a product
+// What bounds the ordinary kernel: a product of the fp64 min-plus ring costs 6.6 clocks per scheduler (add, compare, two
+// selects: 12 register words at two a clock are 6).  But a product
 // matters only if it IMPROVES its element, and the n-th product of an element does so with probability about 1/n.  So
 // each operand tile is also kept as 16-bit fixed-point numbers rounded towards "better" (down for min, up for max): the
 // sum of two such numbers is never worse than the exact sum, and one fused packed add-min instruction handles two
@@ -25,16 +25,15 @@
 // compare-and-swap (pieces > 1; D initialised by an earlier launch).
 //
 // Structure: one persistent CTA per SM.  Warps 8..11 bring exact tiles in (TMA or gather), turn them into 16-bit tiles;
-// warps 0..7 own 64 x 32 blocks of the 128 x 128 tile, 8 x 8 elements per lane.  A stage is 512 bytes of exact operand
-// rows' worth of k: 64 k (fp32) or 32 k (fp64), two stages.
+// warps 0..7 own 64 x 32 blocks of the 128 x 128 tile, 8 x 8 elements per lane.  A stage is a block of 32 k, two stages.
 #pragma once
 
 #include "srgemm_tma.cuh"
 
 namespace cuasr_b200 {
 
-template <typename T>
 struct ScreenParams {
+  using T = double;
   int M, N, K;
   const T* A;  long long lda;      // gathered operands only
   const T* B;  long long ldb;
@@ -50,15 +49,14 @@ struct ScreenParams {
 };
 
 constexpr int kScreenExactBytes = 65536;      // 2 operands x 128 rows x 256 bytes
-template <typename T>
-constexpr int kScreenStageBytes = kScreenExactBytes + 2 * 128 * (256 / (int)sizeof(T)) * 2;
+constexpr int kScreenBlock = 32;                // k per block: 256 bytes of an exact row
+constexpr int kScreenStageBytes = kScreenExactBytes + 2 * 128 * kScreenBlock * 2;
 constexpr int kScreenStages = 2;
 constexpr int kScreenBoundBytes = 8 * 64 * 32 * 2;   // per warp, element and lane: the value a 16-bit sum has to beat
 constexpr int kListGroups = 4;                       // groups of eight elements that a warp recomputes at a time
 constexpr int kListed = 96;                          // elements to recompute that a warp lists at a time
 constexpr int kScreenListBytes = 8 * kListed * 2;
-template <typename T>
-constexpr int kScreenSmemBytes = kScreenStages * kScreenStageBytes<T> + kScreenBoundBytes + kScreenListBytes + 512 + 1024;
+constexpr int kScreenSmemBytes = kScreenStages * kScreenStageBytes + kScreenBoundBytes + kScreenListBytes + 512 + 1024;
 
 __device__ __forceinline__ void sts16(uint32_t addr, uint4 v) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
@@ -90,9 +88,8 @@ struct Screen {
   static constexpr float kFiniteLimit = 16382.0f;
   // scaled fp32 image of an element, rounded towards "better" in both steps (the scaling is inexact where it underflows:
   // rounded to nearest, a tiny negative value would come out as a zero and a tiny maximum would lose its upper bound)
-  static __device__ __forceinline__ float scaled(float x, float scale) { return kMax ? __fmul_ru(x, scale) : __fmul_rd(x, scale); }
   static __device__ __forceinline__ float scaled(double x, float scale) {
-    return scaled(kMax ? __double2float_ru(x) : __double2float_rd(x), scale);
+    return kMax ? __fmul_ru(__double2float_ru(x), scale) : __fmul_rd(__double2float_rd(x), scale);
   }
   static constexpr uint32_t kNever = kMax ? 0x8000u : 0x7FFFu;       // the infinity no sum improves with
   static constexpr uint32_t kNothing = kMax ? 0x7FFFu : 0u;          // bound no sum beats (elements outside the matrix)
@@ -116,38 +113,23 @@ struct Screen {
   // The bound of an element with current value v: a 16-bit sum may stand for an improvement only if it is below
   // (min) or above (max) it.  min: exact sum < v implies (sum of floors) < v * s, i.e. < ceil(v * s); the product is
   // rounded up, so that it only ever gets larger where it is inexact.
-  template <typename T>
-  static __device__ __forceinline__ uint32_t bound(T v, float scale) {
-    const T y = rescaled(v, scale);
+  static __device__ __forceinline__ uint32_t bound(double v, float scale) {
+    const double y = kMax ? __dmul_rd(v, (double)scale) : __dmul_ru(v, (double)scale);
     if (y != y) return kNothing;                                        // a NaN (from C) stays: nothing is better than it
     if (kMax) {
-      if (!(y >= T(0))) return (uint32_t)(uint16_t)-1;                  // any sum of finite values
-      if (y >= T(32766)) return 32766u;
+      if (!(y >= 0.0)) return (uint32_t)(uint16_t)-1;                  // any sum of finite values
+      if (y >= 32766.0) return 32766u;
       return (uint32_t)(int)y;
     }
-    if (!(y < T(32766))) return 32767u;                                 // any sum of finite values
-    if (y < T(0)) return 0u;                                            // nothing: no negative values in a fit stage
+    if (!(y < 32766.0)) return 32767u;                                 // any sum of finite values
+    if (y < 0.0) return 0u;                                             // nothing: no negative values in a fit stage
     return (uint32_t)(int)ceil(y);
   }
-  static __device__ __forceinline__ float rescaled(float v, float scale) { return kMax ? __fmul_rd(v, scale) : __fmul_ru(v, scale); }
-  static __device__ __forceinline__ double rescaled(double v, float scale) {
-    return kMax ? __dmul_rd(v, (double)scale) : __dmul_ru(v, (double)scale);
-  }
   static __device__ __forceinline__ bool sooner(uint32_t a, uint32_t b) { return kMax ? (int16_t)a > (int16_t)b : a < b; }
-  template <typename T>
-  static __device__ __forceinline__ bool better(T candidate, T current) { return kMax ? candidate > current : candidate < current; }
+  static __device__ __forceinline__ bool better(double candidate, double current) { return kMax ? candidate > current : candidate < current; }
 };
 
 // current = better(value, current) in memory other CTAs write too; returns the value that is there afterwards.
-template <bool kMax>
-__device__ __forceinline__ float improve_shared(float* at, float value, float seen) {
-  while (Screen<kMax>::better(value, seen)) {
-    const unsigned int got = atomicCAS(reinterpret_cast<unsigned int*>(at), __float_as_uint(seen), __float_as_uint(value));
-    if (got == __float_as_uint(seen)) return value;
-    seen = __uint_as_float(got);
-  }
-  return seen;
-}
 template <bool kMax>
 __device__ __forceinline__ double improve_shared(double* at, double value, double seen) {
   while (Screen<kMax>::better(value, seen)) {
@@ -158,14 +140,8 @@ __device__ __forceinline__ double improve_shared(double* at, double value, doubl
   return seen;
 }
 
-// *at = better(*at, value) without reading it back.  `value` is not negative, and then the bit patterns of any float
+// *at = better(*at, value) without reading it back.  `value` is not negative, and then the bit patterns of any double
 // compare with it like signed integers; adding zero makes a negative zero a positive one, whose pattern does.
-template <bool kMax>
-__device__ __forceinline__ void merge_into(float* at, float value) {
-  value += 0.0f;
-  if (kMax) atomicMax(reinterpret_cast<int*>(at), __float_as_int(value));
-  else      atomicMin(reinterpret_cast<int*>(at), __float_as_int(value));
-}
 template <bool kMax>
 __device__ __forceinline__ void merge_into(double* at, double value) {
   value += 0.0;
@@ -173,17 +149,19 @@ __device__ __forceinline__ void merge_into(double* at, double value) {
   else      atomicMin(reinterpret_cast<long long*>(at), __double_as_longlong(value));
 }
 
-template <typename T, bool kMax>
+template <bool kMax>
 __global__ void __launch_bounds__(kTmaThreads, 1)
 srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                       const __grid_constant__ ScreenParams<T> p) {
+                       const __grid_constant__ ScreenParams p) {
+  using T = double;
   using S = Screen<kMax>;
   using RingT = Ring<kMax ? CUASR_OP_MAXIMUM : CUASR_OP_MINIMUM, CUASR_OP_PLUS, T>;
   constexpr int EV = 16 / (int)sizeof(T);
   constexpr int TK = 128 / (int)sizeof(T);          // k per 128-byte column
-  constexpr int KB = 2 * TK;                        // k per stage: 64 or 32
-  constexpr int kCoarseRow = KB * 2;                // bytes of a 16-bit row: 128 or 64
-  constexpr int kCoarseChunks = kCoarseRow / 16;    // 8 or 4 chunks of 8 k
+  constexpr int KB = kScreenBlock;                  // k per stage
+  static_assert(KB == 2 * TK, "two 128-byte columns");
+  constexpr int kCoarseRow = KB * 2;                // bytes of a 16-bit row: 64
+  constexpr int kCoarseChunks = kCoarseRow / 16;    // 4 chunks of 8 k
   constexpr int kExactOperand = 32768, kColumn = 16384;
   constexpr int kCoarseOperand = 128 * kCoarseRow;
   // Elements of a warp (of 2048) above which recomputing them one by one costs more than doing the block exactly, and how
@@ -193,7 +171,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* bounds_smem = smem + kScreenStages * kScreenStageBytes<T>;
+  uint8_t* bounds_smem = smem + kScreenStages * kScreenStageBytes;
   uint8_t* list_smem = bounds_smem + kScreenBoundBytes;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(list_smem + kScreenListBytes);   // exact tile landed
   uint64_t* ready_bar = full_bar + kScreenStages;                                     // 16-bit tile written
@@ -263,7 +241,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       const int s = lit % kScreenStages;
       const uint32_t round = lit / kScreenStages;
       if (alive && round > 0) alive = mbar_wait(&empty_bar[s], (round - 1) & 1, p.status, kDeviceTimeoutEmpty);
-      uint8_t* sa = smem + s * kScreenStageBytes<T>;
+      uint8_t* sa = smem + s * kScreenStageBytes;
       uint8_t* sb = sa + kExactOperand;
       const int k0 = (lbegin + lpos) * KB;
       if (s == 0) k0_even = k0;
@@ -307,7 +285,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       if (alive) alive = mbar_wait(&full_bar[s], (it / kScreenStages) & 1, p.status, kDeviceTimeoutFull);
       alive = producers_agree(alive);
       if (!alive) break;
-      const uint32_t exact = smem_u32(smem + s * kScreenStageBytes<T>);
+      const uint32_t exact = smem_u32(smem + s * kScreenStageBytes);
       const uint32_t coarse = exact + kScreenExactBytes;
       const int k_left = p.K - (s == 0 ? k0_even : k0_odd);          // below KB in the block that reaches beyond K
       // No 16-bit tile for a block that all consumers do exactly (what they promise, they keep).
@@ -334,29 +312,14 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
           const int row = block * 8 + r8;                             // 0..127: A, 128..255: B
           const uint32_t src = exact + (row >> 7) * kExactOperand + (row & 127) * 128;
           uint32_t words[4];
-          if constexpr (sizeof(T) == 4) {
-            float x[2][4];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int chunk = 2 * c + h;                            // 4 k
-              lds16(src + (chunk >> 3) * kColumn + (((chunk & 7) ^ r8) << 4), x[h]);
-            }
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-              const float y0 = S::scaled(x[w >> 1][(w & 1) * 2], scale), y1 = S::scaled(x[w >> 1][(w & 1) * 2 + 1], scale);
-              S::survey(y0, y1, largest, smallest);
-              words[w] = S::quantise(y0) | (S::quantise(y1) << 16);
-            }
-          } else {
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-              double x[2];
-              const int chunk = 4 * c + w;                            // 2 k
-              lds16(src + (chunk >> 3) * kColumn + (((chunk & 7) ^ r8) << 4), x);
-              const float y0 = S::scaled(x[0], scale), y1 = S::scaled(x[1], scale);
-              S::survey(y0, y1, largest, smallest);
-              words[w] = S::quantise(y0) | (S::quantise(y1) << 16);
-            }
+          for (int w = 0; w < 4; ++w) {
+            double x[2];
+            const int chunk = 4 * c + w;                            // 2 k
+            lds16(src + (chunk >> 3) * kColumn + (((chunk & 7) ^ r8) << 4), x);
+            const float y0 = S::scaled(x[0], scale), y1 = S::scaled(x[1], scale);
+            S::survey(y0, y1, largest, smallest);
+            words[w] = S::quantise(y0) | (S::quantise(y1) << 16);
           }
           if (k_left < KB) {
             // TMA fills NaN beyond K; the screen shall see the infinity that never improves
@@ -371,7 +334,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             for (int w = 0; w < 4; ++w) words[w] = __vmaxs2(words[w], 0xC000C000u);    // -inf + -inf must not wrap
           }
           const uint32_t dst = coarse + (row >> 7) * kCoarseOperand + (row & 127) * kCoarseRow +
-                               ((kCoarseRow == 128 ? (c ^ r8) : (c ^ ((r8 >> 1) & 3))) << 4);
+                               ((c ^ ((r8 >> 1) & 3)) << 4);
           sts16(dst, make_uint4(words[0], words[1], words[2], words[3]));
         }
 #pragma unroll
@@ -464,7 +427,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
           for (int j = 0; j < 8; ++j) acc[i][j] = p.add_identity;
         for (;;) {
           const int sx = it % kScreenStages;
-          const uint32_t exact = smem_base + sx * kScreenStageBytes<T>;
+          const uint32_t exact = smem_base + sx * kScreenStageBytes;
           const uint32_t a_base = exact + (wm * 64 + lr) * 128, b_base = exact + kExactOperand + (wn * 32 + lc) * 128;
 #pragma unroll 1
           for (int chunk = 0; chunk < 16; ++chunk) {
@@ -534,7 +497,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         __syncwarp();
         continue;
       }
-      const uint32_t exact = smem_base + s * kScreenStageBytes<T>;
+      const uint32_t exact = smem_base + s * kScreenStageBytes;
       const uint32_t coarse = exact + kScreenExactBytes;
 
       if (my_exp != exponent) {
@@ -571,14 +534,8 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         const uint32_t qa = coarse + (wm * 64 + lr) * kCoarseRow, qb = coarse + kCoarseOperand + (wn * 32 + lc) * kCoarseRow;
 #pragma unroll 2
         for (int c = 0; c < kCoarseChunks; ++c) {
-          uint32_t ab, b0, b1;
-          if constexpr (kCoarseRow == 128) {
-            ab = qa + ((c ^ lr) << 4);
-            b0 = qb + ((c ^ lc) << 4); b1 = qb + ((c ^ (lc + 4)) << 4);
-          } else {
-            ab = qa + ((c ^ (lr >> 1)) << 4);                         // rows lr + 8 i: (row >> 1) & 3 == lr >> 1
-            b0 = qb + ((c ^ (lc >> 1)) << 4); b1 = qb + ((c ^ ((lc + 4) >> 1)) << 4);   // rows lc + 4 j
-          }
+          const uint32_t ab = qa + ((c ^ (lr >> 1)) << 4);            // rows lr + 8 i: (row >> 1) & 3 == lr >> 1
+          const uint32_t b0 = qb + ((c ^ (lc >> 1)) << 4), b1 = qb + ((c ^ ((lc + 4) >> 1)) << 4);   // rows lc + 4 j
           uint4 a[8], bv[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) a[i] = lds16u(ab + i * (8 * kCoarseRow));
@@ -652,12 +609,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
               T a[EV], bb[EV];
               lds16(ra + (h >> 1) * kColumn + (((h & 1) << 6) ^ fa), a);
               lds16(rb + (h >> 1) * kColumn + (((h & 1) << 6) ^ fb), bb);
-              if constexpr (RingT::kPackedPairs) {
-                best[u] = RingT::mac_packed(best[u], pack2(a[0], a[1]), pack2(bb[0], bb[1]));
-                best[u] = RingT::mac_packed(best[u], pack2(a[2], a[3]), pack2(bb[2], bb[3]));
-              } else {
-                best[u] = RingT::mac2(best[u], a[0], bb[0], a[1], bb[1]);
-              }
+              best[u] = RingT::mac2(best[u], a[0], bb[0], a[1], bb[1]);
             }
           }
 #pragma unroll
@@ -712,7 +664,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 // D = the start values of a product whose pieces meet in D: the additive identity, folded with beta (x) C.
 template <typename RingT>
 __global__ void __launch_bounds__(256)
-screened_init_kernel(const __grid_constant__ ScreenParams<typename RingT::Element> p) {
+screened_init_kernel(const __grid_constant__ ScreenParams p) {
   using T = typename RingT::Element;
   grid_dependency_wait();
   grid_dependency_launch();
@@ -725,12 +677,9 @@ screened_init_kernel(const __grid_constant__ ScreenParams<typename RingT::Elemen
   }
 }
 
-// Launches srgemm_screened_kernel on `grid` persistent CTAs, and the
-// kernel that prepares D where its pieces share it.
-template <typename T>
-cudaError_t launch_screened(bool maximize, const CUtensorMap& map_a, const CUtensorMap& map_b, const ScreenParams<T>& params,
-                            int grid, cudaStream_t stream);
-template <typename T>
-cudaError_t launch_screened_init(bool maximize, const ScreenParams<T>& params, int sms, cudaStream_t stream);
+// Launches srgemm_screened_kernel on `grid` persistent CTAs, and the kernel that prepares D where its pieces share it.
+cudaError_t launch_screened(bool maximize, const CUtensorMap& map_a, const CUtensorMap& map_b, const ScreenParams& params, int grid,
+                            cudaStream_t stream);
+cudaError_t launch_screened_init(bool maximize, const ScreenParams& params, int sms, cudaStream_t stream);
 
 }  // namespace cuasr_b200
