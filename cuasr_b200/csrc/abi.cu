@@ -626,13 +626,13 @@ int run_path(bool maximize, const Normalised& p, int32_t* parent, long long ld_p
              cudaStream_t stream) {
   constexpr int TK = kTileKBytes / sizeof(T);
   constexpr int small = sizeof(T) == 4 ? kSmallTile : kTinyTile;
-  const double per_k = 2 * 64 * (sizeof(T) == 8 ? 8.2 : 2.1);
   double best = 1e300;
   int tile = kLargeTile, cluster = 1;
   for (int candidate : {(int)kLargeTile, small}) {
     const bool large = candidate == kLargeTile;
     const long long tiles = static_cast<long long>((p.m + kTileRows[candidate] - 1) / kTileRows[candidate]) * ((p.n + kTileCols[candidate] - 1) / kTileCols[candidate]);
     const int step = candidate == kSmallTile ? 2 * TK : TK;
+    const double per_k = 2 * 64 * (sizeof(T) == 4 ? 2.1 : large ? 6.6 : 9.1);
     const double chunks = large ? 2 : candidate == kSmallTile ? 1 : 0.25;           // in fours, of a warp and stage
     const int k_steps = (p.k + step - 1) / step;
     for (int z = 1; z <= (large ? 1 : 8); z *= 2) {
@@ -640,12 +640,12 @@ int run_path(bool maximize, const Normalised& p, int32_t* parent, long long ld_p
       if ((z - 1) * per_piece >= k_steps) break;
       const long long room = z <= 2 ? dev->sms : z == 4 ? dev->sms * 36LL / 37 : dev->sms * 32LL / 37;
       const long long waves = (tiles * z + room - 1) / room;
-      const double per_stage = per_k * step / kTileWk[candidate] + 2 * 256 + 2 * 1.5 * 60 * chunks;
-      // fp64: 180 clocks and 60 per four chunks for each look-up of the slowest lane (1000^3 from +inf: 907 us on 64 x 32 tiles
-      // against 764 on 128 x 128 ones, 300^3: 78 against 340)
-      const double lookups = sizeof(T) == 8 ? 2 * (96 * std::log(1.0 + per_piece) + 4 * per_piece) * (180 + 60 * chunks)
-                                            : 2 * 64 * 60 * chunks * std::log(1.0 + per_piece);
-      const double cost = 3000 + static_cast<double>(waves) * (per_stage * per_piece + lookups + 3000 + (z > 1 ? 3000 : 0));
+      const double per_stage = per_k * step / kTileWk[candidate] + (sizeof(T) == 8 && !large ? 250 : 2 * 256 + 2 * 1.5 * 60 * chunks);
+      // fp64: 300 clocks on the large tile for each look-up of the slowest lane, half of them counted (cold and settled distances are
+      // as common); none on the small one, whose index follows every product
+      const double lookups = sizeof(T) == 4 ? 2 * 64 * 60 * chunks * std::log(1.0 + per_piece)
+                             : large ? (96 * std::log(1.0 + per_piece) + 4 * per_piece) * 300 : 0;
+      const double cost = 3000 + static_cast<double>(waves) * (per_stage * per_piece + lookups + 3000 + (z > 1 ? 3000 + (waves > 1 ? 8000 : 0) : 0));
       if (cost < best) { best = cost; tile = candidate; cluster = z; }
     }
   }

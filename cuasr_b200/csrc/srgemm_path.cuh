@@ -66,6 +66,19 @@ __device__ __forceinline__ uint32_t ld4_cluster(uint32_t addr, int rank) {
   return v;
 }
 
+// If t is better than acc: acc = t, and k to the element's word of shared memory.  Five instructions per product where the product
+// alone takes four, but no test and no look-up per stage: for the fp64 tile whose warps have two k of a stage, where a test costs a
+// quarter of the products and, from a cold start, some lane has an element to look up in nearly every stage.
+template <bool kMaximize>
+__device__ __forceinline__ void improve(double& acc, double t, uint32_t word, int k) {
+  if (kMaximize)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.f64 p, %1, %0;\n\t@p st.shared.b32 [%2], %3;\n\tselp.f64 %0, %1, %0, p;\n\t}"
+                 : "+d"(acc) : "d"(t), "r"(word), "r"(k) : "memory");
+  else
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.f64 p, %1, %0;\n\t@p st.shared.b32 [%2], %3;\n\tselp.f64 %0, %1, %0, p;\n\t}"
+                 : "+d"(acc) : "d"(t), "r"(word), "r"(k) : "memory");
+}
+
 template <typename T, bool kMaximize, typename Tile>
 __global__ void __launch_bounds__(kTmaThreads, 1)
 srgemm_path_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -78,6 +91,7 @@ srgemm_path_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   constexpr int TK = kTileKBytes / (int)sizeof(T);
   constexpr int kStep = TK * kSub;
   constexpr int kChunks = 8 * kSub / WK;          // 16-byte k chunks of a stage that one warp works on
+  constexpr bool kDirect = sizeof(T) == 8 && WK > 1;    // the index follows every product (see improve)
   auto better = [](T candidate, T current) { return kMaximize ? candidate > current : candidate < current; };
 
   extern __shared__ uint8_t smem_raw[];
@@ -210,7 +224,7 @@ srgemm_path_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         // nothing is better than a NaN; the minimum instruction would drop it for the first product
         acc[i][j] = x == x ? x : kMaximize ? static_cast<T>(INFINITY) : -static_cast<T>(INFINITY);
       }
-    keep();
+    if (!kDirect) keep();
 
     for (int kt = kt_begin; kt < kt_end; ++kt, ++it) {
       const int s = it % kStages;
@@ -226,64 +240,79 @@ srgemm_path_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         for (int i = 0; i < 8; ++i) lds16(base + i * 1024, a[i]);
 #pragma unroll
         for (int j = 0; j < 8; ++j) lds16(((j & 1) ? base1 : base0) + j * 512, b[j]);
+        if constexpr (kDirect) {
+          // k stays ascending for every element
+          const int k = kt * kStep + column * TK + first_chunk * EV;
 #pragma unroll
-        for (int e = 0; e < EV; e += 2)
+          for (int j = 0; j < 8; ++j)
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
+            for (int e = 0; e < EV; ++e)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              if constexpr (R::kPackedPairs)
-                acc[i][j] = R::mac_packed(acc[i][j], pack2(a[i][e], a[i][e + 1]), pack2(b[j][e], b[j][e + 1]));
-              else
-                acc[i][j] = R::mac2(acc[i][j], a[i][e], b[j][e], a[i][e + 1], b[j][e + 1]);
-            }
+              for (int i = 0; i < 8; ++i) improve<kMaximize>(acc[i][j], a[i][e] + b[j][e], index + (8 * i + j) * (kConsumerThreads * 4), k + e);
+        } else if constexpr (R::kPackedPairs) {
+#pragma unroll
+          for (int e = 0; e < EV; e += 2)
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+              for (int j = 0; j < 8; ++j) acc[i][j] = R::mac_packed(acc[i][j], pack2(a[i][e], a[i][e + 1]), pack2(b[j][e], b[j][e + 1]));
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)                          // kByColumn of srgemm_tma.cuh
+#pragma unroll
+            for (int e = 0; e < EV; ++e)
+#pragma unroll
+              for (int i = 0; i < 8; ++i) acc[i][j] = R::add(a[i][e] + b[j][e], acc[i][j]);
+        }
       }
       // which elements improved in this stage?  (a minimum only ever moves one way)
-      uint32_t mask_lo = 0, mask_hi = 0;
+      if constexpr (!kDirect) {
+        uint32_t mask_lo = 0, mask_hi = 0;
 #pragma unroll
-      for (int v = 0; v < 64 / EV; ++v) {
-        T x[EV];
-        lds16(kept + v * (kConsumerThreads * 16), x);
+        for (int v = 0; v < 64 / EV; ++v) {
+          T x[EV];
+          lds16(kept + v * (kConsumerThreads * 16), x);
 #pragma unroll
-        for (int e = 0; e < EV; ++e) {
-          const int el = v * EV + e;
-          if (better(acc[el / 8][el % 8], x[e])) {
-            if (el < 32) mask_lo |= 1u << el;
-            else         mask_hi |= 1u << (el - 32);
+          for (int e = 0; e < EV; ++e) {
+            const int el = v * EV + e;
+            if (better(acc[el / 8][el % 8], x[e])) {
+              if (el < 32) mask_lo |= 1u << el;
+              else         mask_hi |= 1u << (el - 32);
+            }
           }
         }
-      }
-      if ((mask_lo | mask_hi) != 0) keep();
-      while ((mask_lo | mask_hi) != 0) {
-        int el;
-        if (mask_lo != 0) { el = __ffs(mask_lo) - 1; mask_lo &= mask_lo - 1; }
-        else              { el = 31 + __ffs(mask_hi); mask_hi &= mask_hi - 1; }
-        const int i = el >> 3, j = el & 7;
-        T value;
-        {
-          const uint32_t at = kept + (el / EV) * (kConsumerThreads * 16) + (el % EV) * (int)sizeof(T);
-          if constexpr (sizeof(T) == 4) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(value) : "r"(at));
-          else                          asm volatile("ld.shared.f64 %0, [%1];" : "=d"(value) : "r"(at));
-        }
-        const uint32_t ra = st + a_base + i * 1024, rb = st + b_base + j * 512;
-        const int bx = lc + 4 * (j & 1);
-        int found = 0;
+        if ((mask_lo | mask_hi) != 0) keep();
+        while ((mask_lo | mask_hi) != 0) {
+          int el;
+          if (mask_lo != 0) { el = __ffs(mask_lo) - 1; mask_lo &= mask_lo - 1; }
+          else              { el = 31 + __ffs(mask_hi); mask_hi &= mask_hi - 1; }
+          const int i = el >> 3, j = el & 7;
+          T value;
+          {
+            const uint32_t at = kept + (el / EV) * (kConsumerThreads * 16) + (el % EV) * (int)sizeof(T);
+            if constexpr (sizeof(T) == 4) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(value) : "r"(at));
+            else                          asm volatile("ld.shared.f64 %0, [%1];" : "=d"(value) : "r"(at));
+          }
+          const uint32_t ra = st + a_base + i * 1024, rb = st + b_base + j * 512;
+          const int bx = lc + 4 * (j & 1);
+          int found = 0;
 #pragma unroll 4
-        for (int c = kChunks - 1; c >= 0; --c) {          // descending: the first k that attains the value stays
-          const int chunk = c + first_chunk;
-          T a[EV], b[EV];
-          lds16(ra + (((chunk ^ lr) & 7) << 4), a);
-          lds16(rb + (((chunk ^ bx) & 7) << 4), b);
+          for (int c = kChunks - 1; c >= 0; --c) {          // descending: the first k that attains the value stays
+            const int chunk = c + first_chunk;
+            T a[EV], b[EV];
+            lds16(ra + (((chunk ^ lr) & 7) << 4), a);
+            lds16(rb + (((chunk ^ bx) & 7) << 4), b);
 #pragma unroll
-          for (int e = EV - 1; e >= 0; --e)
-            if (a[e] + b[e] == value) found = c * EV + e;
-        }
-        const int k = kt * kStep + column * TK + first_chunk * EV + found;
-        if constexpr (WK == 1) {
-          const int m = m_base + lr + 8 * i, n = n_base + lc + 4 * j;
-          if (m < p.M && n < p.N) p.parent[(long long)m * p.ld_parent + n] = k + p.k_offset;
-        } else {
-          asm volatile("st.shared.b32 [%0], %1;" ::"r"(index + el * (kConsumerThreads * 4)), "r"(k) : "memory");
+            for (int e = EV - 1; e >= 0; --e)
+              if (a[e] + b[e] == value) found = c * EV + e;
+          }
+          const int k = kt * kStep + column * TK + first_chunk * EV + found;
+          if constexpr (WK == 1) {
+            const int m = m_base + lr + 8 * i, n = n_base + lc + 4 * j;
+            if (m < p.M && n < p.N) p.parent[(long long)m * p.ld_parent + n] = k + p.k_offset;
+          } else {
+            asm volatile("st.shared.b32 [%0], %1;" ::"r"(index + el * (kConsumerThreads * 4)), "r"(k) : "memory");
+          }
         }
       }
       __syncwarp();
