@@ -361,19 +361,20 @@ bool ring_pads_itself(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& ar
 
 // ---- which tile, and how K is shared ---------------------------------------------------------------------------
 // Clocks the 8 consumer warps of a CTA (two per scheduler, 64 products per lane and k) take for one k: measured per
-// product and scheduler 2.07 (fp32 with a packed add and a three-input minimum, fused integer add-min, one logic
+// product and scheduler 2.15 (fp32 with a packed add and a three-input minimum, fused integer add-min, one logic
 // instruction), 3.0 (two-instruction bottleneck products), 1.55 (fp32 sums), 2.1 (fp64 sums on the tensor cores), and for fp64
 // minima by tile (4096^3 on the large tile, 1000^3 on 128 x 64, 2048^3 on 64 x 64).
 double clocks_per_k(const cuasr_b200_desc_t& desc, int tile) {
   static constexpr double f64_min[4] = {6.6, 7.1, 7.2, 7.3}, f64_bottleneck[4] = {9.1, 9.6, 9.5, 9.7};
   const bool sum = desc.add_op == CUASR_OP_PLUS, logical = desc.add_op == CUASR_OP_BINARY_OR;
   const bool bottleneck = desc.mul_op == CUASR_OP_MINIMUM || desc.mul_op == CUASR_OP_MAXIMUM;
-  double per_product = 2.1;
+  double per_product = 2.15;
   if (logical) per_product = 3.1;
   else if (desc.dtype == CUASR_F64) per_product = sum ? 2.1 : bottleneck ? f64_bottleneck[tile] : f64_min[tile];
   else if (desc.dtype == CUASR_F32 && sum) per_product = 1.55;
   else if (bottleneck) per_product = 3.0;
-  return 2 * 64 * per_product;
+  // the shorter runs of chunks of the smaller tiles: 2048^3 on 64 x 64 522 us where 2.15 a product would be 504
+  return 2 * 64 * per_product * (desc.dtype != CUASR_F64 && tile != kLargeTile ? 1.06 : 1.0);
 }
 
 struct LaunchPlan {
@@ -393,10 +394,11 @@ int tile_sub(int tile, const cuasr_b200_desc_t& desc) {
 }
 
 // The fastest of the launches that need no workspace, by a model in clocks: start of the launch and first tile of
-// operands 3000, then per wave of CTAs the contraction (above) and the tile's end (2000 for the large tile, 1500 for the
+// operands 3000, then per wave of CTAs the contraction (above) and the tile's end (8000 for the large tile, 1500 for the
 // fold of the small ones, twice that for 8-byte elements), 2500 for the exchange inside a cluster.  Clusters of four
 // and eight do not fill every SM (a cluster lives in one GPC): 144 and 128 of the 148.
-// A cluster launch is not persistent: each further wave starts its CTAs anew, 4000.  The 64 x 32 tile hands a stage over
+// A cluster launch is not persistent: each further wave starts its CTAs anew, 4000, and 30000 where eight have to find room in one
+// GPC together (77 x 3001 x 2999 in fp64 as three waves of such clusters: 262 to 434 us where 266 were modelled).  The 64 x 32 tile hands a stage over
 // for every chunk of a warp: 250 clocks a stage, twice that for 8-byte elements (a 512 x 4096 x 4096 product as seven waves of it took 635 us instead of
 // the 514 modelled without; the 128 x 128 tile takes 580).
 // A gathered element costs 0.17 clocks on the small tiles where the contraction is bound by register reads (2048^3
@@ -453,7 +455,7 @@ LaunchPlan plan_without_workspace(const cuasr_b200_desc_t& desc, int m, int n, i
       if ((z - 1) * per_piece >= k_steps) break;                        // every CTA of a cluster has work
       const long long room = z <= 2 ? sms : z == 4 ? sms * 36LL / 37 : sms * 32LL / 37;
       const long long waves = (tiles * z + room - 1) / room;
-      const double end = (tile == kLargeTile ? 2000 : 1500) * wide + (z > 1 ? 2500 + (waves > 1 ? 4000 : 0) : 0);
+      const double end = (tile == kLargeTile ? 8000 : 1500) * wide + (z > 1 ? 2500 + (waves > 1 ? (z == 8 ? 30000 : 4000) : 0) : 0);
       const bool gather_a = tile == kLargeTile ? g.large_a : g.a, gather_b = tile == kLargeTile ? g.large_b : g.b;
       const double gathered = gather_clocks(desc, tile == kLargeTile) * step * ((gather_a ? kTileRows[tile] : 0) + (gather_b ? kTileCols[tile] : 0));
       const double per_stage = clocks_per_k(desc, tile) * step / kTileWk[tile] + gathered + (tile == kTinyTile ? 250 * wide : 0);
@@ -560,8 +562,10 @@ double ticket_plan_cost(const cuasr_b200_desc_t& desc, long long tiles, int whol
   const int k_steps = (k + tk - 1) / tk, per_piece = (k_steps + pieces - 1) / pieces;
   const double per_step = (clocks_per_k(desc, kLargeTile) + gather_clocks(desc, true) * kTileM * gathered) * tk;
   const long long waves = whole_tiles / sms, tail = ((tiles - whole_tiles) * pieces + sms - 1) / sms;
-  // the tickets are cleared by a memset in front of the launch; a piece is parked and read back by the last one
-  return 3000 + 4000 + waves * (per_step * k_steps + 2000 * wide) + tail * (per_step * per_piece + 1000 * wide) + 1000 * wide * pieces;
+  // the tickets are cleared by a memset in front of the launch; a piece is parked and read back by the last one, 20000 clocks a
+  // wave (1000^3 in two pieces 88 us, 2048^3 in four of its last wave 527)
+  const double parked = 10000 * (1 + wide);
+  return 3000 + 4000 + waves * (per_step * k_steps + 8000 * wide) + tail * (per_step * per_piece + parked) + 1000 * wide * pieces;
 }
 
 // How the kernels that can fill in NaN or an infinity bring in one operand, and its tensor map if that is TMA.
@@ -695,14 +699,16 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   constexpr int TK = kTileKBytes / sizeof(T);
   const long long tiles = static_cast<long long>(tile_count(args));
   const bool all_tiles = ring_has_all_tiles<T>(desc);
-  const size_t balance_bytes = slices == 1 && all_tiles ? balance_workspace_bytes(desc, args, plan_sms) : 0;
-  const BalancePlan balance = balance_plan(tiles, plan_sms, (args.k + TK - 1) / TK);
   // an optional workspace buys load balancing and, behind its scratch, copies of operands, as far as it has room for them
-  const bool optional = slices == 1 && args.workspace != nullptr && workspace_aligned;
-  const bool balanced = optional && balance_bytes > 0 && args.workspace_bytes >= balance_bytes;
-  const size_t copies_at = align_up(slices == 1 ? balance_workspace_bytes(desc, args, plan_sms) : 0, 256);
+  BalancePlan balance{0, 1};
+  bool balanced = false;
+  size_t copies_at = 0;
   RepackPlan copies;
-  if (optional) {
+  if (slices == 1 && args.workspace != nullptr && workspace_aligned) {
+    const size_t balance_bytes = balance_workspace_bytes(desc, args, plan_sms);
+    balanced = all_tiles && balance_bytes > 0 && args.workspace_bytes >= balance_bytes;
+    if (balanced) balance = balance_plan(tiles, plan_sms, (args.k + TK - 1) / TK);
+    copies_at = align_up(balance_bytes, 256);
     copies = repack_plan(desc, args, p, plan_sms);
     if (copies.bytes == 0 || args.workspace_bytes < copies_at + copies.bytes) copies = RepackPlan();
   }

@@ -116,6 +116,34 @@ def test_logical_ring_of_any_value(cuda_device, dtype):
         assert (D == (want | (start != 0)).to(D.dtype)).all(), start
 
 
+# pieces of every tile, and whole tiles in front of pieces of the last wave's
+@pytest.mark.parametrize("ring, dtype, m, n, k", [("minimum_plus", "f32", 1500, 1000, 2048), ("maximum_plus", "f64", 1500, 1000, 1024),
+                                                  ("plus_multiplies", "f64", 1500, 2048, 2048), ("maximum_minimum", "s32", 1500, 1000, 2048),
+                                                  ("maximum_minimum", "s32", 1500, 2048, 1024)])
+def test_pieces_meet_through_tickets(cuda_device, ring, dtype, m, n, k):
+    """The optional workspace of a launch that the model cuts along K; twice on the same workspace, whose contents do not matter
+    and whose tickets the first launch has used."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(k)
+    A, B, C = (whole_numbers(g, s, dtype) for s in ((m, k), (k, n), (m, n)))
+    want = by_loop(ring, A, B, C)
+    add, mul = RINGS[ring]
+    true_inf = dtype in ("f32", "f64")
+    one = identity(mul, DTYPE[dtype], true_infinity=true_inf)
+    op = Srgemm(add, mul, DTYPE[dtype], ROW, COL, ROW, add_identity=identity(add, DTYPE[dtype], true_infinity=true_inf))
+    B = B.T.contiguous()
+    ws = None
+    for _ in range(2):
+        D = torch.full_like(C, 77)
+        args = Arguments((m, n, k), (A, k), (B, k), (C, n), (D, n), (one, one))
+        if ws is None:
+            ws = torch.full((op.get_optional_workspace_size(args),), 0x5A, dtype=torch.uint8, device="cuda")
+        assert op(args, ws) == Status.kSuccess
+        assert "tickets=1" in op.last_route(), op.last_route()
+        assert (D == want).all()
+    assert device_status() == 0
+
+
 def test_ragged_k_does_not_lean_on_the_identities(cuda_device):
     """An integer minimum has no neutral padding: a K that ends inside a K step must not bring in products of the
     caller's identities, whatever they are."""
