@@ -32,6 +32,7 @@ struct Route {
   const char* load_a = "";
   const char* load_b = "";
   bool tickets = false, copied_a = false, copied_b = false;
+  int screened_pieces = 0;          // > 0: the screened kernel too, and the operands decided which of the two did the product
 };
 thread_local Route t_route;
 thread_local char t_route_text[160];
@@ -442,12 +443,14 @@ Gathers gathers_of(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args,
   return g;
 }
 
-LaunchPlan plan_without_workspace(const cuasr_b200_desc_t& desc, int m, int n, int k, int sms, bool all_tiles, const Gathers& g) {
+LaunchPlan plan_without_workspace(const cuasr_b200_desc_t& desc, int m, int n, int k, int sms, bool all_tiles, const Gathers& g,
+                                  bool asks = false) {
   const int tk = kTileKBytes / (desc.dtype == CUASR_F64 ? 8 : 4);
   const double wide = desc.dtype == CUASR_F64 ? 2.0 : 1.0;
   LaunchPlan best;
   for (int tile = all_tiles ? kLargeTile : kSmallTile; tile <= kTinyTile; ++tile) {
     const long long tiles = static_cast<long long>((m + kTileRows[tile] - 1) / kTileRows[tile]) * ((n + kTileCols[tile] - 1) / kTileCols[tile]);
+    if (asks && tile == kMediumTile && best.whole_tiles >= sms) break;  // (the variants that ask are slower on smaller tiles: 2048^3 1921 us on 64 x 64)
     const int step = tk * tile_sub(tile, desc);
     const int k_steps = (k + step - 1) / step;
     for (int z = 1; z <= (tile == kLargeTile ? 1 : 8); z *= 2) {
@@ -455,6 +458,7 @@ LaunchPlan plan_without_workspace(const cuasr_b200_desc_t& desc, int m, int n, i
       if ((z - 1) * per_piece >= k_steps) break;                        // every CTA of a cluster has work
       const long long room = z <= 2 ? sms : z == 4 ? sms * 36LL / 37 : sms * 32LL / 37;
       const long long waves = (tiles * z + room - 1) / room;
+      if (asks && z > 1 && waves > 1) break;                            // every CTA looks at the sample: once
       const double end = (tile == kLargeTile ? 8000 : 1500) * wide + (z > 1 ? 2500 + (waves > 1 ? (z == 8 ? 30000 : 4000) : 0) : 0);
       const bool gather_a = tile == kLargeTile ? g.large_a : g.a, gather_b = tile == kLargeTile ? g.large_b : g.b;
       const double gathered = gather_clocks(desc, tile == kLargeTile) * step * ((gather_a ? kTileRows[tile] : 0) + (gather_b ? kTileCols[tile] : 0));
@@ -486,6 +490,40 @@ bool has_all_tiles(const cuasr_b200_desc_t& desc) {
   }
 }
 
+// ---- the screened kernel (srgemm_screened.cuh) -------------------------------------------------------------------
+struct ScreenPlan {
+  int pieces = 1, blocks_per_piece = 0;
+  double cost = 1e300;
+};
+// Modelled clocks: 3.7 per product and scheduler with the tests, the conversions and the usual number of recomputed
+// elements (1000 x 1000 x 3000 takes 250 us more than 1000^3 with 31 blocks more per CTA), and 400000 per tile or piece for
+// its first blocks, which are done exactly or with many recomputed elements; 40000 for the two launches and their samples.  So
+// 2048^3 is screened (1.37 - 1.43 ms against 1.72 exact) and 1000^3 is not (334 - 379 us against 237).
+// An operand that is gathered costs it 4.5 % (4096^3 7760 -> 8066 us with one, 2048^3 1397 -> 1475).
+ScreenPlan screen_plan(int m, int n, int k, int sms, bool may_split, const Gathers& g) {
+  const int blocks = (k + kScreenBlock - 1) / kScreenBlock;
+  const long long tiles = static_cast<long long>((m + kTileM - 1) / kTileM) * ((n + kTileN - 1) / kTileN);
+  const double per_block = 128.0 * kScreenBlock * 3.7;
+  const double first = 400000;
+  ScreenPlan best;
+  for (int pieces = 1; pieces <= (may_split ? 128 : 1) && pieces <= blocks; ++pieces) {
+    const int per_piece = (blocks + pieces - 1) / pieces;
+    if ((pieces - 1) * per_piece >= blocks) continue;                     // every piece has work
+    const long long waves = (tiles * pieces + sms - 1) / sms;
+    const double cost = 40000 + (pieces > 1 ? 4000 : 0) + static_cast<double>(waves) * (per_block * per_piece + first + 2000);
+    if (cost < best.cost) { best.cost = cost; best.pieces = pieces; best.blocks_per_piece = per_piece; }
+  }
+  best.cost *= 1 + 0.045 * (g.a + g.b);
+  return best;
+}
+// The products the screened kernel can do: no factor (alpha is the identity of +) and a start value that compares, so that the running
+// minimum can live in D; and no negative zeros among the factors, so that D holds none and values that compare equal are the same.
+bool can_screen(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args) {
+  if (desc.dtype != CUASR_F64 || desc.mul_op != CUASR_OP_PLUS || (desc.add_op != CUASR_OP_MINIMUM && desc.add_op != CUASR_OP_MAXIMUM)) return false;
+  const double alpha = load_scalar<double>(args.alpha), beta = load_scalar<double>(args.beta), id = load_scalar<double>(args.add_identity);
+  return id == id && alpha == 0.0 && !std::signbit(alpha) && !(beta == 0.0 && std::signbit(beta));
+}
+
 // Every other ring (the integer min/max rings) has no value TMA could fill in.  With the optional workspace both
 // operands are copied and their K range is extended to a whole number of K steps by repeating the last k, as the gather
 // does without the workspace: these rings are idempotent, and nothing depends on the caller's identities.
@@ -515,8 +553,11 @@ RepackPlan repack_plan(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& a
     plan.a = !tma_describable(p.a, p.lda, es);
     plan.b = !tma_describable(p.b, p.ldb, es);
     const bool all_tiles = has_all_tiles(desc);
+    const bool screens = can_screen(desc, args);
     auto cost = [&](bool copy_a, bool copy_b) {
-      return plan_without_workspace(desc, p.m, p.n, p.k, sms, all_tiles, gathers_of(desc, args, p, copy_a, copy_b)).cost;
+      const Gathers g = gathers_of(desc, args, p, copy_a, copy_b);
+      const double exact = plan_without_workspace(desc, p.m, p.n, p.k, sms, all_tiles, g).cost;
+      return screens ? std::min(exact, screen_plan(p.m, p.n, p.k, sms, true, g).cost) : exact;
     };
     for (const bool first : {true, false}) {
       RepackPlan more = plan;
@@ -528,31 +569,6 @@ RepackPlan repack_plan(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& a
   }
   plan.bytes = copies_bytes(plan, p, es);
   return plan;
-}
-
-// ---- the screened kernel (srgemm_screened.cuh) -------------------------------------------------------------------
-struct ScreenPlan {
-  int pieces = 1, blocks_per_piece = 0;
-  double cost = 1e300;
-};
-// Modelled clocks: 3.7 per product and scheduler with the tests, the conversions and the usual number of recomputed
-// elements (1000 x 1000 x 3000 takes 250 us more than 1000^3 with 31 blocks more per CTA), and 400000 per tile or piece for
-// its first blocks, which are done exactly or with many recomputed elements.  So 2048^3 is screened (1.46 - 1.55 ms
-// against 1.90 exact) and 1000^3 is not (334 - 379 us against 276).
-ScreenPlan screen_plan(int m, int n, int k, int sms, bool may_split) {
-  const int blocks = (k + kScreenBlock - 1) / kScreenBlock;
-  const long long tiles = static_cast<long long>((m + kTileM - 1) / kTileM) * ((n + kTileN - 1) / kTileN);
-  const double per_block = 128.0 * kScreenBlock * 3.7;
-  const double first = 400000;
-  ScreenPlan best;
-  for (int pieces = 1; pieces <= (may_split ? 128 : 1) && pieces <= blocks; ++pieces) {
-    const int per_piece = (blocks + pieces - 1) / pieces;
-    if ((pieces - 1) * per_piece >= blocks) continue;                     // every piece has work
-    const long long waves = (tiles * pieces + sms - 1) / sms;
-    const double cost = 4000 + (pieces > 1 ? 4000 : 0) + static_cast<double>(waves) * (per_block * per_piece + first + 2000);
-    if (cost < best.cost) { best.cost = cost; best.pieces = pieces; best.blocks_per_piece = per_piece; }
-  }
-  return best;
 }
 
 // Modelled clocks of a launch of large tiles whose pieces meet through tickets in a workspace.
@@ -591,7 +607,7 @@ bool in_device_memory(const void* ptr) {
 }
 
 // Launches the screened kernel on a normalised problem (row-major D).
-int run_screened(bool maximize, const Normalised& p, double beta, double add_id, bool read_c, const ScreenPlan& plan,
+int run_screened(bool maximize, const Normalised& p, double beta, double add_id, bool read_c, const ScreenPlan& plan, bool if_it_helps,
                  const ExtraOutputs& extra, DeviceState* dev, cudaStream_t stream) {
   ScreenParams sp = {};
   sp.M = p.m; sp.N = p.n; sp.K = p.k;
@@ -606,6 +622,7 @@ int run_screened(bool maximize, const Normalised& p, double beta, double add_id,
   sp.n_extra = extra.count;
   for (int x = 0; x < extra.count; ++x) sp.extra_d[x] = static_cast<double*>(extra.ptr[x]);
   sp.tiles_m = (p.m + kTileM - 1) / kTileM; sp.tiles_n = (p.n + kTileN - 1) / kTileN;
+  sp.if_it_helps = if_it_helps;
   sp.pieces = plan.pieces; sp.blocks_per_piece = plan.blocks_per_piece;
   sp.status = dev->status;
   const long long work = static_cast<long long>(sp.tiles_m) * sp.tiles_n * sp.pieces;
@@ -618,6 +635,7 @@ int run_screened(bool maximize, const Normalised& p, double beta, double add_id,
   if (launch_screened(maximize, map_a, map_b, sp, grid, stream) != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
   g_launches.fetch_add(1);
   t_route = {"screened", kTileM, kTileN, 1, plan.pieces, load_name(sp.a_mode), load_name(sp.b_mode)};
+  t_route.screened_pieces = plan.pieces;
   return CUASR_STATUS_SUCCESS;
 }
 
@@ -678,7 +696,7 @@ int run_path(bool maximize, const Normalised& p, int32_t* parent, long long ld_p
 }
 
 template <typename T>
-int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int slices, const ExtraOutputs& extra) {
+int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int slices, const ExtraOutputs& extra, int screen_pieces) {
   DeviceState* dev = nullptr;
   if (!device_state(&dev)) return CUASR_STATUS_ERROR_INTERNAL;
   cudaStream_t stream = static_cast<cudaStream_t>(args.stream);
@@ -727,9 +745,9 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   // the fastest launch with a given set of copies: without the workspace, or in pieces that meet through tickets in it
   Gathers gathers;
   bool tickets_used = false;
-  auto plan_with = [&](const RepackPlan& c, Gathers& g, bool& tickets) {
+  auto plan_with = [&](const RepackPlan& c, Gathers& g, bool& tickets, bool asks = false) {
     g = gathers_of(desc, args, p, c.a, c.b);
-    LaunchPlan best = plan_without_workspace(desc, p.m, p.n, p.k, plan_sms, all_tiles, g);
+    LaunchPlan best = plan_without_workspace(desc, p.m, p.n, p.k, plan_sms, all_tiles, g, asks);
     tickets = false;
     auto in_pieces = [&](int whole_tiles, int count, bool always) {
       const double cost = ticket_plan_cost(desc, tiles, whole_tiles, count, p.k, plan_sms, g.large_a + g.large_b);
@@ -743,7 +761,17 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
     best.cost += copies_clocks(c, p, sizeof(T));
     return best;
   };
+  // The screened kernel, where it is modelled faster, if the operands are what it helps with: it is launched in front of the exact one,
+  // and a sample of the operands tells either of them whether the product is its own.
+  const bool may_screen = can_screen(desc, args) && !(read_c && std::signbit(beta) && beta == T(0));
+  auto screened_with = [&](const RepackPlan& c, const Gathers& g) {
+    ScreenPlan best;
+    if (may_screen) best = screen_plan(p.m, p.n, p.k, dev->sms, extra.count == 0, g);
+    best.cost += copies_clocks(c, p, sizeof(T));
+    return best;
+  };
   LaunchPlan plan = plan_with(copies, gathers, tickets_used);
+  ScreenPlan screened = screened_with(copies, gathers);
   if (copies.faster_a || copies.faster_b) {          // in pieces the large tile may do as well on the operands as they are
     RepackPlan fewer = copies;
     fewer.a = copies.a && !copies.faster_a; fewer.b = copies.b && !copies.faster_b;
@@ -752,8 +780,13 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
     Gathers g;
     bool tickets;
     const LaunchPlan other = plan_with(fewer, g, tickets);
-    if (other.cost < plan.cost) { plan = other; copies = fewer; gathers = g; tickets_used = tickets; }
+    const ScreenPlan other_screened = screened_with(fewer, g);
+    if (std::min(other.cost, other_screened.cost) < std::min(plan.cost, screened.cost)) {
+      plan = other; screened = other_screened; copies = fewer; gathers = g; tickets_used = tickets;
+    }
   }
+  const bool use_screen = screen_pieces < 0 && screened.cost < plan.cost && in_device_memory(p.d);
+  if (use_screen) plan = plan_with(copies, gathers, tickets_used, true);
   const bool pads_itself = ring_pads_itself(desc, args);
   // operands whose storage lines overlap (leading dimension below the contiguous extent) stay off the TMA path
   const bool dense = p.lda >= (p.a_kcontig ? p.k : p.m) && p.ldb >= (p.b_kcontig ? p.k : p.n);
@@ -786,21 +819,21 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   const char* const name = !aligned_name ? (slices > 1 ? "generic_splitk" : "generic")
                            : slices > 1 ? "tma_splitk" : balanced ? "tma_balanced" : repacked ? "tma_repacked" : "tma";
   if constexpr (std::is_same<T, double>::value) {
-    // the screened kernel, where it is modelled faster: no factor on the product (alpha is the identity of +) and a
-    // start value that compares, so that the running minimum can live in D; and no negative zeros among the factors, so
-    // that D holds none and values that compare equal are the same
-    auto negative_zero = [](T x) { return x == T(0) && std::signbit(x); };
-    if (add_id == add_id && (desc.add_op == CUASR_OP_MINIMUM || desc.add_op == CUASR_OP_MAXIMUM) && desc.mul_op == CUASR_OP_PLUS &&
-        alpha == T(0) && !negative_zero(alpha) && !(read_c && negative_zero(beta))) {
-      const ScreenPlan screened = screen_plan(p.m, p.n, p.k, dev->sms, extra.count == 0);
-      if (screened.cost < plan.cost && in_device_memory(p.d)) {
-        const int st = run_screened(desc.add_op == CUASR_OP_MAXIMUM, p, beta, add_id, read_c, screened, extra, dev, stream);
-        if (st == CUASR_STATUS_SUCCESS) {
-          t_last_kernel = name;
-          t_route.copied_a = copies.a; t_route.copied_b = copies.b;
-        }
-        return st;
+    const bool maximize = desc.add_op == CUASR_OP_MAXIMUM;
+    if (screen_pieces >= 0) {          // cuasr_b200_srgemm_screened
+      if (!may_screen) return CUASR_STATUS_ERROR_NOT_SUPPORTED;
+      if (screen_pieces > 0) {
+        const int blocks = (p.k + kScreenBlock - 1) / kScreenBlock;
+        screened.pieces = screen_pieces; screened.blocks_per_piece = (blocks + screen_pieces - 1) / screen_pieces;
+        if ((screened.pieces - 1LL) * screened.blocks_per_piece >= blocks) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
       }
+    }
+    if (screen_pieces >= 0 || use_screen) {
+      const int st = run_screened(maximize, p, beta, add_id, read_c, screened, use_screen, extra, dev, stream);
+      if (st != CUASR_STATUS_SUCCESS) return st;
+      t_last_kernel = name;
+      t_route.copied_a = copies.a; t_route.copied_b = copies.b;
+      if (!use_screen) return st;
     }
   }
   const int step = TK * tile_sub(plan.tile, desc);
@@ -845,6 +878,7 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   tp.whole_tiles = plan.whole_tiles;
   tp.slices = plan.pieces;
   tp.cluster = plan.cluster > 1;
+  tp.unless_screened = use_screen;
   const int k_steps = (p.k + step - 1) / step;
   tp.k_tiles_per_slice = (k_steps + plan.pieces - 1) / plan.pieces;
   tp.partial = nullptr; tp.tickets = nullptr;
@@ -873,18 +907,18 @@ int run_typed(const cuasr_b200_desc_t& desc, const cuasr_b200_args_t& args, int 
   if (err != cudaSuccess) return CUASR_STATUS_ERROR_INTERNAL;
   t_last_kernel = name;
   t_route = {"product", kTileRows[plan.tile], kTileCols[plan.tile], plan.cluster, plan.pieces, load_name(tp.a_mode), load_name(tp.b_mode),
-             tickets_used && plan.pieces > 1, copies.a, copies.b};
+             tickets_used && plan.pieces > 1, copies.a, copies.b, use_screen ? screened.pieces : 0};
   g_launches.fetch_add(1);
   return CUASR_STATUS_SUCCESS;
 }
 
 int run(const cuasr_b200_desc_t* desc, const cuasr_b200_args_t* args, int slices,
-        const ExtraOutputs& extra = ExtraOutputs()) {
+        const ExtraOutputs& extra = ExtraOutputs(), int screen_pieces = -1) {
   switch (desc->dtype) {
-    case CUASR_F32: return run_typed<float>(*desc, *args, slices, extra);
-    case CUASR_F64: return run_typed<double>(*desc, *args, slices, extra);
-    case CUASR_S32: return run_typed<int32_t>(*desc, *args, slices, extra);
-    case CUASR_U32: return run_typed<uint32_t>(*desc, *args, slices, extra);
+    case CUASR_F32: return run_typed<float>(*desc, *args, slices, extra, screen_pieces);
+    case CUASR_F64: return run_typed<double>(*desc, *args, slices, extra, screen_pieces);
+    case CUASR_S32: return run_typed<int32_t>(*desc, *args, slices, extra, screen_pieces);
+    case CUASR_U32: return run_typed<uint32_t>(*desc, *args, slices, extra, screen_pieces);
     default: return CUASR_STATUS_ERROR_INVALID_DATA_TYPE;
   }
 }
@@ -1008,6 +1042,14 @@ int cuasr_b200_srgemm_push(const cuasr_b200_desc_t* desc, const cuasr_b200_args_
   return run(desc, args, args->split_k_slices, extra);
 }
 
+int cuasr_b200_srgemm_screened(const cuasr_b200_desc_t* desc, const cuasr_b200_args_t* args, int pieces) {
+  const int st = cuasr_b200_srgemm_can_implement(desc, args);
+  if (st != CUASR_STATUS_SUCCESS) return st;
+  if (desc->dtype != CUASR_F64 || args->split_k_slices != 1) return CUASR_STATUS_ERROR_NOT_SUPPORTED;
+  if (pieces < 0) return CUASR_STATUS_ERROR_INVALID_PROBLEM;
+  return run(desc, args, 1, ExtraOutputs(), pieces);
+}
+
 int cuasr_b200_srgemm_splitk_can_implement(const cuasr_b200_desc_t* desc, const cuasr_b200_args_t* args) {
   return validate(desc, args);
 }
@@ -1127,7 +1169,10 @@ const char* cuasr_b200_last_kernel(void) { return t_last_kernel; }
 const char* cuasr_b200_last_route(void) {
   const Route& r = t_route;
   if (r.tile_m == 0) return r.kernel;
-  std::snprintf(t_route_text, sizeof(t_route_text), "%s tile=%dx%d cluster=%d pieces=%d tickets=%d a=%s%s b=%s%s", r.kernel, r.tile_m,
+  char screened[32] = "";
+  if (r.screened_pieces > 0 && std::strcmp(r.kernel, "product") == 0)
+    std::snprintf(screened, sizeof(screened), "screened pieces=%d or ", r.screened_pieces);
+  std::snprintf(t_route_text, sizeof(t_route_text), "%s%s tile=%dx%d cluster=%d pieces=%d tickets=%d a=%s%s b=%s%s", screened, r.kernel, r.tile_m,
                 r.tile_n, r.cluster, r.pieces, (int)r.tickets, r.copied_a ? "copy+" : "", r.load_a, r.copied_b ? "copy+" : "", r.load_b);
   return t_route_text;
 }

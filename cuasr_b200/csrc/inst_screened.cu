@@ -16,9 +16,9 @@ cudaError_t launch_screened(bool maximize, const CUtensorMap& map_a, const CUten
   return maximize ? launch_variant<true>(map_a, map_b, params, grid, stream) : launch_variant<false>(map_a, map_b, params, grid, stream);
 }
 cudaError_t launch_screened_init(bool maximize, const ScreenParams& params, int sms, cudaStream_t stream) {
-  const long long blocks = (static_cast<long long>(params.M) * params.N + 255) / 256;
-  const int grid = static_cast<int>(blocks < 8LL * sms ? blocks : 8LL * sms);
-  return maximize ? launch_overlapped(screened_init_kernel<Ring<CUASR_OP_MAXIMUM, CUASR_OP_PLUS, double>>, grid, 256, 0, 1, stream, params)
-                  : launch_overlapped(screened_init_kernel<Ring<CUASR_OP_MINIMUM, CUASR_OP_PLUS, double>>, grid, 256, 0, 1, stream, params);
+  const long long blocks = (static_cast<long long>(params.M) * params.N + kSampleThreads - 1) / kSampleThreads;
+  const int grid = static_cast<int>(blocks < 2LL * sms ? blocks : 2LL * sms);
+  return maximize ? launch_overlapped(screened_init_kernel<Ring<CUASR_OP_MAXIMUM, CUASR_OP_PLUS, double>>, grid, kSampleThreads, 0, 1, stream, params)
+                  : launch_overlapped(screened_init_kernel<Ring<CUASR_OP_MINIMUM, CUASR_OP_PLUS, double>>, grid, kSampleThreads, 0, 1, stream, params);
 }
 }  // namespace cuasr_b200

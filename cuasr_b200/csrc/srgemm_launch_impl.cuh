@@ -21,16 +21,27 @@ cudaError_t opt_in_shared_memory(Kernel kernel, int bytes, std::atomic<unsigned 
   return err;
 }
 
-template <typename RingT, typename Tile>
-cudaError_t launch_tma_variant(const CUtensorMap& map_a, const CUtensorMap& map_b,
-                               const TmaParams<typename RingT::Element>& params, int grid, int cluster,
-                               cudaStream_t stream) {
+template <typename RingT, typename Tile, bool kAsks>
+cudaError_t launch_tma_kernel(const CUtensorMap& map_a, const CUtensorMap& map_b,
+                              const TmaParams<typename RingT::Element>& params, int grid, int cluster,
+                              cudaStream_t stream) {
   using T = typename RingT::Element;
-  auto kernel = srgemm_tma_kernel<RingT, Tile>;
+  auto kernel = srgemm_tma_kernel<RingT, Tile, kAsks>;
   static std::atomic<unsigned long long> done{0};
   const cudaError_t err = opt_in_shared_memory(kernel, Tile::template kSmemBytes<T>, done);
   if (err != cudaSuccess) return err;
   return launch_overlapped(kernel, grid, kTmaThreads, Tile::template kSmemBytes<T>, cluster, stream, map_a, map_b, params);
+}
+
+template <typename RingT, typename Tile>
+cudaError_t launch_tma_variant(const CUtensorMap& map_a, const CUtensorMap& map_b,
+                               const TmaParams<typename RingT::Element>& params, int grid, int cluster,
+                               cudaStream_t stream) {
+  if constexpr (std::is_same<typename RingT::Element, double>::value && RingT::kMul == CUASR_OP_PLUS &&
+                (RingT::kAdd == CUASR_OP_MINIMUM || RingT::kAdd == CUASR_OP_MAXIMUM)) {
+    if (params.unless_screened) return launch_tma_kernel<RingT, Tile, true>(map_a, map_b, params, grid, cluster, stream);
+  }
+  return launch_tma_kernel<RingT, Tile, false>(map_a, map_b, params, grid, cluster, stream);
 }
 
 template <int ADD, int MUL, typename T>

@@ -16,9 +16,10 @@
 // tiles seen so far.  A stage with a negative or too large finite value is "unfit" and done exactly; a larger 2^-e
 // follows for the next.
 //
-// What the screen saves depends on the data (4096^3, 12.3 ms before it, 14.4 with the exact kernel of srgemm_tma.cuh): sparse
-// edges 7.7 ms, uniform values 8.0, small whole numbers 4.7, sums that improve along k 7.5; values it cannot hold, negative
-// ones or magnitudes over hundreds of decades, are done exactly in runs of blocks, 18.5.
+// What the screen saves depends on the data (4096^3, 12.3 ms with the exact kernel of srgemm_tma.cuh): sparse edges 7.1 ms,
+// uniform values 7.3, small whole numbers 4.6, sums that improve along k 7.5.  Values it cannot hold, negative ones or
+// magnitudes over hundreds of decades, are done exactly in runs of blocks, 15.8 ms; a sample of the operands sends such data to the
+// exact kernel (screen_sample.cuh), and the runs are for what the sample does not show.
 //
 // The running result lives in D itself: an element is written when it improves, by the lane that found it.  Elements
 // and blocks are independent of order, so K may be cut into pieces for different CTAs, which then meet in D by
@@ -45,6 +46,7 @@ struct ScreenParams {
   int n_extra;
   T* extra_d[kMaxDestinations - 1];
   int tiles_m, tiles_n, pieces, blocks_per_piece;
+  int if_it_helps;                 // return at once where screen_helps says no (the exact kernel's launch follows)
   unsigned int* status;
 };
 
@@ -56,7 +58,9 @@ constexpr int kScreenBoundBytes = 8 * 64 * 32 * 2;   // per warp, element and la
 constexpr int kListGroups = 4;                       // groups of eight elements that a warp recomputes at a time
 constexpr int kListed = 96;                          // elements to recompute that a warp lists at a time
 constexpr int kScreenListBytes = 8 * kListed * 2;
-constexpr int kScreenSmemBytes = kScreenStages * kScreenStageBytes + kScreenBoundBytes + kScreenListBytes + 512 + 1024;
+constexpr int kScreenRowBytes = kConsumerThreads * 8 * (int)sizeof(double);   // eight accumulators of every lane, on their way to D
+constexpr int kScreenSmemBytes = kScreenStages * kScreenStageBytes + kScreenBoundBytes + kScreenListBytes + kScreenRowBytes + 512 + 1024;
+static_assert(kScreenSmemBytes <= kMaxSmemBytes, "one CTA's shared memory");
 
 __device__ __forceinline__ void sts16(uint32_t addr, uint4 v) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
@@ -173,7 +177,8 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* bounds_smem = smem + kScreenStages * kScreenStageBytes;
   uint8_t* list_smem = bounds_smem + kScreenBoundBytes;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(list_smem + kScreenListBytes);   // exact tile landed
+  uint8_t* rows_smem = list_smem + kScreenListBytes;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(rows_smem + kScreenRowBytes);   // exact tile landed
   uint64_t* ready_bar = full_bar + kScreenStages;                                     // 16-bit tile written
   uint64_t* empty_bar = ready_bar + kScreenStages;
   // per stage: largest and smallest finite scaled value seen by each producer warp, and the exponent
@@ -199,6 +204,8 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   __syncthreads();
   grid_dependency_wait();
   grid_dependency_launch();
+  if (p.if_it_helps && !screen_helps<kMax>(p.A, p.lda, p.a_mode != kLoadGatherMN, p.M, p.B, p.ldb, p.b_mode != kLoadGatherMN, p.N, p.K))
+    return;
 
   const int blocks_total = (p.K + KB - 1) / KB;
   const int num_work = p.tiles_m * p.tiles_n * p.pieces;
@@ -378,6 +385,7 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   const uint32_t my_bounds = smem_u32(bounds_smem) + warp * (64 * 32 * 2) + lane * 16;   // row i: + i * 512, element j: + 2 j
   const uint32_t warp_bounds = smem_u32(bounds_smem) + warp * (64 * 32 * 2);
   const uint32_t list = smem_u32(list_smem) + warp * (kListed * 2);
+  const uint32_t my_row = smem_u32(rows_smem) + warp * (32 * 8 * (int)sizeof(T)) + lane * 16;   // elements j .. j + EV - 1 of a row: + j * 512 / EV
   const bool shared_d = p.pieces > 1;
 
   uint32_t it = 0;
@@ -442,9 +450,9 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
               T bj[EV];
               lds16(((j & 1) ? b1 : b0) + j * 512, bj);
 #pragma unroll
-              for (int e = 0; e < EV; e += 2)
+              for (int e = 0; e < EV; ++e)               // kByColumn of srgemm_tma.cuh
 #pragma unroll
-                for (int i = 0; i < 8; ++i) acc[i][j] = RingT::mac2(acc[i][j], a[i][e], bj[e], a[i][e + 1], bj[e + 1]);
+                for (int i = 0; i < 8; ++i) acc[i][j] = RingT::add(a[i][e] + bj[e], acc[i][j]);
             }
           }
           __syncwarp();
@@ -454,43 +462,48 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
           // (the 16-bit tile of the next block is not waited for)
           mbar_wait_or_abandon(&full_bar[it % kScreenStages], (it / kScreenStages) & 1, p.status, kDeviceTimeoutFull, abandoned);
         }
-        // (the opaque zero: the addresses are computed here instead of being carried through the contraction)
-        int zero;
-        asm volatile("mov.s32 %0, 0;" : "=r"(zero));
+        // Row by row through the lane's own 64 bytes of shared memory, four elements at a time in a loop that is not unrolled: with
+        // the accumulators in registers the 64 copies of this code spill all of them.
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const int m = m_base + lr + 8 * i + zero;
-          T cur[8];                      // a row's loads together: none of them can pass a store
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int n = n_base + lc + 4 * j;
-            if (m >= p.M || n >= p.N) continue;
-            if (shared_d || opened) cur[j] = __ldcg(p.D + (long long)m * p.ldd + n);   // improved at the L2 by other lanes
-            else if (p.read_c) cur[j] = p.C[(long long)m * p.ldc + n];
-          }
-          uint32_t q[8];
+          for (int j = 0; j < 8; j += EV) sts16(my_row + j * (512 / EV), *reinterpret_cast<const uint4*>(&acc[i][j]));
+          const int m = m_base + lr + 8 * i;
+#pragma unroll 1
+          for (int half = 0; half < 2; ++half) {
+            const int n0 = n_base + lc + 16 * half;
+            T v[4], cur[4];                // loads together: none of them can pass a store
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int n = n_base + lc + 4 * j;
-            T v = acc[i][j] + T(0);                          // alpha (x) product
-            const bool inside = m < p.M && n < p.N;
-            if (inside) {
-              T* at = p.D + (long long)m * p.ldd + n;
-              if (shared_d) {
-                if (!S::better(v, cur[j])) v = cur[j];
-                else if (v >= T(0)) merge_into<kMax>(at, v);       // without waiting for the answer
-                else v = improve_shared<kMax>(at, v, cur[j]);
-              } else if (opened) {
-                if (S::better(v, cur[j])) *at = v;
-                else v = cur[j];
-              } else {
-                if (p.read_c) v = RingT::add(v, RingT::mul(p.beta, cur[j]));
-                *at = v;
-              }
+            for (int j = 0; j < 4; ++j) {
+              if (m >= p.M || n0 + 4 * j >= p.N) continue;
+              if (shared_d || opened) cur[j] = __ldcg(p.D + (long long)m * p.ldd + n0 + 4 * j);   // improved at the L2 by other lanes
+              else if (p.read_c) cur[j] = p.C[(long long)m * p.ldc + n0 + 4 * j];
             }
-            q[j] = inside ? S::bound(v, scale) : S::kNothing;
+#pragma unroll
+            for (int j = 0; j < 4; j += EV) lds16(my_row + (4 * half + j) * (512 / EV), *reinterpret_cast<T(*)[EV]>(&v[j]));
+            uint32_t q[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              v[j] += T(0);                                  // alpha (x) product
+              const bool inside = m < p.M && n0 + 4 * j < p.N;
+              if (inside) {
+                T* at = p.D + (long long)m * p.ldd + n0 + 4 * j;
+                if (shared_d) {
+                  if (!S::better(v[j], cur[j])) v[j] = cur[j];
+                  else if (v[j] >= T(0)) merge_into<kMax>(at, v[j]);       // without waiting for the answer
+                  else v[j] = improve_shared<kMax>(at, v[j], cur[j]);
+                } else if (opened) {
+                  if (S::better(v[j], cur[j])) *at = v[j];
+                  else v[j] = cur[j];
+                } else {
+                  if (p.read_c) v[j] = RingT::add(v[j], RingT::mul(p.beta, cur[j]));
+                  *at = v[j];
+                }
+              }
+              q[j] = inside ? S::bound(v[j], scale) : S::kNothing;
+            }
+            asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(my_bounds + i * 512 + half * 8), "r"(q[0] | (q[1] << 16)), "r"(q[2] | (q[3] << 16)) : "memory");
           }
-          sts16(my_bounds + i * 512, make_uint4(q[0] | (q[1] << 16), q[2] | (q[3] << 16), q[4] | (q[5] << 16), q[6] | (q[7] << 16)));
         }
         opened = true;
         my_exp = exponent;
@@ -663,13 +676,17 @@ srgemm_screened_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 
 // D = the start values of a product whose pieces meet in D: the additive identity, folded with beta (x) C.
 template <typename RingT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kSampleThreads)
 screened_init_kernel(const __grid_constant__ ScreenParams p) {
   using T = typename RingT::Element;
   grid_dependency_wait();
   grid_dependency_launch();
+  // (start values are written for nothing where C is another matrix)
+  if (p.if_it_helps && p.read_c && p.C == p.D && !screen_helps<RingT::kAdd == CUASR_OP_MAXIMUM>(p.A, p.lda, p.a_mode != kLoadGatherMN, p.M, p.B, p.ldb,
+                                                                       p.b_mode != kLoadGatherMN, p.N, p.K))
+    return;
   const long long total = (long long)p.M * p.N;
-  for (long long idx = (long long)blockIdx.x * 256 + threadIdx.x; idx < total; idx += (long long)gridDim.x * 256) {
+  for (long long idx = (long long)blockIdx.x * kSampleThreads + threadIdx.x; idx < total; idx += (long long)gridDim.x * kSampleThreads) {
     const int m = static_cast<int>(idx / p.N), n = static_cast<int>(idx - (long long)m * p.N);
     T v = p.add_identity + T(0);                             // alpha (x) identity
     if (p.read_c) v = RingT::add(v, RingT::mul(p.beta, p.C[(long long)m * p.ldc + n]));

@@ -27,6 +27,7 @@
 #pragma once
 
 #include "gather.cuh"
+#include "screen_sample.cuh"
 
 namespace cuasr_b200 {
 
@@ -123,6 +124,7 @@ struct TmaParams {
   //  * cluster == 1 (WK > 1 only): whole_tiles = 0 and the `slices` CTAs of a cluster hold the pieces of one tile;
   //    CTA r of the cluster folds and writes the r-th part of the tile.
   int whole_tiles, slices, k_tiles_per_slice, cluster;
+  int unless_screened;          // behind the screened kernel: the variant that asks
   T* partial;
   unsigned int* tickets;
 };
@@ -198,7 +200,11 @@ __host__ __device__ constexpr int order_of() {
   return compares_only || Tile::WK == 2 ? kByHalf : kByElement;
 }
 
-template <typename RingT, typename Tile>
+// kAsks: launched behind the screened kernel; returns at once where screen_helps says that that one has done the product.  A variant of
+// its own, because code in front of it takes the fp64 contraction from 12.3 to 14.5 or 15.5 ms at 4096^3, and in the form that
+// the registers of either ring come off best with: 3000^3 on signed data, both operands by TMA / one gathered, min-plus 5130 / 5312 us
+// called and 5173 / 6260 inlined, max-plus 5192 / 6896 called and 5157 / 5160 inlined.
+template <typename RingT, typename Tile, bool kAsks>
 __global__ void __launch_bounds__(kTmaThreads, 1)
 srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                   const __grid_constant__ TmaParams<typename RingT::Element> p) {
@@ -212,6 +218,17 @@ srgemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   constexpr int TK = kTileKBytes / sizeof(T);     // k per 128-byte column: 32 or 16
   constexpr int kStep = TK * kSub;                // k per stage
   constexpr int kChunks = 8 * kSub / WK;          // 16-byte k chunks of a stage that one warp works on
+
+  if constexpr (kAsks) {
+    static_assert(kTmaThreads == kSampleThreads, "the sample is spread over the CTA");
+    grid_dependency_wait();
+    const bool a_along_k = p.a_mode != kLoadGatherMN, b_along_k = p.b_mode != kLoadGatherMN;
+    if constexpr (RingT::kAdd == CUASR_OP_MAXIMUM) {
+      if (screen_helps<true>(p.A, p.lda, a_along_k, p.M, p.B, p.ldb, b_along_k, p.N, p.K)) return;
+    } else {
+      if (screen_helps_called<false>(p.A, p.lda, a_along_k, p.M, p.B, p.ldb, b_along_k, p.N, p.K)) return;
+    }
+  }
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));

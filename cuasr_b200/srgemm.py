@@ -127,8 +127,8 @@ class _Operator:
         return int(self._fn("_workspace_size")(ctypes.byref(self._desc), ctypes.byref(self._pack(args))))
 
     def get_optional_workspace_size(self, args: Arguments) -> int:
-        """Bytes of OPTIONAL workspace for an unsplit launch (0 = nothing to gain): it buys a balanced last wave and,
-        for fp32 min/max-plus/times rings, K-contiguous copies of the operands so that packed adds can be used."""
+        """Bytes of OPTIONAL workspace for an unsplit launch (0 = nothing to gain): it buys a balanced last wave and
+        K-contiguous, aligned copies of operands that would otherwise be gathered element by element."""
         return int(self._lib.cuasr_b200_srgemm_optional_workspace_size(ctypes.byref(self._desc),
                                                                       ctypes.byref(self._pack(args))))
 
@@ -170,6 +170,11 @@ class _Operator:
         ptrs = (ctypes.c_void_p * max(1, len(extra_outputs)))(*[_ptr(x) for x in extra_outputs])
         return Status(self._lib.cuasr_b200_srgemm_push(ctypes.byref(self._desc), ctypes.byref(self._args),
                                                        len(extra_outputs), ptrs))
+
+    def run_screened(self, args: Arguments, pieces: int = 0, workspace=None, stream=None) -> Status:
+        """The product on the kernel that screens in 16 bits, whatever the operands: cuasr_b200_srgemm_screened."""
+        return Status(self._lib.cuasr_b200_srgemm_screened(ctypes.byref(self._desc),
+                                                           ctypes.byref(self._pack(args, workspace, 0, stream)), int(pieces)))
 
     def __call__(self, args: Optional[Arguments] = None, workspace=None, stream=None,
                  workspace_bytes: int = 0) -> Status:

@@ -111,11 +111,14 @@ CUASR_B200_API int cuasr_b200_srgemm_push(const cuasr_b200_desc_t *desc, const c
  * (test/regress/include/fwgpu/cpu_srgemm.hpp:20-48), generalised to both layouts, M x N x K and max-plus.
  * desc: add_op MINIMUM or MAXIMUM, mul_op PLUS, dtype F32 or F64.  args: A, B, D (= the distances, read and
  * written; C, alpha, beta, workspace are ignored), split_k_slices = 1.  parent has D's layout, leading dimension
- * ld_parent, 32-bit signed entries.  fp32 operands with 16-byte aligned storage lines run on the TMA pipeline (the
- * index is looked up, and parent written, only for elements that improved; parent is never read there), everything
- * else on an any-layout kernel. */
+ * ld_parent, 32-bit signed entries; written only where an element improved, and never read. */
 CUASR_B200_API int cuasr_b200_srgemm_path(const cuasr_b200_desc_t *desc, const cuasr_b200_args_t *args, int32_t *parent,
                                           int64_t ld_parent, int32_t k_offset);
+
+/* D of cuasr_b200_srgemm, for fp64 min-plus and max-plus without a factor (alpha and beta not negative zeros) by the kernel
+ * that screens products in 16 bits, whatever the operands and the size: cuasr_b200_srgemm launches that kernel where it is
+ * expected to be the faster one.  For measurements and tests.  pieces: into how many parts K is cut, 0 = chosen by size. */
+CUASR_B200_API int cuasr_b200_srgemm_screened(const cuasr_b200_desc_t *desc, const cuasr_b200_args_t *args, int pieces);
 
 /* SrgemmSplitKParallel::can_implement / get_workspace_size / operator()
  * (device/srgemm_splitk_parallel.h:220-235, :238-279, :333-348).  The reference needs
@@ -185,7 +188,8 @@ CUASR_B200_API const char *cuasr_b200_last_kernel(void);
  * before the first call), its tile, the CTAs that share a tile's K through a cluster or in pieces, whether the pieces meet
  * through tickets in the workspace, and how each operand of the row-major problem came in ("tma", "tma-rows", "gather",
  * "copy+tma"; with a column-major C that problem's operands are B and A), e.g.
- * "product tile=128x128 cluster=1 pieces=3 tickets=1 a=tma b=copy+tma".  For people and tests: the words may change.  The text
+ * "product tile=128x128 cluster=1 pieces=3 tickets=1 a=tma b=copy+tma".  "screened pieces=2 or product ...": both were launched, and
+ * the values of the operands decided on the device which of them did the product.  For people and tests: the words may change.  The text
  * is valid until the next call of this function on the thread. */
 CUASR_B200_API const char *cuasr_b200_last_route(void);
 

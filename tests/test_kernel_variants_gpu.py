@@ -49,7 +49,9 @@ def by_loop(ring, A, B, C):
     return add[a](acc, C)
 
 
-def check_product(ring, dtype, A, B, C, layouts, pads=(0, 0, 0), workspace=False, mul_identity=None, in_place=False):
+def check_product(ring, dtype, A, B, C, layouts, pads=(0, 0, 0), workspace=False, mul_identity=None, in_place=False,
+                  beta=None, screened=None):
+    """screened: on the screened kernel, in that many pieces (0: chosen by size).  Returns the route."""
     import torch
     (m, k), n = A.shape, B.shape[1]
     add, mul = RINGS[ring]
@@ -59,10 +61,11 @@ def check_product(ring, dtype, A, B, C, layouts, pads=(0, 0, 0), workspace=False
                 **({} if mul_identity is None else {"mul_identity": mul_identity}))
     (fa, lda), (fb, ldb), (fc, ldc) = (stored(x, lay, p) for x, lay, p in zip((A, B, C), layouts, pads))
     fd = fc if in_place else torch.full_like(fc, 77)
-    args = Arguments((m, n, k), (fa, lda), (fb, ldb), (fc, ldc), (fd, ldc), (one, one))
+    args = Arguments((m, n, k), (fa, lda), (fb, ldb), (fc, ldc), (fd, ldc), (one, one if beta is None else beta))
     need = op.get_optional_workspace_size(args) if workspace else 0
-    assert op(args, torch.empty(need, dtype=torch.uint8, device="cuda") if need else None) == Status.kSuccess
-    got, want = read(fd, layouts[2], m, n, ldc), by_loop(ring, A, B, C)
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda") if need else None
+    assert (op(args, ws) if screened is None else op.run_screened(args, screened, ws)) == Status.kSuccess
+    got, want = read(fd, layouts[2], m, n, ldc), by_loop(ring, A, B, C if beta is None else C + beta)
     bad = ~((got == want) | ((got != got) & (want != want)))
     assert not bad.any(), (int(bad.sum()), bad.nonzero()[0].tolist(), got[bad][:3].tolist(), want[bad][:3].tolist())
     # nothing beyond the matrix was written
@@ -187,13 +190,10 @@ def distances(kind, g, shape, along):
     return torch.where(x < 0.002, -torch.inf, 100 * x)
 
 
-# Sizes the screened kernel gets: several pieces of K per tile of the output (which then meet in D), on even and odd lines, and
-# one; and sizes just below, which run exactly.
-@pytest.mark.parametrize("m, n, k, screened", [(1000, 1000, 3000, True), (1021, 1023, 4099, True), (400, 390, 12001, True),
-                                               (2049, 2047, 2050, True), (700, 650, 1500, False), (64, 70, 5001, False)])
-@pytest.mark.parametrize("kind", ["edges", "signed", "ties", "falling", "wide", "almost zero", "bursts", "nan", "infinite"])
-@pytest.mark.parametrize("ring", ["minimum_plus", "maximum_plus"])
-def test_double_precision_tropical_products(cuda_device, ring, kind, m, n, k, screened):
+KINDS = ["edges", "signed", "ties", "falling", "wide", "almost zero", "bursts", "nan", "infinite"]
+
+
+def tropical_operands(ring, kind, m, n, k):
     import torch
     g = torch.Generator(device="cuda").manual_seed(k)
     A, B = distances(kind, g, (m, k), 1), distances(kind, g, (k, n), 0)
@@ -204,12 +204,41 @@ def test_double_precision_tropical_products(cuda_device, ring, kind, m, n, k, sc
             A, B = A.flip(1), B.flip(0)
     if ring == "maximum_plus" and kind == "infinite":
         A, B = (torch.where(x == -torch.inf, torch.inf, x) for x in (A, B))
-    want = "screened " if screened else "product "
+    return A, B, C
+
+
+# the screened kernel whatever the data: one piece of K per tile of the output, and several (which then meet in D), one of them of a
+# single block; even and odd lines, every tile and K edge
+@pytest.mark.parametrize("m, n, k, pieces", [(700, 650, 1500, 1), (1021, 1023, 517, 3), (129, 1290, 2000, 5), (64, 70, 5001, 157),
+                                             (2305, 1025, 650, 1), (1, 3, 33, 2), (300, 129, 32, 1)])
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("ring", ["minimum_plus", "maximum_plus"])
+def test_screened_kernel(cuda_device, ring, kind, m, n, k, pieces):
+    import torch
+    A, B, C = tropical_operands(ring, kind, m, n, k)
     for layouts, pads, C, in_place in (((ROW, COL, ROW), (-k % 2, -k % 2, 0), C, False), ((COL, COL, COL), (1, 0, 1), C, True),
                                        ((COL, ROW, ROW), (0, 0, 0), torch.full_like(C, -5.0 if ring == "minimum_plus" else 1e12), False)):
-        route = check_product(ring, "f64", A, B, C, layouts, pads, in_place=in_place)
-        assert route.startswith(want), route
-        assert not screened or ("pieces=1 " in route) == (m == 2049), route
+        route = check_product(ring, "f64", A, B, C, layouts, pads, in_place=in_place, screened=pieces)
+        assert route.startswith("screened tile=128x128") and f"pieces={pieces} " in route, route
+    assert device_status() == 0
+
+
+# Sizes at which both kernels are launched and the operands decide which of them does the product: in several pieces that meet in D
+# and in one; and a size that always runs exactly.  With D in place of C and a factor on it, a product done twice shows.
+@pytest.mark.parametrize("m, n, k, pieces", [(1000, 1000, 3000, 2), (1021, 1023, 4099, 2), (400, 390, 12001, 9), (2049, 2047, 2050, 1),
+                                             (500, 520, 600, 0)])
+@pytest.mark.parametrize("kind", KINDS + ["rare"])
+@pytest.mark.parametrize("ring", ["minimum_plus", "maximum_plus"])
+def test_screened_or_exact(cuda_device, ring, kind, m, n, k, pieces):
+    import torch
+    A, B, C = tropical_operands(ring, "ties" if kind == "rare" else kind, m, n, k)
+    if kind == "rare":               # values the screen cannot hold, few enough for the sample to miss some
+        g = torch.Generator(device="cuda").manual_seed(n)
+        A, B = (torch.where(torch.rand(x.shape, generator=g, device="cuda") < 2e-4, -x - 1, x) for x in (A, B))
+    for layouts, pads, in_place, workspace in (((ROW, COL, ROW), (-k % 2, -k % 2, 0), False, False), ((COL, COL, COL), (1, 0, 1), True, True),
+                                               ((COL, ROW, ROW), (0, 0, 0), True, False)):
+        route = check_product(ring, "f64", A, B, C, layouts, pads, workspace, in_place=in_place, beta=3.0)
+        assert ("or product" in route) == (pieces > 0) and (pieces == 0 or route.startswith(f"screened pieces={pieces} ")), route
     assert device_status() == 0
 
 
@@ -237,6 +266,10 @@ def test_double_precision_tropical_zeros_are_positive(cuda_device, ring, m, n, k
             assert not torch.signbit(D[zero]).any(), (int(torch.signbit(D[zero]).sum()), op.last_route())
         else:
             assert op.last_route().startswith("product ")
+            continue
+        args = Arguments((m, n, k), (A, k), (B, n), (C, n), (D, n), (0.0, beta))
+        assert op.run_screened(args) == Status.kSuccess
+        assert ((D == 0) == zero).all() and not torch.signbit(D[zero]).any()
 
 
 def test_double_precision_tropical_product_into_host_memory(cuda_device):
@@ -255,10 +288,10 @@ def test_double_precision_tropical_product_into_host_memory(cuda_device):
         assert op(args, None, torch.cuda.current_stream()) == Status.kSuccess
         return op.last_route()
     assert product(host).startswith("product ")
-    assert product(here).startswith("screened ")
+    assert product(here).startswith("screened pieces=2 or product ")
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
-        assert product(captured).startswith("screened ")
+        assert product(captured).startswith("screened pieces=2 or product ")
     graph.replay()
     torch.cuda.synchronize()
     want = by_loop("minimum_plus", A, B, C)

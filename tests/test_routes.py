@@ -42,7 +42,7 @@ def test_routes(cuda_device):
     sums = SrgemmSplitKParallel(Op.PLUS, Op.MULTIPLIES, DType.F32, ROW, COL, ROW)
     route = run(sums, 256, 256, 4096, slices=8)
     assert "tile=128x128" in route and "pieces=8 tickets=1" in route, route
-    assert run(Srgemm(Op.MINIMUM, Op.PLUS, DType.F64, ROW, COL, ROW), 4096, 2048, 2048).startswith("screened ")
+    assert run(Srgemm(Op.MINIMUM, Op.PLUS, DType.F64, ROW, COL, ROW), 4096, 2048, 2048).startswith("screened pieces=1 or product ")
     # fp64 minima below the size where the screen pays
     assert run(Srgemm(Op.MINIMUM, Op.PLUS, DType.F64, ROW, COL, ROW), 128, 128, 128).startswith("product ")
     n = 64
