@@ -16,7 +16,7 @@
 // ascending order), and for outputs too small to fill the GPU with those, 64 x 64 (fp32) or 64 x 32 (fp64, whose partial
 // values leave no room for a pipeline beside the larger one) with the k range shared by four or eight warps and, beyond
 // that, by the CTAs of a cluster; their (value, k) candidates meet in shared memory, the smaller k
-// winning ties.
+// winning ties.  On the fp64 one the index follows every product (improve below): 1000^3 from +inf 757 us on the large tile, 370.
 #pragma once
 
 #include "srgemm_tma.cuh"

@@ -12,7 +12,8 @@
 //   warps 8..11         producers: for every K step of every output tile this CTA owns, wait for a free stage and
 //                       fill it: operands that lie contiguous along k on 16-byte storage lines by TMA (one lane),
 //                       all others by the cp.async gather of gather.cuh (all 128 threads).  Either way the stage
-//                       holds [rows][128 bytes of k] with the 128-byte swizzle, so there is one contraction loop.
+//                       holds [rows][128 bytes of k] with the 128-byte swizzle, so there is one contraction loop; only
+//                       its loads differ where the large tile takes an operand along its rows as it lies (LargeRowsTile).
 //   warps 0..7          consumers: WM x WN x WK warps.  A warp owns a 64 x 32 block of the tile (8 x 4 lanes, an
 //                       8 x 8 register micro-tile per lane) and every WK-th part of each stage's k range.
 //                       They wait for a stage, read 16-byte vectors and run the contraction two k steps at a time:

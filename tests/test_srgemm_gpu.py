@@ -237,8 +237,8 @@ def test_unaligned_operands_stay_on_the_tma_kernel_with_the_workspace(cuda_devic
     """The reference accepts any leading dimension and element-aligned pointers
     (include/cuasr/gemm/device/default_srgemm_configuration.h:88-89, test/device/testbed.h:313-319).  TMA cannot
     describe an operand whose address or leading dimension is not a multiple of 16 bytes: without a workspace such
-    a product runs on the generic kernel, with the optional workspace the operand is first copied into aligned
-    scratch and the fast kernel runs.  Either way the result is the host SRGEMM's."""
+    an operand is gathered, with the optional workspace it is first copied into aligned scratch.  Either way the
+    result is the host SRGEMM's."""
     import torch
     rng = np.random.default_rng(97)
     m, n, k = 300, 260, 190
@@ -280,8 +280,7 @@ def test_unaligned_operands_stay_on_the_tma_kernel_with_the_workspace(cuda_devic
                                      ("minimum_maximum", DType.S32), ("maximum_minimum", DType.U32)])
 def test_integer_rings_with_ragged_k_use_padded_copies(cuda_device, ring, dt):
     """Integer min/max rings have no value TMA could fill a ragged last K step with.  With the optional workspace
-    both operands are copied with K extended to whole steps - A by the additive identity, B by the multiplicative
-    one - and the TMA kernel runs; without it the generic kernel does."""
+    both operands are copied with K extended to whole steps by repeating the last k; without it the gather does that."""
     import torch
     rng = np.random.default_rng(5)
     for layouts in (util.ALL_LAYOUTS[0], util.ALL_LAYOUTS[3], util.ALL_LAYOUTS[6]):
@@ -494,8 +493,8 @@ def test_status_codes(cuda_device):
 
 def test_extents_beyond_the_grid_y_limit(cuda_device):
     """The reference accepts any extent.  A 4.3-million-row product with N = K = 1 has more 64-row tiles than the
-    65535 a CUDA grid allows along y or z; tiles are numbered along x here, so it runs (on the generic kernel: a
-    leading dimension of 1 is nothing TMA can describe)."""
+    65535 a CUDA grid allows along y or z; tiles are numbered along x here, so it runs (gathered: a leading dimension
+    of 1 is nothing TMA can describe)."""
     import torch
     m, n, k = 4_300_000, 1, 1
     g = torch.Generator(device="cuda").manual_seed(3)
